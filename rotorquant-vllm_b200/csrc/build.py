@@ -1,8 +1,8 @@
-"""Build librq_b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Build librq_b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a, and ``_host.so``, the
+native side of the Python launchers, with the host compiler against the installed torch.
 
-Usage: ``python rotorquant-vllm_b200/csrc/build.py [--verbose]``.  The library is
-written next to the Python package that loads it
-(``rotorquant-vllm_b200/rotorquant_vllm/librq_b200.so``).
+Usage: ``python rotorquant-vllm_b200/csrc/build.py [--verbose]``.  Both are written next to the
+Python package that loads them (``rotorquant-vllm_b200/rotorquant_vllm/``).
 """
 
 from __future__ import annotations
@@ -11,10 +11,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 CSRC = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.join(os.path.dirname(CSRC), "rotorquant_vllm")
 LIB = os.path.join(PKG, "librq_b200.so")
+HOST_LIB = os.path.join(PKG, "_host.so")
+HOST_SOURCE = os.path.join(CSRC, "rq_host.cpp")
 SOURCES = ["rq_api.cu", "rq_compress.cu", "rq_decode.cu", "rq_peer.cu", "rq_prefill.cu", "rq_probe.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -26,19 +29,39 @@ def _nvcc() -> str:
     return exe
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB):
+def _stale(lib: str) -> bool:
+    if not os.path.exists(lib):
         return True
-    t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))]
+    t = os.path.getmtime(lib)
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".cpp"))]
     deps.append(os.path.join(os.path.dirname(os.path.dirname(CSRC)), "include", "rq_b200.h"))
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_host(force: bool = False) -> str:
+    """Compile the native side of the launchers (a CPython extension module); returns its path."""
+    if not force and not _stale(HOST_LIB):
+        return HOST_LIB
+    from torch._C import _GLIBCXX_USE_CXX11_ABI
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    includes = [f"-I{d}" for d in [*include_paths("cuda"), sysconfig.get_paths()["include"]]]
+    dirs = [flag for d in library_paths("cuda") for flag in (f"-L{d}", f"-Wl,-rpath,{d}")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(_GLIBCXX_USE_CXX11_ABI)}", *includes, HOST_SOURCE, "-o", HOST_LIB, *dirs,
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(" ".join(cmd) + "\n" + proc.stdout + proc.stderr)
+    return HOST_LIB
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    """Compile every ``.cu`` file into one shared library; returns its path."""
+    """Compile every ``.cu`` file into one shared library, and the launchers' native side; returns
+    the path of the former."""
     srcs = [os.path.join(CSRC, s) for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
-    if not force and not _stale():
+    build_host(force)
+    if not force and not _stale(LIB):
         return LIB
     cmd = [_nvcc(), "-O3", "-std=c++17", *ARCH, "-lineinfo", "--shared", "-Xcompiler", "-fPIC",
            "--threads", "0", "-o", LIB, *srcs]

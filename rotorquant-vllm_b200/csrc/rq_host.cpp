@@ -1,0 +1,401 @@
+// Native side of the Python launchers: argument checks, scratch look-up, stream and device of a call, then the
+// C-ABI function.
+//
+// What it replaces and why: written in Python, one launcher call spends its time on attribute reads (about forty
+// tensor properties), a torch.cuda.device context and the conversion of up to 34 ctypes arguments.  A cache
+// write of a few tokens took 17.6 us per call that way, a decode step (cache write + attention, three kernels)
+// 42 us, while the GPU needs about a third of that.  Here a tensor property is a load.
+//
+// Contract with the Python launchers: every function first checks that the call is an ordinary one (CUDA tensors
+// on one device, expected types and layouts, a rotation that has been validated, scratch already in place).  If
+// anything is not, it returns None without having done anything and the launcher takes its Python path, which
+// converts, allocates or raises; so all errors and unusual layouts are handled in one place.  The C-ABI functions
+// are called through the addresses that _lib.py found in the library it loaded.
+#include <Python.h>
+
+#include <torch/csrc/Device.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <cmath>
+#include <unordered_map>
+
+#include "../../include/rq_b200.h"
+
+namespace {
+
+struct Entry {
+    decltype(&rq_compress_store) compress_store;
+    decltype(&rq_compress) compress;
+    decltype(&rq_decompress) decompress;
+    decltype(&rq_decode_workspace_bytes) decode_workspace_bytes;
+    decltype(&rq_decode) decode;
+    decltype(&rq_prefill_workspace_bytes) prefill_workspace_bytes;
+    decltype(&rq_prefill_int8_staged) prefill_int8_staged;
+    decltype(&rq_last_error) last_error;
+};
+Entry fn{};
+bool bound = false;
+
+// Rotation matrices whose structure has been validated: object -> version counter at that time.  The Python side
+// enters an object after its check and removes it when it dies, so an address cannot stand for another tensor.
+// Guarded by the GIL, as everything here outside of the C-ABI calls.
+std::unordered_map<PyObject*, uint32_t>& validated() {
+    static std::unordered_map<PyObject*, uint32_t> table;
+    return table;
+}
+
+const at::Tensor* tensor(PyObject* o) {
+    return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr;
+}
+
+// A call's tensors: all on one CUDA device.
+struct Device {
+    int index = -1;
+    bool ok = true;
+    void add(const at::Tensor& t) {
+        if (!t.is_cuda() || t.layout() != at::kStrided) { ok = false; return; }
+        const int i = t.get_device();
+        if (index < 0) index = i;
+        ok = ok && i == index;
+    }
+};
+
+int dtype_code(at::ScalarType t) {
+    switch (t) {
+        case at::kFloat: return RQ_DTYPE_F32;
+        case at::kHalf: return RQ_DTYPE_F16;
+        case at::kBFloat16: return RQ_DTYPE_BF16;
+        default: return -1;
+    }
+}
+
+bool f32_vector(const at::Tensor& t) { return t.scalar_type() == at::kFloat && t.is_contiguous(); }
+
+bool rotation_ok(PyObject* o, const at::Tensor& t) {
+    const auto it = validated().find(o);
+    return it != validated().end() && it->second == t._version() && t.is_cuda();
+}
+
+// Rows of head-dim elements that may be read with 16-byte loads.
+bool rows16(const at::Tensor& t) {
+    if (t.stride(-1) != 1 || reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 != 0) return false;
+    const int64_t es = t.element_size();
+    for (int64_t d = 0; d + 1 < t.dim(); ++d)
+        if ((t.stride(d) * es) % 16 != 0) return false;
+    return true;
+}
+
+// An int argument; false when it is not a Python int that fits.
+bool integer(PyObject* o, int64_t& v) {
+    if (!PyLong_Check(o)) return false;
+    int overflow = 0;
+    v = PyLong_AsLongLongAndOverflow(o, &overflow);
+    return overflow == 0;
+}
+
+// Scratch buffer of a device in one of the launchers' dictionaries, undefined when it is missing or too small.
+// The caller keeps the tensor over the launch: another thread may put a larger buffer in its place meanwhile.
+at::Tensor scratch(PyObject* dict, const at::Device& dev, size_t need) {
+    PyObject* key = THPDevice_New(dev);
+    PyObject* hit = key != nullptr ? PyDict_GetItemWithError(dict, key) : nullptr;
+    Py_XDECREF(key);
+    if (hit == nullptr) { PyErr_Clear(); return {}; }
+    const at::Tensor* t = tensor(hit);
+    if (t == nullptr || static_cast<size_t>(t->numel()) < need) return {};
+    return *t;
+}
+
+// The exceptions of _lib.check.
+bool raised(int status) {
+    if (status == RQ_OK) return false;
+    PyErr_SetString(status == RQ_ERR_CUDA ? PyExc_RuntimeError : PyExc_ValueError, fn.last_error());
+    return true;
+}
+
+PyObject* none() { Py_RETURN_NONE; }
+
+template <typename F>
+void set(F& f, PyObject* dict, const char* name) {
+    PyObject* v = PyDict_GetItemString(dict, name);
+    f = v != nullptr ? reinterpret_cast<F>(PyLong_AsVoidPtr(v)) : nullptr;
+}
+
+// bind({name: address})
+PyObject* bind(PyObject*, PyObject* dict) {
+    if (!PyDict_Check(dict)) { PyErr_SetString(PyExc_TypeError, "bind: a dict of addresses"); return nullptr; }
+    set(fn.compress_store, dict, "rq_compress_store");
+    set(fn.compress, dict, "rq_compress");
+    set(fn.decompress, dict, "rq_decompress");
+    set(fn.decode_workspace_bytes, dict, "rq_decode_workspace_bytes");
+    set(fn.decode, dict, "rq_decode");
+    set(fn.prefill_workspace_bytes, dict, "rq_prefill_workspace_bytes");
+    set(fn.prefill_int8_staged, dict, "rq_prefill_int8_staged");
+    set(fn.last_error, dict, "rq_last_error");
+    bound = fn.compress_store && fn.compress && fn.decompress && fn.decode_workspace_bytes && fn.decode &&
+            fn.prefill_workspace_bytes && fn.prefill_int8_staged && fn.last_error;
+    if (PyErr_Occurred()) return nullptr;
+    if (!bound) { PyErr_SetString(PyExc_RuntimeError, "bind: an entry point is missing"); return nullptr; }
+    return none();
+}
+
+// mark_valid(rotation), forget(id)
+PyObject* mark_valid(PyObject*, PyObject* o) {
+    if (const at::Tensor* t = tensor(o)) validated()[o] = t->_version();
+    return none();
+}
+PyObject* forget(PyObject*, PyObject* id) {
+    void* p = PyLong_AsVoidPtr(id);
+    if (PyErr_Occurred()) return nullptr;
+    validated().erase(static_cast<PyObject*>(p));
+    return none();
+}
+
+// compress_store(key, value, kv_cache, slot_mapping, rotation, k_boundaries, v_boundaries, write_padding)
+PyObject* compress_store(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    if (n_args != 8 || !bound) return none();
+    const at::Tensor* t[7];
+    Device dev;
+    for (int i = 0; i < 7; ++i) {
+        if ((t[i] = tensor(a[i])) == nullptr) return none();
+        dev.add(*t[i]);
+    }
+    const at::Tensor &key = *t[0], &value = *t[1], &cache = *t[2], &slots = *t[3], &kb = *t[5], &vb = *t[6];
+    const int dtype = dtype_code(key.scalar_type());
+    if (!dev.ok || dtype < 0 || key.dim() != 3 || value.scalar_type() != key.scalar_type() ||
+        key.sizes() != value.sizes() || cache.scalar_type() != at::kByte || cache.dim() != 3 || !cache.is_contiguous() ||
+        slots.scalar_type() != at::kLong || slots.dim() != 1 || !slots.is_contiguous() || !rotation_ok(a[4], *t[4]) ||
+        !f32_vector(kb) || !f32_vector(vb) || !rows16(key) || !rows16(value))
+        return none();
+    const int64_t n = std::min(key.size(0), slots.size(0));
+    if (n == 0) return none();
+    const int padding = PyObject_IsTrue(a[7]);
+    if (padding < 0) return nullptr;
+    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev.index));
+    void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev.index)).stream();
+    int status;
+    Py_BEGIN_ALLOW_THREADS
+    status = fn.compress_store(key.const_data_ptr(), value.const_data_ptr(), dtype, n, static_cast<int>(key.size(1)),
+                               static_cast<int>(key.size(2)), key.stride(0), key.stride(1), value.stride(0),
+                               value.stride(1), static_cast<uint8_t*>(cache.data_ptr()), cache.size(0) * cache.size(1),
+                               static_cast<int>(cache.size(2)), static_cast<const int64_t*>(slots.const_data_ptr()),
+                               static_cast<const float*>(t[4]->const_data_ptr()),
+                               static_cast<const float*>(kb.const_data_ptr()), static_cast<int>(kb.numel()),
+                               static_cast<const float*>(vb.const_data_ptr()), static_cast<int>(vb.numel()), padding,
+                               stream);
+    Py_END_ALLOW_THREADS
+    if (raised(status)) return nullptr;
+    Py_RETURN_TRUE;
+}
+
+// What the two attention launchers have in common: q, kv_cache, block_table, seq_lens, k / v centroids, rotation,
+// num_kv_heads, head_dim, block_size, sm_scale, out (a[0] .. a[11]).
+struct Attention {
+    const at::Tensor* t[7];
+    const at::Tensor* out = nullptr;      // the caller's, or nullptr: allocate
+    int64_t heads = 0, head_dim = 0, block_size = 0, num_seqs = 0;
+    float scale = 0.0f;
+    int dtype = -1;
+    Device dev;
+
+    bool take(PyObject* const* a) {
+        for (int i = 0; i < 7; ++i) {
+            if ((t[i] = tensor(a[i])) == nullptr) return false;
+            dev.add(*t[i]);
+        }
+        if (!integer(a[7], heads) || !integer(a[8], head_dim) || !integer(a[9], block_size)) return false;
+        const at::Tensor &q = *t[0], &cache = *t[1], &table = *t[2], &lens = *t[3];
+        if (a[11] != Py_None) {
+            if ((out = tensor(a[11])) == nullptr) return false;
+            dev.add(*out);
+        }
+        dtype = dtype_code(q.scalar_type());
+        num_seqs = lens.numel();
+        if (!dev.ok || dtype < 0 || q.dim() != 3 || q.numel() == 0 || q.size(2) != head_dim || q.stride(2) != 1 || heads <= 0 ||
+            q.size(1) % heads != 0 || cache.scalar_type() != at::kByte || cache.dim() != 3 || !cache.is_contiguous() ||
+            cache.size(1) != block_size || table.scalar_type() != at::kInt || table.dim() != 2 ||
+            table.size(0) != num_seqs || table.stride(1) != 1 || lens.scalar_type() != at::kInt ||
+            !lens.is_contiguous() || !f32_vector(*t[4]) || !f32_vector(*t[5]) || !rotation_ok(a[6], *t[6]))
+            return false;
+        if (out != nullptr && (out->scalar_type() != q.scalar_type() || out->sizes() != q.sizes() || out->stride(2) != 1))
+            return false;
+        if (a[10] == Py_None) {
+            scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(head_dim)));
+        } else {
+            const double s = PyFloat_AsDouble(a[10]);
+            if (s == -1.0 && PyErr_Occurred()) { PyErr_Clear(); return false; }
+            scale = static_cast<float>(s);
+        }
+        return true;
+    }
+    at::Tensor result() const { return out != nullptr ? *out : at::empty_like(*t[0]); }
+};
+
+// decode(q .. out, max_seq_len, workspace, num_splits, workspaces)
+PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    Attention c;
+    if (n_args != 16 || !bound || !c.take(a)) return none();
+    const at::Tensor &q = *c.t[0], &cache = *c.t[1], &table = *c.t[2];
+    int64_t max_len = table.size(1) * c.block_size, splits = 0;
+    if (q.size(0) != c.num_seqs || (a[12] != Py_None && !integer(a[12], max_len)) || !integer(a[14], splits) ||
+        max_len < 0 || max_len > INT32_MAX || splits < 0 || splits > INT32_MAX)
+        return none();
+    const size_t need = fn.decode_workspace_bytes(static_cast<int>(c.num_seqs), static_cast<int>(q.size(1)),
+                                                  static_cast<int>(c.heads), static_cast<int>(c.head_dim),
+                                                  static_cast<int>(max_len), static_cast<int>(splits));
+    at::Tensor ws;
+    if (a[13] == Py_None) {
+        ws = scratch(a[15], q.device(), need);
+    } else if (const at::Tensor* w = tensor(a[13])) {
+        c.dev.add(*w);
+        ws = *w;
+    }
+    if (!ws.defined() || !c.dev.ok) return none();
+    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(c.dev.index));
+    const at::Tensor out = c.result();
+    void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(c.dev.index)).stream();
+    int status;
+    Py_BEGIN_ALLOW_THREADS
+    status = fn.decode(q.const_data_ptr(), out.data_ptr(), c.dtype, q.stride(0), q.stride(1), out.stride(0), out.stride(1),
+                       static_cast<int>(c.num_seqs), static_cast<int>(q.size(1)), static_cast<int>(c.heads),
+                       static_cast<int>(c.head_dim), static_cast<const uint8_t*>(cache.const_data_ptr()), cache.size(0),
+                       static_cast<int>(c.block_size), static_cast<int>(cache.size(2)),
+                       static_cast<const int32_t*>(table.const_data_ptr()), table.stride(0),
+                       static_cast<const int32_t*>(c.t[3]->const_data_ptr()),
+                       static_cast<const float*>(c.t[4]->const_data_ptr()), static_cast<int>(c.t[4]->numel()),
+                       static_cast<const float*>(c.t[5]->const_data_ptr()), static_cast<int>(c.t[5]->numel()),
+                       static_cast<const float*>(c.t[6]->const_data_ptr()), c.scale, static_cast<int>(max_len),
+                       ws.data_ptr(), static_cast<size_t>(ws.numel()) * ws.element_size(), static_cast<int>(splits), stream);
+    Py_END_ALLOW_THREADS
+    if (raised(status)) return nullptr;
+    return c.out != nullptr ? Py_NewRef(a[11]) : THPVariable_Wrap(out);
+}
+
+// prefill(q .. out, cu_seqlens_q, max_q_len, error_flag, max_seq_len, scratches): the staged path with scratch in place
+PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    Attention c;
+    if (n_args != 17 || !bound || !c.take(a)) return none();
+    const at::Tensor &q = *c.t[0], &cache = *c.t[1], &table = *c.t[2];
+    const at::Tensor *cu = nullptr, *flag = nullptr;
+    if (a[12] != Py_None) {
+        if ((cu = tensor(a[12])) == nullptr) return none();
+        c.dev.add(*cu);
+        if (cu->scalar_type() != at::kInt || !cu->is_contiguous() || cu->numel() != c.num_seqs + 1) return none();
+    } else if (c.num_seqs != 1) {
+        return none();
+    }
+    if (a[14] != Py_None) {
+        if ((flag = tensor(a[14])) == nullptr) return none();
+        c.dev.add(*flag);
+    }
+    int64_t max_q = 0, bound_len = 0;
+    if (!c.dev.ok || (a[13] != Py_None && !integer(a[13], max_q)) || (a[15] != Py_None && !integer(a[15], bound_len)))
+        return none();
+    if (bound_len == 0) bound_len = table.size(1) * c.block_size;
+    if (max_q < 0 || max_q > INT32_MAX || bound_len <= 0 || bound_len > INT32_MAX || q.size(0) > INT32_MAX) return none();
+    const size_t need = fn.prefill_workspace_bytes(static_cast<int>(c.num_seqs), static_cast<int>(c.heads),
+                                                   static_cast<int>(bound_len));
+    const at::Tensor ws = scratch(a[16], q.device(), need);
+    if (!ws.defined()) return none();
+    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(c.dev.index));
+    const at::Tensor out = c.result();
+    void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(c.dev.index)).stream();
+    int status;
+    Py_BEGIN_ALLOW_THREADS
+    status = fn.prefill_int8_staged(
+        q.const_data_ptr(), out.data_ptr(), c.dtype, q.stride(0), q.stride(1), out.stride(0), out.stride(1),
+        cu != nullptr ? static_cast<const int32_t*>(cu->const_data_ptr()) : nullptr, static_cast<int>(q.size(0)),
+        static_cast<int>(c.num_seqs), static_cast<int>(max_q), static_cast<int>(q.size(1)), static_cast<int>(c.heads),
+        static_cast<int>(c.head_dim), static_cast<const uint8_t*>(cache.const_data_ptr()), cache.size(0),
+        static_cast<int>(c.block_size), static_cast<int>(cache.size(2)),
+        static_cast<const int32_t*>(table.const_data_ptr()), table.stride(0),
+        static_cast<const int32_t*>(c.t[3]->const_data_ptr()), static_cast<const float*>(c.t[4]->const_data_ptr()),
+        static_cast<int>(c.t[4]->numel()), static_cast<const float*>(c.t[5]->const_data_ptr()),
+        static_cast<int>(c.t[5]->numel()), static_cast<const float*>(c.t[6]->const_data_ptr()), c.scale,
+        flag != nullptr ? static_cast<int*>(flag->data_ptr()) : nullptr, static_cast<int>(bound_len), ws.data_ptr(),
+        static_cast<size_t>(ws.numel()), stream);
+    Py_END_ALLOW_THREADS
+    if (raised(status)) return nullptr;
+    return c.out != nullptr ? Py_NewRef(a[11]) : THPVariable_Wrap(out);
+}
+
+// compress(x, rotation, boundaries) -> (packed, norms)
+PyObject* compress(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    if (n_args != 3 || !bound) return none();
+    const at::Tensor *x = tensor(a[0]), *rot = tensor(a[1]), *bounds = tensor(a[2]);
+    if (x == nullptr || rot == nullptr || bounds == nullptr) return none();
+    Device dev;
+    dev.add(*x); dev.add(*rot); dev.add(*bounds);
+    const int dtype = dtype_code(x->scalar_type());
+    if (!dev.ok || dtype < 0 || x->dim() != 3 || x->numel() == 0 || !x->is_contiguous() || !rows16(*x) ||
+        !f32_vector(*bounds) || !rotation_ok(a[1], *rot))
+        return none();
+    const int64_t n = x->size(0), h = x->size(1), d = x->size(2);
+    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev.index));
+    const at::Tensor packed = at::empty({n, h, d / 2}, x->options().dtype(at::kByte));
+    const at::Tensor norms = at::empty({n, h, 1}, x->options().dtype(at::kFloat));
+    void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev.index)).stream();
+    int status;
+    Py_BEGIN_ALLOW_THREADS
+    status = fn.compress(x->const_data_ptr(), dtype, n * h, static_cast<int>(d), d,
+                         static_cast<const float*>(rot->const_data_ptr()),
+                         static_cast<const float*>(bounds->const_data_ptr()), static_cast<int>(bounds->numel()),
+                         static_cast<uint8_t*>(packed.data_ptr()), static_cast<float*>(norms.data_ptr()), stream);
+    Py_END_ALLOW_THREADS
+    if (raised(status)) return nullptr;
+    PyObject* p = THPVariable_Wrap(packed);
+    PyObject* m = p != nullptr ? THPVariable_Wrap(norms) : nullptr;
+    if (m == nullptr) { Py_XDECREF(p); return nullptr; }
+    PyObject* pair = PyTuple_Pack(2, p, m);
+    Py_DECREF(p);
+    Py_DECREF(m);
+    return pair;
+}
+
+// decompress(packed, norms, centroids, dtype_code) -> rows
+PyObject* decompress(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    if (n_args != 4 || !bound) return none();
+    const at::Tensor *packed = tensor(a[0]), *norms = tensor(a[1]), *cent = tensor(a[2]);
+    int64_t code;
+    if (packed == nullptr || norms == nullptr || cent == nullptr || !integer(a[3], code)) return none();
+    Device dev;
+    dev.add(*packed); dev.add(*norms); dev.add(*cent);
+    if (!dev.ok || packed->dim() != 3 || packed->numel() == 0 || packed->scalar_type() != at::kByte ||
+        !packed->is_contiguous() || norms->scalar_type() != at::kFloat || !norms->is_contiguous() ||
+        norms->numel() != packed->size(0) * packed->size(1) || !f32_vector(*cent) || code < 0 || code > 2)
+        return none();
+    const at::ScalarType types[3] = {at::kFloat, at::kHalf, at::kBFloat16};
+    const int64_t n = packed->size(0), h = packed->size(1), d = 2 * packed->size(2);
+    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev.index));
+    const at::Tensor out = at::empty({n, h, d}, packed->options().dtype(types[code]));
+    void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev.index)).stream();
+    int status;
+    Py_BEGIN_ALLOW_THREADS
+    status = fn.decompress(static_cast<const uint8_t*>(packed->const_data_ptr()),
+                           static_cast<const float*>(norms->const_data_ptr()), n * h, static_cast<int>(d),
+                           static_cast<const float*>(cent->const_data_ptr()), static_cast<int>(cent->numel()),
+                           out.data_ptr(), static_cast<int>(code), stream);
+    Py_END_ALLOW_THREADS
+    if (raised(status)) return nullptr;
+    return THPVariable_Wrap(out);
+}
+
+PyMethodDef methods[] = {
+    {"bind", bind, METH_O, nullptr},
+    {"mark_valid", mark_valid, METH_O, nullptr},
+    {"forget", forget, METH_O, nullptr},
+    {"compress_store", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(compress_store)), METH_FASTCALL, nullptr},
+    {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(decode)), METH_FASTCALL, nullptr},
+    {"prefill", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(prefill)), METH_FASTCALL, nullptr},
+    {"compress", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(compress)), METH_FASTCALL, nullptr},
+    {"decompress", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(decompress)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }

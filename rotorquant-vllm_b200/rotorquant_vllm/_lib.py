@@ -15,6 +15,7 @@ import torch
 # RQ_B200_LIBRARY: path of another build of the library (A/B comparisons of kernel variants).
 _PATH = os.environ.get("RQ_B200_LIBRARY") or os.path.join(os.path.dirname(os.path.abspath(__file__)), "librq_b200.so")
 _LIB = None
+_HOST = None
 
 RQ_OK = 0
 RQ_ERR_INVALID_ARG, RQ_ERR_UNSUPPORTED, RQ_ERR_ALIGNMENT, RQ_ERR_WORKSPACE, RQ_ERR_CUDA = (
@@ -74,6 +75,23 @@ def lib() -> C.CDLL:
                 fn.restype, fn.argtypes = res, args
         _LIB = handle
     return _LIB
+
+
+def host():
+    """The native side of the launchers (``_host.so``), bound to the loaded library; raises
+    ``RuntimeError`` when it has not been built."""
+    global _HOST
+    if _HOST is None:
+        handle = lib()
+        try:
+            from . import _host
+        except ImportError as exc:
+            raise RuntimeError(
+                f"rotorquant_vllm/_host.so cannot be loaded ({exc}): build it with "
+                "`python rotorquant-vllm_b200/csrc/build.py`.") from exc
+        _host.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in _SIGNATURES})
+        _HOST = _host
+    return _HOST
 
 
 def exported_symbols() -> list[str]:

@@ -44,6 +44,11 @@ def _rows_16b_aligned(x: torch.Tensor) -> bool:
 
 def _compress(x: torch.Tensor, rot_T_even: torch.Tensor, rot_T_odd: torch.Tensor,
               boundaries: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    if x.is_cuda and rot_T_even.is_cuda and rot_T_odd.is_cuda:
+        rotation = _dense_rotation(rot_T_even, rot_T_odd)
+        done = _lib.host().compress(x, rotation, boundaries)
+        if done is not None:
+            return done
     n, h, d = x.shape
     dev = _lib.require_cuda(x, rot_T_even, rot_T_odd, boundaries)
     rotation = _dense_rotation(rot_T_even, rot_T_odd)
@@ -85,6 +90,9 @@ def compress_and_store(key: torch.Tensor, value: torch.Tensor, kv_cache: torch.T
     ``slot_mapping`` (int64) may be shorter than ``N`` (only the first ``len(slot_mapping)``
     tokens are written, as in the reference) and negative entries are skipped.
     """
+    if _lib.host().compress_store(key, value, kv_cache, slot_mapping, rotation, k_boundaries, v_boundaries,
+                                  write_padding):
+        return
     dev = _lib.require_cuda(key, value, kv_cache, slot_mapping, rotation, k_boundaries, v_boundaries)
     validate_rotation(rotation)
     if key.shape != value.shape or key.dim() != 3:

@@ -81,6 +81,11 @@ def fused_paged_rq_decode(
     ``out`` (which must be this GPU's own entry).  The merge kernel then stores every output row into
     all of them; see :class:`rotorquant_vllm.parallel.PeerHeadGather`.
     """
+    if not peer_out_ptrs:
+        done = _lib.host().decode(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v, rotation, num_kv_heads,
+                                  head_dim, block_size, sm_scale, out, max_seq_len, workspace, num_splits, _WORKSPACE)
+        if done is not None:
+            return done
     num_seqs, hq, d = q.shape
     assert d == head_dim, f"D={d} != head_dim={head_dim}"
     assert hq % num_kv_heads == 0

@@ -10,6 +10,9 @@ from .. import _lib
 
 def _decompress(packed: torch.Tensor, norms: torch.Tensor, centroids: torch.Tensor,
                 dtype: torch.dtype) -> torch.Tensor:
+    done = _lib.host().decompress(packed, norms, centroids, _lib.DTYPE_CODE.get(dtype, -1))
+    if done is not None:
+        return done
     n, h, half = packed.shape
     dev = _lib.require_cuda(packed, norms, centroids)
     if packed.dtype != torch.uint8:

@@ -11,6 +11,9 @@ import torch
 from .. import _lib
 from .rotation import validate_rotation
 
+_SCRATCH: dict = {}
+SCRATCH_CAP = 1 << 30          # the per-device buffer never grows beyond this many bytes
+
 
 def fused_paged_rq_int8_prefill(
     q: torch.Tensor,
@@ -49,6 +52,12 @@ def fused_paged_rq_int8_prefill(
     ``SCRATCH_CAP`` bytes but never while a CUDA graph is being captured -- and the fused kernel
     otherwise, so that no call allocates beyond the cap.
     """
+    if staged is None and workspace is None:
+        done = _lib.host().prefill(q, kv_cache, block_table, seq_lens, k_centroids, v_centroids, rotation, num_kv_heads,
+                                   head_dim, block_size, sm_scale, out, cu_seqlens_q, max_q_len, error_flag, max_seq_len,
+                                   _SCRATCH)
+        if done is not None:
+            return done
     num_tokens, hq, d = q.shape
     assert d == head_dim
     assert hq % num_kv_heads == 0
@@ -112,10 +121,6 @@ def fused_paged_rq_int8_prefill(
         else:
             _lib.check(lib.rq_prefill_int8(*common, _lib.stream_ptr(dev)))
     return result
-
-
-_SCRATCH: dict = {}
-SCRATCH_CAP = 1 << 30          # the per-device buffer never grows beyond this many bytes
 
 
 def reserve_prefill_scratch(dev: torch.device, nbytes: int) -> None:

@@ -6,6 +6,8 @@ import weakref
 
 import torch
 
+from .. import _lib
+
 # id(tensor) -> (weak reference, version at validation time).  The table has no size limit: a
 # model builds one matrix per attention layer and every layer must stay validated.  An entry
 # disappears with its tensor (the weak reference's callback), so an id that Python hands to a new
@@ -45,5 +47,8 @@ def validate_rotation(rotation: torch.Tensor) -> None:
         entry = _VALIDATED.get(key)
         if entry is not None and entry[0] is _ref:
             del _VALIDATED[key]
+            host.forget(key)
 
+    host = _lib.host()
+    host.mark_valid(rotation)
     _VALIDATED[key] = (weakref.ref(rotation, _forget), rotation._version)
