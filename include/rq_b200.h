@@ -106,6 +106,23 @@ int rq_decompress_blocks(const uint8_t* kv_cache, int64_t num_blocks, int block_
                          int n_centroids_v, void* out_k, void* out_v, int out_dtype, void* stream);
 
 /*
+ * The physical blocks a batch references (the torch.unique and renumbering part of
+ * RQAttentionImpl._decompress_cache_paged), in one launch.
+ *
+ *   block_table   int32 (num_seqs, max_blocks), rows block_table_stride apart; the first
+ *                 ceil(seq_lens[s] / block_size) entries of row s are referenced
+ *   blocks_out    int32[min(num_seqs * max_blocks, num_blocks)]: the referenced blocks, ascending
+ *   remapped_out  int32 (num_seqs, max_blocks), contiguous: every entry's position in blocks_out, 0 for
+ *                 blocks that are not referenced (negative entries count from the end of the cache)
+ *   count_out     number of referenced blocks; device memory or pinned host memory.  -1 when a referenced
+ *                 entry is not in 0 .. num_blocks - 1
+ *   Limits: num_blocks <= 524288, num_seqs * max_blocks <= 1048576, else RQ_ERR_UNSUPPORTED.
+ */
+int rq_block_union(const int32_t* block_table, int64_t block_table_stride, int num_seqs, int max_blocks,
+                   const int32_t* seq_lens, int block_size, int64_t num_blocks, int32_t* blocks_out,
+                   int32_t* remapped_out, int32_t* count_out, void* stream);
+
+/*
  * Scratch bytes rq_decode needs for `num_splits` context splits (0 = let the library choose
  * from max_seq_len; the same choice rq_decode makes).
  */

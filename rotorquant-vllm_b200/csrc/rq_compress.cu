@@ -14,26 +14,23 @@
 //   rotate : out_j = fma(x3,R[j][3], fma(x2,R[j][2], fma(x1,R[j][1], x0*R[j][0]))) per 4x4 block
 //   bucket : number of boundaries strictly below the value
 //
-// Mapping.  The cache-write path (compress + store) gives a row of 128 values to four threads, 32
-// elements, eight rotation blocks and one 16-byte store each; the plain rows-to-rows path gives it to
-// sixteen threads of 8 elements.  Only the norm needs the whole row: the squares go through shared
-// memory, a few threads of the row form the eight running sums in the prescribed order, and the
-// left-to-right combination is done with shuffles.
+#include <type_traits>
+
 #include "rq_common.cuh"
 
 namespace rq {
 
-constexpr int kCompressThreads = 256;                 // 16 rows per CTA
-constexpr int kRowsPerCta = kCompressThreads / 16;
-constexpr int kCompressGrid = 148 * 4;                // the grid walks the rows: at most 4 CTAs per SM
-constexpr int kRowBatch = 2;                          // rows fetched ahead per 16-thread group and step
-constexpr int64_t kWideFromRows = 16384;              // launches with this many rows per kind use four threads per row
+constexpr int kCompressThreads = 256;
+constexpr int kCompressWarps = kCompressThreads / 32;
+constexpr int kSqPitch = 136;                // floats per row of squares: 128 + 8, so that four rows fall into different banks
+
+constexpr int64_t kWideFrom = 4096;          // rows of all kinds together from which a warp takes eight rows at a time
 
 struct CompressParams {
     const void* src[2];          // key, value (or x, unused)
     int64_t token_stride[2];     // elements
     int64_t head_stride[2];      // elements
-    int64_t num_tokens;          // tokens (store variant) or rows (rows variant)
+    uint32_t rows;               // rows per kind: tokens * H (store variant) or rows (rows variant)
     int H;
     // cache destination (store variant)
     uint8_t* cache;
@@ -49,416 +46,359 @@ struct CompressParams {
     const float* bounds[2];
     int n_bounds[2];
     int h_shift;                 // log2(H) when H is a power of two, else -1
+    int dense;                   // ROWS consecutive rows that start at a multiple of ROWS are 128 elements apart
 };
 
-// Eight consecutive elements of a row, raw (converted only when they are used, so that a load
-// issued ahead of time does not make its issuer wait).
+// Four consecutive elements of a row, raw (converted only when they are used).
 template <typename T>
-struct Raw8 {
-    uint4 a, b;               // b only for 4-byte elements
-};
+struct Raw4 { uint2 a; };
+template <>
+struct Raw4<float> { uint4 a; };
 template <typename T>
-__device__ __forceinline__ Raw8<T> load_raw8(const T* src) {
-    Raw8<T> r;
-    r.a = __ldg(reinterpret_cast<const uint4*>(src));
-    if constexpr (sizeof(T) == 4) r.b = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+__device__ __forceinline__ Raw4<T> load_raw4(const T* src) {
+    Raw4<T> r;
+    if constexpr (sizeof(T) == 4) r.a = __ldg(reinterpret_cast<const uint4*>(src));
+    else r.a = __ldg(reinterpret_cast<const uint2*>(src));
     return r;
 }
-template <typename T>
-__device__ __forceinline__ void unpack8(const Raw8<T>& r, float* x) {
-    if constexpr (sizeof(T) == 4) {
-        Chunk16<float>::unpack(r.a, x);
-        Chunk16<float>::unpack(r.b, x + 4);
-    } else {
-        Chunk16<T>::unpack(r.a, x);
-    }
+__device__ __forceinline__ void unpack4(const Raw4<float>& r, float (&x)[4]) {
+    x[0] = __uint_as_float(r.a.x); x[1] = __uint_as_float(r.a.y);
+    x[2] = __uint_as_float(r.a.z); x[3] = __uint_as_float(r.a.w);
+}
+__device__ __forceinline__ void unpack4(const Raw4<__half>& r, float (&x)[4]) {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.a.x));
+    const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&r.a.y));
+    x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+}
+__device__ __forceinline__ void unpack4(const Raw4<__nv_bfloat16>& r, float (&x)[4]) {
+    x[0] = __uint_as_float(r.a.x << 16); x[1] = __uint_as_float(r.a.x & 0xFFFF0000u);
+    x[2] = __uint_as_float(r.a.y << 16); x[3] = __uint_as_float(r.a.y & 0xFFFF0000u);
 }
 
-// Eight consecutive elements of a row as fp32.
-template <typename T>
-__device__ __forceinline__ void load8(const T* src, float* x) {
-    if constexpr (sizeof(T) == 4) {
-        Chunk16<float>::unpack(__ldg(reinterpret_cast<const uint4*>(src)), x);
-        Chunk16<float>::unpack(__ldg(reinterpret_cast<const uint4*>(src) + 1), x + 4);
-    } else {
-        Chunk16<T>::unpack(__ldg(reinterpret_cast<const uint4*>(src)), x);
-    }
+// Pairs of fp32 values in one 64-bit register.  A packed operation takes the pipe as long as two scalar ones but
+// one issue slot instead of two; every half is rounded as the scalar operation rounds it.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pk(float lo, float hi) {
+    f2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
 }
-
-// What a thread needs of R for the whole launch: the two 4x4 blocks of its elements (thread j of a row owns
-// blocks 2j and 2j + 1), as [half][out jj][in k].  The CTA keeps them in shared memory, 36 floats apart per
-// thread slot so that the 16-byte chunks of eight consecutive threads fall into different banks (the two rows
-// of a warp read the same addresses); keeping them in 32 registers per thread instead costs the fourth CTA per SM.
-constexpr int kRotPitch = 36;
-struct ThreadRotation {
-    const float* s;
-};
-__device__ __forceinline__ ThreadRotation load_rotation(const float* __restrict__ rotation, int j) {
-    __shared__ __align__(16) float rot_s[16 * kRotPitch];
-    for (int i = threadIdx.x; i < 512; i += kCompressThreads) {
-        const int t = i >> 5, e = i & 31;
-        const int g = 2 * t + (e >> 4), jj = (e >> 2) & 3, k = e & 3;
-        rot_s[t * kRotPitch + e] = __ldg(rotation + (4 * g + jj) * kHeadDim + 4 * g + k);
-    }
-    __syncthreads();
-    return ThreadRotation{rot_s + j * kRotPitch};
+__device__ __forceinline__ void upk(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
 }
-
 
 // Number of boundaries strictly below v.  The boundaries ascend, so "bd[b] < v" is true for a
 // prefix of them and a binary search over that prefix gives the count with log2(NB + 1) compares
 // (a NaN compares false everywhere: 0, as the linear count gives).
 template <int NB>
-__device__ __forceinline__ uint32_t count_below(const float (&bd)[NB], float v) {
-    if constexpr (NB == 7) {
-        const bool c1 = bd[3] < v;
-        const bool c2 = (c1 ? bd[5] : bd[1]) < v;
-        const float lo = c2 ? bd[2] : bd[0], hi = c2 ? bd[6] : bd[4];
-        const bool c3 = (c1 ? hi : lo) < v;
-        return (c1 ? 4u : 0u) + (c2 ? 2u : 0u) + (c3 ? 1u : 0u);
-    } else {
-        static_assert(NB == 15, "7 or 15 boundaries");
-        const bool c1 = bd[7] < v;
-        const bool c2 = (c1 ? bd[11] : bd[3]) < v;
-        const float m3a = c2 ? bd[5] : bd[1], m3b = c2 ? bd[13] : bd[9];
-        const bool c3 = (c1 ? m3b : m3a) < v;
-        // fourth level: boundary 8*c1 + 4*c2 + 2*c3
-        const float q0 = c3 ? bd[2] : bd[0], q1 = c3 ? bd[6] : bd[4];
-        const float q2 = c3 ? bd[10] : bd[8], q3 = c3 ? bd[14] : bd[12];
-        const float h0 = c2 ? q1 : q0, h1 = c2 ? q3 : q2;
-        const bool c4 = (c1 ? h1 : h0) < v;
-        return (c1 ? 8u : 0u) + (c2 ? 4u : 0u) + (c3 ? 2u : 0u) + (c4 ? 1u : 0u);
-    }
+__device__ __forceinline__ uint32_t count_below(const float* bd, float v) {
+    constexpr int kTop = (NB + 1) / 2;
+    uint32_t n = 0;
+#pragma unroll
+    for (int step = kTop; step > 0; step >>= 1) n += bd[n + step - 1] < v ? step : 0;
+    return n;
 }
 
-// The 16 threads of a row: returns this thread's packed word (8 indices) and the row norm.
-// `x` are the thread's elements 8j..8j+7, `sq_row` the row's [16][8] exchange area in shared
-// memory, `bd` the NB boundaries; all 32 lanes of the warp must call this.
+// Bucketing by guess and one compare.  guess(v) = the nearest whole number to (v - mid) / delta + NB/2, clamped to
+// 0 .. NB - 1: one saturating multiply-add and one multiply-add whose low mantissa bits are the number.  The guess
+// never decreases when v grows, so if guess(bd[k]) == k for every k, then guess(v) == j means bd[0..j-1] < v and
+// v < bd[j+1..]: the count is j, or j + 1 when bd[j] < v.  The lanes of the warp hold the boundaries (lane k has
+// bd[k]); a shuffle fetches bd[j].  Lloyd-Max codebooks have such a delta (3 and 4 bits: every delta between 0.42
+// and 0.69, 0.284 and 0.314 standard deviations); `fits` is false for boundaries that do not, which take
+// count_below.  Against the binary search this is 5 issue slots per element instead of 11, and 4 cycles of the
+// integer pipe instead of 20.
+struct Guess {
+    float bound;                 // lane k: bd[k]
+    float a, b;                  // saturate(v * a + b) * (NB - 1)
+    bool fits;
+};
+constexpr float kMagic = 12582912.0f;        // 1.5 * 2^23
+__device__ __forceinline__ float sat_fma(float v, float a, float b) {
+    float d;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(v), "f"(a), "f"(b));
+    return d;
+}
 template <int NB>
-__device__ __forceinline__ uint32_t compress_chunk(const float (&x)[8], int j, float* sq_row,
-                                                   const ThreadRotation& rot, const float (&bd)[NB],
-                                                   float& norm_out) {
-    // squares, published for the in-order lane sums
-    float* mine = sq_row + 8 * j;
-    *reinterpret_cast<float4*>(mine) = make_float4(__fmul_rn(x[0], x[0]), __fmul_rn(x[1], x[1]),
-                                                   __fmul_rn(x[2], x[2]), __fmul_rn(x[3], x[3]));
-    *reinterpret_cast<float4*>(mine + 4) = make_float4(__fmul_rn(x[4], x[4]), __fmul_rn(x[5], x[5]),
-                                                       __fmul_rn(x[6], x[6]), __fmul_rn(x[7], x[7]));
-    __syncwarp();
-    float s = 0.0f;
-    if (j < 8) {
-        float v[16];
+__device__ __forceinline__ Guess make_guess(const float* __restrict__ bounds, int lane) {
+    constexpr int kMid = NB / 2;
+    Guess g;
+    g.bound = __ldg(bounds + min(lane, NB - 1));
+    const float mid = __shfl_sync(0xffffffffu, g.bound, kMid);
+    const int k = lane < NB ? lane - kMid : 0, n = k < 0 ? -k : k;
+    const float dist = fabsf(g.bound - mid);
+    // (n - 0.5) delta < dist < (n + 0.5) delta; the outermost buckets are open
+    float lo = (n > 0 && n < kMid) ? dist / (n + 0.5f) : 0.0f;
+    float hi = n > 0 ? dist / (n - 0.5f) : INFINITY;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) v[c] = sq_row[8 * c + j];
-        s = v[0];
-#pragma unroll
-        for (int c = 1; c < 16; ++c) s = __fadd_rn(s, v[c]);
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmaxf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fminf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
-    float tot = __shfl_sync(0xffffffffu, s, 0, 16);
-#pragma unroll
-    for (int l = 1; l < 8; ++l) tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, s, l, 16));
-    __syncwarp();                                   // sq_row may be rewritten by the next row
-    const float norm = __fsqrt_rn(tot);
-    norm_out = norm;
-    const float denom = __fadd_rn(norm, 1e-10f);
-
-    uint32_t word = 0;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const float x0 = __fdiv_rn(x[4 * half], denom), x1 = __fdiv_rn(x[4 * half + 1], denom);
-        const float x2 = __fdiv_rn(x[4 * half + 2], denom), x3 = __fdiv_rn(x[4 * half + 3], denom);
-        uint32_t idx[4];
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            const float4 r4 = *reinterpret_cast<const float4*>(rot.s + 16 * half + 4 * jj);
-            const float r[4] = {r4.x, r4.y, r4.z, r4.w};
-            float acc = __fmul_rn(x0, r[0]);
-            acc = __fmaf_rn(x1, r[1], acc);
-            acc = __fmaf_rn(x2, r[2], acc);
-            acc = __fmaf_rn(x3, r[3], acc);
-            idx[jj] = count_below<NB>(bd, acc);
-        }
-        const uint32_t b0 = (idx[0] << 4) | idx[1];
-        const uint32_t b1 = (idx[2] << 4) | idx[3];
-        word |= (b0 | (b1 << 8)) << (16 * half);
-    }
-    return word;
+    g.a = 1.0f / (0.5f * (lo + hi) * (NB - 1));
+    g.b = 0.5f - mid * g.a;
+    const float m = __fmaf_rn(sat_fma(g.bound, g.a, g.b), NB - 1.0f, kMagic);
+    const bool mine = lane >= NB || __float_as_int(m) == __float_as_int(kMagic) + lane;
+    g.fits = __all_sync(0xffffffffu, mine);
+    return g;
 }
 
-// ---- store variant for small launches: sixteen threads per row -------------------------------------
+struct __align__(16) CompressSmem {
+    union {
+        float sq[8 * kSqPitch];  // squares of the rows of a step, [row][element]
+        uint16_t packed[8][32];  // afterwards: packed indices, [row][lane]
+    };
+    float4 div[4];               // per pair of rows: -denominator a, b, reciprocal a, b
+    const void* src[8];
+    float bd[16];
+};
+
+// One warp walks rows of 128 values, ROWS at a time; lane L has elements 4L .. 4L + 3 of every row, which is one
+// rotation block, so the block's coefficients stay in registers for the whole launch (they were the larger part of
+// the shared-memory traffic when a thread had more of the row).  Rows are worked on two at a time with packed
+// fp32 operations.  Only the norm needs the whole row: the squares go through shared memory, lane 4r + p sums
+// the running sums 2p and 2p + 1 of row r in the prescribed order, and shuffles combine them left to right.
+// The same lane stores 16 of the row's 64 packed bytes.  The rows of the next step are requested before the
+// divisions of this one.
 //
-// The decode step compresses one token per sequence: a few hundred rows.  With 8 elements per thread the
-// dependency chain of a row is a quarter as long as with 32, and the rows spread over four times as many
-// threads, which is what counts when the launch cannot fill the GPU anyway.  A fixed grid walks first all K
-// rows (token-major, head-minor), then all V rows, two rows per warp at a time, the elements of a step's
-// rows all requested before the first is processed.  Every row's 16 threads write its 64 index bytes and its
-// norm straight into the token's cache slot; the K row of head 0 also zeroes the slot's padding.
-template <typename T, int NB>
-__device__ __forceinline__ void store_rows(const CompressParams& p, int kv, const ThreadRotation& rot,
-                                           float* sq_row, int j) {
-    float bd[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) bd[b] = __ldg(p.bounds[kv] + b);
-    const int H = p.H;
+// Division.  q = x / d with r = RN(1 / d): q0 = RN(x r), rem = RN(x - q0 d), q = RN(q0 + rem r) (Markstein's
+// correction step).  That this equals the division instruction was checked for ALL 2^46 pairs of 24-bit
+// significands; exponents do not matter while nothing comes near the subnormal range, which the bounds below
+// ensure (d in 2^-40 .. 2^30, |x| >= 2^-90: q >= 2^-120, rem a multiple of 2^-138).  The bound on x is checked on
+// products of two elements: both are at most d.  A step with a row outside of the bounds, or with a zero element,
+// takes the division instruction.  fp16 inputs cannot be below 2^-24.
+//
+// What bounds it: instruction latency and issue together (23 instructions per element and lane, 64 % of the issue
+// slots at the 16 warps per SM that 125 registers allow; fp32 pipe 46 %, integer pipe 38 %, LSU 36 %).  16384 tokens
+// x 8 heads: bf16 60.5 -> 36.6 us, fp32 73.6 -> 36.8 us against the earlier four-threads-per-row mapping with
+// divisions in double precision and a binary search; 64 tokens: 4.8 -> 3.6 us.
+template <typename T, int NB, int ROWS, bool STORE, bool FITS>
+__device__ __forceinline__ void compress_walk(const CompressParams& p, int kv, CompressSmem& sm, const Guess& guess) {
+    constexpr int kPairs = ROWS / 2;
+    constexpr bool kTiny = !std::is_same<T, __half>::value;                // the type can hold values below 2^-90
+    const int lane = threadIdx.x & 31;
+    const uint32_t H = p.H;
     const SlotLayout lay = slot_layout(H);
-    const uint32_t rows = static_cast<uint32_t>(p.num_tokens) * static_cast<uint32_t>(H);
-    const uint32_t step = gridDim.x * kRowsPerCta;
-    const uint32_t first = blockIdx.x * kRowsPerCta + (threadIdx.x >> 4);
-    const T* src = static_cast<const T*>(p.src[kv]);
+    const uint32_t rows = p.rows;
+    const uint32_t step = gridDim.x * (kCompressWarps * ROWS);
+    const T* const base = static_cast<const T*>(p.src[kv]) + 4 * lane;
+    const int my_row = (lane >> 2) & (ROWS - 1), sub = lane & 3;           // lanes past 4 ROWS repeat the first ones
+    const bool keeper = lane < 4 * ROWS;
+
+    f2 rot[4][4];                                                          // [out][in], both halves alike
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float r = __ldg(p.rotation + (4 * lane + jj) * kHeadDim + 4 * lane + k);
+            rot[jj][k] = pk(r, r);
+        }
+    }
+    const f2 steps = pk(NB - 1.0f, NB - 1.0f), magic = pk(kMagic, kMagic), minus1 = pk(-1.0f, -1.0f);
+
     auto locate = [&](uint32_t r, uint32_t& token, uint32_t& h) {
         if (p.h_shift >= 0) { token = r >> p.h_shift; h = r & (H - 1); }
         else { token = r / H; h = r - token * H; }
     };
-    auto fetch = [&](uint32_t r, Raw8<T>& raw, int64_t& slot) {
+    // The elements of this lane in the rows r0 .. r0 + ROWS - 1 (past the end: the first row again), and the slot of
+    // the row it keeps.
+    Raw4<T> raw[ROWS];
+    int64_t slot = 0;
+    auto fetch = [&](uint32_t r0) {
         uint32_t token, h;
-        locate(r < rows ? r : 0u, token, h);        // rows past the end compute on row 0 and store nothing
-        raw = load_raw8<T>(src + token * p.token_stride[kv] + static_cast<int64_t>(h) * p.head_stride[kv] + 8 * j);
-        slot = __ldg(p.slot_mapping + token);
+        if (p.dense && r0 + ROWS <= rows) {                                // consecutive rows are 128 elements apart
+            locate(r0, token, h);
+            const T* first = base + token * p.token_stride[kv] + static_cast<int64_t>(h * kHeadDim);
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) raw[i] = load_raw4<T>(first + i * kHeadDim);
+            if constexpr (STORE) {
+                locate(r0 + my_row, token, h);
+                slot = __ldg(p.slot_mapping + token);
+            }
+        } else {
+            locate(r0 + my_row < rows ? r0 + my_row : r0, token, h);
+            if (keeper && sub == 0) sm.src[my_row] = base - 4 * lane + token * p.token_stride[kv] + static_cast<int64_t>(h) * p.head_stride[kv];
+            if constexpr (STORE) slot = __ldg(p.slot_mapping + token);
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) raw[i] = load_raw4<T>(static_cast<const T*>(sm.src[i]) + 4 * lane);
+        }
     };
-    // the two rows of a warp run in lock step (shuffles, __syncwarp): loop on the warp's first row.
-    // A step fetches kRowBatch rows per thread group before it works on any of them, so that their
-    // load latencies overlap.
-    constexpr int B = kRowBatch;
-    const uint32_t warp_first = first & ~1u;
-    for (uint32_t wr = warp_first, r = first; wr < rows; wr += B * step, r += B * step) {
-        Raw8<T> raw[B];
-        int64_t slot[B];
+
+    uint32_t r0 = (blockIdx.x * kCompressWarps + (threadIdx.x >> 5)) * ROWS;
+    if (r0 >= rows) return;
+    fetch(r0);
+    for (;;) {
+        // ---- squares and norms ----
+        Raw4<T> cur[ROWS];
+        float least = INFINITY;
 #pragma unroll
-        for (int b = 0; b < B; ++b)
-            if (wr + b * step < rows) fetch(r + b * step, raw[b], slot[b]);
-#pragma unroll
-        for (int b = 0; b < B; ++b) {
-            if (wr + b * step >= rows) break;               // warp-uniform
-            const uint32_t rb = r + b * step;
-            float x[8];
-            unpack8<T>(raw[b], x);
-            float norm;
-            const uint32_t word = compress_chunk<NB>(x, j, sq_row, rot, bd, norm);
-            if (rb < rows) {
-                uint32_t token, h;
-                locate(rb, token, h);
-                if (slot[b] >= 0 && slot[b] < p.num_slots) {
-                    uint8_t* dst = p.cache + slot[b] * p.total_bytes;
-                    *reinterpret_cast<uint32_t*>(dst + (kv ? lay.v_idx : lay.k_idx) + h * kHalfDim + 4 * j) = word;
-                    if (j == 0) *reinterpret_cast<float*>(dst + (kv ? lay.v_norm : lay.k_norm) + 4 * h) = norm;
-                    if (p.write_padding && kv == 0 && h == 0) {
-                        const int units = (lay.total - lay.payload_end) / 8;
-                        for (int u = j; u < units; u += 16)
-                            *reinterpret_cast<uint2*>(dst + lay.payload_end + 8 * u) = make_uint2(0u, 0u);
-                    }
-                }
+        for (int i = 0; i < ROWS; ++i) {
+            cur[i] = raw[i];
+            float x[4];
+            unpack4(cur[i], x);
+            const f2 a = pk(x[0], x[1]), b = pk(x[2], x[3]);
+            *reinterpret_cast<ulonglong2*>(&sm.sq[i * kSqPitch + 4 * lane]) = make_ulonglong2(mul2(a, a), mul2(b, b));
+            if constexpr (kTiny) {
+                float lo, hi;
+                upk(mul2(a, b), lo, hi);
+                asm("min.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(fabsf(lo)), "f"(fabsf(hi)));
             }
         }
-    }
-}
-template <typename T>
-__global__ void __launch_bounds__(kCompressThreads, 4)
-compress_store_kernel(const CompressParams p) {
-    __shared__ __align__(16) float sq[kRowsPerCta][16 * 8];
-    const int j = threadIdx.x & 15;
-    const ThreadRotation rot = load_rotation(p.rotation, j);
-    float* sq_row = sq[threadIdx.x >> 4];
-#pragma unroll 1
-    for (int kv = 0; kv < 2; ++kv) {
-        if (p.n_bounds[kv] <= 7) store_rows<T, 7>(p, kv, rot, sq_row, j);
-        else store_rows<T, 15>(p, kv, rot, sq_row, j);
-    }
-}
-
-// ---- store variant for large launches: four threads per row -----------------------------------------
-//
-// A fixed grid (two CTAs per SM) walks the rows: first all K rows (token-major, head-minor), then all V rows.
-// Every row's threads write its 64 index bytes and its norm straight into the token's cache slot; the K row of
-// head 0 also zeroes the slot's padding.  The arithmetic is that of compress_chunk with 32 elements per thread: thread t of a row owns elements 32t .. 32t + 31 (four
-// 16-byte loads for 2-byte inputs, eight rotation blocks, one 16-byte store of packed indices), a warp works
-// on eight rows at a time.  The per-row and per-thread overhead (addressing, slot lookup, the exchange for the
-// in-order sums, the square root, stores) is spread over four times as many elements as with 16 threads per row.
-// In-order sums: the squares go to shared memory as [c][l] (element 8c + l); thread t forms the running sums
-// of lanes l = 2t and 2t + 1 over c = 0..15, and every thread then adds the eight lane sums left to right.
-constexpr int kWideThreads = 256;
-constexpr int kWideRowsPerWarp = 8;
-constexpr int kWideRowsPerCta = (kWideThreads / 32) * kWideRowsPerWarp;   // 64
-constexpr int kWideSqPitch = 136;            // floats per row of squares: 128 + 8, spreads rows over the banks
-constexpr int kWideRotPitch = 132;           // floats per thread slot of rotation blocks: 8 x 16 + 4
-constexpr int kWideGrid = 148 * 2;           // the grid walks the rows: two CTAs per SM
-
-template <typename T, int NB>
-__device__ __forceinline__ void store_rows_wide(const CompressParams& p, int kv, const float* rot_t, float* sq_row,
-                                                int t) {
-    float bd[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) bd[b] = __ldg(p.bounds[kv] + b);
-    const int H = p.H;
-    const SlotLayout lay = slot_layout(H);
-    const uint32_t rows = static_cast<uint32_t>(p.num_tokens) * static_cast<uint32_t>(H);
-    const uint32_t step = gridDim.x * kWideRowsPerCta;
-    const int lane = threadIdx.x & 31;
-    const uint32_t first = blockIdx.x * kWideRowsPerCta + (threadIdx.x >> 5) * kWideRowsPerWarp + (lane >> 2);
-    const uint32_t warp_first = first - (lane >> 2);
-    const T* src = static_cast<const T*>(p.src[kv]);
-
-    // the eight rows of a warp run in lock step (__syncwarp around the exchange): loop on the warp's first row
-    for (uint32_t wr = warp_first, r = first; wr < rows; wr += step, r += step) {
-        const uint32_t rr = r < rows ? r : 0u;                      // rows past the end compute on row 0, store nothing
-        uint32_t token, h;
-        if (p.h_shift >= 0) { token = rr >> p.h_shift; h = rr & (H - 1); }
-        else { token = rr / H; h = rr - token * H; }
-        const T* row_src = src + token * p.token_stride[kv] + static_cast<int64_t>(h) * p.head_stride[kv] + 32 * t;
-        const int64_t slot = __ldg(p.slot_mapping + token);
-        float x[32];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) load8<T>(row_src + 8 * c, x + 8 * c);
-
-        // squares, published for the in-order lane sums: sq_row[8 c + l], this thread's c = 4t .. 4t + 3
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            float* dst = sq_row + 8 * (4 * t + c);
-            *reinterpret_cast<float4*>(dst) = make_float4(__fmul_rn(x[8 * c], x[8 * c]), __fmul_rn(x[8 * c + 1], x[8 * c + 1]),
-                                                         __fmul_rn(x[8 * c + 2], x[8 * c + 2]), __fmul_rn(x[8 * c + 3], x[8 * c + 3]));
-            *reinterpret_cast<float4*>(dst + 4) = make_float4(__fmul_rn(x[8 * c + 4], x[8 * c + 4]), __fmul_rn(x[8 * c + 5], x[8 * c + 5]),
-                                                             __fmul_rn(x[8 * c + 6], x[8 * c + 6]), __fmul_rn(x[8 * c + 7], x[8 * c + 7]));
+        // the row this lane keeps
+        const bool have = keeper && r0 + my_row < rows;
+        uint8_t* idx_dst = nullptr;
+        float* norm_dst = nullptr;
+        bool pads = false;
+        if constexpr (STORE) {
+            uint32_t token, h;
+            locate(r0 + my_row, token, h);
+            if (have && slot >= 0 && slot < p.num_slots) {
+                uint8_t* const s = p.cache + slot * p.total_bytes;
+                idx_dst = s + (kv ? lay.v_idx : lay.k_idx) + h * kHalfDim + 16 * sub;
+                norm_dst = reinterpret_cast<float*>(s + (kv ? lay.v_norm : lay.k_norm) + 4 * h);
+                pads = kv == 0 && h == 0 && sub == 0 && p.write_padding;
+            }
+        } else if (have) {
+            idx_dst = p.packed_out + static_cast<int64_t>(r0 + my_row) * kHalfDim + 16 * sub;
+            norm_dst = p.norms_out + r0 + my_row;
         }
+        const bool more = r0 + step < rows;
         __syncwarp();
-        float s_even, s_odd;                                        // running sums of lanes 2t and 2t + 1
-        {
-            const float2 v0 = *reinterpret_cast<const float2*>(sq_row + 2 * t);
-            s_even = v0.x; s_odd = v0.y;
-#pragma unroll
-            for (int c = 1; c < 16; ++c) {
-                const float2 v = *reinterpret_cast<const float2*>(sq_row + 8 * c + 2 * t);
-                s_even = __fadd_rn(s_even, v.x);
-                s_odd = __fadd_rn(s_odd, v.y);
-            }
-        }
-        const int row_lane0 = lane & ~3;
-        float tot = __shfl_sync(0xffffffffu, s_even, row_lane0);
-        tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, s_odd, row_lane0));
-#pragma unroll
-        for (int u = 1; u < 4; ++u) {
-            tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, s_even, row_lane0 + u));
-            tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, s_odd, row_lane0 + u));
-        }
-        __syncwarp();                                               // sq_row may be rewritten by the next row
-        const float norm = __fsqrt_rn(tot);
-        const float denom = __fadd_rn(norm, 1e-10f);
+        if (more) fetch(r0 + step);
 
-        // The 32 IEEE divisions x / denom, through double precision: (float)((double)x * (1.0 / (double)denom)) is
-        // the correctly rounded fp32 quotient whenever that quotient is a normal number -- a quotient of two
-        // 24-bit significands stays at least 2^-49 (relative) away from every midpoint between adjacent floats,
-        // and the double-precision value is within 2^-52 of the exact quotient, so both round the same way;
-        // zeros, infinities and NaNs come out as the division gives them.  Quotients in or next to the subnormal
-        // range (coarser grid, exact ties possible) take the division instruction itself.  One reciprocal per
-        // row and no branch per element: the quotients are independent instruction streams, not 32 basic blocks.
+        bool slow = least < 0x1p-60f;
         {
-            const double rcp = __ddiv_rn(1.0, static_cast<double>(denom));
-            float q[32];
-            bool tiny = false;
+            const float* col = &sm.sq[my_row * kSqPitch + 2 * sub];
+            f2 s = *reinterpret_cast<const f2*>(col);                      // running sums 2 sub and 2 sub + 1
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                q[i] = __double2float_rn(__dmul_rn(static_cast<double>(x[i]), rcp));
-                tiny |= fabsf(q[i]) < 0x1p-124f && x[i] != 0.0f;        // (a zero quotient of a nonzero element too)
+            for (int c = 1; c < 16; ++c) s = add2(s, *reinterpret_cast<const f2*>(col + 8 * c));
+            float s_even, s_odd;
+            upk(s, s_even, s_odd);
+            float tot = __shfl_sync(0xffffffffu, s_even, 0, 4);
+            tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, s_odd, 0, 4));
+#pragma unroll
+            for (int u = 1; u < 4; ++u) {
+                tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, s_even, u, 4));
+                tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, s_odd, u, 4));
             }
-            if (tiny) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) q[i] = __fdiv_rn(x[i], denom);
+            const float norm = __fsqrt_rn(tot);
+            const float denom = __fadd_rn(norm, 1e-10f);
+            slow |= !(denom >= 0x1p-40f && denom <= 0x1p30f);
+            if (sub == 0 && keeper) {
+                float* d = reinterpret_cast<float*>(&sm.div[my_row >> 1]) + (my_row & 1);
+                d[0] = -denom;
+                d[2] = __frcp_rn(denom);
+                if (norm_dst != nullptr) *norm_dst = norm;
             }
-#pragma unroll
-            for (int i = 0; i < 32; ++i) x[i] = q[i];
         }
-        uint32_t words[4];
+        slow = __any_sync(0xffffffffu, slow);
+        __syncwarp();                                                      // sm.div is complete, sm.sq has been read
+
+        // ---- divide, rotate, bucket, pack: two rows at a time ----
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {                               // rotation block 8t + b = elements 4b .. 4b + 3 of x
-            const float x0 = x[4 * b], x1 = x[4 * b + 1], x2 = x[4 * b + 2], x3 = x[4 * b + 3];
-            uint32_t idx[4];
+        for (int i = 0; i < kPairs; ++i) {
+            float xa[4], xb[4];
+            unpack4(cur[2 * i], xa);
+            unpack4(cur[2 * i + 1], xb);
+            const float4 dv = sm.div[i];
+            f2 q[4];
+            if (!slow) {
+                const f2 nd = pk(dv.x, dv.y), rcp = pk(dv.z, dv.w);
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-                const float4 r4 = *reinterpret_cast<const float4*>(rot_t + 16 * b + 4 * jj);
-                float acc = __fmul_rn(x0, r4.x);
-                acc = __fmaf_rn(x1, r4.y, acc);
-                acc = __fmaf_rn(x2, r4.z, acc);
-                acc = __fmaf_rn(x3, r4.w, acc);
-                idx[jj] = count_below<NB>(bd, acc);
-            }
-            const uint32_t b0 = (idx[0] << 4) | idx[1];
-            const uint32_t b1 = (idx[2] << 4) | idx[3];
-            const uint32_t half16 = b0 | (b1 << 8);
-            if (b & 1) words[b >> 1] |= half16 << 16;
-            else words[b >> 1] = half16;
-        }
-        if (r < rows && slot >= 0 && slot < p.num_slots) {
-            uint8_t* dst = p.cache + slot * p.total_bytes;
-            uint8_t* idx_dst = dst + (kv ? lay.v_idx : lay.k_idx) + h * kHalfDim + 16 * t;
-            if ((reinterpret_cast<uintptr_t>(idx_dst) & 15u) == 0) {
-                *reinterpret_cast<uint4*>(idx_dst) = make_uint4(words[0], words[1], words[2], words[3]);
+                for (int e = 0; e < 4; ++e) {
+                    const f2 x = pk(xa[e], xb[e]);
+                    const f2 q0 = mul2(x, rcp);
+                    q[e] = fma2(fma2(nd, q0, x), rcp, q0);
+                }
             } else {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) reinterpret_cast<uint32_t*>(idx_dst)[i] = words[i];
+                for (int e = 0; e < 4; ++e) q[e] = pk(__fdiv_rn(xa[e], -dv.x), __fdiv_rn(xb[e], -dv.y));
             }
-            if (t == 0) *reinterpret_cast<float*>(dst + (kv ? lay.v_norm : lay.k_norm) + 4 * h) = norm;
-            if (p.write_padding && kv == 0 && h == 0) {
-                const int units = (lay.total - lay.payload_end) / 8;
-                for (int u = t; u < units; u += 4)
-                    *reinterpret_cast<uint2*>(dst + lay.payload_end + 8 * u) = make_uint2(0u, 0u);
-            }
-        }
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kWideThreads, 2)
-compress_store_wide_kernel(const CompressParams p) {
-    __shared__ __align__(16) float sq[kWideRowsPerCta * kWideSqPitch];
-    __shared__ __align__(16) float rot_s[4 * kWideRotPitch];
-    // rot_s[t][b][jj][k] = R[4g + jj][4g + k], g = 8t + b
-    for (int i = threadIdx.x; i < 512; i += kWideThreads) {
-        const int g = i >> 4, jj = (i >> 2) & 3, k = i & 3;
-        rot_s[(g >> 3) * kWideRotPitch + (g & 7) * 16 + 4 * jj + k] = __ldg(p.rotation + (4 * g + jj) * kHeadDim + 4 * g + k);
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, t = lane & 3;
-    float* sq_row = sq + ((threadIdx.x >> 5) * kWideRowsPerWarp + (lane >> 2)) * kWideSqPitch;
-    const float* rot_t = rot_s + t * kWideRotPitch;
-#pragma unroll 1
-    for (int kv = 0; kv < 2; ++kv) {
-        if (p.n_bounds[kv] <= 7) store_rows_wide<T, 7>(p, kv, rot_t, sq_row, t);
-        else store_rows_wide<T, 15>(p, kv, rot_t, sq_row, t);
-    }
-}
-
-// Rows variant: x (rows, 128) -> packed (rows, 64) + norms, same walk.
-template <typename T, int NB>
-__device__ __forceinline__ void plain_rows(const CompressParams& p, const ThreadRotation& rot, float* sq_row, int j) {
-    float bd[NB];
+            uint32_t ea[4], eb[4];
 #pragma unroll
-    for (int b = 0; b < NB; ++b) bd[b] = __ldg(p.bounds[0] + b);
-    const int64_t rows = p.num_tokens;
-    const int64_t step = static_cast<int64_t>(gridDim.x) * kRowsPerCta;
-    const int64_t first = static_cast<int64_t>(blockIdx.x) * kRowsPerCta + (threadIdx.x >> 4);
-    const T* src = static_cast<const T*>(p.src[0]);
-    for (int64_t wr = first & ~1ll, r = first; wr < rows; wr += step, r += step) {
-        float x[8];
-        load8<T>(src + (r < rows ? r : 0) * p.token_stride[0] + 8 * j, x);
-        float norm;
-        const uint32_t word = compress_chunk<NB>(x, j, sq_row, rot, bd, norm);
-        if (r < rows) {
-            reinterpret_cast<uint32_t*>(p.packed_out + r * kHalfDim)[j] = word;
-            if (j == 0) p.norms_out[r] = norm;
+            for (int jj = 0; jj < 4; ++jj) {
+                f2 acc = mul2(q[0], rot[jj][0]);
+                acc = fma2(q[1], rot[jj][1], acc);
+                acc = fma2(q[2], rot[jj][2], acc);
+                acc = fma2(q[3], rot[jj][3], acc);
+                float va, vb;
+                upk(acc, va, vb);
+                if constexpr (FITS) {
+                    const f2 m = fma2(pk(sat_fma(va, guess.a, guess.b), sat_fma(vb, guess.a, guess.b)), steps, magic);
+                    float ma, mb;
+                    upk(m, ma, mb);
+                    const int ja = __float_as_int(ma), jb = __float_as_int(mb);
+                    // the shuffle looks at the low five bits of the source lane: the guess itself
+                    const f2 bnd = pk(__shfl_sync(0xffffffffu, guess.bound, ja), __shfl_sync(0xffffffffu, guess.bound, jb));
+                    float da, db;                                          // negative exactly when bound < v
+                    upk(fma2(acc, minus1, bnd), da, db);
+                    ea[jj] = ja + (__float_as_uint(da) >> 31);
+                    eb[jj] = jb + (__float_as_uint(db) >> 31);
+                } else {
+                    ea[jj] = count_below<NB>(sm.bd, va);
+                    eb[jj] = count_below<NB>(sm.bd, vb);
+                }
+            }
+            // byte j of a row = index 2j in the high nibble; what the guesses carry above bit 15 drops out
+            sm.packed[2 * i][lane] = static_cast<uint16_t>(((ea[2] * 16 + ea[3]) * 16 + ea[0]) * 16 + ea[1]);
+            sm.packed[2 * i + 1][lane] = static_cast<uint16_t>(((eb[2] * 16 + eb[3]) * 16 + eb[0]) * 16 + eb[1]);
         }
+        __syncwarp();
+        const uint4 w = *reinterpret_cast<const uint4*>(&sm.packed[my_row][8 * sub]);
+        if (idx_dst != nullptr) {
+            if ((reinterpret_cast<uintptr_t>(idx_dst) & 15u) == 0) {
+                *reinterpret_cast<uint4*>(idx_dst) = w;
+            } else {
+                uint32_t* d = reinterpret_cast<uint32_t*>(idx_dst);
+                d[0] = w.x; d[1] = w.y; d[2] = w.z; d[3] = w.w;
+            }
+        }
+        // ---- the padding of the slots whose first K row is among these ----
+        if constexpr (STORE) {
+            unsigned todo = kv == 0 ? __ballot_sync(0xffffffffu, pads) : 0u;
+            while (todo != 0) {
+                const int who = __ffs(todo) - 1;
+                todo &= todo - 1;
+                uint8_t* pad = reinterpret_cast<uint8_t*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(idx_dst), who)) +
+                               (lay.payload_end - lay.k_idx);
+                const int units = (lay.total - lay.payload_end) / 8;
+                for (int u = lane; u < units; u += 32) *reinterpret_cast<uint2*>(pad + 8 * u) = make_uint2(0u, 0u);
+            }
+        }
+        if (!more) return;
+        r0 += step;
+        __syncwarp();                                                      // the next step writes the shared areas again
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kCompressThreads)
-compress_rows_kernel(const CompressParams p) {
-    __shared__ __align__(16) float sq[kRowsPerCta][16 * 8];
-    const int j = threadIdx.x & 15;
-    const ThreadRotation rot = load_rotation(p.rotation, j);
-    float* sq_row = sq[threadIdx.x >> 4];
-    if (p.n_bounds[0] <= 7) plain_rows<T, 7>(p, rot, sq_row, j);
-    else plain_rows<T, 15>(p, rot, sq_row, j);
+template <typename T, int ROWS, bool STORE>
+__global__ void __launch_bounds__(kCompressThreads, 2)
+compress_kernel(const CompressParams p) {
+    __shared__ CompressSmem sm[kCompressWarps];
+    const int kv = blockIdx.y;
+    const int lane = threadIdx.x & 31;
+    CompressSmem& mine = sm[threadIdx.x >> 5];
+    auto walk = [&](auto nb) {
+        constexpr int NB = decltype(nb)::value;
+        const Guess guess = make_guess<NB>(p.bounds[kv], lane);
+        if (lane < NB) mine.bd[lane] = guess.bound;
+        if (guess.fits) compress_walk<T, NB, ROWS, STORE, true>(p, kv, mine, guess);
+        else compress_walk<T, NB, ROWS, STORE, false>(p, kv, mine, guess);
+    };
+    if (p.n_bounds[kv] <= 7) walk(std::integral_constant<int, 7>{});
+    else walk(std::integral_constant<int, 15>{});
 }
 
 // ---- decompress ------------------------------------------------------------
+//
+// A thread makes one 16-byte unit of output: 8 elements from 4 index bytes (2-byte types) or 4 from 2 (fp32), so
+// that a warp's loads and stores are contiguous (a thread with 32 elements of a row stored 16 bytes at a 64-byte
+// stride).  Four units per thread, requested together.  Bound by DRAM / L2 writes.
 
 template <typename T>
 __device__ __forceinline__ uint32_t pack2(float a, float b);
@@ -473,95 +413,162 @@ __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// Four threads per row; each expands 16 packed bytes into 32 output elements.
+constexpr int kExpandThreads = 256;
+constexpr int kExpandUnits = 4;              // per thread
 template <typename T>
-__global__ void decompress_rows_kernel(const uint8_t* __restrict__ packed,
-                                       const float* __restrict__ norms, int64_t num_rows,
-                                       const float* __restrict__ centroids, int n_centroids,
-                                       T* __restrict__ out) {
+struct Expand {
+    static constexpr int kShift = sizeof(T) == 4 ? 5 : 4;               // log2(units per row of 128 elements)
+    static constexpr int kBytes = kHalfDim >> kShift;                   // index bytes per unit
+    // two consecutive centroids per index byte, high nibble first
+    __device__ static uint4 unit(uint32_t w, float norm, const float* cb) {
+        float f[2 * kBytes];
+#pragma unroll
+        for (int b = 0; b < kBytes; ++b) {
+            f[2 * b] = __fmul_rn(cb[(w >> (8 * b + 4)) & 15u], norm);
+            f[2 * b + 1] = __fmul_rn(cb[(w >> (8 * b)) & 15u], norm);
+        }
+        if constexpr (sizeof(T) == 4)
+            return make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+        else
+            return make_uint4(pack2<T>(f[0], f[1]), pack2<T>(f[2], f[3]), pack2<T>(f[4], f[5]), pack2<T>(f[6], f[7]));
+    }
+    __device__ static uint32_t load(const uint8_t* src) {
+        if constexpr (sizeof(T) == 4) return __ldg(reinterpret_cast<const uint16_t*>(src));
+        else return __ldg(reinterpret_cast<const uint32_t*>(src));
+    }
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kExpandThreads)
+decompress_rows_kernel(const uint8_t* __restrict__ packed, const float* __restrict__ norms, int64_t num_rows,
+                       const float* __restrict__ centroids, int n_centroids, T* __restrict__ out) {
+    using E = Expand<T>;
     __shared__ float cb[16];
     if (threadIdx.x < 16) cb[threadIdx.x] = threadIdx.x < n_centroids ? centroids[threadIdx.x] : 0.f;
     __syncthreads();
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t row = i >> 2;
-    const int q = static_cast<int>(i & 3);
-    if (row >= num_rows) return;
-    const uint4 pk = __ldg(reinterpret_cast<const uint4*>(packed + row * kHalfDim) + q);
-    const float norm = __ldg(norms + row);
-    const uint32_t w[4] = {pk.x, pk.y, pk.z, pk.w};
-    T* dst = out + row * kHeadDim + 32 * q;
+    const int64_t units = num_rows << E::kShift;
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * (kExpandThreads * kExpandUnits) + threadIdx.x;
+    uint32_t w[kExpandUnits];
+    float norm[kExpandUnits];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        float f[8];
+    for (int i = 0; i < kExpandUnits; ++i) {
+        const int64_t u = first + i * kExpandThreads;
+        if (u < units) {
+            w[i] = E::load(packed + u * E::kBytes);
+            norm[i] = __ldg(norms + (u >> E::kShift));
+        }
+    }
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const uint32_t byte = (w[k] >> (8 * b)) & 0xFFu;
-            f[2 * b] = __fmul_rn(cb[byte >> 4], norm);
-            f[2 * b + 1] = __fmul_rn(cb[byte & 15u], norm);
-        }
-        if constexpr (sizeof(T) == 4) {
-            reinterpret_cast<float4*>(dst + 8 * k)[0] = make_float4(f[0], f[1], f[2], f[3]);
-            reinterpret_cast<float4*>(dst + 8 * k)[1] = make_float4(f[4], f[5], f[6], f[7]);
-        } else {
-            *reinterpret_cast<uint4*>(dst + 8 * k) =
-                make_uint4(pack2<T>(f[0], f[1]), pack2<T>(f[2], f[3]), pack2<T>(f[4], f[5]),
-                           pack2<T>(f[6], f[7]));
-        }
+    for (int i = 0; i < kExpandUnits; ++i) {
+        const int64_t u = first + i * kExpandThreads;
+        if (u < units) reinterpret_cast<uint4*>(out)[u] = E::unit(w[i], norm[i], cb);
     }
 }
 
-// Paged decompress: the K and V rows of whole cache blocks, picked by a list of physical block
-// numbers, straight out of the slot layout.  Four threads per (token, head, K|V) row; thread q expands
-// index bytes 16q..16q+15.  Output row of (listed block j, position t, head h): (j * block_size + t) * H + h.
+// Paged decompress: the K (blockIdx.y == 0) and V rows of whole cache blocks, picked by a list of physical block
+// numbers, straight out of the slot layout.  Output row of (listed block j, position t, head h):
+// (j * block_size + t) * H + h.
 template <typename T>
-__global__ void decompress_blocks_kernel(const uint8_t* __restrict__ cache, int total_bytes, int block_size, int H,
-                                         const int32_t* __restrict__ blocks, int64_t num_listed, int64_t num_blocks,
-                                         const float* __restrict__ cent_k, int n_k, const float* __restrict__ cent_v,
-                                         int n_v, T* __restrict__ out_k, T* __restrict__ out_v) {
-    __shared__ float cb[2][16];
-    if (threadIdx.x < 32) {
-        const int kv = threadIdx.x >> 4, i = threadIdx.x & 15;
-        cb[kv][i] = i < (kv ? n_v : n_k) ? (kv ? cent_v : cent_k)[i] : 0.f;
-    }
+__global__ void __launch_bounds__(kExpandThreads)
+decompress_blocks_kernel(const uint8_t* __restrict__ cache, int total_bytes, uint32_t block_size, int bs_shift, uint32_t H,
+                         int h_shift, const int32_t* __restrict__ blocks, uint32_t rows, int64_t num_blocks,
+                         const float* __restrict__ cent_k, int n_k, const float* __restrict__ cent_v, int n_v,
+                         T* __restrict__ out_k, T* __restrict__ out_v) {
+    using E = Expand<T>;
+    const int kind = blockIdx.y;
+    __shared__ float cb[16];
+    if (threadIdx.x < 16) cb[threadIdx.x] = threadIdx.x < (kind ? n_v : n_k) ? (kind ? cent_v : cent_k)[threadIdx.x] : 0.f;
     __syncthreads();
-    const int64_t rows_per_kind = num_listed * block_size * H;
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t r2 = i >> 2;
-    const int q = static_cast<int>(i & 3);
-    if (r2 >= 2 * rows_per_kind) return;
-    const int kind = r2 >= rows_per_kind ? 1 : 0;
-    const int64_t r = r2 - kind * rows_per_kind;
-    const int h = static_cast<int>(r % H);
-    const int64_t tok = r / H;
-    const int64_t j = tok / block_size;
-    const int pos = static_cast<int>(tok % block_size);
-    int64_t blk = blocks != nullptr ? static_cast<int64_t>(__ldg(blocks + j)) : j;
-    blk = blk < 0 ? 0 : (blk >= num_blocks ? num_blocks - 1 : blk);
     const SlotLayout lay = slot_layout(H);
-    const uint8_t* slot = cache + (blk * block_size + pos) * total_bytes;
-    const uint8_t* src = slot + (kind ? lay.v_idx : lay.k_idx) + h * kHalfDim + 16 * q;   // 4-byte aligned at least
-    const uint32_t w[4] = {__ldg(reinterpret_cast<const uint32_t*>(src)), __ldg(reinterpret_cast<const uint32_t*>(src) + 1),
-                           __ldg(reinterpret_cast<const uint32_t*>(src) + 2), __ldg(reinterpret_cast<const uint32_t*>(src) + 3)};
-    const float norm = __ldg(reinterpret_cast<const float*>(slot + (kind ? lay.v_norm : lay.k_norm)) + h);
-    const float* c = cb[kind];
-    T* dst = (kind ? out_v : out_k) + r * kHeadDim + 32 * q;
+    const int idx_off = kind ? lay.v_idx : lay.k_idx, norm_off = kind ? lay.v_norm : lay.k_norm;
+    T* out = kind ? out_v : out_k;
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * (kExpandThreads * kExpandUnits) + threadIdx.x;
+    uint32_t w[kExpandUnits];
+    float norm[kExpandUnits];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        float f[8];
+    for (int i = 0; i < kExpandUnits; ++i) {
+        const int64_t u = first + i * kExpandThreads;
+        const uint32_t row = static_cast<uint32_t>(u >> E::kShift);
+        if (row < rows) {
+            const uint32_t tok = h_shift >= 0 ? row >> h_shift : row / H, h = row - tok * H;
+            const uint32_t j = bs_shift >= 0 ? tok >> bs_shift : tok / block_size, pos = tok - j * block_size;
+            int64_t blk = blocks != nullptr ? static_cast<int64_t>(__ldg(blocks + j)) : j;
+            blk = blk < 0 ? 0 : (blk >= num_blocks ? num_blocks - 1 : blk);
+            const uint8_t* slot = cache + (blk * block_size + pos) * total_bytes;
+            const int c = static_cast<int>(u) & ((1 << E::kShift) - 1);
+            w[i] = E::load(slot + idx_off + h * kHalfDim + c * E::kBytes);
+            norm[i] = __ldg(reinterpret_cast<const float*>(slot + norm_off) + h);
+        }
+    }
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const uint32_t byte = (w[k] >> (8 * b)) & 0xFFu;
-            f[2 * b] = __fmul_rn(c[byte >> 4], norm);
-            f[2 * b + 1] = __fmul_rn(c[byte & 15u], norm);
+    for (int i = 0; i < kExpandUnits; ++i) {
+        const int64_t u = first + i * kExpandThreads;
+        if (static_cast<uint32_t>(u >> E::kShift) < rows) reinterpret_cast<uint4*>(out)[u] = E::unit(w[i], norm[i], cb);
+    }
+}
+
+// ---- the blocks that a batch references ---------------------------------------
+//
+// One CTA: a bitmap of the physical blocks in shared memory, its exclusive prefix sums, the referenced blocks in
+// ascending order, and the block table renumbered into that order.  Replaces about fifteen launches (compare,
+// select, sort, unique, scatter, gather) of which two waited for the GPU; the tables of a batch are a few thousand
+// entries, so one CTA takes about 5 us and the launches were the cost.
+constexpr int kUnionThreads = 1024;
+constexpr int64_t kUnionMaxBlocks = 1 << 19;           // bitmap + prefix sums: 128 KB of shared memory
+constexpr int64_t kUnionMaxEntries = 1 << 20;
+
+__global__ void __launch_bounds__(kUnionThreads)
+block_union_kernel(const int32_t* __restrict__ table, int64_t stride, int num_seqs, int width,
+                   const int32_t* __restrict__ seq_lens, int block_size, int num_blocks, int32_t* __restrict__ listed,
+                   int32_t* __restrict__ remapped, int32_t* count) {
+    extern __shared__ uint32_t bits[];
+    const int words = (num_blocks + 31) / 32, tid = threadIdx.x;
+    int* prefix = reinterpret_cast<int*>(bits + words);
+    __shared__ int warp_sums[32];
+    for (int i = tid; i < words; i += kUnionThreads) bits[i] = 0u;
+    __syncthreads();
+    const int entries = num_seqs * width;
+    bool bad = false;
+    for (int e = tid; e < entries; e += kUnionThreads) {
+        const int s = e / width, w = e - s * width;
+        const int64_t need = (static_cast<int64_t>(max(__ldg(seq_lens + s), 0)) + block_size - 1) / block_size;
+        if (w < need) {
+            const int b = __ldg(table + s * stride + w);
+            if (b < 0 || b >= num_blocks) bad = true;
+            else atomicOr(&bits[b >> 5], 1u << (b & 31));
         }
-        if constexpr (sizeof(T) == 4) {
-            reinterpret_cast<float4*>(dst + 8 * k)[0] = make_float4(f[0], f[1], f[2], f[3]);
-            reinterpret_cast<float4*>(dst + 8 * k)[1] = make_float4(f[4], f[5], f[6], f[7]);
-        } else {
-            *reinterpret_cast<uint4*>(dst + 8 * k) =
-                make_uint4(pack2<T>(f[0], f[1]), pack2<T>(f[2], f[3]), pack2<T>(f[4], f[5]),
-                           pack2<T>(f[6], f[7]));
+    }
+    bad = __syncthreads_or(bad);
+    // exclusive prefix sums: a run of words per thread, then over the threads
+    const int per = (words + kUnionThreads - 1) / kUnionThreads, begin = min(tid * per, words), end = min(begin + per, words);
+    int mine = 0;
+    for (int i = begin; i < end; ++i) mine += __popc(bits[i]);
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((tid & 31) >= o) incl += v;
+    }
+    if ((tid & 31) == 31) warp_sums[tid >> 5] = incl;
+    __syncthreads();
+    int at = incl - mine;
+    for (int w = 0; w < (tid >> 5); ++w) at += warp_sums[w];
+    for (int i = begin; i < end; ++i) {
+        prefix[i] = at;
+        for (uint32_t b = bits[i]; b != 0; b &= b - 1) listed[at++] = 32 * i + __ffs(b) - 1;
+    }
+    if (tid == kUnionThreads - 1) *count = bad ? -1 : at;      // every run of the last thread lies behind all others
+    __syncthreads();
+    for (int e = tid; e < entries; e += kUnionThreads) {
+        const int s = e / width, w = e - s * width;
+        int b = __ldg(table + s * stride + w);
+        if (b < 0) b += num_blocks;                            // indices from the end, as tensor indexing takes them
+        int v = 0;
+        if (b >= 0 && b < num_blocks) {
+            const uint32_t word = bits[b >> 5], bit = 1u << (b & 31);
+            if (word & bit) v = prefix[b >> 5] + __popc(word & (bit - 1));
         }
+        remapped[e] = v;
     }
 }
 
@@ -572,24 +579,59 @@ static int check_bounds_count(int n, const char* what) {
     return RQ_OK;
 }
 
-template <typename T>
-static void launch_store(const CompressParams& p, cudaStream_t st) {
-    const int64_t rows = p.num_tokens * p.H;                               // per kind
-    if (rows >= kWideFromRows) {
-        const int64_t want = (rows + kWideRowsPerCta - 1) / kWideRowsPerCta;
-        const unsigned grid = static_cast<unsigned>(want < kWideGrid ? want : kWideGrid);
-        compress_store_wide_kernel<T><<<grid, kWideThreads, 0, st>>>(p);
-        return;
+static int shift_of(int64_t n) {
+    for (int sft = 0; sft < 31; ++sft)
+        if ((1LL << sft) == n) return sft;
+    return -1;
+}
+
+// Rows per warp and step: 8 when that still gives every SM a CTA of each kind (the exchange for the norm and the
+// row's bookkeeping are then shared by four times as many elements), else 2 (a quarter of the dependency chain and
+// four times the warps: a decode step's few hundred rows are latency).  The line is where the two cross: 256 tokens
+// of 8 heads take 4.4 us either way, 64 tokens 4.2 / 3.5 us with 8 / 2 rows, 1024 tokens 5.8 / 8.0 us.  kinds: 2
+// (K and V rows of the store variant) or 1.
+template <typename T, bool STORE>
+static void launch_walk(CompressParams& p, int kinds, cudaStream_t st) {
+    const int sms = 148;
+    const bool wide = p.rows >= static_cast<uint32_t>(kWideFrom / kinds);
+    p.dense = 1;
+    for (int kv = 0; kv < kinds; ++kv) {
+        const bool in_token = p.H % (wide ? 8 : 2) == 0;               // rows of a step belong to one token
+        if (STORE ? p.head_stride[kv] != kHeadDim || (!in_token && p.token_stride[kv] != static_cast<int64_t>(p.H) * kHeadDim)
+                  : p.token_stride[kv] != kHeadDim)
+            p.dense = 0;
     }
-    const int64_t want = (rows + kRowsPerCta - 1) / kRowsPerCta;
-    const unsigned grid = static_cast<unsigned>(want < kCompressGrid ? want : kCompressGrid);
-    compress_store_kernel<T><<<grid, kCompressThreads, 0, st>>>(p);
+    const uint32_t per_cta = kCompressWarps * (wide ? 8 : 2);
+    const uint32_t want = (p.rows + per_cta - 1) / per_cta, most = 2 * sms / kinds;
+    const dim3 grid(want < most ? want : most, kinds);
+    if (wide) compress_kernel<T, 8, STORE><<<grid, kCompressThreads, 0, st>>>(p);
+    else compress_kernel<T, 2, STORE><<<grid, kCompressThreads, 0, st>>>(p);
+}
+template <bool STORE>
+static void dispatch_walk(CompressParams& p, int dtype, int kinds, cudaStream_t st) {
+    switch (dtype) {
+        case RQ_DTYPE_F32: launch_walk<float, STORE>(p, kinds, st); break;
+        case RQ_DTYPE_F16: launch_walk<__half, STORE>(p, kinds, st); break;
+        default: launch_walk<__nv_bfloat16, STORE>(p, kinds, st); break;
+    }
+}
+
+template <typename T>
+static void launch_expand_rows(const uint8_t* packed, const float* norms, int64_t num_rows, const float* centroids,
+                               int n_centroids, void* out, cudaStream_t st) {
+    const int64_t units = num_rows << Expand<T>::kShift, per = kExpandThreads * kExpandUnits;
+    decompress_rows_kernel<T><<<static_cast<unsigned>((units + per - 1) / per), kExpandThreads, 0, st>>>(
+        packed, norms, num_rows, centroids, n_centroids, static_cast<T*>(out));
 }
 template <typename T>
-static void launch_rows(const CompressParams& p, cudaStream_t st) {
-    const int64_t want = (p.num_tokens + kRowsPerCta - 1) / kRowsPerCta;
-    const unsigned grid = static_cast<unsigned>(want < kCompressGrid ? want : kCompressGrid);
-    compress_rows_kernel<T><<<grid, kCompressThreads, 0, st>>>(p);
+static void launch_expand_blocks(const uint8_t* cache, int total_bytes, int block_size, int H, const int32_t* blocks,
+                                 int64_t rows, int64_t num_blocks, const float* cent_k, int n_k, const float* cent_v,
+                                 int n_v, void* out_k, void* out_v, cudaStream_t st) {
+    const int64_t units = rows << Expand<T>::kShift, per = kExpandThreads * kExpandUnits;
+    const dim3 grid(static_cast<unsigned>((units + per - 1) / per), 2);
+    decompress_blocks_kernel<T><<<grid, kExpandThreads, 0, st>>>(
+        cache, total_bytes, block_size, shift_of(block_size), H, shift_of(H), blocks, static_cast<uint32_t>(rows), num_blocks,
+        cent_k, n_k, cent_v, n_v, static_cast<T*>(out_k), static_cast<T*>(out_v));
 }
 
 }  // namespace rq
@@ -633,21 +675,14 @@ extern "C" int rq_compress_store(const void* key, const void* value, int in_dtyp
     p.src[0] = key; p.src[1] = value;
     p.token_stride[0] = k_token_stride; p.token_stride[1] = v_token_stride;
     p.head_stride[0] = k_head_stride; p.head_stride[1] = v_head_stride;
-    p.num_tokens = num_tokens; p.H = num_kv_heads;
-    p.h_shift = -1;
-    for (int sft = 0; sft < 16; ++sft)
-        if ((1 << sft) == num_kv_heads) p.h_shift = sft;
+    p.rows = static_cast<uint32_t>(num_tokens * num_kv_heads); p.H = num_kv_heads;
+    p.h_shift = shift_of(num_kv_heads);
     p.cache = kv_cache; p.num_slots = num_slots; p.total_bytes = total_bytes;
     p.slot_mapping = slot_mapping; p.write_padding = write_padding;
     p.rotation = rotation;
     p.bounds[0] = k_boundaries; p.bounds[1] = v_boundaries;
     p.n_bounds[0] = n_k_boundaries; p.n_bounds[1] = n_v_boundaries;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    switch (in_dtype) {
-        case RQ_DTYPE_F32: launch_store<float>(p, st); break;
-        case RQ_DTYPE_F16: launch_store<__half>(p, st); break;
-        default: launch_store<__nv_bfloat16>(p, st); break;
-    }
+    dispatch_walk<true>(p, in_dtype, 2, static_cast<cudaStream_t>(stream));
     return check_cuda(cudaGetLastError(), "rq_compress_store launch");
 }
 
@@ -665,15 +700,16 @@ extern "C" int rq_compress(const void* x, int in_dtype, int64_t num_rows, int he
         return fail(RQ_ERR_INVALID_ARG, "rq_compress: null pointer");
     if ((row_stride * dtype_bytes(in_dtype)) % 16 != 0 || !aligned(x, 16) || !aligned(packed_out, 4))
         return fail(RQ_ERR_ALIGNMENT, "rq_compress: rows must be 16-byte aligned");
-    CompressParams p{};
-    p.src[0] = x; p.token_stride[0] = row_stride; p.num_tokens = num_rows;
-    p.packed_out = packed_out; p.norms_out = norms_out; p.rotation = rotation;
-    p.bounds[0] = boundaries; p.n_bounds[0] = n_boundaries;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    switch (in_dtype) {
-        case RQ_DTYPE_F32: launch_rows<float>(p, st); break;
-        case RQ_DTYPE_F16: launch_rows<__half>(p, st); break;
-        default: launch_rows<__nv_bfloat16>(p, st); break;
+    constexpr int64_t kChunk = 1 << 30;                    // row numbers are 32-bit
+    for (int64_t at = 0; at < num_rows; at += kChunk) {
+        CompressParams p{};
+        p.src[0] = static_cast<const uint8_t*>(x) + at * row_stride * dtype_bytes(in_dtype);
+        p.token_stride[0] = row_stride;
+        p.H = 1;                                           // a row is a token of one head
+        p.rows = static_cast<uint32_t>(num_rows - at < kChunk ? num_rows - at : kChunk);
+        p.packed_out = packed_out + at * kHalfDim; p.norms_out = norms_out + at; p.rotation = rotation;
+        p.bounds[0] = boundaries; p.n_bounds[0] = n_boundaries;
+        dispatch_walk<false>(p, in_dtype, 1, static_cast<cudaStream_t>(stream));
     }
     return check_cuda(cudaGetLastError(), "rq_compress launch");
 }
@@ -693,22 +729,11 @@ extern "C" int rq_decompress(const uint8_t* packed, const float* norms, int64_t 
         return fail(RQ_ERR_INVALID_ARG, "rq_decompress: null pointer");
     if (!aligned(packed, 16) || !aligned(out, 16))
         return fail(RQ_ERR_ALIGNMENT, "rq_decompress: packed and out must be 16-byte aligned");
-    const int threads = 256;
-    const unsigned grid = static_cast<unsigned>((num_rows * 4 + threads - 1) / threads);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     switch (out_dtype) {
-        case RQ_DTYPE_F32:
-            decompress_rows_kernel<float><<<grid, threads, 0, st>>>(
-                packed, norms, num_rows, centroids, n_centroids, static_cast<float*>(out));
-            break;
-        case RQ_DTYPE_F16:
-            decompress_rows_kernel<__half><<<grid, threads, 0, st>>>(
-                packed, norms, num_rows, centroids, n_centroids, static_cast<__half*>(out));
-            break;
-        default:
-            decompress_rows_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(
-                packed, norms, num_rows, centroids, n_centroids, static_cast<__nv_bfloat16*>(out));
-            break;
+        case RQ_DTYPE_F32: launch_expand_rows<float>(packed, norms, num_rows, centroids, n_centroids, out, st); break;
+        case RQ_DTYPE_F16: launch_expand_rows<__half>(packed, norms, num_rows, centroids, n_centroids, out, st); break;
+        default: launch_expand_rows<__nv_bfloat16>(packed, norms, num_rows, centroids, n_centroids, out, st); break;
     }
     return check_cuda(cudaGetLastError(), "rq_decompress launch");
 }
@@ -734,29 +759,36 @@ extern "C" int rq_decompress_blocks(const uint8_t* kv_cache, int64_t num_blocks,
         return fail(RQ_ERR_INVALID_ARG, "rq_decompress_blocks: null pointer");
     if (!aligned(kv_cache, 16) || !aligned(out_k, 16) || !aligned(out_v, 16))
         return fail(RQ_ERR_ALIGNMENT, "rq_decompress_blocks: kv_cache and outputs must be 16-byte aligned");
-    const int threads = 256;
-    const int64_t work = 2 * num_listed * block_size * num_kv_heads * 4;
-    if ((work + threads - 1) / threads > 0x7fffffffLL)
-        return fail(RQ_ERR_UNSUPPORTED, "rq_decompress_blocks: too many rows for one launch");
-    const unsigned grid = static_cast<unsigned>((work + threads - 1) / threads);
+    const int64_t rows = num_listed * block_size * num_kv_heads;
+    if (rows > 0x7fffffffLL) return fail(RQ_ERR_UNSUPPORTED, "rq_decompress_blocks: too many rows for one launch");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    auto launch = [&](auto tag) {
+        launch_expand_blocks<decltype(tag)>(kv_cache, total_bytes, block_size, num_kv_heads, blocks, rows, num_blocks, centroids_k,
+                                            n_centroids_k, centroids_v, n_centroids_v, out_k, out_v, st);
+    };
     switch (out_dtype) {
-        case RQ_DTYPE_F32:
-            decompress_blocks_kernel<float><<<grid, threads, 0, st>>>(
-                kv_cache, total_bytes, block_size, num_kv_heads, blocks, num_listed, num_blocks, centroids_k,
-                n_centroids_k, centroids_v, n_centroids_v, static_cast<float*>(out_k), static_cast<float*>(out_v));
-            break;
-        case RQ_DTYPE_F16:
-            decompress_blocks_kernel<__half><<<grid, threads, 0, st>>>(
-                kv_cache, total_bytes, block_size, num_kv_heads, blocks, num_listed, num_blocks, centroids_k,
-                n_centroids_k, centroids_v, n_centroids_v, static_cast<__half*>(out_k), static_cast<__half*>(out_v));
-            break;
-        default:
-            decompress_blocks_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(
-                kv_cache, total_bytes, block_size, num_kv_heads, blocks, num_listed, num_blocks, centroids_k,
-                n_centroids_k, centroids_v, n_centroids_v, static_cast<__nv_bfloat16*>(out_k),
-                static_cast<__nv_bfloat16*>(out_v));
-            break;
+        case RQ_DTYPE_F32: launch(float{}); break;
+        case RQ_DTYPE_F16: launch(__half{}); break;
+        default: launch(__nv_bfloat16{}); break;
     }
     return check_cuda(cudaGetLastError(), "rq_decompress_blocks launch");
+}
+
+extern "C" int rq_block_union(const int32_t* block_table, int64_t block_table_stride, int num_seqs, int max_blocks,
+                              const int32_t* seq_lens, int block_size, int64_t num_blocks, int32_t* blocks_out,
+                              int32_t* remapped_out, int32_t* count_out, void* stream) {
+    if (num_seqs <= 0 || max_blocks <= 0 || block_size <= 0 || num_blocks <= 0)
+        return fail(RQ_ERR_INVALID_ARG, "rq_block_union: negative or zero size");
+    if (num_blocks > kUnionMaxBlocks || static_cast<int64_t>(num_seqs) * max_blocks > kUnionMaxEntries)
+        return fail(RQ_ERR_UNSUPPORTED, "rq_block_union: %lld blocks, %lld table entries (at most %lld, %lld)",
+                    static_cast<long long>(num_blocks), static_cast<long long>(num_seqs) * max_blocks,
+                    static_cast<long long>(kUnionMaxBlocks), static_cast<long long>(kUnionMaxEntries));
+    if (!block_table || !seq_lens || !blocks_out || !remapped_out || !count_out)
+        return fail(RQ_ERR_INVALID_ARG, "rq_block_union: null pointer");
+    const size_t smem = static_cast<size_t>((num_blocks + 31) / 32) * 8;
+    if (int e = ensure_smem(block_union_kernel, smem)) return e;
+    block_union_kernel<<<1, kUnionThreads, smem, static_cast<cudaStream_t>(stream)>>>(
+        block_table, block_table_stride, num_seqs, max_blocks, seq_lens, block_size, static_cast<int>(num_blocks), blocks_out,
+        remapped_out, count_out);
+    return check_cuda(cudaGetLastError(), "rq_block_union launch");
 }
