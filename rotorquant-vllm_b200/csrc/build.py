@@ -49,7 +49,7 @@ def build_host(force: bool = False) -> str:
     dirs = [flag for d in library_paths("cuda") for flag in (f"-L{d}", f"-Wl,-rpath,{d}")]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(_GLIBCXX_USE_CXX11_ABI)}", *includes, HOST_SOURCE, "-o", HOST_LIB, *dirs,
-           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-lcudart"]
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
         raise RuntimeError(" ".join(cmd) + "\n" + proc.stdout + proc.stderr)

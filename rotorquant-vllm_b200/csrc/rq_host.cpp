@@ -31,6 +31,8 @@ struct Entry {
     decltype(&rq_compress_store) compress_store;
     decltype(&rq_compress) compress;
     decltype(&rq_decompress) decompress;
+    decltype(&rq_decompress_blocks) decompress_blocks;
+    decltype(&rq_block_union) block_union;
     decltype(&rq_decode_workspace_bytes) decode_workspace_bytes;
     decltype(&rq_decode) decode;
     decltype(&rq_prefill_workspace_bytes) prefill_workspace_bytes;
@@ -130,12 +132,14 @@ PyObject* bind(PyObject*, PyObject* dict) {
     set(fn.compress_store, dict, "rq_compress_store");
     set(fn.compress, dict, "rq_compress");
     set(fn.decompress, dict, "rq_decompress");
+    set(fn.decompress_blocks, dict, "rq_decompress_blocks");
+    set(fn.block_union, dict, "rq_block_union");
     set(fn.decode_workspace_bytes, dict, "rq_decode_workspace_bytes");
     set(fn.decode, dict, "rq_decode");
     set(fn.prefill_workspace_bytes, dict, "rq_prefill_workspace_bytes");
     set(fn.prefill_int8_staged, dict, "rq_prefill_int8_staged");
     set(fn.last_error, dict, "rq_last_error");
-    bound = fn.compress_store && fn.compress && fn.decompress && fn.decode_workspace_bytes && fn.decode &&
+    bound = fn.compress_store && fn.compress && fn.decompress && fn.decompress_blocks && fn.block_union && fn.decode_workspace_bytes && fn.decode &&
             fn.prefill_workspace_bytes && fn.prefill_int8_staged && fn.last_error;
     if (PyErr_Occurred()) return nullptr;
     if (!bound) { PyErr_SetString(PyExc_RuntimeError, "bind: an entry point is missing"); return nullptr; }
@@ -383,6 +387,63 @@ PyObject* decompress(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     return THPVariable_Wrap(out);
 }
 
+// gather(kv_cache, block_table, seq_lens, num_kv_heads, k_centroids, v_centroids, dtype_code) -> (k, v, remapped)
+PyObject* gather(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    if (n_args != 7 || !bound) return none();
+    const at::Tensor *cache = tensor(a[0]), *table = tensor(a[1]), *lens = tensor(a[2]), *ck = tensor(a[4]), *cv = tensor(a[5]);
+    int64_t heads, code;
+    if (!cache || !table || !lens || !ck || !cv || !integer(a[3], heads) || !integer(a[6], code)) return none();
+    Device dev;
+    for (const at::Tensor* t : {cache, table, lens, ck, cv}) dev.add(*t);
+    if (!dev.ok || code < 0 || code > 2 || cache->scalar_type() != at::kByte || cache->dim() != 3 || !cache->is_contiguous() ||
+        cache->numel() == 0 || table->scalar_type() != at::kInt || table->dim() != 2 || table->numel() == 0 ||
+        table->stride(1) != 1 || lens->scalar_type() != at::kInt || lens->dim() != 1 || !lens->is_contiguous() ||
+        lens->numel() != table->size(0) || !f32_vector(*ck) || !f32_vector(*cv) || heads <= 0 || table->numel() > INT32_MAX)
+        return none();
+    const int64_t nb = cache->size(0), bs = cache->size(1);
+    const auto index = static_cast<c10::DeviceIndex>(dev.index);
+    const c10::cuda::CUDAGuard guard(index);
+    const at::Tensor listed = at::empty({std::min(table->numel(), nb)}, table->options());
+    const at::Tensor remapped = at::empty({table->size(0), table->size(1)}, table->options());
+    // the count lands in pinned memory of this thread, which the kernel writes directly
+    static thread_local at::Tensor landing;
+    if (!landing.defined()) landing = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    auto* count = static_cast<volatile int32_t*>(landing.data_ptr());
+    const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(index);
+    int status;
+    Py_BEGIN_ALLOW_THREADS
+    status = fn.block_union(static_cast<const int32_t*>(table->const_data_ptr()), table->stride(0),
+                            static_cast<int>(table->size(0)), static_cast<int>(table->size(1)),
+                            static_cast<const int32_t*>(lens->const_data_ptr()), static_cast<int>(bs), nb,
+                            static_cast<int32_t*>(listed.data_ptr()), static_cast<int32_t*>(remapped.data_ptr()),
+                            static_cast<int32_t*>(landing.data_ptr()), stream.stream());
+    Py_END_ALLOW_THREADS
+    if (status == RQ_ERR_UNSUPPORTED) return none();
+    if (raised(status)) return nullptr;
+    cudaError_t err;
+    Py_BEGIN_ALLOW_THREADS
+    err = cudaStreamSynchronize(stream.stream());
+    Py_END_ALLOW_THREADS
+    if (err != cudaSuccess) { PyErr_SetString(PyExc_RuntimeError, cudaGetErrorString(err)); return nullptr; }
+    const int64_t n = *count;
+    if (n < 0) return none();
+    const at::ScalarType types[3] = {at::kFloat, at::kHalf, at::kBFloat16};
+    const at::Tensor k = at::empty({n, bs, heads, 128}, cache->options().dtype(types[code])), v = at::empty_like(k);
+    Py_BEGIN_ALLOW_THREADS
+    status = fn.decompress_blocks(static_cast<const uint8_t*>(cache->const_data_ptr()), nb, static_cast<int>(bs),
+                                  static_cast<int>(cache->size(2)), static_cast<int>(heads), 128,
+                                  static_cast<const int32_t*>(listed.const_data_ptr()), n,
+                                  static_cast<const float*>(ck->const_data_ptr()), static_cast<int>(ck->numel()),
+                                  static_cast<const float*>(cv->const_data_ptr()), static_cast<int>(cv->numel()),
+                                  k.data_ptr(), v.data_ptr(), static_cast<int>(code), stream.stream());
+    Py_END_ALLOW_THREADS
+    if (raised(status)) return nullptr;
+    PyObject* out[3] = {THPVariable_Wrap(k), THPVariable_Wrap(v), THPVariable_Wrap(remapped)};
+    PyObject* all = out[0] && out[1] && out[2] ? PyTuple_Pack(3, out[0], out[1], out[2]) : nullptr;
+    for (PyObject* o : out) Py_XDECREF(o);
+    return all;
+}
+
 PyMethodDef methods[] = {
     {"bind", bind, METH_O, nullptr},
     {"mark_valid", mark_valid, METH_O, nullptr},
@@ -392,6 +453,7 @@ PyMethodDef methods[] = {
     {"prefill", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(prefill)), METH_FASTCALL, nullptr},
     {"compress", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(compress)), METH_FASTCALL, nullptr},
     {"decompress", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(decompress)), METH_FASTCALL, nullptr},
+    {"gather", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(gather)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

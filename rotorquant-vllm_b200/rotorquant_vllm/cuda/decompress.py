@@ -76,8 +76,14 @@ def decompress_cache_paged(kv_cache: torch.Tensor, block_table: torch.Tensor, se
     """Mirror of ``RQAttentionImpl._decompress_cache_paged`` (vllm/rq_backend.py:737-852 of the
     reference): decompress only the physical blocks the batch references and return
     ``(key_cache, value_cache, remapped_block_table)`` with K/V ``(num_unique, block_size, H, 128)``
-    and the table renumbered into that compact block space.  ``torch.unique`` sizes its result on
-    the host, as upstream; the gather, the per-head split and both decompressions are one launch."""
+    and the table renumbered into that compact block space.  The number of blocks sizes the result,
+    so the host waits for it once, as upstream's ``torch.unique`` does; the union of the blocks is one
+    launch and the gather, the per-head split and both decompressions are another.  Tables the union
+    kernel does not take (entries outside the cache, more than 2**20 entries) go through torch."""
+    done = _lib.host().gather(kv_cache, block_table, seq_lens, num_kv_heads, centroids_k, centroids_v,
+                              _lib.DTYPE_CODE.get(dtype, -1))
+    if done is not None:
+        return done
     nb, bs, _ = kv_cache.shape
     need = (seq_lens.to(torch.int64) + bs - 1) // bs
     cols = torch.arange(block_table.shape[1], device=block_table.device).unsqueeze(0)
