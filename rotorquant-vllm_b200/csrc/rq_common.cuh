@@ -43,6 +43,25 @@ inline int ensure_smem(Kernel k, size_t bytes) {
     return ensure_smem_impl(reinterpret_cast<const void*>(k), bytes);
 }
 
+// Launch with programmatic stream serialization: the kernel may be scheduled while the one before it on the stream
+// drains, as soon as all of that kernel's CTAs have ended or called grid_launch_dependents().  It must not touch
+// memory that earlier kernels write (or read, if it writes it) before grid_dependency_wait() returns.
+template <typename... KArgs, typename... Args>
+inline int launch_dependent(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                            Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...), what);
+}
+
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 inline int dtype_bytes(int dt) { return dt == RQ_DTYPE_F32 ? 4 : 2; }
@@ -61,6 +80,12 @@ __host__ __device__ inline SlotLayout slot_layout(int H) {
     l.total = H * kSlotPerHead;
     return l;
 }
+
+// Programmatic dependent launch.  wait: every kernel before this one on the stream has completed (returns at once in
+// a kernel launched without the attribute).  launch_dependents: the next kernel may be scheduled.  A kernel that
+// waits before it lets the next one start makes everything older visible to the next one from its start.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- device helpers --------------------------------------------------------
 

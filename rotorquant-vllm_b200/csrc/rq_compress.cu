@@ -381,6 +381,7 @@ __global__ void __launch_bounds__(kCompressThreads, 2)
 compress_kernel(const CompressParams p) {
     __shared__ CompressSmem sm[kCompressWarps];
     const int kv = blockIdx.y;
+    grid_launch_dependents();              // the attention kernel's set-up may run beside this; it waits for this grid's end
     const int lane = threadIdx.x & 31;
     CompressSmem& mine = sm[threadIdx.x >> 5];
     auto walk = [&](auto nb) {

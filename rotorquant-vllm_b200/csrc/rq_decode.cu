@@ -82,6 +82,7 @@ struct DecodeParams {
     int32_t* prefix;                       // [num_seqs + 1] exclusive prefix of tiles per sequence (workspace)
     int2* seq_groups;                      // [num_seqs] first and last group whose piece holds tiles of the sequence
     int num_seqs;
+    long long tiles_bound;                 // num_seqs * tiles of the longest sequence the caller admits
     int groups;                            // pieces; CTA = (group, item), item = (KV head, head group)
     int inline_plan;                       // the attention CTAs compute the prefix sums themselves
     int bs_shift;                          // log2(block_size) when it is a power of two, else -1
@@ -106,7 +107,9 @@ __host__ __device__ inline int64_t weight_cum(int64_t n, int layer_ctas, int num
     }
     return acc;
 }
+// A batch with no more tiles than groups (short sequences under a wide block table) gives every group one tile.
 __device__ __forceinline__ int64_t piece_begin(const DecodeParams& p, int64_t g, int64_t total, int J) {
+    if (total <= p.groups) return g < total ? g : total;
     return total * weight_cum(g * J, p.layer_ctas, p.num_layers, p.layer_w) /
            weight_cum(static_cast<int64_t>(p.groups) * J, p.layer_ctas, p.num_layers, p.layer_w);
 }
@@ -180,11 +183,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-
-// Programmatic dependent launch: the merge kernel may be scheduled while the attention kernel
-// drains; it must not read the partial results before this wait returns.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- per-token lookup tables -------------------------------------------------
 //
@@ -336,6 +334,18 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     constexpr int NK = 1 << KB, NV = 1 << VB;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+    // Barriers and TMEM first: they need nothing from the kernels before this one, which may still be running.
+    if (tid == 0) {
+        mbar_init(&sm.bar_s, 1);
+        mbar_init(&sm.bar_o, 1);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) mbar_init(&sm.bar_in[w], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_proxy();
+    }
+    if (warp == 0) tmem_alloc(&sm.tmem_base, kUTmemCols);
+    grid_dependency_wait();
+
     // ---- tiles of every sequence as an exclusive prefix sum; this CTA's piece: CTA = (group, item) ----
     const int J = p.H * p.head_groups;
     const int64_t group = blockIdx.x / J;
@@ -373,17 +383,12 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         x_end = piece_begin(p, group + 1, total, J);
     }
     if (tid == 0) grid_launch_dependents();    // the merge kernel may be scheduled; it waits for this grid's end
-    if (group >= p.groups || x >= x_end) return;
-
-    if (tid == 0) {
-        mbar_init(&sm.bar_s, 1);
-        mbar_init(&sm.bar_o, 1);
-#pragma unroll
-        for (int w = 0; w < 4; ++w) mbar_init(&sm.bar_in[w], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        fence_async_proxy();
+    if (group >= p.groups || x >= x_end) {
+        tc_fence_before();
+        __syncthreads();
+        if (warp == 0) tmem_dealloc(sm.tmem_base, kUTmemCols);
+        return;
     }
-    if (warp == 0) tmem_alloc(&sm.tmem_base, kUTmemCols);
     if (tid < 32) {
         const int kv = tid >> 4, i = tid & 15;
         const int n = kv ? NV : NK;
@@ -862,6 +867,8 @@ __global__ void decode_plan_kernel(const int32_t* __restrict__ seq_lens, int num
                                    int32_t* __restrict__ prefix) {
     __shared__ int warp_sums[32];
     __shared__ int carry;
+    grid_dependency_wait();
+    grid_launch_dependents();
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     for (int base = 0; base < num_seqs; base += blockDim.x) {
@@ -891,24 +898,26 @@ __global__ void decode_plan_kernel(const int32_t* __restrict__ seq_lens, int num
 // query head sits in slot (query head within its group of 8).  Lanes
 // gather the running maxima and row sums of up to 32 parts at a time; then the warp sums the
 // weighted partial outputs.  Which groups those are was recorded per sequence by the attention CTAs.
-// W = 1: a warp per row (the usual few parts per row).  W = 4: a CTA per row, warp s taking every fourth round
-// of 32 parts and the four partial sums combined through shared memory -- for long sequences on few heads,
-// where a row has dozens of parts and there are too few rows to hide the latency of walking them.
-constexpr int kMergeWarps = 4;
+// W = 1: a warp per row (the usual few parts per row).  W = 8: a CTA per row, warp s taking parts s, s + 8, ...
+// and the partial sums combined through shared memory -- for long sequences on few heads, where a row has dozens of
+// parts and there are too few rows to hide the latency of walking them; dealt out one by one, so that 70 parts are
+// nine loads in flight per warp and not four batches of eight in each of two warps.
+constexpr int kMergeWarps = 4;               // rows per CTA of the warp-per-row form
+constexpr int kWideMergeWarps = 8;
 template <typename T, int W>
-__global__ void __launch_bounds__(kMergeWarps * 32)
+__global__ void __launch_bounds__((W > 1 ? W : kMergeWarps) * 32)
 decode_merge_kernel(const DecodeParams p) {
     __shared__ float part_ml[W > 1 ? W : 1][2];
     __shared__ float4 part_acc[W > 1 ? W : 1][32];
     const int lane = threadIdx.x & 31;
-    const int sub = (threadIdx.x >> 5) % W;
+    const int sub = W > 1 ? threadIdx.x >> 5 : 0;
     // the lane's 4x4 block of R does not depend on the attention launch: fetch it before waiting for that
     float4 rr[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
         rr[k] = __ldg(reinterpret_cast<const float4*>(p.rotation + (4 * lane + k) * kHeadDim + 4 * lane));
     grid_dependency_wait();
-    const int64_t wq = static_cast<int64_t>(blockIdx.x) * (kMergeWarps / W) + (threadIdx.x >> 5) / W;
+    const int64_t wq = W > 1 ? static_cast<int64_t>(blockIdx.x) : static_cast<int64_t>(blockIdx.x) * kMergeWarps + (threadIdx.x >> 5);
     if (wq >= static_cast<int64_t>(p.num_seqs) * p.Hq) return;          // (all warps of a row together)
     const int seq = static_cast<int>(wq / p.Hq), qh = static_cast<int>(wq % p.Hq);
     const int J = p.H * p.head_groups;
@@ -933,11 +942,11 @@ decode_merge_kernel(const DecodeParams p) {
             min_w = p.layer_w[0];
             for (int i = 1; i < p.num_layers; ++i) min_w = min(min_w, p.layer_w[i]);
         }
-        const bool dense = total * J * min_w >=
+        const bool dense = total <= p.groups || total * J * min_w >=
                            weight_cum(static_cast<int64_t>(p.groups) * J, p.layer_ctas, p.num_layers, p.layer_w);
         float m_all = -INFINITY;
-        for (int g0 = g_first + 32 * sub; g0 <= g_last; g0 += 32 * W) {             // normally one round
-            const int gi = g0 + lane;
+        for (int g0 = g_first + sub; g0 <= g_last; g0 += 32 * W) {                  // normally one round
+            const int gi = g0 + lane * W;
             const bool live = gi <= g_last &&
                               (dense || piece_begin(p, gi, total, J) < piece_begin(p, gi + 1, total, J));
             const int64_t r = ((static_cast<int64_t>(gi) + seq) * J + item) * slots + slot;
@@ -947,6 +956,7 @@ decode_merge_kernel(const DecodeParams p) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) m_round = fmaxf(m_round, __shfl_xor_sync(0xffffffffu, m_round, o));
             const float m_new = fmaxf(m_all, m_round);
+            if (m_new == -INFINITY) continue;                            // only empty groups so far
             const float w = live ? exp2f(m - m_new) : 0.0f;
             float l_round = w * l;
 #pragma unroll
@@ -955,13 +965,13 @@ decode_merge_kernel(const DecodeParams p) {
             acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
             l_all = l_all * rescale + l_round;
             m_all = m_new;
-            const int n_here = min(32, g_last - g0 + 1);
+            const int n_here = min(32, (g_last - g0) / W + 1);
 #pragma unroll 8
             for (int k = 0; k < n_here; ++k) {
                 const float wk = __shfl_sync(0xffffffffu, w, k);
                 if (wk != 0.0f) {
                     const float4 o = *reinterpret_cast<const float4*>(
-                        p.ws_o + ((((static_cast<int64_t>(g0 + k) + seq) * J + item) * slots + slot) << 7) + 4 * lane);
+                        p.ws_o + ((((static_cast<int64_t>(g0 + k * W) + seq) * J + item) * slots + slot) << 7) + 4 * lane);
                     acc.x += wk * o.x; acc.y += wk * o.y; acc.z += wk * o.z; acc.w += wk * o.w;
                 }
             }
@@ -1180,9 +1190,21 @@ static const DecodeEnv& decode_env() {
 
 template <typename T, int KB, int VB>
 static int launch_decode(DecodeParams& p, int nh, bool tma, cudaStream_t st) {
+    // A launch may start its set-up while the one before (the cache write of the step, for the first) drains: 22.5 ->
+    // 15.5 us for a step of one short sequence.  Not the attention kernel when its CTAs fill every SM with long pieces:
+    // scheduled around the CTAs still running they no longer form launch layers, which their piece weights rely on
+    // (64 x 4096 tokens, 28 tiles per piece: 106 -> 119 us; 16 sequences of up to 32768 on one head, 7 tiles:
+    // 47.6 -> 44.0).  RQ_DECODE_NO_PDL=1 puts full launch boundaries between all of them.
+    const bool layered = p.layer_ctas > 0 && p.tiles_bound > 10LL * p.groups;
+    auto launch = [&](const char* what, bool overlap, auto kernel, dim3 grid, dim3 block, size_t smem, auto... args) -> int {
+        if (overlap && !decode_env().no_pdl) return launch_dependent(what, kernel, grid, block, smem, st, args...);
+        kernel<<<grid, block, smem, st>>>(args...);
+        return check_cuda(cudaGetLastError(), what);
+    };
     if (!p.inline_plan) {
-        decode_plan_kernel<<<1, 1024, 0, st>>>(p.seq_lens, p.num_seqs, kUTile, p.prefix);
-        if (int e = check_cuda(cudaGetLastError(), "rq_decode plan launch")) return e;
+        if (int e = launch("rq_decode plan launch", !layered, decode_plan_kernel, dim3(1), dim3(1024), 0, p.seq_lens, p.num_seqs, kUTile,
+                           p.prefix))
+            return e;
     }
     alignas(64) CUtensorMap map_idx{};
     if (tma)
@@ -1190,41 +1212,26 @@ static int launch_decode(DecodeParams& p, int nh, bool tma, cudaStream_t st) {
     {
         const size_t smem = sizeof(UmmaSmem) + 512;                              // + hand alignment
         const long long ctas = 1LL * p.groups * p.H * p.head_groups;
-        auto launch = [&](auto kernel) -> int {
+        auto attend = [&](auto kernel) -> int {
             if (int e = ensure_smem(kernel, smem)) return e;
-            kernel<<<static_cast<unsigned>(ctas), kUThreads, smem, st>>>(p, map_idx);
-            return check_cuda(cudaGetLastError(), "rq_decode attention launch");
+            return launch("rq_decode attention launch", !layered, kernel, dim3(static_cast<unsigned>(ctas)), dim3(kUThreads), smem, p, map_idx);
         };
         // rows by TMA when the geometry allows; V rows of 1 or 2 KV heads are not 16-byte aligned
         const int mode = !tma ? 0 : (p.H % 4 == 0 ? 1 : 2);
         int e = RQ_OK;
-        if (mode == 0) e = nh == 4 ? launch(decode_attn_kernel<T, KB, VB, 0, 4>) : launch(decode_attn_kernel<T, KB, VB, 0, 8>);
-        else if (mode == 1) e = nh == 4 ? launch(decode_attn_kernel<T, KB, VB, 1, 4>) : launch(decode_attn_kernel<T, KB, VB, 1, 8>);
-        else e = nh == 4 ? launch(decode_attn_kernel<T, KB, VB, 2, 4>) : launch(decode_attn_kernel<T, KB, VB, 2, 8>);
+        if (mode == 0) e = nh == 4 ? attend(decode_attn_kernel<T, KB, VB, 0, 4>) : attend(decode_attn_kernel<T, KB, VB, 0, 8>);
+        else if (mode == 1) e = nh == 4 ? attend(decode_attn_kernel<T, KB, VB, 1, 4>) : attend(decode_attn_kernel<T, KB, VB, 1, 8>);
+        else e = nh == 4 ? attend(decode_attn_kernel<T, KB, VB, 2, 4>) : attend(decode_attn_kernel<T, KB, VB, 2, 8>);
         if (e) return e;
     }
 
     // rows with many parts each (long sequences on few heads): a CTA per row instead of a warp per row
     const long long rows = 1LL * p.num_seqs * p.Hq;
     const bool wide = p.groups > 8LL * p.num_seqs;
-    const unsigned grid = static_cast<unsigned>(wide ? rows : (rows + kMergeWarps - 1) / kMergeWarps);
-    if (decode_env().no_pdl) {
-        if (wide) decode_merge_kernel<T, kMergeWarps><<<grid, kMergeWarps * 32, 0, st>>>(p);
-        else decode_merge_kernel<T, 1><<<grid, kMergeWarps * 32, 0, st>>>(p);
-        return check_cuda(cudaGetLastError(), "rq_decode merge launch");
-    }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kMergeWarps * 32);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return check_cuda(wide ? cudaLaunchKernelEx(&cfg, decode_merge_kernel<T, kMergeWarps>, p)
-                           : cudaLaunchKernelEx(&cfg, decode_merge_kernel<T, 1>, p), "rq_decode merge launch");
+    if (wide) return launch("rq_decode merge launch", true, decode_merge_kernel<T, kWideMergeWarps>, dim3(static_cast<unsigned>(rows)),
+                            dim3(kWideMergeWarps * 32), 0, p);
+    return launch("rq_decode merge launch", true, decode_merge_kernel<T, 1>, dim3(static_cast<unsigned>((rows + kMergeWarps - 1) / kMergeWarps)),
+                  dim3(kMergeWarps * 32), 0, p);
 }
 
 template <typename T>
@@ -1313,6 +1320,7 @@ static int decode_impl(const void* q, void* out, int dtype, int64_t q_stride_seq
     p.ws_m = p.ws_o + slots * kHeadDim;
     p.ws_l = p.ws_m + slots;
     p.num_seqs = num_seqs; p.groups = pl.groups;
+    p.tiles_bound = 1LL * num_seqs * ((max_seq_len + kUTile - 1) / kUTile);
     p.inline_plan = num_seqs <= kInlinePlanSeqs ? 1 : 0;
     p.bs_shift = bs_shift;
     // TMA boxes of 16 tokens: power-of-two blocks of 16 tokens or more (a box never straddles a block),

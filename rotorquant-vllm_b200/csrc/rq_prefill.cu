@@ -636,6 +636,8 @@ prefill_stage_kernel(const PrefillParams p) {
     constexpr int NK = 1 << KB, NV = 1 << VB;
     const int tid = threadIdx.x;
     const int tile = blockIdx.x, kvh = blockIdx.y, seq = blockIdx.z;
+    grid_dependency_wait();                // the cache write of this step
+    grid_launch_dependents();              // the attention kernel prepares its queries meanwhile (after the wait: its inputs are older)
     const int kv_len = max(__ldg(p.seq_lens + seq), 0);
     if (tile * kPfKeys >= kv_len) return;
     uint8_t* rec = p.stage + ((static_cast<int64_t>(seq) * p.stage_tiles_per_seq + tile) * p.H + kvh) * kStageRecord;
@@ -847,6 +849,7 @@ prefill_attn_kernel(const PrefillParams p) {
         mbar_expect_tx(bar, 2 * kPfKeys * kHeadDim);
         bulk_load(smem_u32(sm.v), rec + kPfKeys * kHeadDim, 2 * kPfKeys * kHeadDim, bar);
     };
+    grid_dependency_wait();              // the records
     if (tid == 0) {
         issue_k(0);
         issue_v(0);
@@ -1096,12 +1099,10 @@ static int launch_prefill(const PrefillParams& p, int m_tiles, int num_seqs, cud
     dim3 grid(m_tiles, p.H, num_seqs);
     if (p.stage != nullptr) {
         dim3 sgrid(p.stage_tiles_per_seq, p.H, num_seqs);
-        prefill_stage_kernel<T, KB, VB><<<sgrid, 128, 0, st>>>(p);
-        if (int e = check_cuda(cudaGetLastError(), "rq_prefill_int8 stage launch")) return e;
+        if (int e = launch_dependent("rq_prefill_int8 stage launch", prefill_stage_kernel<T, KB, VB>, sgrid, dim3(128), 0, st, p)) return e;
         const size_t smem = sizeof(AttnSmem);
         if (int e = ensure_smem(prefill_attn_kernel<T>, smem)) return e;
-        prefill_attn_kernel<T><<<grid, kPfThreads, smem, st>>>(p);
-        return check_cuda(cudaGetLastError(), "rq_prefill_int8 attention launch");
+        return launch_dependent("rq_prefill_int8 attention launch", prefill_attn_kernel<T>, grid, dim3(kPfThreads), smem, st, p);
     }
     const size_t smem = sizeof(PrefillSmem);
     if (int e = ensure_smem(prefill_int8_kernel<T, KB, VB>, smem)) return e;
