@@ -75,23 +75,6 @@ __device__ __forceinline__ void unpack4(const Raw4<__nv_bfloat16>& r, float (&x)
     x[2] = __uint_as_float(r.a.y << 16); x[3] = __uint_as_float(r.a.y & 0xFFFF0000u);
 }
 
-// Pairs of fp32 values in one 64-bit register.  A packed operation takes the pipe as long as two scalar ones but
-// one issue slot instead of two; every half is rounded as the scalar operation rounds it.
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 pk(float lo, float hi) {
-    f2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ void upk(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
 // Number of boundaries strictly below v.  The boundaries ascend, so "bd[b] < v" is true for a
 // prefix of them and a binary search over that prefix gives the count with log2(NB + 1) compares
 // (a NaN compares false everywhere: 0, as the linear count gives).

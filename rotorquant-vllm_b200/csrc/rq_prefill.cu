@@ -37,6 +37,7 @@ namespace rq {
 constexpr int kPfThreads = 256;       // two threads per row / key
 constexpr int kPfRows = 128;          // MMA M
 constexpr int kPfKeys = 128;          // keys per tile (MMA N of S, K extent of P V)
+constexpr int kSms = 148;
 constexpr uint32_t kTmemCols = 256;   // S: columns 0..127 (int32), O: columns 128..255 (fp32)
 
 struct PrefillParams {
@@ -44,7 +45,7 @@ struct PrefillParams {
     void* out;
     int64_t q_stride_tok, q_stride_head, o_stride_tok, o_stride_head;
     const int32_t* cu_seqlens_q;      // nullptr: one sequence owning all rows
-    int num_tokens;
+    int num_tokens, num_seqs;
     int H, Hq, G;
     int tokens_per_tile;              // 128 / G
     const uint8_t* cache;
@@ -61,6 +62,7 @@ struct PrefillParams {
     int* error_flag;                  // optional device int, set non-zero when a wait expired
     uint8_t* stage;                   // staged path: scratch records (see prefill_stage_kernel)
     int stage_tiles_per_seq;
+    int tiles_per_unit;               // staged path: MMA tiles per CTA, 1 or 2
 };
 
 template <typename T> using PfType = TcFormat<T>;
@@ -164,6 +166,16 @@ __device__ __forceinline__ float small_int_to_float(uint32_t x) {
 // Barrier of the two warps that share 32 rows (warp w and w ^ 4): ids 1..4.
 __device__ __forceinline__ void pair_sync(int quarter) {
     asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
+}
+
+// The same barrier (by id, 64 threads), and whether any of the threads said yes.
+__device__ __forceinline__ bool pair_any(int id, bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred a, b;\n\tsetp.ne.u32 a, %1, 0;\n\t"
+        "bar.red.or.pred b, %2, 64, a;\n\tselp.u32 %0, 1, 0, b;\n\t}"
+        : "=r"(r) : "r"(static_cast<uint32_t>(v)), "r"(id) : "memory");
+    return r != 0;
 }
 
 // 256 threads: thread (row = tid % 128, half = tid / 128).  Row r is TMEM lane r; the two threads
@@ -451,7 +463,9 @@ prefill_int8_kernel(const PrefillParams p) {
             }
             l_run *= alpha;
             m_run = m_new;
-            // pass B: probabilities -> shared P tile (K-major: 16 chunks of 8 keys per row)
+            // pass B: probabilities -> shared P tile (K-major: 16 chunks of 8 keys per row); the row sum in four
+            // strands (key mod 4), the order in which the staged kernel adds, too
+            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             auto emit_chunk = [&](const uint32_t (&r)[32], int ch) {
                 uint32_t pk[16];
 #pragma unroll
@@ -462,7 +476,8 @@ prefill_int8_kernel(const PrefillParams p) {
                         if (32 * ch + c > limit) p0 = 0.0f;
                         if (32 * ch + c + 1 > limit) p1 = 0.0f;
                     }
-                    l_run += p0 + p1;
+                    sum[c & 2] += p0;
+                    sum[(c & 2) + 1] += p1;
                     pk[c >> 1] = pf_pack<T>(p0, p1);
                 }
 #pragma unroll
@@ -476,6 +491,7 @@ prefill_int8_kernel(const PrefillParams p) {
                 tmem_ld32(lane_base + 64 * half + 32, r1);
                 emit_chunk(r1, 1);
             }
+            l_run += (sum[0] + sum[2]) + (sum[1] + sum[3]);
         };
         // After the first tile the reference maximum rarely has to move, so the tile is first done in ONE
         // pass against the current reference (scaled sums and probabilities together, nothing parked in TMEM,
@@ -484,7 +500,7 @@ prefill_int8_kernel(const PrefillParams p) {
         auto softmax_one_pass = [&](auto masked_tag) -> bool {
             constexpr bool kMasked = decltype(masked_tag)::value;
             const float m_use = (m_run == -INFINITY) ? 0.0f : m_run;
-            float l_try = l_run;
+            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 1
             for (int ch = 0; ch < 2; ++ch) {
                 uint32_t r[32], pk[16];
@@ -501,8 +517,8 @@ prefill_int8_kernel(const PrefillParams p) {
                         pr[e] = pf_ex2(fmaf(sv, row_factor, -m_use));
                         if (kMasked && 32 * ch + c > limit) pr[e] = 0.0f;
                     }
-                    l_try += pr[0] + pr[1];
-                    l_try += pr[2] + pr[3];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) sum[e] += pr[e];
                     pk[2 * c4] = pf_pack<T>(pr[0], pr[1]);
                     pk[2 * c4 + 1] = pf_pack<T>(pr[2], pr[3]);
                 }
@@ -511,17 +527,15 @@ prefill_int8_kernel(const PrefillParams p) {
                     *reinterpret_cast<uint4*>(prow + (8 * half + 4 * ch + kc) * 128) =
                         make_uint4(pk[4 * kc], pk[4 * kc + 1], pk[4 * kc + 2], pk[4 * kc + 3]);
             }
-            // The maximum is not tracked here: a row whose probabilities of this tile add up to more than 2^15
-            // has outgrown its reference (every probability is below 2^15 otherwise, harmless for P in T
+            // The maximum is not tracked here: a row whose probabilities of this half tile add up to more than 2^14
+            // has outgrown its reference (every probability is below 2^14 otherwise, harmless for P in T
             // precision and for the fp32 sums), and so has a row that met its first visible key (its
             // reference is still -inf and some probability is exp2(score), unbounded): redo those tiles.
-            sm.xch[half][row] = l_try - l_run;
-            pair_sync(quarter);
-            const float tile_sum = (l_try - l_run) + sm.xch[half ^ 1][row];
-            // both warps that share these rows see the same sums, hence take the same decision
-            const bool outgrown = !(tile_sum <= 32768.0f) || (m_run == -INFINITY && tile_sum > 0.0f);
-            if (__any_sync(0xffffffffu, outgrown)) return false;
-            l_run = l_try;
+            const float half_sum = (sum[0] + sum[2]) + (sum[1] + sum[3]);
+            // both warps that share these rows take the same decision
+            const bool outgrown = !(half_sum <= 16384.0f) || (m_run == -INFINITY && half_sum > 0.0f);
+            if (pair_any(quarter + 1, outgrown)) return false;
+            l_run += half_sum;
             return true;
         };
         bool done = false;
@@ -607,28 +621,6 @@ prefill_int8_kernel(const PrefillParams p) {
 // the attention kernel, then the 128 key scales.  Record index: (seq * tiles_per_seq + tile) * H + head.
 constexpr int kStageRecord = 3 * kPfKeys * kHeadDim + kPfKeys * 4;      // 16 KB + 32 KB + 512 B
 
-struct __align__(128) AttnSmem {
-    uint8_t q[kPfRows * kHeadDim];
-    uint8_t k[kPfKeys * kHeadDim];
-    uint16_t v[kPfKeys * kHeadDim];
-    uint16_t p[kPfRows * kPfKeys];
-    float k_scale[2][kPfKeys];
-    float xch[2][kPfRows];
-    float rot[32 * 16];
-    uint64_t bar_s, bar_o, bar_k, bar_v;
-    uint32_t tmem_base;
-};
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar_addr, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_addr), "r"(bytes) : "memory");
-}
-// Contiguous global -> shared copy of `bytes` (multiple of 16, both addresses 16-byte aligned),
-// completing on the mbarrier.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar_addr) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar_addr) : "memory");
-}
-
 // One CTA of 128 threads per (tile, KV head, sequence): thread = key.  Writes the record of the tile.
 template <typename T, int KB, int VB>
 __global__ void __launch_bounds__(128)
@@ -704,406 +696,544 @@ prefill_stage_kernel(const PrefillParams p) {
     }
 }
 
-// The attention kernel of the staged path: the same CTA shape, query set-up, softmax and epilogue
-// as prefill_int8_kernel, but the K codes, key scales and V values of a tile arrive ready-made from
-// the scratch written by prefill_stage_kernel: one thread starts three bulk copies per tile
-// (cp.async.bulk, 16 KB + 512 B + 32 KB, already in operand order) that complete on mbarriers.  K of
-// tile j+1 and V of tile j are requested as soon as S_j is finished, so both land under the softmax.
+// ---- staged path: attention --------------------------------------------------------------------
+//
+// One CTA = two MMA tiles of 128 rows (2 x (128 / G) query tokens x G heads of one (sequence, KV head)) that
+// share every K/V tile they read.  Eighteen warps with fixed roles:
+//   warps 0-7, 8-15 softmax of tile 0 and tile 1: two threads per row (= TMEM lane), 64 keys each; they also prepare
+//                   their rows of Q and write their rows of the output;
+//   warp 16         issues every MMA: S_x(j) = Q_x K(j) (int8, shared memory -> int32 in TMEM) and O_x += P_x(j) V(j)
+//                   (P from TMEM, fp32 in TMEM);
+//   warp 17         keeps three stages of K codes, V values and key scales in flight (cp.async.bulk of the staged
+//                   records, already in operand order).
+// TMEM (all 512 columns): S_0 0-127, S_1 128-255, O_0 256-383, O_1 384-511; a thread's probabilities overwrite the
+// first half of the sums it read.  While one tile is in its softmax the tensor core works for the other: the order of
+// issue is PV_0(j) S_0(j+1) PV_1(j) S_1(j+1).  MMAs run in the order of issue, so S_x(j+1) cannot overwrite P_x(j)
+// before it has been read, and the commit behind S_x(j+1) also says that PV_x(j) is done.
+//
+// Softmax: the scaled sums are exponentiated against a lazy reference maximum in one pass over the half row; the tile
+// is redone (the sums are still in TMEM) after finding the row's maximum when it is the row's first tile, when the
+// probabilities add up to more than 2^14 (the reference has been outgrown by more than 2^8), or when a row meets its
+// first visible key.  Packed fp32 operations on key pairs: 4.75 issue slots per score.
+//
+// Bound by the softmax (exponentials and the fp32 pipe: about 1.1 us per 256 x 128 scores against 0.3 us of MMAs), and for
+// short sequences by what a CTA does outside the loop, about 10 us of a 32 us life at 2048 tokens.  Against one tile per
+// CTA, two CTAs per SM, P through shared memory (us, whole call): 2048 tokens after 30000, 32 heads 1140 -> 942-1000;
+// 8 x 2048 tokens 519 -> 479; 2 prompts of up to 1500 and 30 single tokens after 4000, 28 heads 286 -> 225.
+// Slower than this (the attention kernel of the first, 920 here): one thread per row 968; steps of 64 keys with two S
+// buffers 1192; S released early and P in shared memory 1210; an MMA thread per tile 1077; persistent CTAs whose
+// queries are prepared by two more warps 964.
+constexpr int kAttnThreads = 576;
+constexpr int kSoftmaxWarps = 16;
+constexpr int kAttnStages = 3;
+constexpr uint32_t kAttnTmemCols = 512;
+// Q tile in core-matrix order with 16 bytes between the core matrices: the 8 head-dim chunks of a row then fall into
+// different banks when a warp writes a row.
+constexpr int kQCore = 128 + 16, kQGroup = 8 * kQCore;
+
+struct __align__(128) AttnSmem {
+    uint8_t q[2][(kPfRows / 8) * kQGroup];              // (the epilogue passes O through it: 128 rows of 144 bytes)
+    uint8_t k[kAttnStages][kPfKeys * kHeadDim];
+    uint16_t v[kAttnStages][kPfKeys * kHeadDim];
+    float k_scale[kAttnStages][kPfKeys];
+    float rot[32 * 16];
+    float q_scale[2][kPfRows];
+    float xch[2][2][kPfRows];                           // [tile][half]: exchange between the two threads of a row
+    uint64_t q_ready;                                   // both Q tiles are in shared memory
+    uint64_t s_ready[2], p_ready[2];                    // per tile: S complete (and the PV before it), P written
+    uint64_t full[kAttnStages], empty[kAttnStages];     // per stage: record landed, record used up
+    uint64_t drained;                                   // after a failed wait: every MMA issued has completed
+    uint32_t tmem_base;
+};
+
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar_addr, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_addr), "r"(bytes) : "memory");
+}
+// Contiguous global -> shared copy of `bytes` (multiple of 16, both addresses 16-byte aligned),
+// completing on the mbarrier.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar_addr) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar_addr) : "memory");
+}
+// Barrier of the 256 softmax threads of a tile, and of all softmax threads.
+__device__ __forceinline__ void tile_sync(int x) { asm volatile("bar.sync %0, 256;" ::"r"(10 + x) : "memory"); }
+__device__ __forceinline__ void softmax_sync() { asm volatile("bar.sync 9, 512;" ::: "memory"); }
+
+// Which (sequence, tile or pair of tiles) the `index`-th unit of work is; sequences in order, their units from the
+// last (longest) to the first.  Every warp finds it by itself.  False when there are fewer units.
+__device__ __forceinline__ bool find_unit(const PrefillParams& p, int index, int& seq, int& unit) {
+    const int per = p.tokens_per_tile * p.tiles_per_unit, lane = threadIdx.x & 31;
+    if (p.cu_seqlens_q == nullptr) {
+        seq = 0;
+        const int n = (p.num_tokens + per - 1) / per;
+        unit = n - 1 - index;
+        return index < n;
+    }
+    int before = 0;
+    for (int s0 = 0; s0 < p.num_seqs; s0 += 128) {
+        int cu[4], next[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int s = s0 + 32 * i + lane;
+            cu[i] = next[i] = 0;
+            if (s < p.num_seqs) { cu[i] = __ldg(p.cu_seqlens_q + s); next[i] = __ldg(p.cu_seqlens_q + s + 1); }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (s0 + 32 * i >= p.num_seqs) break;
+            int incl = (max(next[i] - cu[i], 0) + per - 1) / per;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const unsigned hit = __ballot_sync(0xffffffffu, before + incl > index);
+            if (hit) {
+                const int l = __ffs(hit) - 1;
+                seq = s0 + 32 * i + l;
+                unit = __shfl_sync(0xffffffffu, before + incl, l) - 1 - index;
+                return true;
+            }
+            before += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    return false;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(kPfThreads, 2)
+__global__ void __launch_bounds__(kAttnThreads, 1)
 prefill_attn_kernel(const PrefillParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     AttnSmem& sm = *reinterpret_cast<AttnSmem*>(smem_raw);
 
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int row = tid & (kPfRows - 1), half = tid >> 7, quarter = warp & 3;
-    const int kvh = blockIdx.y, seq = blockIdx.z;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int kvh = blockIdx.x % p.H;
+    int seq, unit;
+    if (!find_unit(p, blockIdx.x / p.H, seq, unit)) return;
     const int q_begin = p.cu_seqlens_q ? __ldg(p.cu_seqlens_q + seq) : 0;
     const int q_end = p.cu_seqlens_q ? __ldg(p.cu_seqlens_q + seq + 1) : p.num_tokens;
-    const int q_len = max(q_end - q_begin, 0);
+    const int q_len = q_end - q_begin;
     const int kv_len = max(__ldg(p.seq_lens + seq), 0);
-    const int tiles_m = (q_len + p.tokens_per_tile - 1) / p.tokens_per_tile;
-    // heavy (late) query tiles first
-    const int m_tile = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);
-    if (m_tile >= tiles_m || kv_len == 0) {
-        // rows of an empty sequence still get a defined (zero) output
-        if (m_tile < tiles_m && half == 0) {
-            const int tl = row / p.G, h = row % p.G;
-            const int tok = m_tile * p.tokens_per_tile + tl;
-            if (tl < p.tokens_per_tile && tok < q_len) {
-                T* dst = static_cast<T*>(p.out) + (q_begin + tok) * p.o_stride_tok +
-                         static_cast<int64_t>(kvh * p.G + h) * p.o_stride_head;
-                for (int d = 0; d < kHeadDim; d += 8) *reinterpret_cast<uint4*>(dst + d) = make_uint4(0, 0, 0, 0);
-            }
-        }
-        return;
-    }
+    // K/V tiles that each of the two tiles needs: up to its last row's position, never past the staged records
+    auto tiles_of = [&](int x) {
+        const int first = (unit * p.tiles_per_unit + x) * p.tokens_per_tile;
+        const int last = min(q_len, first + p.tokens_per_tile) - 1;
+        const int last_pos = min(kv_len - q_len + last, kv_len - 1);
+        const bool any = x < p.tiles_per_unit && first < q_len && last_pos >= 0;
+        return any ? min(last_pos / kPfKeys + 1, p.stage_tiles_per_seq) : 0;
+    };
+    const int n0 = tiles_of(0), n1 = tiles_of(1), n_all = max(n0, n1);
 
-    // this thread's query row: token and head; absolute position of the token in its sequence
-    const int tok_local = row / p.G, head_local = row % p.G;
-    const int tok = m_tile * p.tokens_per_tile + tok_local;
-    const bool row_valid = tok_local < p.tokens_per_tile && tok < q_len;
-    const int pos = row_valid ? kv_len - q_len + tok : -1;
-    const int last_tok = min(q_len, (m_tile + 1) * p.tokens_per_tile) - 1;
-    const int max_pos = kv_len - q_len + last_tok;                  // >= 0 for the CTA
-    // never past the staged records (max_seq_len of the call bounds every sequence)
-    const int n_tiles = min(min(max_pos, kv_len - 1) / kPfKeys + 1, p.stage_tiles_per_seq);
-
-    // ---- set-up: barriers, TMEM, parameters ----
+    // ---- set-up: barriers, TMEM, rotation blocks ----
     if (tid == 0) {
-        mbar_init(&sm.bar_s, 1);
-        mbar_init(&sm.bar_o, 1);
-        mbar_init(&sm.bar_k, 1);
-        mbar_init(&sm.bar_v, 1);
+        mbar_init(&sm.q_ready, kSoftmaxWarps);
+        mbar_init(&sm.drained, 1);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            mbar_init(&sm.s_ready[x], 1);
+            mbar_init(&sm.p_ready[x], kSoftmaxWarps / 2);
+        }
+#pragma unroll
+        for (int s = 0; s < kAttnStages; ++s) {
+            mbar_init(&sm.full[s], 1);
+            mbar_init(&sm.empty[s], 1);
+        }
         fence_async_proxy();
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tmem_alloc(&sm.tmem_base, kTmemCols);
-    for (int i = tid; i < 32 * 16; i += kPfThreads) {
+    if (warp == kSoftmaxWarps) tmem_alloc(&sm.tmem_base, kAttnTmemCols);
+    for (int i = tid; i < 32 * 16; i += kAttnThreads) {
         const int g = i >> 4, j = (i >> 2) & 3, k = i & 3;
         sm.rot[i] = __ldg(p.rotation + (4 * g + j) * kHeadDim + 4 * g + k);      // R[4g+j][4g+k]
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = sm.tmem_base;
-    const uint32_t lane_base = tmem + (static_cast<uint32_t>(quarter * 32) << 16);   // this warp's TMEM lanes
-    const uint32_t core_row_off = (row >> 3) * 1024 + (row & 7) * 16;                // q/k tiles: 8 chunks per row group
+    bool failed = false;
 
-    // ---- Q: rotate, round, quantise the row to int8; each of the row's two threads handles half
-    //      of the head-dims (16 rotation blocks, 4 chunks) and they exchange their maxima ----
-    float q_scale = 0.0f;
-    {
-        uint32_t packed[32];                    // this half of the rotated, rounded row as T pairs (d, d+1)
-        float mx = 0.0f;
-        if (row_valid) {
-            const T* src = static_cast<const T*>(p.q) + (q_begin + tok) * p.q_stride_tok +
-                           static_cast<int64_t>(kvh * p.G + head_local) * p.q_stride_head + 64 * half;
-#pragma unroll
-            for (int b = 0; b < 16; ++b) {
-                const uint2 raw = __ldg(reinterpret_cast<const uint2*>(src + 4 * b));
-                const float2 x01 = pf_unpack<T>(raw.x), x23 = pf_unpack<T>(raw.y);
-                float r[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float4 rr = *reinterpret_cast<const float4*>(&sm.rot[(16 * half + b) * 16 + j * 4]);
-                    float acc = __fmul_rn(x01.x, rr.x);
-                    acc = __fmaf_rn(x01.y, rr.y, acc);
-                    acc = __fmaf_rn(x23.x, rr.z, acc);
-                    acc = __fmaf_rn(x23.y, rr.w, acc);
-                    r[j] = acc;
-                }
-                packed[2 * b] = pf_pack<T>(r[0], r[1]);
-                packed[2 * b + 1] = pf_pack<T>(r[2], r[3]);
-                const float2 a = pf_unpack<T>(packed[2 * b]), c = pf_unpack<T>(packed[2 * b + 1]);
-                mx = fmaxf(mx, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(c.x), fabsf(c.y))));
+    if (warp == kSoftmaxWarps + 1) {
+        // ---- loads: record of 128 keys = [K codes 16 KB | V values 32 KB | key scales 512 B] ----
+        if (lane == 0) {
+            grid_dependency_wait();                           // the records
+            const uint8_t* rec = p.stage + (static_cast<int64_t>(seq) * p.stage_tiles_per_seq * p.H + kvh) * kStageRecord;
+            const int64_t record_stride = static_cast<int64_t>(p.H) * kStageRecord;
+            int issued = 0;
+            for (; issued < n_all; ++issued, rec += record_stride) {
+                const int s = issued % kAttnStages;
+                if (issued >= kAttnStages) failed = !mbar_wait(&sm.empty[s], static_cast<uint32_t>(issued / kAttnStages - 1) & 1u);
+                if (failed) break;
+                const uint32_t bar = smem_u32(&sm.full[s]);
+                mbar_expect_tx(bar, kStageRecord);
+                bulk_load(smem_u32(sm.k[s]), rec, kPfKeys * kHeadDim, bar);
+                bulk_load(smem_u32(sm.v[s]), rec + kPfKeys * kHeadDim, 2 * kPfKeys * kHeadDim, bar);
+                bulk_load(smem_u32(sm.k_scale[s]), rec + 3 * kPfKeys * kHeadDim, kPfKeys * 4, bar);
             }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) packed[i] = 0u;
+            if (failed)                                       // copies in flight land before the CTA ends
+                for (int j = max(0, issued - kAttnStages); j < issued; ++j)
+                    mbar_wait(&sm.full[j % kAttnStages], static_cast<uint32_t>(j / kAttnStages) & 1u);
         }
-        sm.xch[half][row] = mx;
-        pair_sync(quarter);
-        mx = fmaxf(mx, sm.xch[half ^ 1][row]);
-        pair_sync(quarter);                     // xch is reused by the softmax
-        const bool ok = mx > 0.0f && mx <= 3.0e38f;
-        const float inv = ok ? __fdiv_rn(127.0f, mx) : 0.0f;
-        q_scale = ok ? __fdiv_rn(mx, 127.0f) : 0.0f;
+        __syncwarp();
+    } else if (warp == kSoftmaxWarps) {
+        // ---- MMAs ----
+        // Unrolled over the stages, so that every operand of an MMA is a constant plus the shared-memory base (and the
+        // TMEM base, 0 as all columns are allocated): an MMA blocks its issuing thread while the tensor core works on the
+        // one before, so whatever the thread computes between two of them is added to the tensor core's time.
+        if (lane == 0 && n_all > 0) {
+            constexpr uint32_t idesc_s = (2u << 4) | (1u << 7) | (1u << 10) | ((kPfKeys >> 3) << 17) | ((kPfRows >> 4) << 24);
+            constexpr uint32_t idesc_o = (1u << 4) | (TcFormat<T>::kFmt << 7) | (TcFormat<T>::kFmt << 10) | (1u << 16) |
+                                         ((kHeadDim >> 3) << 17) | ((kPfRows >> 4) << 24);
+            auto scores = [&](int x, int stage) {
+                const uint32_t q_addr = smem_u32(sm.q[x]), k_addr = smem_u32(sm.k[stage]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {           // 16 head-dims = 16 bytes per chunk; chunks 4*half .. 4*half + 3
-            uint32_t wds[4];
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                const float2 a = pf_unpack<T>(packed[8 * c + 2 * w]), b = pf_unpack<T>(packed[8 * c + 2 * w + 1]);
-                const int i0 = __float2int_rn(a.x * inv), i1 = __float2int_rn(a.y * inv);
-                const int i2 = __float2int_rn(b.x * inv), i3 = __float2int_rn(b.y * inv);
-                // position x holds head-dim x ^ 1
-                wds[w] = (i1 & 0xFF) | ((i0 & 0xFF) << 8) | ((i3 & 0xFF) << 16) | ((i2 & 0xFF) << 24);
+                for (int s = 0; s < 4; ++s)
+                    tc_mma_i8(128u * x, smem_desc(q_addr + 2 * kQCore * s, kQCore, kQGroup), smem_desc(k_addr + 256 * s, 128, 1024),
+                              idesc_s, s > 0 ? 1u : 0u);
+            };
+            failed |= !mbar_wait(&sm.q_ready, 0);
+            failed |= !mbar_wait(&sm.full[0], 0);
+            if (!failed) {
+                tc_fence_after();
+                if (n0 > 0) { scores(0, 0); tc_commit(&sm.s_ready[0]); }
+                if (n1 > 0) { scores(1, 0); tc_commit(&sm.s_ready[1]); }
             }
-            *reinterpret_cast<uint4*>(&sm.q[core_row_off + (4 * half + c) * 128]) = make_uint4(wds[0], wds[1], wds[2], wds[3]);
-        }
-    }
-    const float row_factor = q_scale * p.qk_scale;
-    fence_async_proxy();                 // the Q tile is read by the tensor core
-    __syncthreads();
-
-    // descriptors and instruction words
-    const uint32_t idesc_s = (2u << 4) | (1u << 7) | (1u << 10) | ((kPfKeys >> 3) << 17) | ((kPfRows >> 4) << 24);
-    const uint32_t idesc_o = (1u << 4) | (PfType<T>::kFmt << 7) | (PfType<T>::kFmt << 10) | (1u << 16) |
-                             ((kHeadDim >> 3) << 17) | ((kPfRows >> 4) << 24);
-    const uint32_t q_addr = smem_u32(sm.q), k_addr = smem_u32(sm.k), v_addr = smem_u32(sm.v), p_addr = smem_u32(sm.p);
-
-    // scratch records of this (sequence, KV head): [K codes 16 KB | V values 32 KB | key scales 512 B] per tile
-    const uint8_t* const records = p.stage + (static_cast<int64_t>(seq) * p.stage_tiles_per_seq * p.H + kvh) * kStageRecord;
-    const int64_t record_stride = static_cast<int64_t>(p.H) * kStageRecord;
-    auto issue_k = [&](int tile) {                  // thread 0 only
-        const uint8_t* rec = records + tile * record_stride;
-        const uint32_t bar = smem_u32(&sm.bar_k);
-        mbar_expect_tx(bar, kPfKeys * kHeadDim + kPfKeys * 4);
-        bulk_load(smem_u32(sm.k), rec, kPfKeys * kHeadDim, bar);
-        bulk_load(smem_u32(sm.k_scale[tile & 1]), rec + 3 * kPfKeys * kHeadDim, kPfKeys * 4, bar);
-    };
-    auto issue_v = [&](int tile) {                  // thread 0 only
-        const uint8_t* rec = records + tile * record_stride;
-        const uint32_t bar = smem_u32(&sm.bar_v);
-        mbar_expect_tx(bar, 2 * kPfKeys * kHeadDim);
-        bulk_load(smem_u32(sm.v), rec + kPfKeys * kHeadDim, 2 * kPfKeys * kHeadDim, bar);
-    };
-    grid_dependency_wait();              // the records
-    if (tid == 0) {
-        issue_k(0);
-        issue_v(0);
-    }
-
-    float m_run = -INFINITY, l_run = 0.0f;      // l_run: sum over this thread's half of the keys
-    uint32_t ph_s = 0, ph_o = 0, ph_k = 0, ph_v = 0;
-    bool pv_pending = false, failed = false;
-
-#pragma unroll 1
-    for (int j = 0; j < n_tiles; ++j) {
-        // ---- 1, 2. K codes and key scales of this tile have landed: S = Q K^T ----
-        failed |= !mbar_wait(&sm.bar_k, ph_k);
-        ph_k ^= 1u;
-        if (tid == 0) {
-            tc_fence_after();
+            // tile j: PV_x(j), then S_x(j + 1); the commit is there without an S, too
+            auto step = [&](auto unrolled, int j, uint32_t phase) {
+                constexpr int stage = decltype(unrolled)::value, next = (stage + 1) % kAttnStages;
+                if (j + 1 < n_all && !failed) failed |= !mbar_wait(&sm.full[next], next == 0 ? phase ^ 1u : phase);
+                const uint32_t v_addr = smem_u32(sm.v[stage]);
 #pragma unroll
-            for (int s = 0; s < 4; ++s)
-                tc_mma_i8(tmem, smem_desc(q_addr + 256 * s, 128, 1024), smem_desc(k_addr + 256 * s, 128, 1024),
-                          idesc_s, s > 0 ? 1u : 0u);
-            tc_commit(&sm.bar_s);
-        }
-        failed |= !mbar_wait(&sm.bar_s, ph_s);
-        ph_s ^= 1u;
-        tc_fence_after();
-        // the previous tile's P V has normally finished by now: its V tile and the P tile are free
-        if (pv_pending) {
-            failed |= !mbar_wait(&sm.bar_o, ph_o);
-            ph_o ^= 1u;
-            tc_fence_after();
-            pv_pending = false;
-        }
-        if (tid == 0) {
-            if (j + 1 < n_tiles) issue_k(j + 1);
-            if (j > 0) issue_v(j);
-        }
-        const float* const k_scale = sm.k_scale[j & 1];
-
-        // ---- 3. online softmax: this thread's row, keys 64*half .. 64*half + 63 of the tile ----
-        // keys of this half that the row may see: columns 0 .. limit (>= 63: all of them)
-        const int limit = pos - (j * kPfKeys + 64 * half);
-        const bool unmasked = __all_sync(0xffffffffu, limit >= 63);
-        uint8_t* prow = reinterpret_cast<uint8_t*>(sm.p) + (row >> 3) * (16 * 128) + (row & 7) * 16;
-        auto softmax_half = [&](auto masked_tag) {
-            constexpr bool kMasked = decltype(masked_tag)::value;
-            // pass A: scale the integer sums by the key scales, row maximum.  The first 32 scaled sums
-            // stay in registers, the other 32 go back to TMEM as floats until pass B.
-            float m_half = -INFINITY;
-            uint32_t r0[32];
-            auto scale_chunk = [&](uint32_t (&r)[32], int ch) {
+                for (int x = 0; x < 2; ++x) {
+                    const int nx = x == 0 ? n0 : n1;
+                    if (j >= nx || failed) continue;
+                    failed |= !mbar_wait(&sm.p_ready[x], static_cast<uint32_t>(j) & 1u);
+                    if (failed) continue;
+                    tc_fence_after();
 #pragma unroll
-                for (int c4 = 0; c4 < 8; ++c4) {
-                    const float4 ks = *reinterpret_cast<const float4*>(&k_scale[64 * half + 32 * ch + 4 * c4]);
-                    const float kk[4] = {ks.x, ks.y, ks.z, ks.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int c = 4 * c4 + e;
-                        const float sv = small_int_to_float(r[c]) * kk[e];
-                        r[c] = __float_as_uint(sv);
-                        if (!kMasked || 32 * ch + c <= limit) m_half = fmaxf(m_half, sv);
-                    }
+                    for (int c = 0; c < 8; ++c)
+                        tc_mma_f16_ta(256u + 128u * x, 128u * x + 64u * (c >> 2) + 8u * (c & 3), smem_desc(v_addr + 4096 * c, 2048, 128),
+                                      idesc_o, c > 0 ? 1u : static_cast<uint32_t>(j > 0));
+                    if (j + 1 < nx) scores(x, next);
+                    tc_commit(&sm.s_ready[x]);
                 }
             };
-            {
-                uint32_t r1[32];
-                tmem_ld32(lane_base + 64 * half + 32, r1);
-                scale_chunk(r1, 1);
-                tmem_st32(lane_base + 64 * half + 32, r1);
+            uint32_t phase = 0;
+            for (int j = 0; j < n_all && !failed; j += kAttnStages, phase ^= 1u) {
+                step(std::integral_constant<int, 0>{}, j, phase);
+                step(std::integral_constant<int, 1>{}, j + 1, phase);
+                step(std::integral_constant<int, 2>{}, j + 2, phase);
             }
-            tmem_ld32(lane_base + 64 * half, r0);
-            scale_chunk(r0, 0);
-            sm.xch[half][row] = m_half;
-            pair_sync(quarter);
-            const float m_tile = fmaxf(m_half, sm.xch[half ^ 1][row]) * row_factor;     // row_factor >= 0
-            // lazy reference: it moves only when the tile maximum exceeds it by more than 2^8
-            const bool grew = m_tile > m_run + 8.0f;
-            const float m_new = grew ? m_tile : m_run;
-            const float m_use = (m_new == -INFINITY) ? 0.0f : m_new;
-            const float alpha = grew ? ((m_run == -INFINITY) ? 0.0f : pf_ex2(m_run - m_use)) : 1.0f;
-            if (j > 0 && __any_sync(0xffffffffu, grew)) {                // this thread's half of the O columns
+            if (failed) {                                     // what was issued ends before TMEM is freed
+                tc_commit(&sm.drained);
+                mbar_wait(&sm.drained, 0);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---- softmax: tile x, row = thread of its warp group, half of the tile's keys ----
+        const int x = warp >> 3, half = (warp >> 2) & 1, row = tid & (kPfRows - 1);
+        const int pair_id = 1 + 4 * x + (warp & 3);           // named barrier of the two warps with the same rows
+        const int n = x == 0 ? n0 : n1;
+        const uint32_t lanes = (static_cast<uint32_t>((warp & 3) * 32) << 16) + 128u * x;
+        const uint32_t s_cols = lanes + 64u * half, o_cols = lanes + 256u + 64u * half;
+        float* const xch = sm.xch[x][half] + row;
+        const float* const xch_other = sm.xch[x][half ^ 1] + row;
+        const int first_tok = (unit * p.tiles_per_unit + x) * p.tokens_per_tile;
+        // Q and the output are handled by whole rows: a warp has rows row0 .. row0 + rows - 1 of tile xr, lane i < 16 knows
+        // where row row0 + i is (-1: no such row).  Queries of a single tile are shared by all the warps.
+        auto row_offset = [&](int xr, int r, int64_t tok_stride, int64_t head_stride) -> long long {
+            const int tl = r / p.G, tk = (unit * p.tiles_per_unit + xr) * p.tokens_per_tile + tl;
+            if (xr >= p.tiles_per_unit || tl >= p.tokens_per_tile || tk >= q_len) return -1;
+            return (q_begin + tk) * tok_stride + static_cast<int64_t>(kvh * p.G + r % p.G) * head_stride;
+        };
+
+        // Q: rotate, round, quantise the rows to int8.  Lane L has head-dims 4L .. 4L + 3 (one rotation block, in
+        // registers), so that loads are contiguous.  Bound by latency, so eight rows are in flight while eight are converted.
+        {
+            constexpr int kRows = 8;
+            const int rows = kRows * p.tiles_per_unit, xq = (warp * rows) >> 7, row_q = (warp * rows) & (kPfRows - 1);
+            f2 rot[4][2];                                     // [in][outs 0, 1 | outs 2, 3]
+            {
+                float r[4][4];
+#pragma unroll
+                for (int jj = 0; jj < 4; ++jj) *reinterpret_cast<float4*>(r[jj]) = *reinterpret_cast<const float4*>(&sm.rot[lane * 16 + 4 * jj]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) { rot[k][0] = pk(r[0][k], r[1][k]); rot[k][1] = pk(r[2][k], r[3][k]); }
+            }
+            const long long at_row = row_offset(xq, row_q + (lane & 15), p.q_stride_tok, p.q_stride_head);
+            uint2 next[kRows];
+            auto fetch = [&](int i0) {
+#pragma unroll
+                for (int i = 0; i < kRows; ++i) {
+                    const long long at = __shfl_sync(0xffffffffu, at_row, i0 + i);
+                    next[i] = at >= 0 ? __ldg(reinterpret_cast<const uint2*>(static_cast<const T*>(p.q) + at + 4 * lane)) : make_uint2(0u, 0u);
+                }
+            };
+            // Adding 1.5 * 2^23 rounds to the nearest integer, in the low bits.  Scalar operations: the assembler contracts a
+            // packed product and sum, and a product that is a tie after its own rounding would go the other way.
+            auto code = [](float v, float scale) { return __float_as_uint(__fadd_rn(__fmul_rn(v, scale), 12582912.0f)); };
+            if ((xq == 0 ? n0 : n1) > 0) {
+                fetch(0);
+#pragma unroll 1
+                for (int i0 = 0; i0 < rows; i0 += kRows) {
+                    uint2 raw[kRows];
+#pragma unroll
+                    for (int i = 0; i < kRows; ++i) raw[i] = next[i];
+                    if (i0 + kRows < rows) fetch(i0 + kRows);
+                    float mx = 0.0f;                          // lane i < 8: largest |value| of row i0 + i
+#pragma unroll
+                    for (int i = 0; i < kRows; ++i) {
+                        const float2 a = pf_unpack<T>(raw[i].x), b = pf_unpack<T>(raw[i].y);
+                        const float in[4] = {a.x, a.y, b.x, b.y};
+                        f2 y01 = mul2(pk(in[0], in[0]), rot[0][0]), y23 = mul2(pk(in[0], in[0]), rot[0][1]);
+#pragma unroll
+                        for (int k = 1; k < 4; ++k) { y01 = fma2(pk(in[k], in[k]), rot[k][0], y01); y23 = fma2(pk(in[k], in[k]), rot[k][1], y23); }
+                        float y[4];
+                        upk(y01, y[0], y[1]);
+                        upk(y23, y[2], y[3]);
+                        raw[i] = make_uint2(pf_pack<T>(y[0], y[1]), pf_pack<T>(y[2], y[3]));
+                        const float2 c = pf_unpack<T>(raw[i].x), d = pf_unpack<T>(raw[i].y);
+                        const float m = fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y)));
+                        const uint32_t m_row = __reduce_max_sync(0xffffffffu, __float_as_uint(m));   // non-negative floats order as integers
+                        if (lane == i) mx = __uint_as_float(m_row);
+                    }
+                    const bool ok = mx > 0.0f && mx <= 3.0e38f;
+                    const float inv = ok ? __fdiv_rn(127.0f, mx) : 0.0f;
+                    if (lane < kRows) sm.q_scale[xq][row_q + i0 + lane] = ok ? __fdiv_rn(mx, 127.0f) : 0.0f;
+#pragma unroll
+                    for (int i = 0; i < kRows; ++i) {
+                        const float inv_row = __shfl_sync(0xffffffffu, inv, i);
+                        const float2 a = pf_unpack<T>(raw[i].x), b = pf_unpack<T>(raw[i].y);
+                        // position d holds head-dim d ^ 1
+                        const uint32_t w = prmt(prmt(code(a.y, inv_row), code(a.x, inv_row), 0x0040), prmt(code(b.y, inv_row), code(b.x, inv_row), 0x0040), 0x5410);
+                        const int r = row_q + i0 + i;
+                        *reinterpret_cast<uint32_t*>(&sm.q[xq][(r >> 3) * kQGroup + (lane >> 2) * kQCore + (r & 7) * 16 + 4 * (lane & 3)]) = w;
+                    }
+                }
+            }
+        }
+        fence_async_proxy();                                  // the Q tile is read by the tensor core
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.q_ready);
+        softmax_sync();                                       // every row's scale is there
+        const float row_factor = n > 0 ? sm.q_scale[x][row] * p.qk_scale : 0.0f;
+        int pos;                                              // of the row's token in its sequence
+        {
+            const int tl = row / p.G, tk = first_tok + tl;
+            pos = x < p.tiles_per_unit && tl < p.tokens_per_tile && tk < q_len ? kv_len - q_len + tk : -1;
+        }
+
+        const f2 factor2 = pk(row_factor, row_factor), unbias2 = pk(-12582912.0f, -12582912.0f);
+        float m_run = -INFINITY, l_run = 0.0f;                // l_run: this half of the keys
+        for (int j = 0; j < n; ++j) {
+            // After an expired wait the warp keeps its step (its partner meets it at the named barrier) without waiting.
+            const int stage = j % kAttnStages;
+            if (!failed) failed = !mbar_wait(&sm.s_ready[x], static_cast<uint32_t>(j) & 1u);
+            if (!failed) failed = !mbar_wait(&sm.full[stage], static_cast<uint32_t>(j / kAttnStages) & 1u);   // key scales
+            failed = __any_sync(0xffffffffu, failed);
+            tc_fence_after();
+            // S(j) is complete, so PV(j - 1) is: the later tile of the two frees the record that PV used up
+            if (j > 0 && tid == (n1 > 0 ? 256 : 0)) mbar_arrive(&sm.empty[(j - 1) % kAttnStages]);
+            const float* const k_scale = sm.k_scale[stage] + 64 * half;
+            const int limit = pos - (j * kPfKeys + 64 * half);    // the row sees keys 0 .. limit of this half tile
+            const bool unmasked = __all_sync(0xffffffffu, limit >= 63);
+
+            // scaled sums of four keys, in pairs: (float)S * key scale
+            auto scaled = [&](const uint32_t* r, int key, f2& a, f2& b) {
+                const float4 ks = *reinterpret_cast<const float4*>(&k_scale[key]);
+                // int -> float: |S| < 2^22, so adding it to the bits of 1.5 * 2^23 gives 1.5 * 2^23 + S exactly
+                const f2 r01 = pk(__uint_as_float(r[0] + 0x4B400000u), __uint_as_float(r[1] + 0x4B400000u));
+                const f2 r23 = pk(__uint_as_float(r[2] + 0x4B400000u), __uint_as_float(r[3] + 0x4B400000u));
+                a = mul2(add2(r01, unbias2), pk(ks.x, ks.y));
+                b = mul2(add2(r23, unbias2), pk(ks.z, ks.w));
+            };
+            // the row's maximum over the tile becomes the reference if it exceeds it by 2^8 or more
+            auto move_reference = [&]() {
+                float m_half = -INFINITY;
+#pragma unroll 1
+                for (int ch = 0; ch < 4; ++ch) {
+                    uint32_t r[16];
+                    tmem_ld16_nowait(s_cols + 16 * ch, r);
+                    tmem_wait_ld();
+                    tmem_ld16_landed(r);
+#pragma unroll
+                    for (int c4 = 0; c4 < 4; ++c4) {
+                        f2 a, b;
+                        scaled(&r[4 * c4], 16 * ch + 4 * c4, a, b);
+                        float v[4];
+                        upk(a, v[0], v[1]);
+                        upk(b, v[2], v[3]);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (16 * ch + 4 * c4 + e <= limit) m_half = fmaxf(m_half, v[e]);
+                    }
+                }
+                *xch = m_half;
+                pair_any(pair_id, false);
+                const float m_tile = fmaxf(m_half, *xch_other) * row_factor;                // row_factor >= 0
+                const bool grew = m_tile > m_run + 8.0f;
+                const float m_new = grew ? m_tile : m_run;
+                const float alpha = grew ? (m_run == -INFINITY ? 0.0f : pf_ex2(m_run - m_new)) : 1.0f;
+                if (j > 0 && __any_sync(0xffffffffu, grew)) { // O_x is at rest: the commit behind S_x(j) covered PV_x(j - 1)
+#pragma unroll 1
+                    for (int ch = 0; ch < 4; ++ch) {
+                        uint32_t r[16];
+                        tmem_ld16_nowait(o_cols + 16 * ch, r);
+                        tmem_wait_ld();
+                        tmem_ld16_landed(r);
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * alpha);
+                        tmem_st16_nowait(o_cols + 16 * ch, r);
+                    }
+                    tmem_wait_st();
+                }
+                l_run *= alpha;
+                m_run = m_new;
+                pair_any(pair_id, false);                     // xch has been read
+            };
+            uint32_t prob[32];                                // probabilities of the half row as T pairs
+            float half_sum;
+            auto exponentiate = [&](auto masked_tag) {
+                constexpr bool kMasked = decltype(masked_tag)::value;
+                const float m_use = (m_run == -INFINITY) ? 0.0f : m_run;
+                const f2 minus_m = pk(-m_use, -m_use);
+                f2 sum_a = pk(0.0f, 0.0f), sum_b = sum_a;
+                uint32_t buf[2][8];
+                tmem_ld8_nowait(s_cols, buf[0]);
+#pragma unroll
+                for (int it = 0; it < 8; ++it) {
+                    tmem_wait_ld();
+                    tmem_ld8_landed(buf[it & 1]);
+                    if (it < 7) tmem_ld8_nowait(s_cols + 8 * (it + 1), buf[(it + 1) & 1]);
+#pragma unroll
+                    for (int c4 = 0; c4 < 2; ++c4) {
+                        f2 a, b;
+                        scaled(&buf[it & 1][4 * c4], 8 * it + 4 * c4, a, b);
+                        float e[4];
+                        upk(fma2(a, factor2, minus_m), e[0], e[1]);
+                        upk(fma2(b, factor2, minus_m), e[2], e[3]);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            e[i] = pf_ex2(e[i]);
+                            if (kMasked && 8 * it + 4 * c4 + i > limit) e[i] = 0.0f;
+                        }
+                        sum_a = add2(sum_a, pk(e[0], e[1]));
+                        sum_b = add2(sum_b, pk(e[2], e[3]));
+                        prob[4 * it + 2 * c4] = pf_pack<T>(e[0], e[1]);
+                        prob[4 * it + 2 * c4 + 1] = pf_pack<T>(e[2], e[3]);
+                    }
+                }
+                float lo, hi;
+                upk(add2(sum_a, sum_b), lo, hi);
+                half_sum = lo + hi;
+            };
+            if (j == 0) move_reference();
+#pragma unroll 1
+            for (int attempt = 0;; ++attempt) {
+                if (unmasked) exponentiate(std::false_type{});
+                else exponentiate(std::true_type{});
+                // both threads of every row take the same decision
+                const bool outgrown = !(half_sum <= 16384.0f) || (m_run == -INFINITY && half_sum > 0.0f);
+                if (!pair_any(pair_id, outgrown) || attempt == 1) break;
+                move_reference();
+            }
+            l_run += half_sum;
+            tmem_st32_nowait(s_cols, prob);                   // over the half row's own sums
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.p_ready[x]);
+        }
+
+        // ---- epilogue: O / l, round, rotate by R, round, store ----
+        // The rows go through shared memory (the Q tile's space, half of the head-dims at a time), so that a warp stores
+        // whole half rows: 16 lanes per row, one rotation block each.
+        if (n > 0) {
+            if (!failed) failed = !mbar_wait(&sm.s_ready[x], static_cast<uint32_t>(n) & 1u);     // the last PV
+            failed = __any_sync(0xffffffffu, failed);
+            tc_fence_after();
+            *xch = l_run;
+            pair_any(pair_id, false);
+            l_run += *xch_other;
+        }
+        const float inv_l = l_run > 0.0f ? 1.0f / l_run : 0.0f;
+        const int row0 = 16 * (warp & 7);
+        const long long mine = failed ? -1 : row_offset(x, row0 + (lane & 15), p.o_stride_tok, p.o_stride_head);
+        uint8_t* const tile_rows = sm.q[x];
+#pragma unroll 1
+        for (int h = 0; h < 2 && x < p.tiles_per_unit; ++h) {
+            if (half == h) {
 #pragma unroll 1
                 for (int ch = 0; ch < 2; ++ch) {
                     uint32_t r[32];
-                    tmem_ld32(lane_base + kPfKeys + 64 * half + 32 * ch, r);
+                    if (n > 0) {
+                        tmem_ld32(o_cols + 32 * ch, r);
+                    } else {                                  // rows that see no key are zero
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * alpha);
-                    tmem_st32(lane_base + kPfKeys + 64 * half + 32 * ch, r);
-                }
-            }
-            l_run *= alpha;
-            m_run = m_new;
-            // pass B: probabilities -> shared P tile (K-major: 16 chunks of 8 keys per row)
-            auto emit_chunk = [&](const uint32_t (&r)[32], int ch) {
-                uint32_t pk[16];
-#pragma unroll
-                for (int c = 0; c < 32; c += 2) {
-                    float p0 = pf_ex2(fmaf(__uint_as_float(r[c]), row_factor, -m_use));
-                    float p1 = pf_ex2(fmaf(__uint_as_float(r[c + 1]), row_factor, -m_use));
-                    if (kMasked) {
-                        if (32 * ch + c > limit) p0 = 0.0f;
-                        if (32 * ch + c + 1 > limit) p1 = 0.0f;
+                        for (int i = 0; i < 32; ++i) r[i] = 0u;
                     }
-                    l_run += p0 + p1;
-                    pk[c >> 1] = pf_pack<T>(p0, p1);
-                }
 #pragma unroll
-                for (int kc = 0; kc < 4; ++kc)
-                    *reinterpret_cast<uint4*>(prow + (8 * half + 4 * ch + kc) * 128) =
-                        make_uint4(pk[4 * kc], pk[4 * kc + 1], pk[4 * kc + 2], pk[4 * kc + 3]);
-            };
-            emit_chunk(r0, 0);
-            {
-                uint32_t r1[32];
-                tmem_ld32(lane_base + 64 * half + 32, r1);
-                emit_chunk(r1, 1);
-            }
-        };
-        // After the first tile the reference maximum rarely has to move, so the tile is first done in ONE
-        // pass against the current reference (scaled sums and probabilities together, nothing parked in TMEM,
-        // the raw sums left untouched); only when some row of the warp has outgrown its reference is the
-        // tile redone by the two-pass code above, which also finds the new maximum.
-        auto softmax_one_pass = [&](auto masked_tag) -> bool {
-            constexpr bool kMasked = decltype(masked_tag)::value;
-            const float m_use = (m_run == -INFINITY) ? 0.0f : m_run;
-            float l_try = l_run;
-#pragma unroll 1
-            for (int ch = 0; ch < 2; ++ch) {
-                uint32_t r[32], pk[16];
-                tmem_ld32(lane_base + 64 * half + 32 * ch, r);
+                    for (int c = 0; c < 4; ++c) {             // column d of O holds head-dim d ^ 1
+                        uint32_t w[4];
 #pragma unroll
-                for (int c4 = 0; c4 < 8; ++c4) {
-                    const float4 ks = *reinterpret_cast<const float4*>(&k_scale[64 * half + 32 * ch + 4 * c4]);
-                    const float kk[4] = {ks.x, ks.y, ks.z, ks.w};
-                    float pr[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int c = 4 * c4 + e;
-                        const float sv = small_int_to_float(r[c]) * kk[e];
-                        pr[e] = pf_ex2(fmaf(sv, row_factor, -m_use));
-                        if (kMasked && 32 * ch + c > limit) pr[e] = 0.0f;
+                        for (int i = 0; i < 4; ++i)
+                            w[i] = pf_pack<T>(__uint_as_float(r[8 * c + 2 * i + 1]) * inv_l, __uint_as_float(r[8 * c + 2 * i]) * inv_l);
+                        *reinterpret_cast<uint4*>(tile_rows + row * kQCore + 64 * ch + 16 * c) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
-                    l_try += pr[0] + pr[1];
-                    l_try += pr[2] + pr[3];
-                    pk[2 * c4] = pf_pack<T>(pr[0], pr[1]);
-                    pk[2 * c4 + 1] = pf_pack<T>(pr[2], pr[3]);
                 }
-#pragma unroll
-                for (int kc = 0; kc < 4; ++kc)
-                    *reinterpret_cast<uint4*>(prow + (8 * half + 4 * ch + kc) * 128) =
-                        make_uint4(pk[4 * kc], pk[4 * kc + 1], pk[4 * kc + 2], pk[4 * kc + 3]);
             }
-            // The maximum is not tracked here: a row whose probabilities of this tile add up to more than 2^15
-            // has outgrown its reference (every probability is below 2^15 otherwise, harmless for P in T
-            // precision and for the fp32 sums), and so has a row that met its first visible key (its
-            // reference is still -inf and some probability is exp2(score), unbounded): redo those tiles.
-            sm.xch[half][row] = l_try - l_run;
-            pair_sync(quarter);
-            const float tile_sum = (l_try - l_run) + sm.xch[half ^ 1][row];
-            // both warps that share these rows see the same sums, hence take the same decision
-            const bool outgrown = !(tile_sum <= 32768.0f) || (m_run == -INFINITY && tile_sum > 0.0f);
-            if (__any_sync(0xffffffffu, outgrown)) return false;
-            l_run = l_try;
-            return true;
-        };
-        bool done = false;
-        if (j > 0) done = unmasked ? softmax_one_pass(std::false_type{}) : softmax_one_pass(std::true_type{});
-        if (!done) {
-            if (unmasked) softmax_half(std::false_type{});
-            else softmax_half(std::true_type{});
-        }
-        failed |= !mbar_wait(&sm.bar_v, ph_v);                   // the V tile has landed
-        ph_v ^= 1u;
-        fence_async_proxy();
-        tc_fence_before();
-        if (__syncthreads_or(failed)) { failed = true; break; }      // uniform exit
-
-        // ---- 4. O += P V (completes under the next tile's S and row maxima) ----
-        if (tid == 0) {
-            tc_fence_after();
+            tile_sync(x);
+            const float* rb = &sm.rot[(16 * h + (lane & 15)) * 16];              // rb[k * 4 + jj] = R[4g+k][4g+jj]
+            float4 rr[4];
 #pragma unroll
-            for (int s = 0; s < 8; ++s)
-                tc_mma_f16(tmem + kPfKeys, smem_desc(p_addr + 256 * s, 128, 2048),
-                           smem_desc(v_addr + 4096 * s, 2048, 128), idesc_o, (j > 0 || s > 0) ? 1u : 0u);
-            tc_commit(&sm.bar_o);
-        }
-        pv_pending = true;
-    }
-    if (pv_pending) {
-        failed |= !mbar_wait(&sm.bar_o, ph_o);
-        tc_fence_after();
-    }
-    failed = __syncthreads_or(failed);
-
-    // ---- epilogue: O / l, round, rotate by R, round, store; this thread's half of the head-dims ----
-    if (!failed) {
-        sm.xch[half][row] = l_run;
-        pair_sync(quarter);
-        const float l_all = l_run + sm.xch[half ^ 1][row];
-        const float inv_l = l_all > 0.0f ? 1.0f / l_all : 0.0f;
-        T* dst = row_valid ? static_cast<T*>(p.out) + (q_begin + tok) * p.o_stride_tok +
-                                 static_cast<int64_t>(kvh * p.G + head_local) * p.o_stride_head
-                           : nullptr;
-#pragma unroll 1
-        for (int c2 = 0; c2 < 2; ++c2) {
-            const int ch = 2 * half + c2;
-            uint32_t r[32];
-            tmem_ld32(lane_base + kPfKeys + 32 * ch, r);
-            uint32_t outw[16];
+            for (int k = 0; k < 4; ++k) rr[k] = *reinterpret_cast<const float4*>(rb + 4 * k);
+#pragma unroll 2
+            for (int i = 0; i < 8; ++i) {
+                const int r = row0 + 2 * i + (lane >> 4);
+                const long long at = __shfl_sync(0xffffffffu, mine, 2 * i + (lane >> 4));
+                const uint2 o4 = *reinterpret_cast<const uint2*>(tile_rows + r * kQCore + 8 * (lane & 15));
+                const float2 o01 = pf_unpack<T>(o4.x), o23 = pf_unpack<T>(o4.y);
+                float y[4] = {__fmul_rn(o01.x, rr[0].x), __fmul_rn(o01.x, rr[0].y), __fmul_rn(o01.x, rr[0].z), __fmul_rn(o01.x, rr[0].w)};
+                const float o[3] = {o01.y, o23.x, o23.y};
 #pragma unroll
-            for (int b = 0; b < 8; ++b) {       // rotation block = head-dims 32ch + 4b .. + 3
-                float o[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e)    // column x of O holds head-dim x ^ 1
-                    o[e] = pf_round<T>(__uint_as_float(r[(4 * b + e) ^ 1]) * inv_l);
-                const float* rb = &sm.rot[(8 * ch + b) * 16];      // rb[k*4 + jj] = R[4g+k][4g+jj]
-                float y[4];
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    float acc = __fmul_rn(o[0], rb[jj]);
-                    acc = __fmaf_rn(o[1], rb[4 + jj], acc);
-                    acc = __fmaf_rn(o[2], rb[8 + jj], acc);
-                    acc = __fmaf_rn(o[3], rb[12 + jj], acc);
-                    y[jj] = acc;
+                for (int k = 0; k < 3; ++k) {
+                    y[0] = __fmaf_rn(o[k], rr[k + 1].x, y[0]); y[1] = __fmaf_rn(o[k], rr[k + 1].y, y[1]);
+                    y[2] = __fmaf_rn(o[k], rr[k + 1].z, y[2]); y[3] = __fmaf_rn(o[k], rr[k + 1].w, y[3]);
                 }
-                outw[2 * b] = pf_pack<T>(y[0], y[1]);
-                outw[2 * b + 1] = pf_pack<T>(y[2], y[3]);
+                if (at >= 0)
+                    *reinterpret_cast<uint2*>(static_cast<T*>(p.out) + at + 64 * h + 4 * (lane & 15)) = make_uint2(pf_pack<T>(y[0], y[1]), pf_pack<T>(y[2], y[3]));
             }
-            if (dst != nullptr) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    *reinterpret_cast<uint4*>(dst + 32 * ch + 8 * i) =
-                        make_uint4(outw[4 * i], outw[4 * i + 1], outw[4 * i + 2], outw[4 * i + 3]);
-            }
+            tile_sync(x);
         }
-    } else if (tid == 0 && p.error_flag != nullptr) {
-        atomicExch(p.error_flag, 1);
     }
+    if (failed && p.error_flag != nullptr) atomicExch(p.error_flag, 1);
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, kTmemCols);
+    if (warp == kSoftmaxWarps) tmem_dealloc(sm.tmem_base, kAttnTmemCols);
 }
 
 // ---- host side --------------------------------------------------------------------------------
 
 template <typename T, int KB, int VB>
-static int launch_prefill(const PrefillParams& p, int m_tiles, int num_seqs, cudaStream_t st) {
-    dim3 grid(m_tiles, p.H, num_seqs);
+static int launch_prefill(PrefillParams& p, int m_tiles, int num_seqs, cudaStream_t st) {
     if (p.stage != nullptr) {
         dim3 sgrid(p.stage_tiles_per_seq, p.H, num_seqs);
         if (int e = launch_dependent("rq_prefill_int8 stage launch", prefill_stage_kernel<T, KB, VB>, sgrid, dim3(128), 0, st, p)) return e;
         const size_t smem = sizeof(AttnSmem);
         if (int e = ensure_smem(prefill_attn_kernel<T>, smem)) return e;
-        return launch_dependent("rq_prefill_int8 attention launch", prefill_attn_kernel<T>, grid, dim3(kPfThreads), smem, st, p);
+        // Units of work: at most tokens / (tokens of a unit) + one partial unit per sequence, found by the CTAs
+        // themselves (a grid of longest sequence x sequences was mostly empty CTAs for batches of mixed lengths).  Two
+        // tiles per CTA share the K/V tiles and keep the tensor core busy under each other's softmax; with no more
+        // tiles than SMs a CTA per tile finishes earlier.
+        auto units = [&](long long per) {
+            const long long by_tokens = p.num_tokens / per + num_seqs;
+            const long long by_longest = num_seqs * ((1LL * m_tiles * p.tokens_per_tile + per - 1) / per);
+            return (by_tokens < by_longest ? by_tokens : by_longest) * p.H;
+        };
+        p.tiles_per_unit = units(p.tokens_per_tile) > kSms ? 2 : 1;
+        const dim3 grid(static_cast<unsigned>(units(1LL * p.tokens_per_tile * p.tiles_per_unit)));
+        return launch_dependent("rq_prefill_int8 attention launch", prefill_attn_kernel<T>, grid, dim3(kAttnThreads), smem, st, p);
     }
+    dim3 grid(m_tiles, p.H, num_seqs);
     const size_t smem = sizeof(PrefillSmem);
     if (int e = ensure_smem(prefill_int8_kernel<T, KB, VB>, smem)) return e;
     prefill_int8_kernel<T, KB, VB><<<grid, kPfThreads, smem, st>>>(p);
@@ -1111,7 +1241,7 @@ static int launch_prefill(const PrefillParams& p, int m_tiles, int num_seqs, cud
 }
 
 template <typename T>
-static int dispatch_prefill(const PrefillParams& p, int m_tiles, int num_seqs, int kb, int vb, cudaStream_t st) {
+static int dispatch_prefill(PrefillParams& p, int m_tiles, int num_seqs, int kb, int vb, cudaStream_t st) {
     if (kb == 3 && vb == 3) return launch_prefill<T, 3, 3>(p, m_tiles, num_seqs, st);
     if (kb == 4 && vb == 3) return launch_prefill<T, 4, 3>(p, m_tiles, num_seqs, st);
     if (kb == 3 && vb == 4) return launch_prefill<T, 3, 4>(p, m_tiles, num_seqs, st);
@@ -1179,7 +1309,7 @@ static int prefill_impl(const void* q, void* out, int dtype, int64_t q_stride_to
     p.q = q; p.out = out;
     p.q_stride_tok = q_stride_tok; p.q_stride_head = q_stride_head;
     p.o_stride_tok = o_stride_tok; p.o_stride_head = o_stride_head;
-    p.cu_seqlens_q = cu_seqlens_q; p.num_tokens = num_tokens;
+    p.cu_seqlens_q = cu_seqlens_q; p.num_tokens = num_tokens; p.num_seqs = num_seqs;
     p.H = num_kv_heads; p.Hq = num_q_heads; p.G = G;
     p.tokens_per_tile = kPfRows / G;
     p.cache = kv_cache; p.num_blocks = num_blocks; p.block_size = block_size;
