@@ -716,10 +716,12 @@ prefill_stage_kernel(const PrefillParams p) {
 // probabilities add up to more than 2^14 (the reference has been outgrown by more than 2^8), or when a row meets its
 // first visible key.  Packed fp32 operations on key pairs: 4.75 issue slots per score.
 //
-// Bound by the softmax (exponentials and the fp32 pipe: about 1.1 us per 256 x 128 scores against 0.3 us of MMAs), and for
-// short sequences by what a CTA does outside the loop, about 10 us of a 32 us life at 2048 tokens.  Against one tile per
-// CTA, two CTAs per SM, P through shared memory (us, whole call): 2048 tokens after 30000, 32 heads 1140 -> 942-1000;
-// 8 x 2048 tokens 519 -> 479; 2 prompts of up to 1500 and 30 single tokens after 4000, 28 heads 286 -> 225.
+// What bounds it: 256 x 128 scores take 1.8 us; their exponentials alone take 1.06 (16 a clock), their MMAs 0.8, and
+// with two tiles in TMEM the two overlap only in part.  For short sequences also what a CTA does outside the loop, about
+// 10 us of a 32 us life at 2048 tokens; and the last wave (2048 tokens of 8 KV heads are 256 CTAs on 148 SMs).  Against
+// one tile per CTA, two CTAs per SM, P through shared memory (us, whole call): 2048 tokens after 30000, 32 heads
+// 1140 -> 942-1000; 8 x 2048 tokens 519 -> 480; 2 prompts of up to 1500 and 30 single tokens after 4000, 28 heads
+// 286 -> 195.
 // Slower than this (the attention kernel of the first, 920 here): one thread per row 968; steps of 64 keys with two S
 // buffers 1192; S released early and P in shared memory 1210; an MMA thread per tile 1077; persistent CTAs whose
 // queries are prepared by two more warps 964.
@@ -759,8 +761,9 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 __device__ __forceinline__ void tile_sync(int x) { asm volatile("bar.sync %0, 256;" ::"r"(10 + x) : "memory"); }
 __device__ __forceinline__ void softmax_sync() { asm volatile("bar.sync 9, 512;" ::: "memory"); }
 
-// Which (sequence, tile or pair of tiles) the `index`-th unit of work is; sequences in order, their units from the
-// last (longest) to the first.  Every warp finds it by itself.  False when there are fewer units.
+// Which (sequence, tile or pair of tiles) the `index`-th unit of work is; sequences from the last to the first
+// (schedulers put running requests with one token before prompts), their units from the last (longest) to the first, so
+// that long units start early (217 -> 195 us for 30 single tokens and 2 prompts).  Every warp finds it by itself.  False when there are fewer units.
 __device__ __forceinline__ bool find_unit(const PrefillParams& p, int index, int& seq, int& unit) {
     const int per = p.tokens_per_tile * p.tiles_per_unit, lane = threadIdx.x & 31;
     if (p.cu_seqlens_q == nullptr) {
@@ -774,9 +777,9 @@ __device__ __forceinline__ bool find_unit(const PrefillParams& p, int index, int
         int cu[4], next[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int s = s0 + 32 * i + lane;
+            const int s = p.num_seqs - 1 - (s0 + 32 * i + lane);
             cu[i] = next[i] = 0;
-            if (s < p.num_seqs) { cu[i] = __ldg(p.cu_seqlens_q + s); next[i] = __ldg(p.cu_seqlens_q + s + 1); }
+            if (s >= 0) { cu[i] = __ldg(p.cu_seqlens_q + s); next[i] = __ldg(p.cu_seqlens_q + s + 1); }
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -790,7 +793,7 @@ __device__ __forceinline__ bool find_unit(const PrefillParams& p, int index, int
             const unsigned hit = __ballot_sync(0xffffffffu, before + incl > index);
             if (hit) {
                 const int l = __ffs(hit) - 1;
-                seq = s0 + 32 * i + l;
+                seq = p.num_seqs - 1 - (s0 + 32 * i + l);
                 unit = __shfl_sync(0xffffffffu, before + incl, l) - 1 - index;
                 return true;
             }
@@ -1016,10 +1019,13 @@ prefill_attn_kernel(const PrefillParams p) {
         if (lane == 0) mbar_arrive(&sm.q_ready);
         softmax_sync();                                       // every row's scale is there
         const float row_factor = n > 0 ? sm.q_scale[x][row] * p.qk_scale : 0.0f;
-        int pos;                                              // of the row's token in its sequence
+        // Position of the row's token in its sequence.  Rows without a token (zero queries, never stored) see every key: as
+        // rows that see none they would send their whole warp through the masked path at every tile (with 7 heads a tile
+        // has 126 rows, with a single query token 7: 225 -> 217 us for the batch of 28 heads).
+        int pos;
         {
             const int tl = row / p.G, tk = first_tok + tl;
-            pos = x < p.tiles_per_unit && tl < p.tokens_per_tile && tk < q_len ? kv_len - q_len + tk : -1;
+            pos = tl < p.tokens_per_tile && tk < q_len ? kv_len - q_len + tk : (1 << 30);
         }
 
         const f2 factor2 = pk(row_factor, row_factor), unbias2 = pk(-12582912.0f, -12582912.0f);
