@@ -62,7 +62,6 @@ struct PrefillParams {
     int* error_flag;                  // optional device int, set non-zero when a wait expired
     uint8_t* stage;                   // staged path: scratch records (see prefill_stage_kernel)
     int stage_tiles_per_seq;
-    int tiles_per_unit;               // staged path: MMA tiles per CTA, 1 or 2
 };
 
 template <typename T> using PfType = TcFormat<T>;
@@ -698,7 +697,7 @@ prefill_stage_kernel(const PrefillParams p) {
 
 // ---- staged path: attention --------------------------------------------------------------------
 //
-// One CTA = two MMA tiles of 128 rows (2 x (128 / G) query tokens x G heads of one (sequence, KV head)) that
+// One CTA = two MMA tiles (TILES = 2) of 128 rows (2 x (128 / G) query tokens x G heads of one (sequence, KV head)) that
 // share every K/V tile they read.  Eighteen warps with fixed roles:
 //   warps 0-7, 8-15 softmax of tile 0 and tile 1: two threads per row (= TMEM lane), 64 keys each; they also prepare
 //                   their rows of Q and write their rows of the output;
@@ -720,30 +719,33 @@ prefill_stage_kernel(const PrefillParams p) {
 // with two tiles in TMEM the two overlap only in part.  For short sequences also what a CTA does outside the loop, about
 // 10 us of a 32 us life at 2048 tokens; and the last wave (2048 tokens of 8 KV heads are 256 CTAs on 148 SMs).  Against
 // one tile per CTA, two CTAs per SM, P through shared memory (us, whole call): 2048 tokens after 30000, 32 heads
-// 1140 -> 942-1000; 8 x 2048 tokens 519 -> 480; 2 prompts of up to 1500 and 30 single tokens after 4000, 28 heads
-// 286 -> 195.
+// 1140 -> 942-1000; 8 x 2048 tokens 519 -> 480, with TILES = 1 470; 2 prompts of up to 1500 and 30 single tokens after 4000, 28 heads
+// 286 -> 202 (TILES = 1).
 // Slower than this (the attention kernel of the first, 920 here): one thread per row 968; steps of 64 keys with two S
 // buffers 1192; S released early and P in shared memory 1210; an MMA thread per tile 1077; persistent CTAs whose
 // queries are prepared by two more warps 964.
-constexpr int kAttnThreads = 576;
-constexpr int kSoftmaxWarps = 16;
-constexpr int kAttnStages = 3;
-constexpr uint32_t kAttnTmemCols = 512;
+//
+// With TILES = 1 a CTA has one tile, half the warps and columns, and one buffer each for K codes and V values, reloaded
+// as soon as the MMAs that read them are done: two CTAs per SM, which hide each other's gaps.
+constexpr int kAttnStages = 3;        // TILES = 2
 // Q tile in core-matrix order with 16 bytes between the core matrices: the 8 head-dim chunks of a row then fall into
 // different banks when a warp writes a row.
 constexpr int kQCore = 128 + 16, kQGroup = 8 * kQCore;
 
+template <int TILES>
 struct __align__(128) AttnSmem {
-    uint8_t q[2][(kPfRows / 8) * kQGroup];              // (the epilogue passes O through it: 128 rows of 144 bytes)
-    uint8_t k[kAttnStages][kPfKeys * kHeadDim];
-    uint16_t v[kAttnStages][kPfKeys * kHeadDim];
-    float k_scale[kAttnStages][kPfKeys];
+    static constexpr int kStages = TILES == 2 ? kAttnStages : 1;
+    uint8_t q[TILES][(kPfRows / 8) * kQGroup];          // (the epilogue passes O through it: 128 rows of 144 bytes)
+    uint8_t k[kStages][kPfKeys * kHeadDim];
+    uint16_t v[kStages][kPfKeys * kHeadDim];
+    float k_scale[TILES == 2 ? kStages : 2][kPfKeys];
     float rot[32 * 16];
-    float q_scale[2][kPfRows];
-    float xch[2][2][kPfRows];                           // [tile][half]: exchange between the two threads of a row
-    uint64_t q_ready;                                   // both Q tiles are in shared memory
-    uint64_t s_ready[2], p_ready[2];                    // per tile: S complete (and the PV before it), P written
-    uint64_t full[kAttnStages], empty[kAttnStages];     // per stage: record landed, record used up
+    float q_scale[TILES][kPfRows];
+    float xch[TILES][2][kPfRows];                       // [tile][half]: exchange between the two threads of a row
+    uint64_t q_ready;                                   // the Q tiles are in shared memory
+    uint64_t s_ready[TILES], p_ready[TILES];            // per tile: S complete (and the PV before it), P written
+    uint64_t full[kAttnStages], empty[kAttnStages];     // two tiles; per stage: record landed, record used up
+    uint64_t k_full, v_full, scale_full[2];             // one tile: K codes, V values, key scales (two buffers) landed
     uint64_t drained;                                   // after a failed wait: every MMA issued has completed
     uint32_t tmem_base;
 };
@@ -757,15 +759,14 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar_addr) : "memory");
 }
-// Barrier of the 256 softmax threads of a tile, and of all softmax threads.
-__device__ __forceinline__ void tile_sync(int x) { asm volatile("bar.sync %0, 256;" ::"r"(10 + x) : "memory"); }
-__device__ __forceinline__ void softmax_sync() { asm volatile("bar.sync 9, 512;" ::: "memory"); }
+// Barrier of the 256 softmax threads of a tile.
+__device__ __forceinline__ void tile_sync(int x) { asm volatile("bar.sync %0, 256;" ::"r"(9 + x) : "memory"); }
 
 // Which (sequence, tile or pair of tiles) the `index`-th unit of work is; sequences from the last to the first
 // (schedulers put running requests with one token before prompts), their units from the last (longest) to the first, so
-// that long units start early (217 -> 195 us for 30 single tokens and 2 prompts).  Every warp finds it by itself.  False when there are fewer units.
-__device__ __forceinline__ bool find_unit(const PrefillParams& p, int index, int& seq, int& unit) {
-    const int per = p.tokens_per_tile * p.tiles_per_unit, lane = threadIdx.x & 31;
+// that long units start early; `per` tokens a unit (217 -> 195 us with two tiles per CTA for 30 single tokens and 2 prompts).  Every warp finds it by itself.  False when there are fewer units.
+__device__ __forceinline__ bool find_unit(const PrefillParams& p, int per, int index, int& seq, int& unit) {
+    const int lane = threadIdx.x & 31;
     if (p.cu_seqlens_q == nullptr) {
         seq = 0;
         const int n = (p.num_tokens + per - 1) / per;
@@ -803,26 +804,30 @@ __device__ __forceinline__ bool find_unit(const PrefillParams& p, int index, int
     return false;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kAttnThreads, 1)
+template <int TILES> constexpr int kAttnThreads = 256 * TILES + 64;
+
+template <typename T, int TILES>
+__global__ void __launch_bounds__(kAttnThreads<TILES>, TILES == 2 ? 1 : 2)
 prefill_attn_kernel(const PrefillParams p) {
+    constexpr int kSoftmaxWarps = 8 * TILES, kThreads = kAttnThreads<TILES>;
+    constexpr uint32_t kCols = 256u * TILES, kOutCols = 128u * TILES;       // O_x behind the sums
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    AttnSmem& sm = *reinterpret_cast<AttnSmem*>(smem_raw);
+    AttnSmem<TILES>& sm = *reinterpret_cast<AttnSmem<TILES>*>(smem_raw);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = blockIdx.x % p.H;
     int seq, unit;
-    if (!find_unit(p, blockIdx.x / p.H, seq, unit)) return;
+    if (!find_unit(p, p.tokens_per_tile * TILES, blockIdx.x / p.H, seq, unit)) return;
     const int q_begin = p.cu_seqlens_q ? __ldg(p.cu_seqlens_q + seq) : 0;
     const int q_end = p.cu_seqlens_q ? __ldg(p.cu_seqlens_q + seq + 1) : p.num_tokens;
     const int q_len = q_end - q_begin;
     const int kv_len = max(__ldg(p.seq_lens + seq), 0);
     // K/V tiles that each of the two tiles needs: up to its last row's position, never past the staged records
     auto tiles_of = [&](int x) {
-        const int first = (unit * p.tiles_per_unit + x) * p.tokens_per_tile;
+        const int first = (unit * TILES + x) * p.tokens_per_tile;
         const int last = min(q_len, first + p.tokens_per_tile) - 1;
         const int last_pos = min(kv_len - q_len + last, kv_len - 1);
-        const bool any = x < p.tiles_per_unit && first < q_len && last_pos >= 0;
+        const bool any = x < TILES && first < q_len && last_pos >= 0;
         return any ? min(last_pos / kPfKeys + 1, p.stage_tiles_per_seq) : 0;
     };
     const int n0 = tiles_of(0), n1 = tiles_of(1), n_all = max(n0, n1);
@@ -832,10 +837,14 @@ prefill_attn_kernel(const PrefillParams p) {
         mbar_init(&sm.q_ready, kSoftmaxWarps);
         mbar_init(&sm.drained, 1);
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
+        for (int x = 0; x < TILES; ++x) {
             mbar_init(&sm.s_ready[x], 1);
-            mbar_init(&sm.p_ready[x], kSoftmaxWarps / 2);
+            mbar_init(&sm.p_ready[x], 8);
         }
+        mbar_init(&sm.k_full, 1);
+        mbar_init(&sm.v_full, 1);
+        mbar_init(&sm.scale_full[0], 1);
+        mbar_init(&sm.scale_full[1], 1);
 #pragma unroll
         for (int s = 0; s < kAttnStages; ++s) {
             mbar_init(&sm.full[s], 1);
@@ -844,14 +853,15 @@ prefill_attn_kernel(const PrefillParams p) {
         fence_async_proxy();
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == kSoftmaxWarps) tmem_alloc(&sm.tmem_base, kAttnTmemCols);
-    for (int i = tid; i < 32 * 16; i += kAttnThreads) {
+    if (warp == kSoftmaxWarps) tmem_alloc(&sm.tmem_base, kCols);
+    for (int i = tid; i < 32 * 16; i += kThreads) {
         const int g = i >> 4, j = (i >> 2) & 3, k = i & 3;
         sm.rot[i] = __ldg(p.rotation + (4 * g + j) * kHeadDim + 4 * g + k);      // R[4g+j][4g+k]
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    const uint32_t base = TILES == 2 ? 0u : sm.tmem_base;     // all columns, or half of them
     bool failed = false;
 
     if (warp == kSoftmaxWarps + 1) {
@@ -860,6 +870,36 @@ prefill_attn_kernel(const PrefillParams p) {
             grid_dependency_wait();                           // the records
             const uint8_t* rec = p.stage + (static_cast<int64_t>(seq) * p.stage_tiles_per_seq * p.H + kvh) * kStageRecord;
             const int64_t record_stride = static_cast<int64_t>(p.H) * kStageRecord;
+            if constexpr (TILES == 1) {
+                int k_next = 0, v_next = 0;
+                auto load_k = [&] {
+                    const uint8_t* const src = rec + k_next * record_stride;
+                    const uint32_t bar = smem_u32(&sm.k_full), bar_s = smem_u32(&sm.scale_full[k_next & 1]);
+                    mbar_expect_tx(bar, kPfKeys * kHeadDim);
+                    bulk_load(smem_u32(sm.k[0]), src, kPfKeys * kHeadDim, bar);
+                    mbar_expect_tx(bar_s, kPfKeys * 4);
+                    bulk_load(smem_u32(sm.k_scale[k_next & 1]), src + 3 * kPfKeys * kHeadDim, kPfKeys * 4, bar_s);
+                    ++k_next;
+                };
+                auto load_v = [&] {
+                    const uint32_t bar = smem_u32(&sm.v_full);
+                    mbar_expect_tx(bar, 2 * kPfKeys * kHeadDim);
+                    bulk_load(smem_u32(sm.v[0]), rec + v_next * record_stride + kPfKeys * kHeadDim, 2 * kPfKeys * kHeadDim, bar);
+                    ++v_next;
+                };
+                if (n0 > 0) { load_k(); load_v(); }
+                for (int j = 0; j < n0; ++j) {                // S(j) complete: K(j) and, before it, V(j - 1) have been read
+                    failed = !mbar_wait(&sm.s_ready[0], static_cast<uint32_t>(j) & 1u);
+                    if (failed) break;
+                    if (j > 0) load_v();
+                    if (j + 1 < n0) load_k();
+                }
+                if (n0 > 0) {                                 // copies in flight land before the CTA ends
+                    mbar_wait(&sm.k_full, static_cast<uint32_t>(k_next - 1) & 1u);
+                    mbar_wait(&sm.v_full, static_cast<uint32_t>(v_next - 1) & 1u);
+                    mbar_wait(&sm.scale_full[(k_next - 1) & 1], static_cast<uint32_t>((k_next - 1) / 2) & 1u);
+                }
+            } else {
             int issued = 0;
             for (; issued < n_all; ++issued, rec += record_stride) {
                 const int s = issued % kAttnStages;
@@ -874,6 +914,7 @@ prefill_attn_kernel(const PrefillParams p) {
             if (failed)                                       // copies in flight land before the CTA ends
                 for (int j = max(0, issued - kAttnStages); j < issued; ++j)
                     mbar_wait(&sm.full[j % kAttnStages], static_cast<uint32_t>(j / kAttnStages) & 1u);
+            }
         }
         __syncwarp();
     } else if (warp == kSoftmaxWarps) {
@@ -889,10 +930,36 @@ prefill_attn_kernel(const PrefillParams p) {
                 const uint32_t q_addr = smem_u32(sm.q[x]), k_addr = smem_u32(sm.k[stage]);
 #pragma unroll
                 for (int s = 0; s < 4; ++s)
-                    tc_mma_i8(128u * x, smem_desc(q_addr + 2 * kQCore * s, kQCore, kQGroup), smem_desc(k_addr + 256 * s, 128, 1024),
+                    tc_mma_i8(base + 128u * x, smem_desc(q_addr + 2 * kQCore * s, kQCore, kQGroup), smem_desc(k_addr + 256 * s, 128, 1024),
                               idesc_s, s > 0 ? 1u : 0u);
             };
+            auto values = [&](int x, int stage, int j) {
+                const uint32_t v_addr = smem_u32(sm.v[stage]);
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    tc_mma_f16_ta(base + kOutCols + 128u * x, base + 128u * x + 64u * (c >> 2) + 8u * (c & 3),
+                                  smem_desc(v_addr + 4096 * c, 2048, 128), idesc_o, c > 0 ? 1u : static_cast<uint32_t>(j > 0));
+            };
             failed |= !mbar_wait(&sm.q_ready, 0);
+            if constexpr (TILES == 1) {
+                for (int j = -1; j < n0 && !failed; ++j) {    // PV(j), S(j + 1)
+                    const uint32_t parity = static_cast<uint32_t>(j) & 1u;
+                    if (j >= 0) {
+                        failed |= !mbar_wait(&sm.v_full, parity);
+                        failed |= !mbar_wait(&sm.p_ready[0], parity);
+                        if (failed) break;
+                        tc_fence_after();
+                        values(0, 0, j);
+                    }
+                    if (j + 1 < n0) {
+                        failed |= !mbar_wait(&sm.k_full, parity ^ 1u);
+                        if (failed) break;
+                        tc_fence_after();
+                        scores(0, 0);
+                    }
+                    tc_commit(&sm.s_ready[0]);
+                }
+            } else {
             failed |= !mbar_wait(&sm.full[0], 0);
             if (!failed) {
                 tc_fence_after();
@@ -903,7 +970,6 @@ prefill_attn_kernel(const PrefillParams p) {
             auto step = [&](auto unrolled, int j, uint32_t phase) {
                 constexpr int stage = decltype(unrolled)::value, next = (stage + 1) % kAttnStages;
                 if (j + 1 < n_all && !failed) failed |= !mbar_wait(&sm.full[next], next == 0 ? phase ^ 1u : phase);
-                const uint32_t v_addr = smem_u32(sm.v[stage]);
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
                     const int nx = x == 0 ? n0 : n1;
@@ -911,10 +977,7 @@ prefill_attn_kernel(const PrefillParams p) {
                     failed |= !mbar_wait(&sm.p_ready[x], static_cast<uint32_t>(j) & 1u);
                     if (failed) continue;
                     tc_fence_after();
-#pragma unroll
-                    for (int c = 0; c < 8; ++c)
-                        tc_mma_f16_ta(256u + 128u * x, 128u * x + 64u * (c >> 2) + 8u * (c & 3), smem_desc(v_addr + 4096 * c, 2048, 128),
-                                      idesc_o, c > 0 ? 1u : static_cast<uint32_t>(j > 0));
+                    values(x, stage, j);
                     if (j + 1 < nx) scores(x, next);
                     tc_commit(&sm.s_ready[x]);
                 }
@@ -924,6 +987,7 @@ prefill_attn_kernel(const PrefillParams p) {
                 step(std::integral_constant<int, 0>{}, j, phase);
                 step(std::integral_constant<int, 1>{}, j + 1, phase);
                 step(std::integral_constant<int, 2>{}, j + 2, phase);
+            }
             }
             if (failed) {                                     // what was issued ends before TMEM is freed
                 tc_commit(&sm.drained);
@@ -936,16 +1000,17 @@ prefill_attn_kernel(const PrefillParams p) {
         const int x = warp >> 3, half = (warp >> 2) & 1, row = tid & (kPfRows - 1);
         const int pair_id = 1 + 4 * x + (warp & 3);           // named barrier of the two warps with the same rows
         const int n = x == 0 ? n0 : n1;
-        const uint32_t lanes = (static_cast<uint32_t>((warp & 3) * 32) << 16) + 128u * x;
-        const uint32_t s_cols = lanes + 64u * half, o_cols = lanes + 256u + 64u * half;
+        const uint32_t lanes = (static_cast<uint32_t>((warp & 3) * 32) << 16) + base + 128u * x;
+        const uint32_t s_cols = lanes + 64u * half, o_cols = lanes + kOutCols + 64u * half;
         float* const xch = sm.xch[x][half] + row;
         const float* const xch_other = sm.xch[x][half ^ 1] + row;
-        const int first_tok = (unit * p.tiles_per_unit + x) * p.tokens_per_tile;
-        // Q and the output are handled by whole rows: a warp has rows row0 .. row0 + rows - 1 of tile xr, lane i < 16 knows
-        // where row row0 + i is (-1: no such row).  Queries of a single tile are shared by all the warps.
-        auto row_offset = [&](int xr, int r, int64_t tok_stride, int64_t head_stride) -> long long {
-            const int tl = r / p.G, tk = (unit * p.tiles_per_unit + xr) * p.tokens_per_tile + tl;
-            if (xr >= p.tiles_per_unit || tl >= p.tokens_per_tile || tk >= q_len) return -1;
+        const int first_tok = (unit * TILES + x) * p.tokens_per_tile;
+        // Q and the output are handled by whole rows: a warp has rows row0 .. row0 + 15, lane i < 16 knows where row
+        // row0 + i is (-1: no such row)
+        const int row0 = 16 * (warp & 7);
+        auto row_offset = [&](int64_t tok_stride, int64_t head_stride) -> long long {
+            const int r = row0 + (lane & 15), tl = r / p.G, tk = first_tok + tl;
+            if (tl >= p.tokens_per_tile || tk >= q_len) return -1;
             return (q_begin + tk) * tok_stride + static_cast<int64_t>(kvh * p.G + r % p.G) * head_stride;
         };
 
@@ -953,7 +1018,6 @@ prefill_attn_kernel(const PrefillParams p) {
         // registers), so that loads are contiguous.  Bound by latency, so eight rows are in flight while eight are converted.
         {
             constexpr int kRows = 8;
-            const int rows = kRows * p.tiles_per_unit, xq = (warp * rows) >> 7, row_q = (warp * rows) & (kPfRows - 1);
             f2 rot[4][2];                                     // [in][outs 0, 1 | outs 2, 3]
             {
                 float r[4][4];
@@ -962,7 +1026,7 @@ prefill_attn_kernel(const PrefillParams p) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) { rot[k][0] = pk(r[0][k], r[1][k]); rot[k][1] = pk(r[2][k], r[3][k]); }
             }
-            const long long at_row = row_offset(xq, row_q + (lane & 15), p.q_stride_tok, p.q_stride_head);
+            const long long at_row = row_offset(p.q_stride_tok, p.q_stride_head);
             uint2 next[kRows];
             auto fetch = [&](int i0) {
 #pragma unroll
@@ -974,14 +1038,14 @@ prefill_attn_kernel(const PrefillParams p) {
             // Adding 1.5 * 2^23 rounds to the nearest integer, in the low bits.  Scalar operations: the assembler contracts a
             // packed product and sum, and a product that is a tie after its own rounding would go the other way.
             auto code = [](float v, float scale) { return __float_as_uint(__fadd_rn(__fmul_rn(v, scale), 12582912.0f)); };
-            if ((xq == 0 ? n0 : n1) > 0) {
+            if (n > 0) {
                 fetch(0);
 #pragma unroll 1
-                for (int i0 = 0; i0 < rows; i0 += kRows) {
+                for (int i0 = 0; i0 < 16; i0 += kRows) {
                     uint2 raw[kRows];
 #pragma unroll
                     for (int i = 0; i < kRows; ++i) raw[i] = next[i];
-                    if (i0 + kRows < rows) fetch(i0 + kRows);
+                    if (i0 + kRows < 16) fetch(i0 + kRows);
                     float mx = 0.0f;                          // lane i < 8: largest |value| of row i0 + i
 #pragma unroll
                     for (int i = 0; i < kRows; ++i) {
@@ -1001,15 +1065,15 @@ prefill_attn_kernel(const PrefillParams p) {
                     }
                     const bool ok = mx > 0.0f && mx <= 3.0e38f;
                     const float inv = ok ? __fdiv_rn(127.0f, mx) : 0.0f;
-                    if (lane < kRows) sm.q_scale[xq][row_q + i0 + lane] = ok ? __fdiv_rn(mx, 127.0f) : 0.0f;
+                    if (lane < kRows) sm.q_scale[x][row0 + i0 + lane] = ok ? __fdiv_rn(mx, 127.0f) : 0.0f;
 #pragma unroll
                     for (int i = 0; i < kRows; ++i) {
                         const float inv_row = __shfl_sync(0xffffffffu, inv, i);
                         const float2 a = pf_unpack<T>(raw[i].x), b = pf_unpack<T>(raw[i].y);
                         // position d holds head-dim d ^ 1
                         const uint32_t w = prmt(prmt(code(a.y, inv_row), code(a.x, inv_row), 0x0040), prmt(code(b.y, inv_row), code(b.x, inv_row), 0x0040), 0x5410);
-                        const int r = row_q + i0 + i;
-                        *reinterpret_cast<uint32_t*>(&sm.q[xq][(r >> 3) * kQGroup + (lane >> 2) * kQCore + (r & 7) * 16 + 4 * (lane & 3)]) = w;
+                        const int r = row0 + i0 + i;
+                        *reinterpret_cast<uint32_t*>(&sm.q[x][(r >> 3) * kQGroup + (lane >> 2) * kQCore + (r & 7) * 16 + 4 * (lane & 3)]) = w;
                     }
                 }
             }
@@ -1017,7 +1081,7 @@ prefill_attn_kernel(const PrefillParams p) {
         fence_async_proxy();                                  // the Q tile is read by the tensor core
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.q_ready);
-        softmax_sync();                                       // every row's scale is there
+        tile_sync(x);                                       // every row's scale is there
         const float row_factor = n > 0 ? sm.q_scale[x][row] * p.qk_scale : 0.0f;
         // Position of the row's token in its sequence.  Rows without a token (zero queries, never stored) see every key: as
         // rows that see none they would send their whole warp through the masked path at every tile (with 7 heads a tile
@@ -1032,13 +1096,14 @@ prefill_attn_kernel(const PrefillParams p) {
         float m_run = -INFINITY, l_run = 0.0f;                // l_run: this half of the keys
         for (int j = 0; j < n; ++j) {
             // After an expired wait the warp keeps its step (its partner meets it at the named barrier) without waiting.
-            const int stage = j % kAttnStages;
+            const int stage = TILES == 2 ? j % kAttnStages : j & 1;
             if (!failed) failed = !mbar_wait(&sm.s_ready[x], static_cast<uint32_t>(j) & 1u);
-            if (!failed) failed = !mbar_wait(&sm.full[stage], static_cast<uint32_t>(j / kAttnStages) & 1u);   // key scales
+            if (!failed) failed = TILES == 2 ? !mbar_wait(&sm.full[stage], static_cast<uint32_t>(j / kAttnStages) & 1u)   // key scales
+                                             : !mbar_wait(&sm.scale_full[stage], static_cast<uint32_t>(j / 2) & 1u);
             failed = __any_sync(0xffffffffu, failed);
             tc_fence_after();
             // S(j) is complete, so PV(j - 1) is: the later tile of the two frees the record that PV used up
-            if (j > 0 && tid == (n1 > 0 ? 256 : 0)) mbar_arrive(&sm.empty[(j - 1) % kAttnStages]);
+            if (TILES == 2 && j > 0 && tid == (n1 > 0 ? 256 : 0)) mbar_arrive(&sm.empty[(j - 1) % kAttnStages]);
             const float* const k_scale = sm.k_scale[stage] + 64 * half;
             const int limit = pos - (j * kPfKeys + 64 * half);    // the row sees keys 0 .. limit of this half tile
             const bool unmasked = __all_sync(0xffffffffu, limit >= 63);
@@ -1162,11 +1227,10 @@ prefill_attn_kernel(const PrefillParams p) {
             l_run += *xch_other;
         }
         const float inv_l = l_run > 0.0f ? 1.0f / l_run : 0.0f;
-        const int row0 = 16 * (warp & 7);
-        const long long mine = failed ? -1 : row_offset(x, row0 + (lane & 15), p.o_stride_tok, p.o_stride_head);
+        const long long mine = failed ? -1 : row_offset(p.o_stride_tok, p.o_stride_head);
         uint8_t* const tile_rows = sm.q[x];
 #pragma unroll 1
-        for (int h = 0; h < 2 && x < p.tiles_per_unit; ++h) {
+        for (int h = 0; h < 2; ++h) {
             if (half == h) {
 #pragma unroll 1
                 for (int ch = 0; ch < 2; ++ch) {
@@ -1214,30 +1278,37 @@ prefill_attn_kernel(const PrefillParams p) {
     if (failed && p.error_flag != nullptr) atomicExch(p.error_flag, 1);
     tc_fence_before();
     __syncthreads();
-    if (warp == kSoftmaxWarps) tmem_dealloc(sm.tmem_base, kAttnTmemCols);
+    if (warp == kSoftmaxWarps) tmem_dealloc(sm.tmem_base, kCols);
 }
 
 // ---- host side --------------------------------------------------------------------------------
 
 template <typename T, int KB, int VB>
-static int launch_prefill(PrefillParams& p, int m_tiles, int num_seqs, cudaStream_t st) {
+static int launch_prefill(const PrefillParams& p, int m_tiles, int num_seqs, cudaStream_t st) {
     if (p.stage != nullptr) {
         dim3 sgrid(p.stage_tiles_per_seq, p.H, num_seqs);
         if (int e = launch_dependent("rq_prefill_int8 stage launch", prefill_stage_kernel<T, KB, VB>, sgrid, dim3(128), 0, st, p)) return e;
-        const size_t smem = sizeof(AttnSmem);
-        if (int e = ensure_smem(prefill_attn_kernel<T>, smem)) return e;
         // Units of work: at most tokens / (tokens of a unit) + one partial unit per sequence, found by the CTAs
-        // themselves (a grid of longest sequence x sequences was mostly empty CTAs for batches of mixed lengths).  Two
-        // tiles per CTA share the K/V tiles and keep the tensor core busy under each other's softmax; with no more
-        // tiles than SMs a CTA per tile finishes earlier.
+        // themselves (a grid of longest sequence x sequences was mostly empty CTAs for batches of mixed lengths).
+        // One tile per CTA, two CTAs per SM, is the faster form up to some thousand keys, as one CTA's queries and output
+        // run under the other's loop (8 x 2048 tokens 480 -> 470 us, 19 prompts of 34 to 283 85 -> 73).  Two tiles per CTA
+        // read K/V half as often, which pays where contexts may be long (2048 tokens after 30000: 1010-1030 -> 950), unless
+        // most sequences have no second tile or there are too few tiles for every SM.
         auto units = [&](long long per) {
             const long long by_tokens = p.num_tokens / per + num_seqs;
             const long long by_longest = num_seqs * ((1LL * m_tiles * p.tokens_per_tile + per - 1) / per);
             return (by_tokens < by_longest ? by_tokens : by_longest) * p.H;
         };
-        p.tiles_per_unit = units(p.tokens_per_tile) > kSms ? 2 : 1;
-        const dim3 grid(static_cast<unsigned>(units(1LL * p.tokens_per_tile * p.tiles_per_unit)));
-        return launch_dependent("rq_prefill_int8 attention launch", prefill_attn_kernel<T>, grid, dim3(kAttnThreads), smem, st, p);
+        auto attend = [&](auto tiles) {
+            constexpr int kTiles = decltype(tiles)::value;
+            const size_t smem = sizeof(AttnSmem<kTiles>);
+            if (int e = ensure_smem(prefill_attn_kernel<T, kTiles>, smem)) return e;
+            return launch_dependent("rq_prefill_int8 attention launch", prefill_attn_kernel<T, kTiles>,
+                                    dim3(static_cast<unsigned>(units(1LL * p.tokens_per_tile * kTiles))), dim3(kAttnThreads<kTiles>), smem, st, p);
+        };
+        const bool one = p.stage_tiles_per_seq <= 16384 / kPfKeys || units(p.tokens_per_tile) <= kSms ||
+                         p.num_tokens <= 1LL * num_seqs * p.tokens_per_tile;
+        return one ? attend(std::integral_constant<int, 1>{}) : attend(std::integral_constant<int, 2>{});
     }
     dim3 grid(m_tiles, p.H, num_seqs);
     const size_t smem = sizeof(PrefillSmem);
@@ -1247,7 +1318,7 @@ static int launch_prefill(PrefillParams& p, int m_tiles, int num_seqs, cudaStrea
 }
 
 template <typename T>
-static int dispatch_prefill(PrefillParams& p, int m_tiles, int num_seqs, int kb, int vb, cudaStream_t st) {
+static int dispatch_prefill(const PrefillParams& p, int m_tiles, int num_seqs, int kb, int vb, cudaStream_t st) {
     if (kb == 3 && vb == 3) return launch_prefill<T, 3, 3>(p, m_tiles, num_seqs, st);
     if (kb == 4 && vb == 3) return launch_prefill<T, 4, 3>(p, m_tiles, num_seqs, st);
     if (kb == 3 && vb == 4) return launch_prefill<T, 3, 4>(p, m_tiles, num_seqs, st);

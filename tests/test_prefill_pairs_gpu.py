@@ -1,24 +1,32 @@
-"""Prefill batches whose sequences end at every remainder of the pairs of 128-row tiles the staged
-path works on (and of single tiles, for small grids), with empty sequences, single-token rows and
-more sequences than one step of the search for a unit of work covers."""
+"""Prefill batches whose sequences end at every remainder of the 128-row tiles the staged path works
+on -- one tile per CTA, and pairs of tiles where contexts may be long -- with empty sequences,
+single-token rows and more sequences than one step of the search for a unit of work covers."""
 
 import pytest
 import torch
 
 import test_prefill_gpu as base
+from gpu_util import on_gpu
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("H,HQ,ctx,q", [
-    (8, 32, [130, 300, 64, 65, 0, 31, 700], [1, 97, 64, 65, 0, 31, 161]),         # 32 tokens a tile: pairs
-    (8, 32, [500], [33]), (8, 32, [129, 5], [1, 5]),                              # single tiles
-    (4, 28, [400, 1, 0, 290, 37, 19], [400, 1, 0, 126, 37, 19]),                   # 18 tokens a tile, 2 rows without one
+    (8, 32, [130, 300, 64, 65, 0, 31, 700], [1, 97, 64, 65, 0, 31, 161]),         # 32 tokens a tile
+    (8, 32, [500], [33]), (8, 32, [129, 5], [1, 5]),                              # always single tiles
+    (4, 28, [400, 1, 0, 290, 37, 19], [400, 1, 0, 126, 37, 19]),                  # 18 tokens a tile, 2 rows without one
     (32, 32, [257, 129, 300], [257, 129, 1]),                                     # 128 tokens a tile
-    (1, 128, [40 + i % 3 for i in range(150)], [i % 3 for i in range(150)]),      # one token a tile, 150 sequences
+    (1, 128, [40 + i % 4 for i in range(150)], [i % 4 for i in range(150)]),      # one token a tile, 150 sequences
 ])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_unit_remainders(H, HQ, ctx, q, dtype):
+@pytest.mark.parametrize("bound", [1024, 16385])
+def test_unit_remainders(H, HQ, ctx, q, dtype, bound):
     # (seed 5 has a rotated query on a rounding boundary, where the kernels and the oracle add in different orders)
     c, cu = base._fresh("iso_fast", 3, 4, H, HQ, ctx, q, 16, dtype, 6)
-    base._check(base._run(c, cu, staged=True), c, cu)
+    g = on_gpu(c)
+    flag = torch.zeros(1, dtype=torch.int32, device=g["q"].device)
+    out = base._prefill(g["q"], g["kv_cache"], g["block_table"], g["seq_lens"], g["k_centroids"], g["v_centroids"], g["R"],
+                        H, 128, 16, sm_scale=c["sm_scale"], cu_seqlens_q=cu.to(flag.device), error_flag=flag, staged=True,
+                        max_seq_len=bound).cpu()
+    assert int(flag.item()) == 0, "a bounded device-side wait expired"
+    base._check(out, c, cu)
