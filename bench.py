@@ -754,7 +754,7 @@ def measure_compress(job: GpuJob, device, tokens: int = 16384) -> dict:
     bytes_per_token = job.H * (2 * w.head_dim * 2 + 136)
     gbs = tokens * bytes_per_token / (ms * 1e-3) / 1e9
     return {"tokens": tokens, "kv_heads": job.H, "ms": ms, "mtok_per_s": tokens / (ms * 1e-3) / 1e6,
-            "roofline": {"bound": "hbm", "kernel": "compress_store_kernel", "achieved": gbs, "peak": peak["hbm_gbs"],
+            "roofline": {"bound": "hbm", "kernel": "compress_kernel", "achieved": gbs, "peak": peak["hbm_gbs"],
                          "unit": "GB/s", "frac": gbs / peak["hbm_gbs"], "peak_kind": peak["kind"] + " copy bandwidth",
                          "algorithmic_bytes_per_token": bytes_per_token},
             "_inputs": (k, v, slots)}
