@@ -10,10 +10,12 @@
 // on one device, expected types and layouts, a rotation that has been validated, scratch already in place).  If
 // anything is not, it returns None without having done anything and the launcher takes its Python path, which
 // converts, allocates or raises; so all errors and unusual layouts are handled in one place.  The C-ABI functions
-// are called through the addresses that _lib.py found in the library it loaded.
+// are called through the addresses that _lib.py found in the library it loaded.  C++ exceptions (memory that cannot
+// be had, tensors without storage or version counter) leave as the Python exceptions torch makes of them.
 #include <Python.h>
 
 #include <torch/csrc/Device.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <ATen/ATen.h>
@@ -21,6 +23,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <cmath>
+#include <exception>
 #include <unordered_map>
 
 #include "../../include/rq_b200.h"
@@ -50,8 +53,22 @@ std::unordered_map<PyObject*, uint32_t>& validated() {
     return table;
 }
 
+// Tensors and parameters themselves; a subclass may mean anything by its operations, so it takes the Python path.
 const at::Tensor* tensor(PyObject* o) {
-    return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr;
+    return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr;
+}
+
+// The GIL is released for the life of this object, also when an exception passes.
+struct Unlocked {
+    PyThreadState* const state = PyEval_SaveThread();
+    Unlocked() = default;
+    Unlocked(const Unlocked&) = delete;
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+template <typename F>
+auto unlocked(F&& call) {
+    const Unlocked no_gil;
+    return call();
 }
 
 // A call's tensors: all on one CUDA device.
@@ -148,7 +165,10 @@ PyObject* bind(PyObject*, PyObject* dict) {
 
 // mark_valid(rotation), forget(id)
 PyObject* mark_valid(PyObject*, PyObject* o) {
-    if (const at::Tensor* t = tensor(o)) validated()[o] = t->_version();
+    if (const at::Tensor* t = tensor(o)) {
+        const uint32_t version = t->_version();          // throws for tensors without a counter: no entry then
+        validated()[o] = version;
+    }
     return none();
 }
 PyObject* forget(PyObject*, PyObject* id) {
@@ -180,17 +200,16 @@ PyObject* compress_store(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (padding < 0) return nullptr;
     const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev.index));
     void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev.index)).stream();
-    int status;
-    Py_BEGIN_ALLOW_THREADS
-    status = fn.compress_store(key.const_data_ptr(), value.const_data_ptr(), dtype, n, static_cast<int>(key.size(1)),
-                               static_cast<int>(key.size(2)), key.stride(0), key.stride(1), value.stride(0),
-                               value.stride(1), static_cast<uint8_t*>(cache.data_ptr()), cache.size(0) * cache.size(1),
-                               static_cast<int>(cache.size(2)), static_cast<const int64_t*>(slots.const_data_ptr()),
-                               static_cast<const float*>(t[4]->const_data_ptr()),
-                               static_cast<const float*>(kb.const_data_ptr()), static_cast<int>(kb.numel()),
-                               static_cast<const float*>(vb.const_data_ptr()), static_cast<int>(vb.numel()), padding,
-                               stream);
-    Py_END_ALLOW_THREADS
+    const int status = unlocked([&] {
+        return fn.compress_store(key.const_data_ptr(), value.const_data_ptr(), dtype, n, static_cast<int>(key.size(1)),
+                                 static_cast<int>(key.size(2)), key.stride(0), key.stride(1), value.stride(0),
+                                 value.stride(1), static_cast<uint8_t*>(cache.data_ptr()), cache.size(0) * cache.size(1),
+                                 static_cast<int>(cache.size(2)), static_cast<const int64_t*>(slots.const_data_ptr()),
+                                 static_cast<const float*>(t[4]->const_data_ptr()),
+                                 static_cast<const float*>(kb.const_data_ptr()), static_cast<int>(kb.numel()),
+                                 static_cast<const float*>(vb.const_data_ptr()), static_cast<int>(vb.numel()), padding,
+                                 stream);
+    });
     if (raised(status)) return nullptr;
     Py_RETURN_TRUE;
 }
@@ -261,19 +280,18 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(c.dev.index));
     const at::Tensor out = c.result();
     void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(c.dev.index)).stream();
-    int status;
-    Py_BEGIN_ALLOW_THREADS
-    status = fn.decode(q.const_data_ptr(), out.data_ptr(), c.dtype, q.stride(0), q.stride(1), out.stride(0), out.stride(1),
-                       static_cast<int>(c.num_seqs), static_cast<int>(q.size(1)), static_cast<int>(c.heads),
-                       static_cast<int>(c.head_dim), static_cast<const uint8_t*>(cache.const_data_ptr()), cache.size(0),
-                       static_cast<int>(c.block_size), static_cast<int>(cache.size(2)),
-                       static_cast<const int32_t*>(table.const_data_ptr()), table.stride(0),
-                       static_cast<const int32_t*>(c.t[3]->const_data_ptr()),
-                       static_cast<const float*>(c.t[4]->const_data_ptr()), static_cast<int>(c.t[4]->numel()),
-                       static_cast<const float*>(c.t[5]->const_data_ptr()), static_cast<int>(c.t[5]->numel()),
-                       static_cast<const float*>(c.t[6]->const_data_ptr()), c.scale, static_cast<int>(max_len),
-                       ws.data_ptr(), static_cast<size_t>(ws.numel()) * ws.element_size(), static_cast<int>(splits), stream);
-    Py_END_ALLOW_THREADS
+    const int status = unlocked([&] {
+        return fn.decode(q.const_data_ptr(), out.data_ptr(), c.dtype, q.stride(0), q.stride(1), out.stride(0), out.stride(1),
+                         static_cast<int>(c.num_seqs), static_cast<int>(q.size(1)), static_cast<int>(c.heads),
+                         static_cast<int>(c.head_dim), static_cast<const uint8_t*>(cache.const_data_ptr()), cache.size(0),
+                         static_cast<int>(c.block_size), static_cast<int>(cache.size(2)),
+                         static_cast<const int32_t*>(table.const_data_ptr()), table.stride(0),
+                         static_cast<const int32_t*>(c.t[3]->const_data_ptr()),
+                         static_cast<const float*>(c.t[4]->const_data_ptr()), static_cast<int>(c.t[4]->numel()),
+                         static_cast<const float*>(c.t[5]->const_data_ptr()), static_cast<int>(c.t[5]->numel()),
+                         static_cast<const float*>(c.t[6]->const_data_ptr()), c.scale, static_cast<int>(max_len),
+                         ws.data_ptr(), static_cast<size_t>(ws.numel()) * ws.element_size(), static_cast<int>(splits), stream);
+    });
     if (raised(status)) return nullptr;
     return c.out != nullptr ? Py_NewRef(a[11]) : THPVariable_Wrap(out);
 }
@@ -307,21 +325,20 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(c.dev.index));
     const at::Tensor out = c.result();
     void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(c.dev.index)).stream();
-    int status;
-    Py_BEGIN_ALLOW_THREADS
-    status = fn.prefill_int8_staged(
-        q.const_data_ptr(), out.data_ptr(), c.dtype, q.stride(0), q.stride(1), out.stride(0), out.stride(1),
-        cu != nullptr ? static_cast<const int32_t*>(cu->const_data_ptr()) : nullptr, static_cast<int>(q.size(0)),
-        static_cast<int>(c.num_seqs), static_cast<int>(max_q), static_cast<int>(q.size(1)), static_cast<int>(c.heads),
-        static_cast<int>(c.head_dim), static_cast<const uint8_t*>(cache.const_data_ptr()), cache.size(0),
-        static_cast<int>(c.block_size), static_cast<int>(cache.size(2)),
-        static_cast<const int32_t*>(table.const_data_ptr()), table.stride(0),
-        static_cast<const int32_t*>(c.t[3]->const_data_ptr()), static_cast<const float*>(c.t[4]->const_data_ptr()),
-        static_cast<int>(c.t[4]->numel()), static_cast<const float*>(c.t[5]->const_data_ptr()),
-        static_cast<int>(c.t[5]->numel()), static_cast<const float*>(c.t[6]->const_data_ptr()), c.scale,
-        flag != nullptr ? static_cast<int*>(flag->data_ptr()) : nullptr, static_cast<int>(bound_len), ws.data_ptr(),
-        static_cast<size_t>(ws.numel()), stream);
-    Py_END_ALLOW_THREADS
+    const int status = unlocked([&] {
+        return fn.prefill_int8_staged(
+            q.const_data_ptr(), out.data_ptr(), c.dtype, q.stride(0), q.stride(1), out.stride(0), out.stride(1),
+            cu != nullptr ? static_cast<const int32_t*>(cu->const_data_ptr()) : nullptr, static_cast<int>(q.size(0)),
+            static_cast<int>(c.num_seqs), static_cast<int>(max_q), static_cast<int>(q.size(1)), static_cast<int>(c.heads),
+            static_cast<int>(c.head_dim), static_cast<const uint8_t*>(cache.const_data_ptr()), cache.size(0),
+            static_cast<int>(c.block_size), static_cast<int>(cache.size(2)),
+            static_cast<const int32_t*>(table.const_data_ptr()), table.stride(0),
+            static_cast<const int32_t*>(c.t[3]->const_data_ptr()), static_cast<const float*>(c.t[4]->const_data_ptr()),
+            static_cast<int>(c.t[4]->numel()), static_cast<const float*>(c.t[5]->const_data_ptr()),
+            static_cast<int>(c.t[5]->numel()), static_cast<const float*>(c.t[6]->const_data_ptr()), c.scale,
+            flag != nullptr ? static_cast<int*>(flag->data_ptr()) : nullptr, static_cast<int>(bound_len), ws.data_ptr(),
+            static_cast<size_t>(ws.numel()), stream);
+    });
     if (raised(status)) return nullptr;
     return c.out != nullptr ? Py_NewRef(a[11]) : THPVariable_Wrap(out);
 }
@@ -342,13 +359,12 @@ PyObject* compress(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const at::Tensor packed = at::empty({n, h, d / 2}, x->options().dtype(at::kByte));
     const at::Tensor norms = at::empty({n, h, 1}, x->options().dtype(at::kFloat));
     void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev.index)).stream();
-    int status;
-    Py_BEGIN_ALLOW_THREADS
-    status = fn.compress(x->const_data_ptr(), dtype, n * h, static_cast<int>(d), d,
-                         static_cast<const float*>(rot->const_data_ptr()),
-                         static_cast<const float*>(bounds->const_data_ptr()), static_cast<int>(bounds->numel()),
-                         static_cast<uint8_t*>(packed.data_ptr()), static_cast<float*>(norms.data_ptr()), stream);
-    Py_END_ALLOW_THREADS
+    const int status = unlocked([&] {
+        return fn.compress(x->const_data_ptr(), dtype, n * h, static_cast<int>(d), d,
+                           static_cast<const float*>(rot->const_data_ptr()),
+                           static_cast<const float*>(bounds->const_data_ptr()), static_cast<int>(bounds->numel()),
+                           static_cast<uint8_t*>(packed.data_ptr()), static_cast<float*>(norms.data_ptr()), stream);
+    });
     if (raised(status)) return nullptr;
     PyObject* p = THPVariable_Wrap(packed);
     PyObject* m = p != nullptr ? THPVariable_Wrap(norms) : nullptr;
@@ -376,13 +392,12 @@ PyObject* decompress(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev.index));
     const at::Tensor out = at::empty({n, h, d}, packed->options().dtype(types[code]));
     void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev.index)).stream();
-    int status;
-    Py_BEGIN_ALLOW_THREADS
-    status = fn.decompress(static_cast<const uint8_t*>(packed->const_data_ptr()),
-                           static_cast<const float*>(norms->const_data_ptr()), n * h, static_cast<int>(d),
-                           static_cast<const float*>(cent->const_data_ptr()), static_cast<int>(cent->numel()),
-                           out.data_ptr(), static_cast<int>(code), stream);
-    Py_END_ALLOW_THREADS
+    const int status = unlocked([&] {
+        return fn.decompress(static_cast<const uint8_t*>(packed->const_data_ptr()),
+                             static_cast<const float*>(norms->const_data_ptr()), n * h, static_cast<int>(d),
+                             static_cast<const float*>(cent->const_data_ptr()), static_cast<int>(cent->numel()),
+                             out.data_ptr(), static_cast<int>(code), stream);
+    });
     if (raised(status)) return nullptr;
     return THPVariable_Wrap(out);
 }
@@ -410,33 +425,29 @@ PyObject* gather(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (!landing.defined()) landing = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
     auto* count = static_cast<volatile int32_t*>(landing.data_ptr());
     const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(index);
-    int status;
-    Py_BEGIN_ALLOW_THREADS
-    status = fn.block_union(static_cast<const int32_t*>(table->const_data_ptr()), table->stride(0),
-                            static_cast<int>(table->size(0)), static_cast<int>(table->size(1)),
-                            static_cast<const int32_t*>(lens->const_data_ptr()), static_cast<int>(bs), nb,
-                            static_cast<int32_t*>(listed.data_ptr()), static_cast<int32_t*>(remapped.data_ptr()),
-                            static_cast<int32_t*>(landing.data_ptr()), stream.stream());
-    Py_END_ALLOW_THREADS
+    int status = unlocked([&] {
+        return fn.block_union(static_cast<const int32_t*>(table->const_data_ptr()), table->stride(0),
+                              static_cast<int>(table->size(0)), static_cast<int>(table->size(1)),
+                              static_cast<const int32_t*>(lens->const_data_ptr()), static_cast<int>(bs), nb,
+                              static_cast<int32_t*>(listed.data_ptr()), static_cast<int32_t*>(remapped.data_ptr()),
+                              static_cast<int32_t*>(landing.data_ptr()), stream.stream());
+    });
     if (status == RQ_ERR_UNSUPPORTED) return none();
     if (raised(status)) return nullptr;
-    cudaError_t err;
-    Py_BEGIN_ALLOW_THREADS
-    err = cudaStreamSynchronize(stream.stream());
-    Py_END_ALLOW_THREADS
+    const cudaError_t err = unlocked([&] { return cudaStreamSynchronize(stream.stream()); });
     if (err != cudaSuccess) { PyErr_SetString(PyExc_RuntimeError, cudaGetErrorString(err)); return nullptr; }
     const int64_t n = *count;
     if (n < 0) return none();
     const at::ScalarType types[3] = {at::kFloat, at::kHalf, at::kBFloat16};
     const at::Tensor k = at::empty({n, bs, heads, 128}, cache->options().dtype(types[code])), v = at::empty_like(k);
-    Py_BEGIN_ALLOW_THREADS
-    status = fn.decompress_blocks(static_cast<const uint8_t*>(cache->const_data_ptr()), nb, static_cast<int>(bs),
-                                  static_cast<int>(cache->size(2)), static_cast<int>(heads), 128,
-                                  static_cast<const int32_t*>(listed.const_data_ptr()), n,
-                                  static_cast<const float*>(ck->const_data_ptr()), static_cast<int>(ck->numel()),
-                                  static_cast<const float*>(cv->const_data_ptr()), static_cast<int>(cv->numel()),
-                                  k.data_ptr(), v.data_ptr(), static_cast<int>(code), stream.stream());
-    Py_END_ALLOW_THREADS
+    status = unlocked([&] {
+        return fn.decompress_blocks(static_cast<const uint8_t*>(cache->const_data_ptr()), nb, static_cast<int>(bs),
+                                    static_cast<int>(cache->size(2)), static_cast<int>(heads), 128,
+                                    static_cast<const int32_t*>(listed.const_data_ptr()), n,
+                                    static_cast<const float*>(ck->const_data_ptr()), static_cast<int>(ck->numel()),
+                                    static_cast<const float*>(cv->const_data_ptr()), static_cast<int>(cv->numel()),
+                                    k.data_ptr(), v.data_ptr(), static_cast<int>(code), stream.stream());
+    });
     if (raised(status)) return nullptr;
     PyObject* out[3] = {THPVariable_Wrap(k), THPVariable_Wrap(v), THPVariable_Wrap(remapped)};
     PyObject* all = out[0] && out[1] && out[2] ? PyTuple_Pack(3, out[0], out[1], out[2]) : nullptr;
@@ -444,16 +455,31 @@ PyObject* gather(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     return all;
 }
 
+// The functions as Python calls them: an exception must not reach the interpreter's C frames, which end the process.
+template <auto F, typename... Args>
+PyObject* guarded(PyObject* self, Args... args) {
+    try {
+        return F(self, args...);
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());
+        return nullptr;
+    }
+}
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyCFunction several_arguments() {
+    return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<F, PyObject* const*, Py_ssize_t>));
+}
+
 PyMethodDef methods[] = {
-    {"bind", bind, METH_O, nullptr},
-    {"mark_valid", mark_valid, METH_O, nullptr},
-    {"forget", forget, METH_O, nullptr},
-    {"compress_store", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(compress_store)), METH_FASTCALL, nullptr},
-    {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(decode)), METH_FASTCALL, nullptr},
-    {"prefill", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(prefill)), METH_FASTCALL, nullptr},
-    {"compress", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(compress)), METH_FASTCALL, nullptr},
-    {"decompress", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(decompress)), METH_FASTCALL, nullptr},
-    {"gather", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(gather)), METH_FASTCALL, nullptr},
+    {"bind", guarded<bind, PyObject*>, METH_O, nullptr},
+    {"mark_valid", guarded<mark_valid, PyObject*>, METH_O, nullptr},
+    {"forget", guarded<forget, PyObject*>, METH_O, nullptr},
+    {"compress_store", several_arguments<compress_store>(), METH_FASTCALL, nullptr},
+    {"decode", several_arguments<decode>(), METH_FASTCALL, nullptr},
+    {"prefill", several_arguments<prefill>(), METH_FASTCALL, nullptr},
+    {"compress", several_arguments<compress>(), METH_FASTCALL, nullptr},
+    {"decompress", several_arguments<decompress>(), METH_FASTCALL, nullptr},
+    {"gather", several_arguments<gather>(), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
