@@ -110,7 +110,8 @@ template <int NB>
 __device__ __forceinline__ Guess make_guess(const float* __restrict__ bounds, int lane) {
     constexpr int kMid = NB / 2;
     Guess g;
-    g.bound = __ldg(bounds + min(lane, NB - 1));
+    // + 0: a boundary of -0 becomes +0, which compares alike; the sign of bound - v would be set for v = 0 otherwise
+    g.bound = __fadd_rn(__ldg(bounds + min(lane, NB - 1)), 0.0f);
     const float mid = __shfl_sync(0xffffffffu, g.bound, kMid);
     const int k = lane < NB ? lane - kMid : 0, n = k < 0 ? -k : k;
     const float dist = fabsf(g.bound - mid);

@@ -49,6 +49,26 @@ def test_cache_write_edges(tokens, heads, kind, bounds, bits, dtype):
     assert bool((got[untouched] == 0xAB).all())
 
 
+@pytest.mark.parametrize("tokens", [3, 300])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_a_boundary_of_minus_zero_is_zero(tokens, dtype):
+    """Values of +0 and -0 are not above a boundary of -0; zero rows have nothing else."""
+    p = gpu_util.params("iso_fast", 4, 4)
+    gen = torch.Generator().manual_seed(tokens)
+    x = torch.randn(tokens, 8, 128, generator=gen)
+    x[::2] = 0.0
+    x[::4, :, ::3] = -0.0
+    x = x.to(dtype)
+    bounds = p["k_boundaries"].clone()
+    bounds[7] = -0.0
+    cache = torch.zeros(tokens, 1, 2048, dtype=torch.uint8, device=DEV)
+    rq.compress_and_store(x.to(DEV), x.to(DEV), cache, torch.arange(tokens, device=DEV), p["R"].to(DEV), bounds.to(DEV),
+                          p["v_boundaries"].to(DEV))
+    want = rq_exact.build_slots(x.float().numpy(), x.float().numpy(), p["R"].numpy(), bounds.numpy(),
+                                p["v_boundaries"].numpy())
+    assert np.array_equal(cache.cpu().reshape(tokens, -1).numpy(), want)
+
+
 @pytest.mark.parametrize("blocks,bs,lens,width", [(31, 16, [5, 300], 20), (32, 16, [512], 32), (33, 8, [0, 264], 40),
                                                   (1, 1, [1, 1, 1], 1), (1500, 16, [5000, 4000, 1], 700)])
 @pytest.mark.parametrize("unused", [0, -1])
