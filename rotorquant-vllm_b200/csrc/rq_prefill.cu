@@ -817,7 +817,12 @@ prefill_attn_kernel(const PrefillParams p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = blockIdx.x % p.H;
     int seq, unit;
-    if (!find_unit(p, p.tokens_per_tile * TILES, blockIdx.x / p.H, seq, unit)) return;
+    if (!find_unit(p, p.tokens_per_tile * TILES, blockIdx.x / p.H, seq, unit)) {
+        // The next launch waits for the end of this grid and takes everything older as done: a grid whose CTAs all
+        // leave here (no sequence has a query) must not end before the records of its stage launch are written.
+        grid_dependency_wait();
+        return;
+    }
     const int q_begin = p.cu_seqlens_q ? __ldg(p.cu_seqlens_q + seq) : 0;
     const int q_end = p.cu_seqlens_q ? __ldg(p.cu_seqlens_q + seq + 1) : p.num_tokens;
     const int q_len = q_end - q_begin;

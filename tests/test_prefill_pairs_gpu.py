@@ -30,3 +30,19 @@ def test_unit_remainders(H, HQ, ctx, q, dtype, bound):
                         max_seq_len=bound).cpu()
     assert int(flag.item()) == 0, "a bounded device-side wait expired"
     base._check(out, c, cu)
+
+
+def test_a_batch_without_queries_does_not_disturb_the_next_one():
+    """Calls whose sequences have no query row still write scratch records; the call behind them uses the same
+    scratch.  (That the empty grid waits for its stage launch was shown by reading: the order is a matter of
+    microseconds.)"""
+    c, cu = base._fresh("iso_fast", 3, 3, 8, 32, [300, 900], [65, 161], 16, torch.bfloat16, 1)
+    g = on_gpu(c)
+    args = (g["kv_cache"], g["block_table"], g["seq_lens"], g["k_centroids"], g["v_centroids"], g["R"], 8, 128, 16)
+    cu = cu.to(g["q"].device)
+    want = base._prefill(g["q"], *args, cu_seqlens_q=cu, max_seq_len=1024)
+    out = torch.full_like(want, 7.0)
+    for _ in range(3):
+        base._prefill(g["q"], *args, cu_seqlens_q=torch.zeros_like(cu), max_seq_len=1024, out=out)
+        assert torch.equal(base._prefill(g["q"], *args, cu_seqlens_q=cu, max_seq_len=1024), want)
+    assert bool((out == 7.0).all())
