@@ -1064,7 +1064,10 @@ prefill_attn_kernel(const PrefillParams p) {
                         upk(y23, y[2], y[3]);
                         raw[i] = make_uint2(pf_pack<T>(y[0], y[1]), pf_pack<T>(y[2], y[3]));
                         const float2 c = pf_unpack<T>(raw[i].x), d = pf_unpack<T>(raw[i].y);
-                        const float m = fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y)));
+                        float m = fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y)));
+                        // A NaN element makes its whole rotation block NaN, which then counts as zero: its codes are 0
+                        // and the row's scale comes from the others.  (Next to an infinity the row's scale is 0.)
+                        if (!(m >= 0.0f)) { m = 0.0f; raw[i] = make_uint2(0u, 0u); }
                         const uint32_t m_row = __reduce_max_sync(0xffffffffu, __float_as_uint(m));   // non-negative floats order as integers
                         if (lane == i) mx = __uint_as_float(m_row);
                     }

@@ -46,3 +46,26 @@ def test_a_batch_without_queries_does_not_disturb_the_next_one():
         base._prefill(g["q"], *args, cu_seqlens_q=torch.zeros_like(cu), max_seq_len=1024, out=out)
         assert torch.equal(base._prefill(g["q"], *args, cu_seqlens_q=cu, max_seq_len=1024), want)
     assert bool((out == 7.0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bound", [1024, 16385])
+def test_queries_that_are_not_finite(dtype, bound):
+    """NaN and infinite query elements: the staged kernels give the bits of the fused one, and the other rows theirs."""
+    c, cu = base._fresh("iso_fast", 3, 4, 4, 28, [700, 90], [200, 40], 16, dtype, 2)
+    plain = c["q"].clone()
+    c["q"][3, 5, 7] = float("nan")
+    c["q"][50, 0, 0:4] = float("nan")
+    c["q"][60, 27] = float("nan")
+    c["q"][70, 9, 100] = float("inf")
+    c["q"][71, 9, 8:12] = float("-inf")
+    c["q"][210, 1, [3, 64]] = torch.tensor([float("inf"), float("nan")], dtype=dtype)
+    g = on_gpu(c)
+    args = (g["kv_cache"], g["block_table"], g["seq_lens"], g["k_centroids"], g["v_centroids"], g["R"], 4, 128, 16)
+    cu = cu.to(g["q"].device)
+    fused, staged, usual = (base._prefill(q, *args, cu_seqlens_q=cu, staged=s, max_seq_len=bound) for q, s in
+                            ((g["q"], False), (g["q"], True), (plain.to(g["q"].device), True)))
+    assert torch.equal(staged, fused)
+    same = torch.ones(plain.shape[:2], dtype=torch.bool)
+    same[[3, 50, 60, 70, 71, 210], [5, 0, 27, 9, 9, 1]] = False
+    assert torch.equal(staged[same.to(staged.device)], usual[same.to(staged.device)])
