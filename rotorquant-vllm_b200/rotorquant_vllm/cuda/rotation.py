@@ -47,8 +47,9 @@ def validate_rotation(rotation: torch.Tensor) -> None:
         entry = _VALIDATED.get(key)
         if entry is not None and entry[0] is _ref:
             del _VALIDATED[key]
-            host.forget(key)
+            native_forget(key)
 
     host = _lib.host()
+    native_forget = host.forget          # by itself: at interpreter exit the module's names may be gone
     host.mark_valid(rotation)
     _VALIDATED[key] = (weakref.ref(rotation, _forget), rotation._version)

@@ -54,6 +54,20 @@ def test_exceptions_are_python_exceptions(body):
     assert done.returncode == 0 and "refused" in done.stdout, (done.returncode, done.stdout, done.stderr[-2000:])
 
 
+def test_a_rotation_that_outlives_the_modules_is_silent():
+    """A validated matrix that dies at interpreter exit, after the native module was cleared."""
+    done = _run("""
+        import functools
+        @functools.lru_cache(None)
+        def layer():
+            r = torch.eye(128)
+            rq.validate_rotation(r)
+            return {"rotation": r}
+        layer()
+    """)
+    assert done.returncode == 0 and "_forget" not in done.stderr, done.stderr[-2000:]
+
+
 @pytest.mark.gpu
 def test_no_memory_for_the_result():
     done = _run("""
