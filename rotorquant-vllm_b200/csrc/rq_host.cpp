@@ -94,9 +94,11 @@ int dtype_code(at::ScalarType t) {
 
 bool f32_vector(const at::Tensor& t) { return t.scalar_type() == at::kFloat && t.is_contiguous(); }
 
+// The object has been validated, and still is what the kernels read (the object may have been given other data).
 bool rotation_ok(PyObject* o, const at::Tensor& t) {
     const auto it = validated().find(o);
-    return it != validated().end() && it->second == t._version() && t.is_cuda();
+    return it != validated().end() && it->second == t._version() && t.is_cuda() && f32_vector(t) && t.dim() == 2 &&
+           t.size(0) == 128 && t.size(1) == 128;
 }
 
 // Rows of head-dim elements that may be read with 16-byte loads.

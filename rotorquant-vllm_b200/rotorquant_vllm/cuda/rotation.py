@@ -29,14 +29,16 @@ def validate_rotation(rotation: torch.Tensor) -> None:
     touch the device, so they are legal inside a CUDA graph capture.
     """
     global validations
-    key = id(rotation)
-    hit = _VALIDATED.get(key)
-    if hit is not None and hit[0]() is rotation and hit[1] == rotation._version:
-        return
+    # what the kernels read of the tensor's memory is looked at in every call: giving the object other data
+    # (``rotation.data = ...``) leaves its version as it was
     if rotation.dtype != torch.float32 or tuple(rotation.shape) != (128, 128):
         raise ValueError(f"rotation must be fp32 (128, 128), got {rotation.dtype} {tuple(rotation.shape)}")
     if not rotation.is_contiguous():
         raise ValueError("rotation must be contiguous")
+    key = id(rotation)
+    hit = _VALIDATED.get(key)
+    if hit is not None and hit[0]() is rotation and hit[1] == rotation._version:
+        return
     validations += 1
     r = rotation.detach().to("cpu")
     blocks = torch.block_diag(*[torch.ones(4, 4) for _ in range(32)]).bool()

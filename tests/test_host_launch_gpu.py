@@ -51,6 +51,19 @@ def test_a_rotation_changed_in_place_is_checked_again():
         rq.compress_and_store(*args)
 
 
+@pytest.mark.parametrize("other", [lambda r: r[:64, :64].contiguous(), lambda r: r.double(), lambda r: r[:, ::2]])
+def test_a_validated_rotation_that_was_given_other_data_is_refused(other):
+    """Such an assignment does not change the version of the tensor."""
+    p = _layer()
+    x = torch.randn(5, 8, 128, device=DEV)
+    cache = torch.zeros(5, 1, 2048, dtype=torch.uint8, device=DEV)
+    args = (x, x, cache, torch.arange(5, device=DEV), p["R"], p["k_boundaries"], p["v_boundaries"])
+    rq.compress_and_store(*args)
+    p["R"].data = other(p["R"].clone())
+    with pytest.raises(ValueError, match="rotation must be"):
+        rq.compress_and_store(*args)
+
+
 def test_errors_of_the_library_keep_their_types():
     p = _layer()
     q = torch.randn(1, 8, 128, device=DEV)                      # fp32 queries are not supported
