@@ -837,7 +837,8 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
 #pragma unroll
             for (int h = 1; h < NH; ++h) m = tid == h ? m_ref[h] : m;
             const float l = (sm.red[0][tid] + sm.red[1][tid]) + (sm.red[2][tid] + sm.red[3][tid]);
-            p.ws_m[row * kHeadsPerCta + tid] = m;
+            // (a finite maximum with the NaN sum: the merge passes over parts whose maximum is -inf)
+            p.ws_m[row * kHeadsPerCta + tid] = dead ? 0.0f : m;
             p.ws_l[row * kHeadsPerCta + tid] = dead ? __int_as_float(0x7fc00000) : l;
         }
         if (!dead) {
