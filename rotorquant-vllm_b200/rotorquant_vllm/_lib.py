@@ -8,7 +8,10 @@ been built (``python rotorquant-vllm_b200/csrc/build.py``).
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
+import sys
 
 import torch
 
@@ -78,20 +81,28 @@ def lib() -> C.CDLL:
     return _LIB
 
 
+def host_path() -> str:
+    """The native side of the launchers for this interpreter and torch; another torch has another file."""
+    return os.path.join(os.path.dirname(os.path.abspath(__file__)),
+                        f"_host-{sys.implementation.cache_tag}-torch{torch.__version__}.so")
+
+
 def host():
-    """The native side of the launchers (``_host.so``), bound to the loaded library; raises
-    ``RuntimeError`` when it has not been built."""
+    """The native side of the launchers, bound to the loaded library; raises ``RuntimeError`` when it has
+    not been built against this torch."""
     global _HOST
     if _HOST is None:
         handle = lib()
+        name, path = __package__ + "._host", host_path()
         try:
-            from . import _host
+            spec = importlib.util.spec_from_loader(name, importlib.machinery.ExtensionFileLoader(name, path))
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
         except ImportError as exc:
             raise RuntimeError(
-                f"rotorquant_vllm/_host.so cannot be loaded ({exc}): build it with "
-                "`python rotorquant-vllm_b200/csrc/build.py`.") from exc
-        _host.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in _SIGNATURES})
-        _HOST = _host
+                f"{path} cannot be loaded ({exc}): build it with `python rotorquant-vllm_b200/csrc/build.py`.") from exc
+        module.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in _SIGNATURES})
+        _HOST = module
     return _HOST
 
 

@@ -68,6 +68,27 @@ def test_a_rotation_that_outlives_the_modules_is_silent():
     assert done.returncode == 0 and "_forget" not in done.stderr, done.stderr[-2000:]
 
 
+def test_another_torch_wants_another_module(monkeypatch):
+    """The native side is built against one torch: with another installed it is missing, and the build makes it."""
+    import importlib.util
+    import os
+
+    import torch
+
+    from rotorquant_vllm import _lib
+
+    path = os.path.join(os.path.dirname(os.path.dirname(GOLDEN)), "rotorquant-vllm_b200", "csrc", "build.py")
+    spec = importlib.util.spec_from_file_location("rq_build", path)
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    assert _lib.host_path() == build.host_library() and os.path.exists(_lib.host_path())
+    monkeypatch.setattr(torch, "__version__", "0.1.0")
+    monkeypatch.setattr(_lib, "_HOST", None)
+    assert _lib.host_path() == build.host_library() and build._stale(build.host_library())
+    with pytest.raises(RuntimeError, match="build it with"):
+        _lib.host()
+
+
 @pytest.mark.gpu
 def test_no_memory_for_the_result():
     done = _run("""

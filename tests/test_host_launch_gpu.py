@@ -1,4 +1,4 @@
-"""The launchers' native side (``_host.so``) takes ordinary calls; everything else goes through the
+"""The launchers' native side (``_host-*.so``) takes ordinary calls; everything else goes through the
 Python path.  Both must give the same bytes, and the native side must not take what it may not."""
 
 import pytest
