@@ -43,6 +43,9 @@ inline int ensure_smem(Kernel k, size_t bytes) {
     return ensure_smem_impl(reinterpret_cast<const void*>(k), bytes);
 }
 
+// SM count of the current device (148 on a B200), looked up once per device.
+int sm_count();
+
 // Launch with programmatic stream serialization: the kernel may be scheduled while the one before it on the stream
 // drains, as soon as all of that kernel's CTAs have ended or called grid_launch_dependents().  It must not touch
 // memory that earlier kernels write (or read, if it writes it) before grid_dependency_wait() returns.

@@ -577,7 +577,6 @@ static int shift_of(int64_t n) {
 // (K and V rows of the store variant) or 1.
 template <typename T, bool STORE>
 static void launch_walk(CompressParams& p, int kinds, cudaStream_t st) {
-    const int sms = 148;
     const bool wide = p.rows >= static_cast<uint32_t>(kWideFrom / kinds);
     p.dense = 1;
     for (int kv = 0; kv < kinds; ++kv) {
@@ -587,7 +586,7 @@ static void launch_walk(CompressParams& p, int kinds, cudaStream_t st) {
             p.dense = 0;
     }
     const uint32_t per_cta = kCompressWarps * (wide ? 8 : 2);
-    const uint32_t want = (p.rows + per_cta - 1) / per_cta, most = 2 * sms / kinds;
+    const uint32_t want = (p.rows + per_cta - 1) / per_cta, most = 2 * sm_count() / kinds;
     const dim3 grid(want < most ? want : most, kinds);
     if (wide) compress_kernel<T, 8, STORE><<<grid, kCompressThreads, 0, st>>>(p);
     else compress_kernel<T, 2, STORE><<<grid, kCompressThreads, 0, st>>>(p);

@@ -1043,21 +1043,6 @@ static int env_int(const char* name, int fallback) {
     return (e != nullptr && e[0] != '\0') ? std::atoi(e) : fallback;
 }
 
-// SM count of the current device (148 on a B200), looked up once per device.
-static int sm_count() {
-    static std::mutex mu;
-    static int cached[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    std::lock_guard<std::mutex> lock(mu);
-    if (cached[dev] == 0) {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        cached[dev] = n;
-    }
-    return cached[dev];
-}
-
 // Grid and scratch of one decode call.  The (sequence, tile) space is cut into `groups` pieces and
 // each piece is walked by J CTAs, one per (KV head, group of 8 query heads).
 struct DecodePlan {

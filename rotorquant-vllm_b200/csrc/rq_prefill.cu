@@ -37,7 +37,6 @@ namespace rq {
 constexpr int kPfThreads = 256;       // two threads per row / key
 constexpr int kPfRows = 128;          // MMA M
 constexpr int kPfKeys = 128;          // keys per tile (MMA N of S, K extent of P V)
-constexpr int kSms = 148;
 constexpr uint32_t kTmemCols = 256;   // S: columns 0..127 (int32), O: columns 128..255 (fp32)
 
 struct PrefillParams {
@@ -1314,7 +1313,7 @@ static int launch_prefill(const PrefillParams& p, int m_tiles, int num_seqs, cud
             return launch_dependent("rq_prefill_int8 attention launch", prefill_attn_kernel<T, kTiles>,
                                     dim3(static_cast<unsigned>(units(1LL * p.tokens_per_tile * kTiles))), dim3(kAttnThreads<kTiles>), smem, st, p);
         };
-        const bool one = p.stage_tiles_per_seq <= 16384 / kPfKeys || units(p.tokens_per_tile) <= kSms ||
+        const bool one = p.stage_tiles_per_seq <= 16384 / kPfKeys || units(p.tokens_per_tile) <= sm_count() ||
                          p.num_tokens <= 1LL * num_seqs * p.tokens_per_tile;
         return one ? attend(std::integral_constant<int, 1>{}) : attend(std::integral_constant<int, 2>{});
     }
