@@ -92,53 +92,11 @@ __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddep
 
 // ---- device helpers --------------------------------------------------------
 
-__device__ __forceinline__ float to_f32(float v) { return v; }
-__device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }
-__device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
-
-// fp32 value of element i of a 16-byte chunk holding `T` elements.
-template <typename T>
-struct Chunk16;
-template <>
-struct Chunk16<float> {
-    static constexpr int kElems = 4;
-    __device__ static void unpack(const uint4& c, float* out) {
-        out[0] = __uint_as_float(c.x); out[1] = __uint_as_float(c.y);
-        out[2] = __uint_as_float(c.z); out[3] = __uint_as_float(c.w);
-    }
-};
-template <>
-struct Chunk16<__half> {
-    static constexpr int kElems = 8;
-    __device__ static void unpack(const uint4& c, float* out) {
-        const uint32_t w[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            __half2 h = *reinterpret_cast<const __half2*>(&w[i]);
-            float2 f = __half22float2(h);
-            out[2 * i] = f.x; out[2 * i + 1] = f.y;
-        }
-    }
-};
-template <>
-struct Chunk16<__nv_bfloat16> {
-    static constexpr int kElems = 8;
-    __device__ static void unpack(const uint4& c, float* out) {
-        const uint32_t w[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {  // bf16 -> fp32 is a 16-bit shift
-            out[2 * i] = __uint_as_float(w[i] << 16);
-            out[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-        }
-    }
-};
-
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     uint32_t d;
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
     return d;
 }
-
 
 // Pairs of fp32 values in one 64-bit register.  A packed operation takes the pipe as long as two scalar ones but
 // one issue slot instead of two.  The assembler may contract a packed product and a packed sum into one operation.
@@ -157,7 +115,6 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
     return d;
 }
 
-
 // ---- mbarrier (shared-memory barrier objects) -----------------------------------------------
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -171,16 +128,6 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 // Wait until the phase with the given parity has completed.  Every wait in this library is
 // bounded (about one second of SM clocks); false means the bound expired.
-// One non-blocking look: has the phase with the given parity completed?
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return done != 0;
-}
 constexpr long long kWaitCycles = 2000000000LL;
 __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, long long limit_cycles) {
     const uint32_t addr = smem_u32(bar);

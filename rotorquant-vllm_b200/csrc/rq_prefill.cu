@@ -904,20 +904,20 @@ prefill_attn_kernel(const PrefillParams p) {
                     mbar_wait(&sm.scale_full[(k_next - 1) & 1], static_cast<uint32_t>((k_next - 1) / 2) & 1u);
                 }
             } else {
-            int issued = 0;
-            for (; issued < n_all; ++issued, rec += record_stride) {
-                const int s = issued % kAttnStages;
-                if (issued >= kAttnStages) failed = !mbar_wait(&sm.empty[s], static_cast<uint32_t>(issued / kAttnStages - 1) & 1u);
-                if (failed) break;
-                const uint32_t bar = smem_u32(&sm.full[s]);
-                mbar_expect_tx(bar, kStageRecord);
-                bulk_load(smem_u32(sm.k[s]), rec, kPfKeys * kHeadDim, bar);
-                bulk_load(smem_u32(sm.v[s]), rec + kPfKeys * kHeadDim, 2 * kPfKeys * kHeadDim, bar);
-                bulk_load(smem_u32(sm.k_scale[s]), rec + 3 * kPfKeys * kHeadDim, kPfKeys * 4, bar);
-            }
-            if (failed)                                       // copies in flight land before the CTA ends
-                for (int j = max(0, issued - kAttnStages); j < issued; ++j)
-                    mbar_wait(&sm.full[j % kAttnStages], static_cast<uint32_t>(j / kAttnStages) & 1u);
+                int issued = 0;
+                for (; issued < n_all; ++issued, rec += record_stride) {
+                    const int s = issued % kAttnStages;
+                    if (issued >= kAttnStages) failed = !mbar_wait(&sm.empty[s], static_cast<uint32_t>(issued / kAttnStages - 1) & 1u);
+                    if (failed) break;
+                    const uint32_t bar = smem_u32(&sm.full[s]);
+                    mbar_expect_tx(bar, kStageRecord);
+                    bulk_load(smem_u32(sm.k[s]), rec, kPfKeys * kHeadDim, bar);
+                    bulk_load(smem_u32(sm.v[s]), rec + kPfKeys * kHeadDim, 2 * kPfKeys * kHeadDim, bar);
+                    bulk_load(smem_u32(sm.k_scale[s]), rec + 3 * kPfKeys * kHeadDim, kPfKeys * 4, bar);
+                }
+                if (failed)                                   // copies in flight land before the CTA ends
+                    for (int j = max(0, issued - kAttnStages); j < issued; ++j)
+                        mbar_wait(&sm.full[j % kAttnStages], static_cast<uint32_t>(j / kAttnStages) & 1u);
             }
         }
         __syncwarp();
@@ -964,34 +964,34 @@ prefill_attn_kernel(const PrefillParams p) {
                     tc_commit(&sm.s_ready[0]);
                 }
             } else {
-            failed |= !mbar_wait(&sm.full[0], 0);
-            if (!failed) {
-                tc_fence_after();
-                if (n0 > 0) { scores(0, 0); tc_commit(&sm.s_ready[0]); }
-                if (n1 > 0) { scores(1, 0); tc_commit(&sm.s_ready[1]); }
-            }
-            // tile j: PV_x(j), then S_x(j + 1); the commit is there without an S, too
-            auto step = [&](auto unrolled, int j, uint32_t phase) {
-                constexpr int stage = decltype(unrolled)::value, next = (stage + 1) % kAttnStages;
-                if (j + 1 < n_all && !failed) failed |= !mbar_wait(&sm.full[next], next == 0 ? phase ^ 1u : phase);
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    const int nx = x == 0 ? n0 : n1;
-                    if (j >= nx || failed) continue;
-                    failed |= !mbar_wait(&sm.p_ready[x], static_cast<uint32_t>(j) & 1u);
-                    if (failed) continue;
+                failed |= !mbar_wait(&sm.full[0], 0);
+                if (!failed) {
                     tc_fence_after();
-                    values(x, stage, j);
-                    if (j + 1 < nx) scores(x, next);
-                    tc_commit(&sm.s_ready[x]);
+                    if (n0 > 0) { scores(0, 0); tc_commit(&sm.s_ready[0]); }
+                    if (n1 > 0) { scores(1, 0); tc_commit(&sm.s_ready[1]); }
                 }
-            };
-            uint32_t phase = 0;
-            for (int j = 0; j < n_all && !failed; j += kAttnStages, phase ^= 1u) {
-                step(std::integral_constant<int, 0>{}, j, phase);
-                step(std::integral_constant<int, 1>{}, j + 1, phase);
-                step(std::integral_constant<int, 2>{}, j + 2, phase);
-            }
+                // tile j: PV_x(j), then S_x(j + 1); the commit is there without an S, too
+                auto step = [&](auto unrolled, int j, uint32_t phase) {
+                    constexpr int stage = decltype(unrolled)::value, next = (stage + 1) % kAttnStages;
+                    if (j + 1 < n_all && !failed) failed |= !mbar_wait(&sm.full[next], next == 0 ? phase ^ 1u : phase);
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        const int nx = x == 0 ? n0 : n1;
+                        if (j >= nx || failed) continue;
+                        failed |= !mbar_wait(&sm.p_ready[x], static_cast<uint32_t>(j) & 1u);
+                        if (failed) continue;
+                        tc_fence_after();
+                        values(x, stage, j);
+                        if (j + 1 < nx) scores(x, next);
+                        tc_commit(&sm.s_ready[x]);
+                    }
+                };
+                uint32_t phase = 0;
+                for (int j = 0; j < n_all && !failed; j += kAttnStages, phase ^= 1u) {
+                    step(std::integral_constant<int, 0>{}, j, phase);
+                    step(std::integral_constant<int, 1>{}, j + 1, phase);
+                    step(std::integral_constant<int, 2>{}, j + 2, phase);
+                }
             }
             if (failed) {                                     // what was issued ends before TMEM is freed
                 tc_commit(&sm.drained);
