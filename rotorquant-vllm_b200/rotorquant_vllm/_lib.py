@@ -54,6 +54,8 @@ _SIGNATURES = {
                                     _L, _P, _P, _I, _P, _I, _P, _F, _P, _I, _P, _Z, _P]),
 }
 
+_OPTIONAL: dict = {}
+
 
 def library_path() -> str:
     return _PATH
@@ -71,6 +73,10 @@ def lib() -> C.CDLL:
         for name, (res, args) in _SIGNATURES.items():
             fn = getattr(handle, name)
             fn.restype, fn.argtypes = res, args
+        for name, (res, args) in _OPTIONAL.items():
+            if hasattr(handle, name):
+                fn = getattr(handle, name)
+                fn.restype, fn.argtypes = res, args
         _LIB = handle
     return _LIB
 
