@@ -150,9 +150,11 @@ struct __align__(16) CompressSmem {
 // divisions of this one.
 //
 // Division.  q = x / d with r = RN(1 / d): q0 = RN(x r), rem = RN(x - q0 d), q = RN(q0 + rem r) (Markstein's
-// correction step).  That this equals the division instruction was checked for ALL 2^46 pairs of 24-bit
-// significands; exponents do not matter while nothing comes near the subnormal range, which the bounds below
-// ensure (d in 2^-40 .. 2^30, |x| >= 2^-90: q >= 2^-120, rem a multiple of 2^-138).  The bound on x is checked on
+// correction step).  It equals the IEEE quotient for all pairs of significands: the value before the last rounding is so near
+// to x / d that only quotients next to a midpoint of two floats could round another way, and all of those were tried
+// (tests/test_compress_division.py does, and has the bounds; Markstein's theorem itself asks for a q0 within one unit, and
+// q0 is within one and a half where x < d).  Exponents do not matter while nothing comes near the subnormal range, which the
+// bounds below ensure (d in 2^-40 .. 2^30, |x| >= 2^-90: q >= 2^-120, rem a multiple of 2^-138).  The bound on x is checked on
 // products of two elements: both are at most d.  A step with a row outside of the bounds, or with a zero element,
 // takes the division instruction.  fp16 inputs cannot be below 2^-24.
 //

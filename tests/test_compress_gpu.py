@@ -174,15 +174,15 @@ def test_full_size_prefill_compress_properties():
 
 
 def test_large_launch_divisions_equal_the_ieee_quotients_on_extreme_rows():
-    """The large-launch mapping forms x / (norm + 1e-10) through double precision where the quotient is a
-    normal number and with the division instruction next to the subnormal range.  Rows built to hit both
+    """Steps of ordinary rows divide by reciprocal and correction; a step with a row next to the subnormal range,
+    outside of the normal one, or with a zero element takes the division instruction.  Rows built to hit both
     sides: one huge element beside tiny ones (quotients of 1e-38 .. 1e-45 and exact zeros), whole rows of
     tiny or huge magnitude, all-zero rows (denominator 1e-10), and ordinary rows; every byte and norm must equal
-    the exact-arithmetic oracle on a sample, and the small-launch kernel (other mapping, plain divisions)
-    must give the same bytes for the same tokens."""
+    the exact-arithmetic oracle on a sample, and small launches (two rows per step of a warp instead of
+    eight) must give the same bytes for the same tokens."""
     p = gpu_util.params("iso_fast", 3, 3)
     gen = torch.Generator(device=DEV).manual_seed(7)
-    N, H = 4096, 8                                    # 32768 rows per kind: the large-launch mapping
+    N, H = 4096, 8                                    # 32768 rows per kind: eight rows per step
     key = torch.randn(N, H, 128, generator=gen, device=DEV)
     value = torch.randn(N, H, 128, generator=gen, device=DEV)
     key[0::8] *= 1e-30
@@ -205,8 +205,29 @@ def test_large_launch_divisions_equal_the_ieee_quotients_on_extreme_rows():
     rows = rq_exact.build_slots(key[sample].float().cpu().numpy(), value[sample].float().cpu().numpy(),
                                 p["R"].numpy(), p["k_boundaries"].numpy(), p["v_boundaries"].numpy())
     assert np.array_equal(flat[slots[sample]].cpu().numpy(), rows)
-    # the same tokens in launches of 256 tokens (2048 rows per kind: the small-launch mapping)
+    # the same tokens in launches of 128 tokens (1024 rows per kind: two rows per step)
     small = torch.zeros_like(big)
-    for lo in range(0, N, 256):
-        _cuda().compress_and_store(key[lo:lo + 256], value[lo:lo + 256], small, slots[lo:lo + 256], *args)
+    for lo in range(0, N, 128):
+        _cuda().compress_and_store(key[lo:lo + 128], value[lo:lo + 128], small, slots[lo:lo + 128], *args)
     assert torch.equal(big, small)
+
+
+def test_rows_beside_a_zero_element_have_the_same_bytes():
+    """A zero element sends the rows of its step (here a token's eight heads) to the division instruction: the other
+    seven must not change."""
+    p = gpu_util.params("iso_full", 4, 3)
+    gen = torch.Generator(device=DEV).manual_seed(8)
+    N, H = 8192, 8
+    key, value = (torch.randn(N, H, 128, generator=gen, device=DEV).to(torch.bfloat16) for _ in range(2))
+    key[key == 0], value[value == 0] = 1.0, 1.0
+    slots = torch.arange(N, device=DEV)
+    args = (p["R"].to(DEV), p["k_boundaries"].to(DEV), p["v_boundaries"].to(DEV))
+    corrected, divided = (torch.zeros(N, 1, 2048, dtype=torch.uint8, device=DEV) for _ in range(2))
+    _cuda().compress_and_store(key, value, corrected, slots, *args)
+    key[:, 3, 17], value[:, 3, 99] = 0.0, 0.0
+    _cuda().compress_and_store(key, value, divided, slots, *args)
+    others = [0, 1, 2, 4, 5, 6, 7]
+    for first in (0, 544):                            # K and V index bytes of a slot
+        a, b = (c[:, 0, first:first + 512].reshape(N, H, 64) for c in (corrected, divided))
+        assert torch.equal(a[:, others], b[:, others])
+        assert not torch.equal(a[:, 3], b[:, 3])
