@@ -11,7 +11,8 @@ Parity status: unpinned against the reference (nothing in the reference computes
 pinned to the kernel's documented arithmetic only.
 
 Scheme, per (sequence, KV head), queries and keys in rotated space:
-  q_rot       = round_T(q @ R^T)
+  q_rot       = round_T(q @ R^T), the products of a 4x4 block as one chain of fused multiply-adds, ascending (another
+                order moves a query that lies on a rounding boundary by a unit of T, and its code with it)
   q_i8[m]     = rint(q_rot[m] * (127 / max|q_rot[m]|)),       q_scale[m] = max|q_rot[m]| / 127
   table[t][i] = round_T(centroid_k[i] * norm_k[t]);  code[t][i] = rint(table * (127 / max_i|table|))
   k_i8[t][d]  = code[t][idx[t][d]],                           k_scale[t] = max_i|table[t][i]| / 127
@@ -28,7 +29,7 @@ import math
 
 import torch
 
-from . import rq_oracle
+from . import rq_exact, rq_oracle
 
 TILE = 128
 
@@ -39,7 +40,12 @@ def _f32(x):
 
 def prefill_int8(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v, rotation,
                  num_kv_heads, head_dim, block_size, sm_scale=None, cu_seqlens_q=None,
-                 return_rotated_fp32=False):
+                 return_rotated_fp32=False, return_flip=False):
+    """``return_flip``: instead of the output, how far it moves when ONE probability rounds the other way:
+    max over the keys of (its weight) x (its value in original space) x (the largest unit of T relative to a
+    value: 2^-7 for bf16, 2^-10 for fp16).  Kernel and restatement round the same probabilities, but compute
+    them with relative differences of about 1e-6 (fused scaling, the GPU's exp2), so one that lies that near to a
+    rounding boundary may go either way: one in some thousand does, and in rows with few keys it shows."""
     t_all, hq, d = q.shape
     g = hq // num_kv_heads
     dtype = q.dtype
@@ -48,8 +54,10 @@ def prefill_int8(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v, r
     qk_scale = _f32(sm_scale) * _f32(1.4426950408889634)
     cu = [0, t_all] if cu_seqlens_q is None else [int(x) for x in cu_seqlens_q]
     rot = rotation.to(torch.float32)
-    q_rot = (q.to(torch.float32) @ rot.T).to(dtype).to(torch.float32)
+    q_rot = rq_exact.rotate_rows(q.to(torch.float32).reshape(-1, d).numpy(), rq_exact.rotation_blocks(rot.numpy()), transpose=True)
+    q_rot = torch.from_numpy(q_rot).reshape(q.shape).to(dtype).to(torch.float32)
     o_rot = torch.zeros(t_all, hq, d, dtype=torch.float32)
+    flip = torch.zeros_like(o_rot)
     ck = centroids_k.to(torch.float32)
     c127 = _f32(127.0)
 
@@ -87,6 +95,7 @@ def prefill_int8(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v, r
             m_run = torch.full((tq, g), float("-inf"))
             l_run = torch.zeros(tq, g)
             acc = torch.zeros(tq, g, d)
+            scores = []
             for j in range((n + TILE - 1) // TILE):
                 k0, k1 = j * TILE, min(n, (j + 1) * TILE)
                 dots = torch.einsum("tgd,kd->tgk", q_i8, k_i8[k0:k1, h])                    # exact integers
@@ -94,6 +103,8 @@ def prefill_int8(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v, r
                 allowed = (torch.arange(k0, k1).view(1, 1, -1) <= pos.view(-1, 1, 1))
                 sk_max = torch.where(allowed, sk, torch.full_like(sk, float("-inf"))).amax(-1)
                 sc = torch.where(allowed, sk * row_factor.unsqueeze(-1), torch.full_like(sk, float("-inf")))
+                if return_flip:
+                    scores.append(sc)
                 # lazy reference: it moves only when the tile maximum exceeds it by more than 2^8
                 m_tile = sk_max * row_factor
                 grew = m_tile > m_run + 8.0
@@ -107,7 +118,14 @@ def prefill_int8(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v, r
                 acc = acc * alpha.unsqueeze(-1) + torch.einsum("tgk,kd->tgd", p, v_all[k0:k1, h])
                 m_run = m_new
             inv_l = torch.where(l_run > 0, 1.0 / l_run, torch.zeros_like(l_run))
+            if return_flip:
+                v_orig = (v_all[:, h] @ rot).abs()
+                weight = torch.exp2(torch.cat(scores, -1) - torch.nan_to_num(m_run, neginf=0.0).unsqueeze(-1)) * inv_l.unsqueeze(-1)
+                for t in range(tq):
+                    flip[lo + t, h * g:(h + 1) * g] = (weight[t].unsqueeze(-1) * v_orig).amax(1)
             o_rot[lo:hi, h * g:(h + 1) * g] = acc * inv_l.unsqueeze(-1)
+    if return_flip:
+        return flip * (2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10)
     if return_rotated_fp32:
         return o_rot
     return (o_rot.to(dtype).to(torch.float32) @ rot).to(dtype)
