@@ -92,7 +92,7 @@ def fused_paged_rq_decode(
     assert kv_cache.dtype == torch.uint8
     assert block_table.dtype == torch.int32
     assert seq_lens.dtype == torch.int32
-    dev = _lib.require_cuda(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v, rotation, out)
+    dev = _lib.require_cuda(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v, rotation, out, workspace)
     validate_rotation(rotation)
     if kv_cache.dim() != 3 or kv_cache.shape[1] != block_size or not kv_cache.is_contiguous():
         raise ValueError("kv_cache must be contiguous (num_blocks, block_size, total_bytes)")

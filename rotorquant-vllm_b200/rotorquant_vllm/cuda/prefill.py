@@ -69,7 +69,7 @@ def fused_paged_rq_int8_prefill(
             "fused_paged_rq_int8_prefill supports only a single sequence without cu_seqlens_q, "
             f"but got seq_lens.numel() == {seq_lens.numel()}.")
     dev = _lib.require_cuda(q, kv_cache, block_table, seq_lens, k_centroids, v_centroids, rotation,
-                            out, cu_seqlens_q, error_flag)
+                            out, cu_seqlens_q, error_flag, workspace)
     validate_rotation(rotation)
     num_seqs = seq_lens.numel()
     if kv_cache.dim() != 3 or kv_cache.shape[1] != block_size or not kv_cache.is_contiguous():
@@ -112,10 +112,8 @@ def fused_paged_rq_int8_prefill(
         if staged:
             if workspace is None:
                 workspace = _scratch(dev, need)
-            else:
-                _lib.require_cuda(workspace)
-                if workspace.dtype != torch.uint8 or not workspace.is_contiguous():
-                    raise ValueError("workspace must be a contiguous uint8 tensor")
+            elif workspace.dtype != torch.uint8 or not workspace.is_contiguous():
+                raise ValueError("workspace must be a contiguous uint8 tensor")
             _lib.check(lib.rq_prefill_int8_staged(*common, bound, workspace.data_ptr(), workspace.numel(),
                                                    _lib.stream_ptr(dev)))
         else:

@@ -73,3 +73,14 @@ def test_errors_of_the_library_keep_their_types():
         with pytest.raises(ValueError, match="dtype"):
             rq.fused_paged_rq_decode(q, cache, table, lens, p["k_centroids"], p["v_centroids"], p["R"], 1, 128, 16)
         rq.fused_paged_rq_decode(q.half(), cache, table, lens, p["k_centroids"], p["v_centroids"], p["R"], 1, 128, 16)
+
+
+def test_scratch_must_be_on_the_device_of_the_call():
+    p = _layer()
+    q = torch.randn(1, 8, 128, device=DEV).half()
+    cache = torch.zeros(4, 16, 256, dtype=torch.uint8, device=DEV)
+    table, lens = torch.zeros(1, 4, dtype=torch.int32, device=DEV), torch.ones(1, dtype=torch.int32, device=DEV)
+    args = (q, cache, table, lens, p["k_centroids"], p["v_centroids"], p["R"], 1, 128, 16)
+    for call in (rq.fused_paged_rq_decode, rq.fused_paged_rq_int8_prefill):
+        with pytest.raises(RuntimeError, match="CUDA tensors only"):
+            call(*args, workspace=torch.empty(1 << 22, dtype=torch.uint8))
