@@ -69,7 +69,7 @@ def fused_paged_rq_int8_prefill(
             "fused_paged_rq_int8_prefill supports only a single sequence without cu_seqlens_q, "
             f"but got seq_lens.numel() == {seq_lens.numel()}.")
     dev = _lib.require_cuda(q, kv_cache, block_table, seq_lens, k_centroids, v_centroids, rotation,
-                            out, cu_seqlens_q, error_flag, workspace)
+                            out, cu_seqlens_q, error_flag, workspace if staged is not False else None)
     validate_rotation(rotation)
     num_seqs = seq_lens.numel()
     if kv_cache.dim() != 3 or kv_cache.shape[1] != block_size or not kv_cache.is_contiguous():
