@@ -78,8 +78,9 @@ def decompress_cache_paged(kv_cache: torch.Tensor, block_table: torch.Tensor, se
     ``(key_cache, value_cache, remapped_block_table)`` with K/V ``(num_unique, block_size, H, 128)``
     and the table renumbered into that compact block space.  The number of blocks sizes the result,
     so the host waits for it once, as upstream's ``torch.unique`` does; the union of the blocks is one
-    launch and the gather, the per-head split and both decompressions are another.  Tables the union
-    kernel does not take (entries outside the cache, more than 2**20 entries) go through torch."""
+    launch and the gather, the per-head split and both decompressions are another.  What the union
+    kernel does not take (negative entries, more than 2**20 entries, more than 2**19 cache blocks) goes through torch;
+    an entry outside the cache that a sequence needs is a ``ValueError``."""
     done = _lib.host().gather(kv_cache, block_table, seq_lens, num_kv_heads, centroids_k, centroids_v,
                               _lib.DTYPE_CODE.get(dtype, -1))
     if done is not None:
@@ -88,8 +89,12 @@ def decompress_cache_paged(kv_cache: torch.Tensor, block_table: torch.Tensor, se
     need = (seq_lens.to(torch.int64) + bs - 1) // bs
     cols = torch.arange(block_table.shape[1], device=block_table.device).unsqueeze(0)
     unique_blocks = torch.unique(block_table[cols < need.unsqueeze(1)], sorted=True).to(torch.int32)
+    if unique_blocks.numel() and (int(unique_blocks[0]) < -nb or int(unique_blocks[-1]) >= nb):
+        raise ValueError(f"block_table refers to block {int(unique_blocks[0])} or {int(unique_blocks[-1])} of a cache of {nb} blocks")
     k, v = decompress_blocks(kv_cache, unique_blocks, num_kv_heads, centroids_k, centroids_v, dtype)
     remap = torch.zeros(nb, dtype=block_table.dtype, device=block_table.device)
     remap[unique_blocks.long()] = torch.arange(unique_blocks.numel(), dtype=block_table.dtype,
                                                device=block_table.device)
-    return k, v, remap[block_table.long()]
+    table = block_table.long()
+    inside = (table >= -nb) & (table < nb)                  # entries that no sequence reaches may be anything
+    return k, v, remap[torch.where(inside, table, 0)] * inside.to(remap.dtype)

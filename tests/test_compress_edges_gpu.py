@@ -98,3 +98,18 @@ def test_referenced_blocks_are_listed_once_in_order(blocks, bs, lens, width, unu
         idx = torch.stack([rows[:, 136:264] >> 4, rows[:, 136:264] & 15], -1).view(-1, 2, 128).long()
         norm = rows[:, 264:272].contiguous().view(torch.float32).view(-1, 2, 1)
         assert torch.equal(v.cpu().view(-1, 2, 128), (p["v_centroids"].cpu()[idx] * norm).to(dtype))
+
+
+@pytest.mark.parametrize("tables", ["plain", "many"])        # "many" entries: the way through torch
+def test_blocks_outside_the_cache(tables):
+    """Needed entries outside the cache are an error of the host; entries that no sequence reaches may be anything."""
+    p = {k: v.to(DEV) for k, v in gpu_util.params("iso_fast", 3, 3).items()}
+    cache = torch.randint(0, 255, (6, 4, 256), dtype=torch.uint8, device=DEV)
+    table = torch.full((2, 8 if tables == "plain" else (1 << 19) + 1), 1 << 20, dtype=torch.int32, device=DEV)
+    table[0, :3], table[1, :2] = torch.tensor([5, 0, 3]).to(table), torch.tensor([3, 4]).to(table)
+    args = (1, p["k_centroids"], p["v_centroids"], torch.bfloat16)
+    k, _, remapped = rq.decompress_cache_paged(cache, table, torch.tensor([12, 5], dtype=torch.int32, device=DEV), *args)
+    assert k.shape[0] == 4 and remapped[0, :3].tolist() == [3, 0, 1] and remapped[1, :2].tolist() == [1, 2]
+    assert int(remapped[:, 3:].abs().max()) == 0
+    with pytest.raises(ValueError, match="of a cache of 6 blocks"):
+        rq.decompress_cache_paged(cache, table, torch.tensor([12, 9], dtype=torch.int32, device=DEV), *args)
