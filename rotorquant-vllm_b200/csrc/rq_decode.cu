@@ -1143,7 +1143,7 @@ static bool encode_cache_map(CUtensorMap* map, const uint8_t* cache, int64_t num
 
 // Environment switches, read once per process:
 //   RQ_DECODE_NO_TMA=1            every thread loads its own rows (the path of odd block sizes)
-//   RQ_DECODE_NO_PDL=1            launch the merge without programmatic dependent launch
+//   RQ_DECODE_NO_PDL=1            no programmatic dependent launch (plan, attention, merge)
 //   RQ_DECODE_EQUAL_PIECES=1      no launch-layer weights
 //   RQ_DECODE_LAYER_WEIGHTS=a,b   weights of the launch layers (defaults below)
 struct DecodeEnv {
@@ -1178,9 +1178,14 @@ template <typename T, int KB, int VB>
 static int launch_decode(DecodeParams& p, int nh, bool tma, cudaStream_t st) {
     // A launch may start its set-up while the one before (the cache write of the step, for the first) drains: 22.5 ->
     // 15.5 us for a step of one short sequence.  Not the attention kernel when its CTAs fill every SM with long pieces:
-    // scheduled around the CTAs still running they no longer form launch layers, which their piece weights rely on
-    // (64 x 4096 tokens, 28 tiles per piece: 106 -> 119 us; 16 sequences of up to 32768 on one head, 7 tiles:
-    // 47.6 -> 44.0).  RQ_DECODE_NO_PDL=1 puts full launch boundaries between all of them.
+    // scheduled around the CTAs still running they no longer form launch layers, which their piece weights rely on.  Both, in us
+    // (overlapped / full boundary; tiles per piece in front): 2.6: 64 x 300 tokens, 8 KV heads 27.5 / 29.9; 3.7: 16 of 2048 to 32768
+    // on one head 38.0 / 41.4; 6.9: 64 x 1000 45.0 / 43.5, 256 x 512 on 4 heads 62.6 / 67.4, 8 x 8192 on 8 42.5 / 46.9, 16 x 32768
+    // on one 62.4 / 62.7; 10.4: 64 x 1500 59.6 / 55.5; 13.8: 256 x 1024 92.3 / 97.2, 8 x 16384 67.6 / 67.7, 16 x 65536 95.7 / 93.4;
+    // 28: 256 x 2048 151 / 154, 8 x 32768 113 / 108, 16 x 131072 165 / 156, 64 x 4096 118 / 105.  No line on tiles per piece is right
+    // for all; at 10 what is lost on either side is about equal.  The tiles are those of the longest sequence that the caller
+    // admits: short sequences under a bound that was not lowered get the full boundary (64 x 300 tokens with
+    // max_seq_len 8192: 29.9).  RQ_DECODE_NO_PDL=1 puts full launch boundaries between all of them.
     const bool layered = p.layer_ctas > 0 && p.tiles_bound > 10LL * p.groups;
     auto launch = [&](const char* what, bool overlap, auto kernel, dim3 grid, dim3 block, size_t smem, auto... args) -> int {
         if (overlap && !decode_env().no_pdl) return launch_dependent(what, kernel, grid, block, smem, st, args...);

@@ -8,15 +8,17 @@
 // MMA M dimension so that a K/V tile is dequantised once per GQA group, and skips KV tiles that
 // are entirely masked.
 //
-// One CTA = 128 MMA rows = (128 / G) query tokens x G heads of one (sequence, KV head); one
-// thread owns one row (= one TMEM lane).  Per 128-key tile:
-//   1. every thread dequantises one key: K -> int8 codes with a per-key scale (8/16-entry code
-//      table, PRMT lookup), V -> exact round_T(centroid * norm) values; both go to shared memory
-//      in the tcgen05 core-matrix layout (no swizzle);
-//   2. S = Q K^T   tcgen05.mma kind::i8, int32 accumulator in TMEM (4 instructions, K = 32 each);
-//   3. each thread reads its row of S from TMEM, scales by q_scale[row] * k_scale[key], applies
-//      the causal mask, runs the online softmax, writes P (bf16/f16) to shared memory;
-//   4. O += P V    tcgen05.mma kind::f16, fp32 accumulator in TMEM (8 instructions, K = 16 each).
+// Two ways, with the same results bit for bit; 128 MMA rows are (128 / G) query tokens x G heads of one (sequence, KV head).
+//   staged (prefill_stage_kernel + prefill_attn_kernel, where scratch is lent): every 128-key tile is dequantised once, into a
+//     record in operand order; attention CTAs with fixed warp roles (softmax, MMA issue, loads) stream the records, the
+//     probabilities stay in tensor memory.
+//   fused (prefill_int8_kernel, no scratch): a CTA of 256 threads, two per row, does everything of a tile in sequence:
+//     1. every thread dequantises half a key: K -> int8 codes with a per-key scale (8/16-entry code table, PRMT lookup), V ->
+//        exact round_T(centroid * norm) values; both go to shared memory in the tcgen05 core-matrix layout (no swizzle);
+//     2. S = Q K^T   tcgen05.mma kind::i8, int32 accumulator in TMEM (4 instructions, K = 32 each);
+//     3. the two threads of a row read their halves of S from TMEM, scale by q_scale[row] * k_scale[key], apply the causal
+//        mask, run the online softmax, write P (bf16/f16) to shared memory;
+//     4. O += P V    tcgen05.mma kind::f16, fp32 accumulator in TMEM (8 instructions, K = 16 each).
 // The epilogue divides by the row sum, rounds, applies R, rounds and stores.
 //
 // INT8 scheme (the reference quantises Q per 64x128 tile and K per BLOCK_N x 128 tile with
@@ -714,12 +716,14 @@ prefill_stage_kernel(const PrefillParams p) {
 // probabilities add up to more than 2^14 (the reference has been outgrown by more than 2^8), or when a row meets its
 // first visible key.  Packed fp32 operations on key pairs: 4.75 issue slots per score.
 //
-// What bounds it: 256 x 128 scores take 1.8 us; their exponentials alone take 1.06 (16 a clock), their MMAs 0.8, and
-// with two tiles in TMEM the two overlap only in part.  For short sequences also what a CTA does outside the loop, about
-// 10 us of a 32 us life at 2048 tokens; and the last wave (2048 tokens of 8 KV heads are 256 CTAs on 148 SMs).  Against
+// What bounds it: no unit is saturated.  With two tiles per CTA (2048 tokens after 18000) the exponential unit is busy for
+// 58 % of the time, the tensor pipe 43 %, the issue slots 54 %; 256 x 128 scores take 1.8 us, their exponentials alone 1.06 (16 a
+// clock), their MMAs 0.8, and with two tiles in TMEM the two overlap only in part.  With one tile per CTA (8 x 2048 tokens) 33 %,
+// 24 % and 53 %: the chains of the two CTAs on an SM cover half of the issue slots, and about 10 us of a CTA's 32 lie outside
+// the loop.  For few long sequences also the last wave (2048 tokens of 8 KV heads are 256 CTAs on 148 SMs).  Against
 // one tile per CTA, two CTAs per SM, P through shared memory (us, whole call): 2048 tokens after 30000, 32 heads
-// 1140 -> 942-1000; 8 x 2048 tokens 519 -> 480, with TILES = 1 470; 2 prompts of up to 1500 and 30 single tokens after 4000, 28 heads
-// 286 -> 202 (TILES = 1).
+// 1140 -> 950-1040 between GPUs; 8 x 2048 tokens 519 -> 480, with TILES = 1 472; 2 prompts of up to 1500 and 30 single tokens after
+// 4000, 28 heads 286 -> 197, with TILES = 1 204.
 // Slower than this (the attention kernel of the first, 920 here): one thread per row 968; steps of 64 keys with two S
 // buffers 1192; S released early and P in shared memory 1210; an MMA thread per tile 1077; persistent CTAs whose
 // queries are prepared by two more warps 964.
@@ -1318,10 +1322,16 @@ static int launch_prefill(const PrefillParams& p, int m_tiles, int num_seqs, cud
         if (int e = launch_dependent("rq_prefill_int8 stage launch", prefill_stage_kernel<T, KB, VB>, sgrid, dim3(128), 0, st, p)) return e;
         // Units of work: at most tokens / (tokens of a unit) + one partial unit per sequence, found by the CTAs
         // themselves (a grid of longest sequence x sequences was mostly empty CTAs for batches of mixed lengths).
-        // One tile per CTA, two CTAs per SM, is the faster form up to some thousand keys, as one CTA's queries and output
-        // run under the other's loop (8 x 2048 tokens 480 -> 470 us, 19 prompts of 34 to 283 85 -> 73).  Two tiles per CTA
-        // read K/V half as often, which pays where contexts may be long (2048 tokens after 30000: 1010-1030 -> 950), unless
-        // most sequences have no second tile or there are too few tiles for every SM.
+        // One tile per CTA, two CTAs per SM, is the faster form for short contexts, as one CTA's queries and output run under
+        // the other's loop; two tiles per CTA read K/V half as often.  Both, in us (one / two): 300 tokens 20.5 / 24.6,
+        // 19 prompts of 34 to 283 67 / 77, 64 x 256 282 / 300, 16 x 1024 371 / 377, 8 x 2048 480 / 479, 4 x 4096 696 / 687; 2048 tokens
+        // after 2000 141 / 135, 8192 327 / 314, 12000 453 / 437, 18000 653 / 625, 30000 1042 / 999.  So for prompts alone the
+        // two cross near 2000 to 4000 keys, and the line at 16384 gives up 2 to 5 % between there and itself.  It stands there
+        // for the sake of batches that also have running requests of one token, where the form with fewer, longer units
+        // wins or loses with the last wave: after up to 6000, 28 heads, one prompt of 2048 with 12 of them 265 / 253, with 30 284 / 313,
+        // one of 512 with 60 231 / 256; 32 heads, 2048 with 12 300 / 328, with 30 420 / 410 (and 30 with 2 prompts of up to 1500 after
+        // 4000, 28 heads 205 / 197).  Behind the line one tile is kept where most sequences have no second one (4 x 64 after
+        // 16000 277 / 284) or there are too few tiles for every SM.
         auto units = [&](long long per) {
             const long long by_tokens = p.num_tokens / per + num_seqs;
             const long long by_longest = num_seqs * ((1LL * m_tiles * p.tokens_per_tile + per - 1) / per);
