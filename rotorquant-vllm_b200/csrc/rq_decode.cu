@@ -1216,7 +1216,10 @@ static int launch_decode(DecodeParams& p, int nh, bool tma, cudaStream_t st) {
         if (e) return e;
     }
 
-    // rows with many parts each (long sequences on few heads): a CTA per row instead of a warp per row
+    // Rows with many parts each (long sequences on few heads): a CTA per row instead of a warp per row.  Whole step in us, warp /
+    // CTA per row, by pieces per sequence: 74: one of 131072 tokens 74.9 / 64.1, 8 on one head 51.5 / 36.8; 37: 71.1 / 63.9; 18:
+    // 66.1 / 63.7; 9: 8 of 32768 105.7 / 103.7, 8 of 131072 384 / 377; 7: 124.0 / 123.3; 6: 146 / 144, but with many rows 59.5 /
+    // 61.5 (24 x 28 heads) and 79.4 / 80.9 (96 x 8).
     const long long rows = 1LL * p.num_seqs * p.Hq;
     const bool wide = p.groups > 8LL * p.num_seqs;
     if (wide) return launch("rq_decode merge launch", true, decode_merge_kernel<T, kWideMergeWarps>, dim3(static_cast<unsigned>(rows)),
