@@ -317,6 +317,7 @@ struct __align__(512) UmmaSmem {
     int64_t piece[2];                        // this CTA's piece of the tile line
     uint64_t bar_s, bar_o;
     uint64_t bar_in[4];                      // per warp: "staged rows landed"
+    uint64_t drained;                        // after an expired wait: every MMA issued has completed
     uint32_t tmem_base;
 };
 
@@ -338,6 +339,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     if (tid == 0) {
         mbar_init(&sm.bar_s, 1);
         mbar_init(&sm.bar_o, 1);
+        mbar_init(&sm.drained, 1);
 #pragma unroll
         for (int w = 0; w < 4; ++w) mbar_init(&sm.bar_in[w], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -491,14 +493,15 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
             const int t = tile * kUTile + 32 * warp + (lane & 16);
             return (tile < t_end && t < seq_len) ? __ldg(bt_row + (t >> p.bs_shift)) : 0;
         };
-        [[maybe_unused]] auto issue_tile = [&](int tile, int blk) {      // completes one phase of bar_in[warp]
+        // Completes one phase of bar_in[warp].  Not after a wait for the phase before has expired (stop): it may be open still.
+        [[maybe_unused]] auto issue_tile = [&](int tile, int blk, bool stop) {
             const int t = tile * kUTile + 32 * warp + (lane & 16);
             blk = blk < 0 ? 0 : (blk > last_blk ? last_blk : blk);
             const int gslot = (blk << p.bs_shift) + (t & (p.block_size - 1));
             const int s0 = __shfl_sync(0xffffffffu, gslot, 0), s1 = __shfl_sync(0xffffffffu, gslot, 16);
             const bool on0 = tile * kUTile + 32 * warp < seq_len, on1 = tile * kUTile + 32 * warp + 16 < seq_len;
             staged_slot = (t + (lane & 15) < seq_len) ? gslot + (lane & 15) : -1;
-            if (lane == 0) {
+            if (lane == 0 && !stop) {
                 const uint32_t bar = smem_u32(&sm.bar_in[warp]);
                 if (on0) {
                     const uint32_t group_bytes = v_by_tma ? 2048u : 1024u;
@@ -559,7 +562,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         // the first tile's rows are requested before the query set-up, which hides most of their latency
         if (!dead) {
             if constexpr (TMA) {
-                issue_tile(t_begin, load_blk(t_begin));
+                issue_tile(t_begin, load_blk(t_begin), false);
                 pf_blk = load_blk(t_begin + 1);
             } else {
                 const uint8_t* first = slot_of(t_begin);
@@ -616,7 +619,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
                 fetch_staged(0, kw, nk);
                 fetch_staged(1, vw, nv);
                 __syncwarp();
-                if (t_begin + 1 < t_end) issue_tile(t_begin + 1, pf_blk);
+                if (t_begin + 1 < t_end) issue_tile(t_begin + 1, pf_blk, failed_in);
                 pf_blk = load_blk(t_begin + 2);
             }
         }
@@ -719,7 +722,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
                 v_rows_landed();
                 if (tile + 1 < t_end) fetch_staged(1, vw, nv);
                 __syncwarp();                            // the staging rows are free again
-                if (tile + 2 < t_end) issue_tile(tile + 2, pf_blk);
+                if (tile + 2 < t_end) issue_tile(tile + 2, pf_blk, failed);
                 pf_blk = load_blk(tile + 3);
             } else {
                 fetch_direct(1, next_slot, vw, nv);
@@ -858,10 +861,24 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         if (t_end == n_s) ++seq;
     }
 
+    if (dead) {
+        // What is in flight lands before shared and tensor memory are given back, within limits of their own: copies (the
+        // staging barrier's open phase is one of the two) and MMAs.
+        if constexpr (TMA) {
+            mbar_wait_for(&sm.bar_in[warp], 0u, kWaitCycles / 8);
+            mbar_wait_for(&sm.bar_in[warp], 1u, kWaitCycles / 8);
+            if constexpr (!v_by_tma) cp_async_wait_all();
+        }
+        if (tid == 0) {
+            tc_commit(&sm.drained);
+            mbar_wait(&sm.drained, 0u);
+        }
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, kUTmemCols);
 }
+
 // Tiles of every sequence as an exclusive prefix sum, for batches too large for the attention CTAs
 // to scan themselves: prefix[s] = sum_{s' < s} ceil(len[s'] / tile_tokens), prefix[num_seqs] = total.
 __global__ void decode_plan_kernel(const int32_t* __restrict__ seq_lens, int num_seqs, int tile_tokens,
