@@ -119,6 +119,7 @@ struct __align__(128) PrefillSmem {
     float rot[32 * 16];
     float cb[2][16];
     uint64_t bar_s, bar_o;
+    uint64_t drained;                 // after an expired wait: every MMA issued has completed
     uint32_t tmem_base;
 };
 
@@ -226,6 +227,7 @@ prefill_int8_kernel(const PrefillParams p) {
     if (tid == 0) {
         mbar_init(&sm.bar_s, 1);
         mbar_init(&sm.bar_o, 1);
+        mbar_init(&sm.drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tmem_alloc(&sm.tmem_base, kTmemCols);
@@ -606,8 +608,10 @@ prefill_int8_kernel(const PrefillParams p) {
                         make_uint4(outw[4 * i], outw[4 * i + 1], outw[4 * i + 2], outw[4 * i + 3]);
             }
         }
-    } else if (tid == 0 && p.error_flag != nullptr) {
-        atomicExch(p.error_flag, 1);
+    } else if (tid == 0) {
+        if (p.error_flag != nullptr) atomicExch(p.error_flag, 1);
+        tc_commit(&sm.drained);                      // what was issued ends before TMEM is freed
+        mbar_wait(&sm.drained, 0);
     }
     tc_fence_before();
     __syncthreads();
