@@ -248,11 +248,14 @@ int rq_prefill_int8(const void* q, void* out, int dtype, int64_t q_stride_tok,
  * rq_prefill_int8 in two steps, for callers that can lend scratch memory: every (sequence, KV head,
  * 128-key tile) is decompressed once into `workspace` (int8 K codes, key scales, V values, already
  * in tensor-core operand order) and the attention kernel streams those records with bulk copies
- * instead of rebuilding them for every block of query rows.  Same results as rq_prefill_int8.
+ * instead of rebuilding them for every block of query rows.  Where a batch has few query tiles with long contexts, their keys
+ * are divided between CTAs and the parts put together in fp32.  Rows of tiles that are not divided have the results of
+ * rq_prefill_int8 bit for bit, the others up to the rounding of their probabilities.
  *
  *   max_seq_len      upper bound of seq_lens (host value); sequences longer than it are truncated
- *   workspace        >= rq_prefill_workspace_bytes(num_seqs, num_kv_heads, max_seq_len) bytes,
- *                    128-byte aligned; contents are scratch
+ *   workspace        rq_prefill_workspace_bytes(num_seqs, num_kv_heads, max_seq_len) bytes, 128-byte aligned; contents are
+ *                    scratch.  num_seqs * ceil(max_seq_len / 128) * num_kv_heads * 49664 bytes are enough, but then no
+ *                    tile is divided.
  */
 size_t rq_prefill_workspace_bytes(int num_seqs, int num_kv_heads, int max_seq_len);
 int rq_prefill_int8_staged(const void* q, void* out, int dtype, int64_t q_stride_tok,

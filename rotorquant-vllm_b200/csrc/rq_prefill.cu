@@ -8,10 +8,10 @@
 // MMA M dimension so that a K/V tile is dequantised once per GQA group, and skips KV tiles that
 // are entirely masked.
 //
-// Two ways, with the same results bit for bit; 128 MMA rows are (128 / G) query tokens x G heads of one (sequence, KV head).
+// Two ways; 128 MMA rows are (128 / G) query tokens x G heads of one (sequence, KV head).
 //   staged (prefill_stage_kernel + prefill_attn_kernel, where scratch is lent): every 128-key tile is dequantised once, into a
 //     record in operand order; attention CTAs with fixed warp roles (softmax, MMA issue, loads) stream the records, the
-//     probabilities stay in tensor memory.
+//     probabilities stay in tensor memory.  Few tiles with long contexts are divided by keys (prefill_merge_kernel).
 //   fused (prefill_int8_kernel, no scratch): a CTA of 256 threads, two per row, does everything of a tile in sequence:
 //     1. every thread dequantises half a key: K -> int8 codes with a per-key scale (8/16-entry code table, PRMT lookup), V ->
 //        exact round_T(centroid * norm) values; both go to shared memory in the tcgen05 core-matrix layout (no swizzle);
@@ -29,6 +29,7 @@
 //
 // Every wait on an mbarrier is bounded; on expiry the CTA records an error, frees its TMEM and
 // returns.
+#include <algorithm>
 #include <type_traits>
 
 #include "rq_common.cuh"
@@ -63,6 +64,10 @@ struct PrefillParams {
     int* error_flag;                  // optional device int, set non-zero when a wait expired
     uint8_t* stage;                   // staged path: scratch records (see prefill_stage_kernel)
     int stage_tiles_per_seq;
+    // staged path: units of the attention (a tile of query rows and a KV head), how many of them are not divided, and into how
+    // many parts the others may be (see find_work); the results of the parts
+    int units, whole, max_parts;
+    float* parts;
 };
 
 template <typename T> using PfType = TcFormat<T>;
@@ -702,47 +707,365 @@ prefill_stage_kernel(const PrefillParams p) {
 
 // ---- staged path: attention --------------------------------------------------------------------
 //
-// One CTA = two MMA tiles (TILES = 2) of 128 rows (2 x (128 / G) query tokens x G heads of one (sequence, KV head)) that
-// share every K/V tile they read.  Eighteen warps with fixed roles:
-//   warps 0-7, 8-15 softmax of tile 0 and tile 1: two threads per row (= TMEM lane), 64 keys each; they also prepare
-//                   their rows of Q and write their rows of the output;
-//   warp 16         issues every MMA: S_x(j) = Q_x K(j) (int8, shared memory -> int32 in TMEM) and O_x += P_x(j) V(j)
-//                   (P from TMEM, fp32 in TMEM);
-//   warp 17         keeps three stages of K codes, V values and key scales in flight (cp.async.bulk of the staged
-//                   records, already in operand order).
-// TMEM (all 512 columns): S_0 0-127, S_1 128-255, O_0 256-383, O_1 384-511; a thread's probabilities overwrite the
-// first half of the sums it read.  While one tile is in its softmax the tensor core works for the other: the order of
-// issue is PV_0(j) S_0(j+1) PV_1(j) S_1(j+1).  MMAs run in the order of issue, so S_x(j+1) cannot overwrite P_x(j)
-// before it has been read, and the commit behind S_x(j+1) also says that PV_x(j) is done.
+// A tile is 128 MMA rows: (128 / G) query tokens x G heads of one (sequence, KV head).  Fixed warp roles:
+//   softmax, eight warps per tile: two threads per row (= TMEM lane), 64 keys each; they also prepare the rows of Q and write those
+//     of the output;
+//   one warp issues every MMA: S(j) = Q K(j) (int8, shared memory -> int32 in TMEM) and O += P(j) V(j) (P from TMEM, fp32 in TMEM);
+//   one loads K codes, V values and key scales (cp.async.bulk of the staged records, already in operand order).
+// A thread's probabilities overwrite the first half of the sums it read.  MMAs run in the order of issue, so S(j+1) cannot
+// overwrite P(j) before it has been read, and the commit behind S(j+1) also says that PV(j) is done.
+//   TILES = 1: one tile per CTA, two CTAs per SM.  K codes and V values have one buffer each, reloaded as soon as the MMAs
+//     that read them are done; the other CTA covers the gaps, the set-up and the epilogue.
+//   TILES = 2: two tiles of consecutive tokens per CTA, which share every K/V tile they read, out of three stages.  While one tile is in
+//     its softmax the tensor core works for the other: the order of issue is PV_0(j) S_0(j+1) PV_1(j) S_1(j+1).  For long contexts
+//     and many tiles: half of the traffic from L2, which counts where the GPU runs at its power limit.
+// TMEM: S_x in columns 128 x, O_x behind them.
 //
 // Softmax: the scaled sums are exponentiated against a lazy reference maximum in one pass over the half row; the tile
 // is redone (the sums are still in TMEM) after finding the row's maximum when it is the row's first tile, when the
 // probabilities add up to more than 2^14 (the reference has been outgrown by more than 2^8), or when a row meets its
 // first visible key.  Packed fp32 operations on key pairs: 4.75 issue slots per score.
 //
-// What bounds it: no unit is saturated.  With two tiles per CTA (2048 tokens after 18000) the exponential unit is busy for
-// 58 % of the time, the tensor pipe 43 %, the issue slots 54 %; 256 x 128 scores take 1.8 us, their exponentials alone 1.06 (16 a
-// clock), their MMAs 0.8, and with two tiles in TMEM the two overlap only in part.  With one tile per CTA (8 x 2048 tokens) 33 %,
-// 24 % and 53 %: the chains of the two CTAs on an SM cover half of the issue slots, and about 10 us of a CTA's 32 lie outside
-// the loop.  For few long sequences also the last wave (2048 tokens of 8 KV heads are 256 CTAs on 148 SMs).  Against
-// one tile per CTA, two CTAs per SM, P through shared memory (us, whole call): 2048 tokens after 30000, 32 heads
-// 1140 -> 950-1040 between GPUs; 8 x 2048 tokens 519 -> 480, with TILES = 1 472; 2 prompts of up to 1500 and 30 single tokens after
-// 4000, 28 heads 286 -> 197, with TILES = 1 204.
-// Slower than this (the attention kernel of the first, 920 here): one thread per row 968; steps of 64 keys with two S
-// buffers 1192; S released early and P in shared memory 1210; an MMA thread per tile 1077; persistent CTAs whose
-// queries are prepared by two more warps 964.
-//
-// With TILES = 1 a CTA has one tile, half the warps and columns, and one buffer each for K codes and V values, reloaded
-// as soon as the MMAs that read them are done: two CTAs per SM, which hide each other's gaps.
-constexpr int kAttnStages = 3;        // TILES = 2
 // Q tile in core-matrix order with 16 bytes between the core matrices: the 8 head-dim chunks of a row then fall into
 // different banks when a warp writes a row.
-constexpr int kQCore = 128 + 16, kQGroup = 8 * kQCore;
+constexpr int kQCore = 128 + 16, kQGroup = 8 * kQCore, kQTile = (kPfRows / 8) * kQGroup;
+// A softmax warp passes its output rows through shared memory, 32 rows of 32 head-dims at a time.
+constexpr int kOutPitch = 72, kOutWarp = 32 * kOutPitch;
 
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar_addr, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_addr), "r"(bytes) : "memory");
+}
+// Contiguous global -> shared copy of `bytes` (multiple of 16, both addresses 16-byte aligned),
+// completing on the mbarrier.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar_addr) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar_addr) : "memory");
+}
+// Barrier of the 256 softmax threads of tile x, and whether any of them said yes.
+__device__ __forceinline__ bool tile_any(int x, bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred a, b;\n\tsetp.ne.u32 a, %1, 0;\n\t"
+        "bar.red.or.pred b, %2, 256, a;\n\tselp.u32 %0, 1, 0, b;\n\t}"
+        : "=r"(r) : "r"(static_cast<uint32_t>(v)), "r"(9 + x) : "memory");
+    return r != 0;
+}
+
+// The query rows of a tile in the order of its MMA rows, from `row0` on.  `first`: the first row of the tile's first token,
+// `tokens` of which the tile has (at least one).  The rows behind them are the last token's again (their outputs go
+// nowhere): where a row lies is then the same for all lanes and follows from the row before, and no load is under a condition.
+// (With places shuffled out of the lanes that know them, and zeros for rows without a token, every load waited for the
+// one before: the 128 rows of a tile took one warp 50000 clocks against 31000.)
+template <typename T>
+struct QueryRows {
+    const T* at;
+    int64_t head_step, next_token, same_token;
+    int head, G, left;                                // the row's head; tokens behind its own
+    __device__ __forceinline__ QueryRows(const PrefillParams& p, long long first, int tokens, int row0) {
+        const int tl = min(row0 / p.G, tokens - 1);
+        G = p.G;
+        head = row0 % p.G;
+        left = tokens - 1 - tl;
+        head_step = p.q_stride_head;
+        same_token = -(p.G - 1) * p.q_stride_head;
+        next_token = p.q_stride_tok + same_token;
+        at = static_cast<const T*>(p.q) + first + tl * p.q_stride_tok + head * p.q_stride_head + 4 * (threadIdx.x & 31);
+    }
+    __device__ __forceinline__ uint2 load() {         // this lane's four elements; on to the next row
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(at));
+        const bool wraps = ++head == G;
+        at += wraps ? (left > 0 ? next_token : same_token) : head_step;
+        if (wraps) { head = 0; --left; }
+        return v;
+    }
+};
+// Q: rotate, round, quantise the rows row0 .. row0 + 15 of a tile to int8, by the 32 lanes of a warp.  Lane L has head-dims
+// 4L .. 4L + 3 (one rotation block, in registers), so that loads are contiguous.  Rows are worked on two at a time with packed operations, and eight are in flight while eight are converted.  Rows
+// without a token get the scale 0, so that their scores are 0 and they never outgrow a reference maximum (which would have their
+// warp do the tile again: 338 -> 302 us for 12 single tokens and one prompt of 2048 after up to 6000, 32 heads).
+template <typename T>
+__device__ __forceinline__ void prepare_queries(const PrefillParams& p, const float* rot_blocks, uint8_t* q_tile, float* q_scale, int row0,
+                                                long long first, int tokens) {
+    const int lane = threadIdx.x & 31, valid = tokens * p.G;
+    constexpr int kRows = 8;
+    f2 rot[4][4];                                     // [out][in], both halves alike
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+        const float4 r = *reinterpret_cast<const float4*>(&rot_blocks[lane * 16 + 4 * jj]);
+        rot[jj][0] = pk(r.x, r.x); rot[jj][1] = pk(r.y, r.y); rot[jj][2] = pk(r.z, r.z); rot[jj][3] = pk(r.w, r.w);
+    }
+    // Adding 1.5 * 2^23 rounds to the nearest integer, in the low bits.  Scalar operations: the assembler contracts a
+    // packed product and sum, and a product that is a tie after its own rounding would go the other way.
+    auto code = [](float v, float scale) { return __float_as_uint(__fadd_rn(__fmul_rn(v, scale), 12582912.0f)); };
+    auto rotate = [&](uint2& va, uint2& vb) {
+        const float2 a01 = pf_unpack<T>(va.x), a23 = pf_unpack<T>(va.y), b01 = pf_unpack<T>(vb.x), b23 = pf_unpack<T>(vb.y);
+        const f2 in[4] = {pk(a01.x, b01.x), pk(a01.y, b01.y), pk(a23.x, b23.x), pk(a23.y, b23.y)};
+        float ya[4], yb[4];
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+            f2 y = mul2(in[0], rot[jj][0]);
+#pragma unroll
+            for (int k = 1; k < 4; ++k) y = fma2(in[k], rot[jj][k], y);
+            upk(y, ya[jj], yb[jj]);
+        }
+        va = make_uint2(pf_pack<T>(ya[0], ya[1]), pf_pack<T>(ya[2], ya[3]));
+        vb = make_uint2(pf_pack<T>(yb[0], yb[1]), pf_pack<T>(yb[2], yb[3]));
+    };
+    auto largest = [](uint2 v) {
+        const float2 c = pf_unpack<T>(v.x), d = pf_unpack<T>(v.y);
+        return fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y)));
+    };
+    auto store_codes = [&](uint2 v, float inv_row, int r) {
+        const float2 a = pf_unpack<T>(v.x), b = pf_unpack<T>(v.y);
+        // position d holds head-dim d ^ 1
+        const uint32_t w = prmt(prmt(code(a.y, inv_row), code(a.x, inv_row), 0x0040), prmt(code(b.y, inv_row), code(b.x, inv_row), 0x0040), 0x5410);
+        *reinterpret_cast<uint32_t*>(&q_tile[(r >> 3) * kQGroup + (lane >> 2) * kQCore + (r & 7) * 16 + 4 * (lane & 3)]) = w;
+    };
+    bool nan = false;                                 // one of the rows that lane i < 8 keeps the maximum of
+    QueryRows<T> rows(p, first, tokens, row0);
+    uint2 next[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) next[i] = rows.load();
+#pragma unroll 1
+    for (int i0 = 0; i0 < 16; i0 += kRows) {
+        uint2 raw[kRows];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) raw[i] = next[i];
+        if (i0 + kRows < 16) {
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) next[i] = rows.load();
+        }
+        float mx = 0.0f;                              // lane i < 8: largest |value| of row i0 + i
+#pragma unroll
+        for (int i = 0; i < kRows; i += 2) {
+            rotate(raw[i], raw[i + 1]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const uint32_t m_row = __reduce_max_sync(0xffffffffu, __float_as_uint(largest(raw[i + e])));     // non-negative floats order as integers
+                if (lane == i + e) mx = __uint_as_float(m_row);
+            }
+        }
+        nan |= mx != mx;
+        const bool ok = mx > 0.0f && mx <= 3.0e38f;
+        const float inv = ok ? __fdiv_rn(127.0f, mx) : 0.0f;
+        if (lane < kRows) q_scale[row0 + i0 + lane] = ok && row0 + i0 + lane < valid ? __fdiv_rn(mx, 127.0f) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) store_codes(raw[i], __shfl_sync(0xffffffffu, inv, i), row0 + i0 + i);
+    }
+    // A NaN element makes its whole rotation block NaN, and a NaN is larger than infinity as an integer.  Such a block
+    // counts as zero: its codes are 0 and the row's scale comes from the others.  (A block with infinities has an
+    // infinite maximum, and its row the scale 0.)  The rows are done again, one by one.  What the look at them takes, of
+    // the call for 8 x 2048 tokens: 2 % at every row, 0.6 % per eight rows before their codes, 0.2 % here.
+    if (__any_sync(0xffffffffu, nan)) {
+        rows = QueryRows<T>(p, first, tokens, row0);
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i) {
+            uint2 v = rows.load(), same = v;
+            rotate(v, same);
+            float m = largest(v);
+            if (m != m) { m = 0.0f; v = make_uint2(0u, 0u); }
+            m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+            const bool ok = m > 0.0f && m <= 3.0e38f;
+            if (lane == 0) q_scale[row0 + i] = ok && row0 + i < valid ? __fdiv_rn(m, 127.0f) : 0.0f;
+            store_codes(v, ok ? __fdiv_rn(127.0f, m) : 0.0f, row0 + i);
+        }
+    }
+}
+
+// What the two threads of a row keep over the tiles.
+struct SoftmaxRow {
+    uint32_t s_cols, o_cols;          // this half's columns of S and O, in the row's TMEM lane
+    float *xch;                       // exchange with the other thread of the row: this half's place ...
+    const float *xch_other;           // ... and the other's
+    int pair_id;                      // named barrier of the two warps with the same rows
+    float row_factor;                 // query scale * softmax scale
+    float m_run, l_run;               // reference maximum; sum over this half of the keys
+};
+
+// Probabilities of a tile: this thread's 64 keys (k_scale: their scales; keys 0 .. limit are visible), written over the half row's
+// own sums.  `first`: O holds nothing yet.
+template <typename T>
+__device__ __forceinline__ void softmax_tile(SoftmaxRow& s, const float* k_scale, int limit, bool first) {
+    const f2 factor2 = pk(s.row_factor, s.row_factor), unbias2 = pk(-12582912.0f, -12582912.0f);
+    const bool unmasked = __all_sync(0xffffffffu, limit >= 63);
+
+    // scaled sums of four keys, in pairs: (float)S * key scale
+    auto scaled = [&](const uint32_t* r, float4 ks, f2& a, f2& b) {
+        // int -> float: |S| < 2^22, so adding it to the bits of 1.5 * 2^23 gives 1.5 * 2^23 + S exactly
+        const f2 r01 = pk(__uint_as_float(r[0] + 0x4B400000u), __uint_as_float(r[1] + 0x4B400000u));
+        const f2 r23 = pk(__uint_as_float(r[2] + 0x4B400000u), __uint_as_float(r[3] + 0x4B400000u));
+        a = mul2(add2(r01, unbias2), pk(ks.x, ks.y));
+        b = mul2(add2(r23, unbias2), pk(ks.z, ks.w));
+    };
+    auto scales = [&](int key) { return *reinterpret_cast<const float4*>(&k_scale[key]); };
+    // the row's maximum over the tile becomes the reference if it exceeds it by 2^8 or more
+    auto move_reference = [&]() {
+        float m_half = -INFINITY;
+#pragma unroll 1
+        for (int ch = 0; ch < 4; ++ch) {
+            uint32_t r[16];
+            tmem_ld16_nowait(s.s_cols + 16 * ch, r);
+            tmem_wait_ld();
+            tmem_ld16_landed(r);
+#pragma unroll
+            for (int c4 = 0; c4 < 4; ++c4) {
+                f2 a, b;
+                scaled(&r[4 * c4], scales(16 * ch + 4 * c4), a, b);
+                float v[4];
+                upk(a, v[0], v[1]);
+                upk(b, v[2], v[3]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (16 * ch + 4 * c4 + e <= limit) m_half = fmaxf(m_half, v[e]);
+            }
+        }
+        *s.xch = m_half;
+        pair_any(s.pair_id, false);
+        const float m_tile = fmaxf(m_half, *s.xch_other) * s.row_factor;            // row_factor >= 0
+        const bool grew = m_tile > s.m_run + 8.0f;
+        const float m_new = grew ? m_tile : s.m_run;
+        const float alpha = grew ? (s.m_run == -INFINITY ? 0.0f : pf_ex2(s.m_run - m_new)) : 1.0f;
+        if (!first && __any_sync(0xffffffffu, grew)) {    // O is at rest: the commit behind S covered the PV before it
+#pragma unroll 1
+            for (int ch = 0; ch < 4; ++ch) {
+                uint32_t r[16];
+                tmem_ld16_nowait(s.o_cols + 16 * ch, r);
+                tmem_wait_ld();
+                tmem_ld16_landed(r);
+#pragma unroll
+                for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * alpha);
+                tmem_st16_nowait(s.o_cols + 16 * ch, r);
+            }
+            tmem_wait_st();
+        }
+        s.l_run *= alpha;
+        s.m_run = m_new;
+        pair_any(s.pair_id, false);                       // xch has been read
+    };
+    uint32_t prob[32];                                    // probabilities of the half row as T pairs
+    float half_sum;
+    auto exponentiate = [&](auto masked_tag) {
+        constexpr bool kMasked = decltype(masked_tag)::value;
+        const float m_use = (s.m_run == -INFINITY) ? 0.0f : s.m_run;
+        const f2 minus_m = pk(-m_use, -m_use);
+        f2 sum_a = pk(0.0f, 0.0f), sum_b = sum_a;
+        uint32_t buf[2][8];
+        tmem_ld8_nowait(s.s_cols, buf[0]);
+        float4 ks[2] = {scales(0), scales(4)};
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            tmem_wait_ld();
+            tmem_ld8_landed(buf[it & 1]);
+            const float4 now[2] = {ks[0], ks[1]};
+            if (it < 7) {
+                tmem_ld8_nowait(s.s_cols + 8 * (it + 1), buf[(it + 1) & 1]);
+                ks[0] = scales(8 * (it + 1));
+                ks[1] = scales(8 * (it + 1) + 4);
+            }
+#pragma unroll
+            for (int c4 = 0; c4 < 2; ++c4) {
+                f2 a, b;
+                scaled(&buf[it & 1][4 * c4], now[c4], a, b);
+                float e[4];
+                upk(fma2(a, factor2, minus_m), e[0], e[1]);
+                upk(fma2(b, factor2, minus_m), e[2], e[3]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    e[i] = pf_ex2(e[i]);
+                    if (kMasked && 8 * it + 4 * c4 + i > limit) e[i] = 0.0f;
+                }
+                sum_a = add2(sum_a, pk(e[0], e[1]));
+                sum_b = add2(sum_b, pk(e[2], e[3]));
+                prob[4 * it + 2 * c4] = pf_pack<T>(e[0], e[1]);
+                prob[4 * it + 2 * c4 + 1] = pf_pack<T>(e[2], e[3]);
+            }
+        }
+        float lo, hi;
+        upk(add2(sum_a, sum_b), lo, hi);
+        half_sum = lo + hi;
+    };
+    if (first) move_reference();
+#pragma unroll 1
+    for (int attempt = 0;; ++attempt) {
+        if (unmasked) exponentiate(std::false_type{});
+        else exponentiate(std::true_type{});
+        // both threads of every row take the same decision
+        const bool outgrown = !(half_sum <= 16384.0f) || (s.m_run == -INFINITY && half_sum > 0.0f);
+        if (!pair_any(s.pair_id, outgrown) || attempt == 1) break;
+        move_reference();
+    }
+    s.l_run += half_sum;
+    tmem_st32_nowait(s.s_cols, prob);                     // over the half row's own sums
+    tmem_wait_st();
+}
+
+// Output rows of a warp: O / l, round, rotate by R, round, store.  Lane = row of the warp's 32 TMEM lanes; `mine` is where the
+// lane's row goes (-1: nowhere), `half` which 64 head-dims the warp has, `any` false for rows that saw no key (zeros).  A lane
+// rotates its own row, whose rotation blocks are then the same for all lanes; the rows pass through the warp's own shared
+// memory, so that four lanes store 64 contiguous bytes.
+template <typename T>
+__device__ __forceinline__ void store_rows(const PrefillParams& p, uint32_t o_cols, int half, float inv_l, bool any, long long mine,
+                                           const float* rot_blocks, uint8_t* rows) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int ch = 0; ch < 2; ++ch) {
+        uint32_t r[32];
+        if (any) {
+            tmem_ld32(o_cols + 32 * ch, r);
+            tmem_ld32_landed(r);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) r[i] = 0u;
+        }
+        const float* rb = &rot_blocks[(16 * half + 8 * ch) * 16];                    // rb[16 b + 4 k + j] = R[4g+k][4g+j]
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {                     // column d of O holds head-dim d ^ 1
+            const float2 o01 = pf_unpack<T>(pf_pack<T>(__uint_as_float(r[4 * b + 1]) * inv_l, __uint_as_float(r[4 * b]) * inv_l));
+            const float2 o23 = pf_unpack<T>(pf_pack<T>(__uint_as_float(r[4 * b + 3]) * inv_l, __uint_as_float(r[4 * b + 2]) * inv_l));
+            const float o[4] = {o01.x, o01.y, o23.x, o23.y};
+            f2 y01 = 0, y23 = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const ulonglong2 rr = *reinterpret_cast<const ulonglong2*>(rb + 16 * b + 4 * k);
+                const f2 ok = pk(o[k], o[k]);
+                y01 = k == 0 ? mul2(ok, rr.x) : fma2(ok, rr.x, y01);
+                y23 = k == 0 ? mul2(ok, rr.y) : fma2(ok, rr.y, y23);
+            }
+            float y[4];
+            upk(y01, y[0], y[1]);
+            upk(y23, y[2], y[3]);
+            r[2 * b] = pf_pack<T>(y[0], y[1]);
+            r[2 * b + 1] = pf_pack<T>(y[2], y[3]);
+        }
+        __syncwarp();                                     // the rows of the pass before have been read
+#pragma unroll
+        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint2*>(rows + lane * kOutPitch + 8 * c) = make_uint2(r[2 * c], r[2 * c + 1]);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r_of = 8 * i + (lane >> 2);
+            const long long at = __shfl_sync(0xffffffffu, mine, r_of);
+            const uint2 lo = *reinterpret_cast<const uint2*>(rows + r_of * kOutPitch + 16 * (lane & 3));
+            const uint2 hi = *reinterpret_cast<const uint2*>(rows + r_of * kOutPitch + 16 * (lane & 3) + 8);
+            if (at >= 0)
+                *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + at + 64 * half + 32 * ch + 8 * (lane & 3)) = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        }
+    }
+}
+
+// K/V tiles that the rows of the tokens first .. first + count - 1 of a sequence need: up to the last one's position, never past
+// the staged records.
+__device__ __forceinline__ int key_tiles(const PrefillParams& p, int q_len, int kv_len, int first, int count) {
+    const int last = min(q_len, first + count) - 1;
+    const int last_pos = min(kv_len - q_len + last, kv_len - 1);
+    return first < q_len && last_pos >= 0 ? min(last_pos / kPfKeys + 1, p.stage_tiles_per_seq) : 0;
+}
+
+constexpr int kAttnStages = 3;        // TILES = 2
 template <int TILES>
 struct __align__(128) AttnSmem {
     static constexpr int kStages = TILES == 2 ? kAttnStages : 1;
-    uint8_t q[TILES][(kPfRows / 8) * kQGroup];          // (the epilogue passes O through it: 128 rows of 144 bytes)
+    uint8_t q[TILES][kQTile];                           // (the epilogue passes the output rows through it)
     uint8_t k[kStages][kPfKeys * kHeadDim];
     uint16_t v[kStages][kPfKeys * kHeadDim];
     float k_scale[TILES == 2 ? kStages : 2][kPfKeys];
@@ -756,22 +1079,11 @@ struct __align__(128) AttnSmem {
     uint64_t drained;                                   // after a failed wait: every MMA issued has completed
     uint32_t tmem_base;
 };
+static_assert(8 * kOutWarp <= kQTile, "the output rows of eight warps fit into a Q tile");
 
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar_addr, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_addr), "r"(bytes) : "memory");
-}
-// Contiguous global -> shared copy of `bytes` (multiple of 16, both addresses 16-byte aligned),
-// completing on the mbarrier.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar_addr) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar_addr) : "memory");
-}
-// Barrier of the 256 softmax threads of a tile.
-__device__ __forceinline__ void tile_sync(int x) { asm volatile("bar.sync %0, 256;" ::"r"(9 + x) : "memory"); }
-
-// Which (sequence, tile or pair of tiles) the `index`-th unit of work is; sequences from the last to the first
+// Which (sequence, tile) the `index`-th unit of work is; sequences from the last to the first
 // (schedulers put running requests with one token before prompts), their units from the last (longest) to the first, so
-// that long units start early; `per` tokens a unit (217 -> 195 us with two tiles per CTA for 30 single tokens and 2 prompts).  Every warp finds it by itself.  False when there are fewer units.
+// that long units start early; `per` tokens a unit.  Every warp finds it by itself.  False when there are fewer units.
 __device__ __forceinline__ bool find_unit(const PrefillParams& p, int per, int index, int& seq, int& unit) {
     const int lane = threadIdx.x & 31;
     if (p.cu_seqlens_q == nullptr) {
@@ -811,38 +1123,89 @@ __device__ __forceinline__ bool find_unit(const PrefillParams& p, int per, int i
     return false;
 }
 
+// The units behind the first `whole` (in the order of find_unit, every KV head on its own) may be divided by keys into parts of
+// kMinPart tiles or more.  Every part is a CTA of its own, which leaves unnormalised outputs [column][row], reference maxima
+// and row sums, and prefill_merge_kernel puts them together.
+constexpr int kMinPart = 8;
+constexpr int kPartFloats = kPfRows * kHeadDim + 2 * kPfRows;
+
+struct AttnWork {
+    int seq, kvh, first_tok, q_begin, q_len, kv_len;
+    int part, parts;
+    int t0, tiles;                    // key tiles t0 .. t0 + tiles - 1
+    int64_t slot;                     // number of the unit's first partial result
+};
+// The work of CTA `index`: whole units, then the first parts of the others, their second parts and so on.  DIVIDED false: no
+// unit is divided (registers and set-up of a short CTA: 442 -> 433 us for 8 x 2048 tokens, 20.5 -> 19.5 for 300).
+template <bool DIVIDED>
+__device__ __forceinline__ bool find_work(const PrefillParams& p, int per, int index, AttnWork& w) {
+    int unit, flat = index;
+    w.part = 0;
+    if constexpr (DIVIDED) {
+        const int tail = p.units - p.whole;
+        if (index >= p.units) w.part = (index - p.whole) / tail;
+        flat -= w.part * tail;
+    }
+    w.kvh = flat % p.H;
+    if (!find_unit(p, per, flat / p.H, w.seq, unit)) return false;
+    w.q_begin = p.cu_seqlens_q ? __ldg(p.cu_seqlens_q + w.seq) : 0;
+    w.q_len = (p.cu_seqlens_q ? __ldg(p.cu_seqlens_q + w.seq + 1) : p.num_tokens) - w.q_begin;
+    w.kv_len = max(__ldg(p.seq_lens + w.seq), 0);
+    w.first_tok = unit * per;
+    w.t0 = 0;
+    w.tiles = key_tiles(p, w.q_len, w.kv_len, w.first_tok, per);
+    w.parts = 1;
+    if (DIVIDED && flat >= p.whole) {
+        w.slot = static_cast<int64_t>(flat - p.whole) * p.max_parts;
+        w.parts = max(1, min(p.max_parts, w.tiles / kMinPart));
+        if (w.part >= w.parts) return false;
+        const int n = w.tiles;
+        w.t0 = w.part * n / w.parts;
+        w.tiles = (w.part + 1) * n / w.parts - w.t0;
+    }
+    return true;
+}
+
+constexpr uint32_t kIdescS = (2u << 4) | (1u << 7) | (1u << 10) | ((kPfKeys >> 3) << 17) | ((kPfRows >> 4) << 24);
+template <typename T>
+constexpr uint32_t kIdescO = (1u << 4) | (TcFormat<T>::kFmt << 7) | (TcFormat<T>::kFmt << 10) | (1u << 16) |
+                             ((kHeadDim >> 3) << 17) | ((kPfRows >> 4) << 24);
+// S = Q K^T and O (+)= P V of one tile; s_cols, o_cols: its TMEM columns, q_addr, k_addr, v_addr: operands in shared memory
+__device__ __forceinline__ void issue_scores(uint32_t s_cols, uint32_t q_addr, uint32_t k_addr) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+        tc_mma_i8(s_cols, smem_desc(q_addr + 2 * kQCore * s, kQCore, kQGroup), smem_desc(k_addr + 256 * s, 128, 1024), kIdescS, s > 0 ? 1u : 0u);
+}
+template <typename T>
+__device__ __forceinline__ void issue_values(uint32_t s_cols, uint32_t o_cols, uint32_t v_addr, bool accumulate) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        tc_mma_f16_ta(o_cols, s_cols + 64u * (c >> 2) + 8u * (c & 3), smem_desc(v_addr + 4096 * c, 2048, 128), kIdescO<T>,
+                      c > 0 ? 1u : static_cast<uint32_t>(accumulate));
+}
+
 template <int TILES> constexpr int kAttnThreads = 256 * TILES + 64;
 
-template <typename T, int TILES>
+template <typename T, int TILES, bool DIVIDED>
 __global__ void __launch_bounds__(kAttnThreads<TILES>, TILES == 2 ? 1 : 2)
 prefill_attn_kernel(const PrefillParams p) {
+    static_assert(TILES == 1 || !DIVIDED);
     constexpr int kSoftmaxWarps = 8 * TILES, kThreads = kAttnThreads<TILES>;
     constexpr uint32_t kCols = 256u * TILES, kOutCols = 128u * TILES;       // O_x behind the sums
     extern __shared__ __align__(128) uint8_t smem_raw[];
     AttnSmem<TILES>& sm = *reinterpret_cast<AttnSmem<TILES>*>(smem_raw);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int kvh = blockIdx.x % p.H;
-    int seq, unit;
-    if (!find_unit(p, p.tokens_per_tile * TILES, blockIdx.x / p.H, seq, unit)) {
+    AttnWork w;
+    if (!find_work<DIVIDED>(p, p.tokens_per_tile * TILES, blockIdx.x, w)) {
         // The next launch waits for the end of this grid and takes everything older as done: a grid whose CTAs all
         // leave here (no sequence has a query) must not end before the records of its stage launch are written.
-        grid_dependency_wait();
+        if (w.part == 0) grid_dependency_wait();
         return;
     }
-    const int q_begin = p.cu_seqlens_q ? __ldg(p.cu_seqlens_q + seq) : 0;
-    const int q_end = p.cu_seqlens_q ? __ldg(p.cu_seqlens_q + seq + 1) : p.num_tokens;
-    const int q_len = q_end - q_begin;
-    const int kv_len = max(__ldg(p.seq_lens + seq), 0);
-    // K/V tiles that each of the two tiles needs: up to its last row's position, never past the staged records
-    auto tiles_of = [&](int x) {
-        const int first = (unit * TILES + x) * p.tokens_per_tile;
-        const int last = min(q_len, first + p.tokens_per_tile) - 1;
-        const int last_pos = min(kv_len - q_len + last, kv_len - 1);
-        const bool any = x < TILES && first < q_len && last_pos >= 0;
-        return any ? min(last_pos / kPfKeys + 1, p.stage_tiles_per_seq) : 0;
-    };
-    const int n0 = tiles_of(0), n1 = tiles_of(1), n_all = max(n0, n1);
+    // key tiles of the two tiles (of one, w.tiles)
+    const int n0 = TILES == 1 ? w.tiles : key_tiles(p, w.q_len, w.kv_len, w.first_tok, p.tokens_per_tile);
+    const int n1 = TILES == 1 ? 0 : key_tiles(p, w.q_len, w.kv_len, w.first_tok + p.tokens_per_tile, p.tokens_per_tile), n_all = max(n0, n1);
 
     // ---- set-up: barriers, TMEM, rotation blocks ----
     if (tid == 0) {
@@ -853,15 +1216,15 @@ prefill_attn_kernel(const PrefillParams p) {
             mbar_init(&sm.s_ready[x], 1);
             mbar_init(&sm.p_ready[x], 8);
         }
-        mbar_init(&sm.k_full, 1);
-        mbar_init(&sm.v_full, 1);
-        mbar_init(&sm.scale_full[0], 1);
-        mbar_init(&sm.scale_full[1], 1);
 #pragma unroll
         for (int s = 0; s < kAttnStages; ++s) {
             mbar_init(&sm.full[s], 1);
             mbar_init(&sm.empty[s], 1);
         }
+        mbar_init(&sm.k_full, 1);
+        mbar_init(&sm.v_full, 1);
+        mbar_init(&sm.scale_full[0], 1);
+        mbar_init(&sm.scale_full[1], 1);
         fence_async_proxy();
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -875,12 +1238,13 @@ prefill_attn_kernel(const PrefillParams p) {
     tc_fence_after();
     const uint32_t base = TILES == 2 ? 0u : sm.tmem_base;     // all columns, or half of them
     bool failed = false;
+    if (DIVIDED && tid == 0) grid_launch_dependents();         // the merge launch, which waits for this grid's end
 
     if (warp == kSoftmaxWarps + 1) {
         // ---- loads: record of 128 keys = [K codes 16 KB | V values 32 KB | key scales 512 B] ----
         if (lane == 0) {
             grid_dependency_wait();                           // the records
-            const uint8_t* rec = p.stage + (static_cast<int64_t>(seq) * p.stage_tiles_per_seq * p.H + kvh) * kStageRecord;
+            const uint8_t* rec = p.stage + ((static_cast<int64_t>(w.seq) * p.stage_tiles_per_seq + w.t0) * p.H + w.kvh) * kStageRecord;
             const int64_t record_stride = static_cast<int64_t>(p.H) * kStageRecord;
             if constexpr (TILES == 1) {
                 int k_next = 0, v_next = 0;
@@ -900,13 +1264,13 @@ prefill_attn_kernel(const PrefillParams p) {
                     ++v_next;
                 };
                 if (n0 > 0) { load_k(); load_v(); }
-                for (int j = 0; j < n0; ++j) {                // S(j) complete: K(j) and, before it, V(j - 1) have been read
+                for (int j = 0; j < n0; ++j) {                     // S(j) complete: K(j) and, before it, V(j - 1) have been read
                     failed = !mbar_wait(&sm.s_ready[0], static_cast<uint32_t>(j) & 1u);
                     if (failed) break;
                     if (j > 0) load_v();
                     if (j + 1 < n0) load_k();
                 }
-                if (n0 > 0) {                                 // copies in flight land before the CTA ends
+                if (n0 > 0) {                                      // copies in flight land before the CTA ends
                     mbar_wait(&sm.k_full, static_cast<uint32_t>(k_next - 1) & 1u);
                     mbar_wait(&sm.v_full, static_cast<uint32_t>(v_next - 1) & 1u);
                     mbar_wait(&sm.scale_full[(k_next - 1) & 1], static_cast<uint32_t>((k_next - 1) / 2) & 1u);
@@ -935,22 +1299,9 @@ prefill_attn_kernel(const PrefillParams p) {
         // TMEM base, 0 as all columns are allocated): an MMA blocks its issuing thread while the tensor core works on the
         // one before, so whatever the thread computes between two of them is added to the tensor core's time.
         if (lane == 0 && n_all > 0) {
-            constexpr uint32_t idesc_s = (2u << 4) | (1u << 7) | (1u << 10) | ((kPfKeys >> 3) << 17) | ((kPfRows >> 4) << 24);
-            constexpr uint32_t idesc_o = (1u << 4) | (TcFormat<T>::kFmt << 7) | (TcFormat<T>::kFmt << 10) | (1u << 16) |
-                                         ((kHeadDim >> 3) << 17) | ((kPfRows >> 4) << 24);
-            auto scores = [&](int x, int stage) {
-                const uint32_t q_addr = smem_u32(sm.q[x]), k_addr = smem_u32(sm.k[stage]);
-#pragma unroll
-                for (int s = 0; s < 4; ++s)
-                    tc_mma_i8(base + 128u * x, smem_desc(q_addr + 2 * kQCore * s, kQCore, kQGroup), smem_desc(k_addr + 256 * s, 128, 1024),
-                              idesc_s, s > 0 ? 1u : 0u);
-            };
+            auto scores = [&](int x, int stage) { issue_scores(base + 128u * x, smem_u32(sm.q[x]), smem_u32(sm.k[stage])); };
             auto values = [&](int x, int stage, int j) {
-                const uint32_t v_addr = smem_u32(sm.v[stage]);
-#pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    tc_mma_f16_ta(base + kOutCols + 128u * x, base + 128u * x + 64u * (c >> 2) + 8u * (c & 3),
-                                  smem_desc(v_addr + 4096 * c, 2048, 128), idesc_o, c > 0 ? 1u : static_cast<uint32_t>(j > 0));
+                issue_values<T>(base + 128u * x, base + kOutCols + 128u * x, smem_u32(sm.v[stage]), j > 0);
             };
             failed |= !mbar_wait(&sm.q_ready, 0);
             if constexpr (TILES == 1) {
@@ -1009,128 +1360,31 @@ prefill_attn_kernel(const PrefillParams p) {
         __syncwarp();
     } else {
         // ---- softmax: tile x, row = thread of its warp group, half of the tile's keys ----
-        const int x = warp >> 3, half = (warp >> 2) & 1, row = tid & (kPfRows - 1);
-        const int pair_id = 1 + 4 * x + (warp & 3);           // named barrier of the two warps with the same rows
-        const int n = x == 0 ? n0 : n1;
+        const int x = TILES == 1 ? 0 : warp >> 3, half = (warp >> 2) & 1, row = tid & (kPfRows - 1);
+        const int n = x == 0 ? n0 : n1, first_tok = w.first_tok + x * p.tokens_per_tile;
         const uint32_t lanes = (static_cast<uint32_t>((warp & 3) * 32) << 16) + base + 128u * x;
-        const uint32_t s_cols = lanes + 64u * half, o_cols = lanes + kOutCols + 64u * half;
-        float* const xch = sm.xch[x][half] + row;
-        const float* const xch_other = sm.xch[x][half ^ 1] + row;
-        const int first_tok = (unit * TILES + x) * p.tokens_per_tile;
-        // Q and the output are handled by whole rows: a warp has rows row0 .. row0 + 15, lane i < 16 knows where row
-        // row0 + i is (-1: no such row)
         const int row0 = 16 * (warp & 7);
-        auto row_offset = [&](int64_t tok_stride, int64_t head_stride) -> long long {
-            const int r = row0 + (lane & 15), tl = r / p.G, tk = first_tok + tl;
-            if (tl >= p.tokens_per_tile || tk >= q_len) return -1;
-            return (q_begin + tk) * tok_stride + static_cast<int64_t>(kvh * p.G + r % p.G) * head_stride;
-        };
-
-        // Q: rotate, round, quantise the rows to int8.  Lane L has head-dims 4L .. 4L + 3 (one rotation block, in
-        // registers), so that loads are contiguous.  Bound by latency, so eight rows are in flight while eight are converted.
-        {
-            constexpr int kRows = 8;
-            f2 rot[4][2];                                     // [in][outs 0, 1 | outs 2, 3]
-            {
-                float r[4][4];
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) *reinterpret_cast<float4*>(r[jj]) = *reinterpret_cast<const float4*>(&sm.rot[lane * 16 + 4 * jj]);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) { rot[k][0] = pk(r[0][k], r[1][k]); rot[k][1] = pk(r[2][k], r[3][k]); }
-            }
-            const long long at_row = row_offset(p.q_stride_tok, p.q_stride_head);
-            uint2 next[kRows];
-            auto fetch = [&](int i0) {
-#pragma unroll
-                for (int i = 0; i < kRows; ++i) {
-                    const long long at = __shfl_sync(0xffffffffu, at_row, i0 + i);
-                    next[i] = at >= 0 ? __ldg(reinterpret_cast<const uint2*>(static_cast<const T*>(p.q) + at + 4 * lane)) : make_uint2(0u, 0u);
-                }
-            };
-            // Adding 1.5 * 2^23 rounds to the nearest integer, in the low bits.  Scalar operations: the assembler contracts a
-            // packed product and sum, and a product that is a tie after its own rounding would go the other way.
-            auto code = [](float v, float scale) { return __float_as_uint(__fadd_rn(__fmul_rn(v, scale), 12582912.0f)); };
-            auto rotate = [&](uint2 v) {
-                const float2 a = pf_unpack<T>(v.x), b = pf_unpack<T>(v.y);
-                const float in[4] = {a.x, a.y, b.x, b.y};
-                f2 y01 = mul2(pk(in[0], in[0]), rot[0][0]), y23 = mul2(pk(in[0], in[0]), rot[0][1]);
-#pragma unroll
-                for (int k = 1; k < 4; ++k) { y01 = fma2(pk(in[k], in[k]), rot[k][0], y01); y23 = fma2(pk(in[k], in[k]), rot[k][1], y23); }
-                float y[4];
-                upk(y01, y[0], y[1]);
-                upk(y23, y[2], y[3]);
-                return make_uint2(pf_pack<T>(y[0], y[1]), pf_pack<T>(y[2], y[3]));
-            };
-            auto largest = [](uint2 v) {
-                const float2 c = pf_unpack<T>(v.x), d = pf_unpack<T>(v.y);
-                return fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y)));
-            };
-            auto store_codes = [&](uint2 v, float inv_row, int r) {
-                const float2 a = pf_unpack<T>(v.x), b = pf_unpack<T>(v.y);
-                // position d holds head-dim d ^ 1
-                const uint32_t w = prmt(prmt(code(a.y, inv_row), code(a.x, inv_row), 0x0040), prmt(code(b.y, inv_row), code(b.x, inv_row), 0x0040), 0x5410);
-                *reinterpret_cast<uint32_t*>(&sm.q[x][(r >> 3) * kQGroup + (lane >> 2) * kQCore + (r & 7) * 16 + 4 * (lane & 3)]) = w;
-            };
-            bool nan = false;                                 // one of the rows that lane i < 8 keeps the maximum of
-            if (n > 0) {
-                fetch(0);
-#pragma unroll 1
-                for (int i0 = 0; i0 < 16; i0 += kRows) {
-                    uint2 raw[kRows];
-#pragma unroll
-                    for (int i = 0; i < kRows; ++i) raw[i] = next[i];
-                    if (i0 + kRows < 16) fetch(i0 + kRows);
-                    float mx = 0.0f;                          // lane i < 8: largest |value| of row i0 + i
-#pragma unroll
-                    for (int i = 0; i < kRows; ++i) {
-                        raw[i] = rotate(raw[i]);
-                        const uint32_t m_row = __reduce_max_sync(0xffffffffu, __float_as_uint(largest(raw[i])));   // non-negative floats order as integers
-                        if (lane == i) mx = __uint_as_float(m_row);
-                    }
-                    nan |= mx != mx;
-                    const bool ok = mx > 0.0f && mx <= 3.0e38f;
-                    const float inv = ok ? __fdiv_rn(127.0f, mx) : 0.0f;
-                    if (lane < kRows) sm.q_scale[x][row0 + i0 + lane] = ok ? __fdiv_rn(mx, 127.0f) : 0.0f;
-#pragma unroll
-                    for (int i = 0; i < kRows; ++i) store_codes(raw[i], __shfl_sync(0xffffffffu, inv, i), row0 + i0 + i);
-                }
-            }
-            // A NaN element makes its whole rotation block NaN, and a NaN is larger than infinity as an integer.  Such a block
-            // counts as zero: its codes are 0 and the row's scale comes from the others.  (A block with infinities has an
-            // infinite maximum, and its row the scale 0.)  The rows are done again, one by one.  What the look at them takes, of
-            // the call for 8 x 2048 tokens: 2 % at every row, 0.6 % per eight rows before their codes, 0.2 % here.
-            if (__any_sync(0xffffffffu, nan)) {
-#pragma unroll 1
-                for (int i = 0; i < 16; ++i) {
-                    const long long at = __shfl_sync(0xffffffffu, at_row, i);
-                    uint2 v = at >= 0 ? __ldg(reinterpret_cast<const uint2*>(static_cast<const T*>(p.q) + at + 4 * lane)) : make_uint2(0u, 0u);
-                    v = rotate(v);
-                    float m = largest(v);
-                    if (m != m) { m = 0.0f; v = make_uint2(0u, 0u); }
-                    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-                    const bool ok = m > 0.0f && m <= 3.0e38f;
-                    if (lane == 0) sm.q_scale[x][row0 + i] = ok ? __fdiv_rn(m, 127.0f) : 0.0f;
-                    store_codes(v, ok ? __fdiv_rn(127.0f, m) : 0.0f, row0 + i);
-                }
-            }
+        if (n > 0) {
+            const long long first = (w.q_begin + first_tok) * p.q_stride_tok + static_cast<int64_t>(w.kvh * p.G) * p.q_stride_head;
+            const int tokens = min(p.tokens_per_tile, w.q_len - first_tok);
+            if (row0 < tokens * p.G) prepare_queries<T>(p, sm.rot, sm.q[x], sm.q_scale[x], row0, first, tokens);
+            else if (lane < 16) sm.q_scale[x][row0 + lane] = 0.0f;              // (whatever is in Q)
         }
         fence_async_proxy();                                  // the Q tile is read by the tensor core
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.q_ready);
-        tile_sync(x);                                       // every row's scale is there
-        const float row_factor = n > 0 ? sm.q_scale[x][row] * p.qk_scale : 0.0f;
-        // Position of the row's token in its sequence.  Rows without a token (zero queries, never stored) see every key: as
-        // rows that see none they would send their whole warp through the masked path at every tile (with 7 heads a tile
-        // has 126 rows, with a single query token 7: 225 -> 217 us for the batch of 28 heads).
-        int pos;
+        tile_any(x, false);                                     // every row's scale is there
+        SoftmaxRow s{lanes + 64u * half, lanes + kOutCols + 64u * half, &sm.xch[x][half][row], &sm.xch[x][half ^ 1][row], 1 + 4 * x + (warp & 3),
+                     n > 0 ? sm.q_scale[x][row] * p.qk_scale : 0.0f, -INFINITY, 0.0f};
+        // Position of the row's token in its sequence.  Rows without a token (never stored) see every key: as rows that see none
+        // they would send their whole warp through the masked path at every tile (with 7 heads a tile has 126 rows, with a
+        // single query token 7: 225 -> 217 us for the batch of 28 heads).
+        int limit;                                            // the row sees this half's keys 0 .. limit of the tile
         {
             const int tl = row / p.G, tk = first_tok + tl;
-            pos = tl < p.tokens_per_tile && tk < q_len ? kv_len - q_len + tk : (1 << 30);
+            limit = (tl < p.tokens_per_tile && tk < w.q_len ? w.kv_len - w.q_len + tk : (1 << 30)) - (w.t0 * kPfKeys + 64 * half);
         }
-
-        const f2 factor2 = pk(row_factor, row_factor), unbias2 = pk(-12582912.0f, -12582912.0f);
-        float m_run = -INFINITY, l_run = 0.0f;                // l_run: this half of the keys
-        for (int j = 0; j < n; ++j) {
+        for (int j = 0; j < n; ++j, limit -= kPfKeys) {
             // After an expired wait the warp keeps its step (its partner meets it at the named barrier) without waiting.
             const int stage = TILES == 2 ? j % kAttnStages : j & 1;
             if (!failed) failed = !mbar_wait(&sm.s_ready[x], static_cast<uint32_t>(j) & 1u);
@@ -1140,175 +1394,42 @@ prefill_attn_kernel(const PrefillParams p) {
             tc_fence_after();
             // S(j) is complete, so PV(j - 1) is: the later tile of the two frees the record that PV used up
             if (TILES == 2 && j > 0 && tid == (n1 > 0 ? 256 : 0)) mbar_arrive(&sm.empty[(j - 1) % kAttnStages]);
-            const float* const k_scale = sm.k_scale[stage] + 64 * half;
-            const int limit = pos - (j * kPfKeys + 64 * half);    // the row sees keys 0 .. limit of this half tile
-            const bool unmasked = __all_sync(0xffffffffu, limit >= 63);
-
-            // scaled sums of four keys, in pairs: (float)S * key scale
-            auto scaled = [&](const uint32_t* r, int key, f2& a, f2& b) {
-                const float4 ks = *reinterpret_cast<const float4*>(&k_scale[key]);
-                // int -> float: |S| < 2^22, so adding it to the bits of 1.5 * 2^23 gives 1.5 * 2^23 + S exactly
-                const f2 r01 = pk(__uint_as_float(r[0] + 0x4B400000u), __uint_as_float(r[1] + 0x4B400000u));
-                const f2 r23 = pk(__uint_as_float(r[2] + 0x4B400000u), __uint_as_float(r[3] + 0x4B400000u));
-                a = mul2(add2(r01, unbias2), pk(ks.x, ks.y));
-                b = mul2(add2(r23, unbias2), pk(ks.z, ks.w));
-            };
-            // the row's maximum over the tile becomes the reference if it exceeds it by 2^8 or more
-            auto move_reference = [&]() {
-                float m_half = -INFINITY;
-#pragma unroll 1
-                for (int ch = 0; ch < 4; ++ch) {
-                    uint32_t r[16];
-                    tmem_ld16_nowait(s_cols + 16 * ch, r);
-                    tmem_wait_ld();
-                    tmem_ld16_landed(r);
-#pragma unroll
-                    for (int c4 = 0; c4 < 4; ++c4) {
-                        f2 a, b;
-                        scaled(&r[4 * c4], 16 * ch + 4 * c4, a, b);
-                        float v[4];
-                        upk(a, v[0], v[1]);
-                        upk(b, v[2], v[3]);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            if (16 * ch + 4 * c4 + e <= limit) m_half = fmaxf(m_half, v[e]);
-                    }
-                }
-                *xch = m_half;
-                pair_any(pair_id, false);
-                const float m_tile = fmaxf(m_half, *xch_other) * row_factor;                // row_factor >= 0
-                const bool grew = m_tile > m_run + 8.0f;
-                const float m_new = grew ? m_tile : m_run;
-                const float alpha = grew ? (m_run == -INFINITY ? 0.0f : pf_ex2(m_run - m_new)) : 1.0f;
-                if (j > 0 && __any_sync(0xffffffffu, grew)) { // O_x is at rest: the commit behind S_x(j) covered PV_x(j - 1)
-#pragma unroll 1
-                    for (int ch = 0; ch < 4; ++ch) {
-                        uint32_t r[16];
-                        tmem_ld16_nowait(o_cols + 16 * ch, r);
-                        tmem_wait_ld();
-                        tmem_ld16_landed(r);
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * alpha);
-                        tmem_st16_nowait(o_cols + 16 * ch, r);
-                    }
-                    tmem_wait_st();
-                }
-                l_run *= alpha;
-                m_run = m_new;
-                pair_any(pair_id, false);                     // xch has been read
-            };
-            uint32_t prob[32];                                // probabilities of the half row as T pairs
-            float half_sum;
-            auto exponentiate = [&](auto masked_tag) {
-                constexpr bool kMasked = decltype(masked_tag)::value;
-                const float m_use = (m_run == -INFINITY) ? 0.0f : m_run;
-                const f2 minus_m = pk(-m_use, -m_use);
-                f2 sum_a = pk(0.0f, 0.0f), sum_b = sum_a;
-                uint32_t buf[2][8];
-                tmem_ld8_nowait(s_cols, buf[0]);
-#pragma unroll
-                for (int it = 0; it < 8; ++it) {
-                    tmem_wait_ld();
-                    tmem_ld8_landed(buf[it & 1]);
-                    if (it < 7) tmem_ld8_nowait(s_cols + 8 * (it + 1), buf[(it + 1) & 1]);
-#pragma unroll
-                    for (int c4 = 0; c4 < 2; ++c4) {
-                        f2 a, b;
-                        scaled(&buf[it & 1][4 * c4], 8 * it + 4 * c4, a, b);
-                        float e[4];
-                        upk(fma2(a, factor2, minus_m), e[0], e[1]);
-                        upk(fma2(b, factor2, minus_m), e[2], e[3]);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            e[i] = pf_ex2(e[i]);
-                            if (kMasked && 8 * it + 4 * c4 + i > limit) e[i] = 0.0f;
-                        }
-                        sum_a = add2(sum_a, pk(e[0], e[1]));
-                        sum_b = add2(sum_b, pk(e[2], e[3]));
-                        prob[4 * it + 2 * c4] = pf_pack<T>(e[0], e[1]);
-                        prob[4 * it + 2 * c4 + 1] = pf_pack<T>(e[2], e[3]);
-                    }
-                }
-                float lo, hi;
-                upk(add2(sum_a, sum_b), lo, hi);
-                half_sum = lo + hi;
-            };
-            if (j == 0) move_reference();
-#pragma unroll 1
-            for (int attempt = 0;; ++attempt) {
-                if (unmasked) exponentiate(std::false_type{});
-                else exponentiate(std::true_type{});
-                // both threads of every row take the same decision
-                const bool outgrown = !(half_sum <= 16384.0f) || (m_run == -INFINITY && half_sum > 0.0f);
-                if (!pair_any(pair_id, outgrown) || attempt == 1) break;
-                move_reference();
-            }
-            l_run += half_sum;
-            tmem_st32_nowait(s_cols, prob);                   // over the half row's own sums
-            tmem_wait_st();
+            softmax_tile<T>(s, sm.k_scale[stage] + 64 * half, limit, j == 0);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.p_ready[x]);
         }
-
-        // ---- epilogue: O / l, round, rotate by R, round, store ----
-        // The rows go through shared memory (the Q tile's space, half of the head-dims at a time), so that a warp stores
-        // whole half rows: 16 lanes per row, one rotation block each.
         if (n > 0) {
             if (!failed) failed = !mbar_wait(&sm.s_ready[x], static_cast<uint32_t>(n) & 1u);     // the last PV
             failed = __any_sync(0xffffffffu, failed);
             tc_fence_after();
-            *xch = l_run;
-            pair_any(pair_id, false);
-            l_run += *xch_other;
+            *s.xch = s.l_run;
+            pair_any(s.pair_id, false);
+            s.l_run += *s.xch_other;
         }
-        const float inv_l = l_run > 0.0f ? 1.0f / l_run : 0.0f;
-        const long long mine = failed ? -1 : row_offset(p.o_stride_tok, p.o_stride_head);
-        uint8_t* const tile_rows = sm.q[x];
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-            if (half == h) {
-#pragma unroll 1
-                for (int ch = 0; ch < 2; ++ch) {
-                    uint32_t r[32];
-                    if (n > 0) {
-                        tmem_ld32(o_cols + 32 * ch, r);
-                    } else {                                  // rows that see no key are zero
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) r[i] = 0u;
-                    }
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {             // column d of O holds head-dim d ^ 1
-                        uint32_t w[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            w[i] = pf_pack<T>(__uint_as_float(r[8 * c + 2 * i + 1]) * inv_l, __uint_as_float(r[8 * c + 2 * i]) * inv_l);
-                        *reinterpret_cast<uint4*>(tile_rows + row * kQCore + 64 * ch + 16 * c) = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                }
+        failed = tile_any(x, failed);                           // (every warp's rows have been read)
+        if (DIVIDED && w.parts > 1) {
+            float* const dst = p.parts + (w.slot + w.part) * kPartFloats + row;
+            const bool there = row < min(p.tokens_per_tile, w.q_len - first_tok) * p.G;
+            if (half == 0 && there) {
+                dst[kPfRows * kHeadDim] = s.m_run;
+                dst[kPfRows * kHeadDim + kPfRows] = s.l_run;
             }
-            tile_sync(x);
-            const float* rb = &sm.rot[(16 * h + (lane & 15)) * 16];              // rb[k * 4 + jj] = R[4g+k][4g+jj]
-            float4 rr[4];
+#pragma unroll 1
+            for (int ch = 0; ch < 2; ++ch) {
+                uint32_t r[32];
+                tmem_ld32(s.o_cols + 32 * ch, r);
+                tmem_ld32_landed(r);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) rr[k] = *reinterpret_cast<const float4*>(rb + 4 * k);
-#pragma unroll 2
-            for (int i = 0; i < 8; ++i) {
-                const int r = row0 + 2 * i + (lane >> 4);
-                const long long at = __shfl_sync(0xffffffffu, mine, 2 * i + (lane >> 4));
-                const uint2 o4 = *reinterpret_cast<const uint2*>(tile_rows + r * kQCore + 8 * (lane & 15));
-                const float2 o01 = pf_unpack<T>(o4.x), o23 = pf_unpack<T>(o4.y);
-                float y[4] = {__fmul_rn(o01.x, rr[0].x), __fmul_rn(o01.x, rr[0].y), __fmul_rn(o01.x, rr[0].z), __fmul_rn(o01.x, rr[0].w)};
-                const float o[3] = {o01.y, o23.x, o23.y};
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    y[0] = __fmaf_rn(o[k], rr[k + 1].x, y[0]); y[1] = __fmaf_rn(o[k], rr[k + 1].y, y[1]);
-                    y[2] = __fmaf_rn(o[k], rr[k + 1].z, y[2]); y[3] = __fmaf_rn(o[k], rr[k + 1].w, y[3]);
-                }
-                if (at >= 0)
-                    *reinterpret_cast<uint2*>(static_cast<T*>(p.out) + at + 64 * h + 4 * (lane & 15)) = make_uint2(pf_pack<T>(y[0], y[1]), pf_pack<T>(y[2], y[3]));
+                for (int c = 0; c < 32; ++c)
+                    if (there) dst[(64 * half + 32 * ch + c) * kPfRows] = __uint_as_float(r[c]);
             }
-            tile_sync(x);
+        } else {
+            const int tl = row / p.G, tk = first_tok + tl;
+            const bool stored = !failed && tl < p.tokens_per_tile && tk < w.q_len;
+            const long long out_row = stored ? (w.q_begin + tk) * p.o_stride_tok + static_cast<int64_t>(w.kvh * p.G + row % p.G) * p.o_stride_head : -1;
+            store_rows<T>(p, s.o_cols, half, s.l_run > 0.0f ? 1.0f / s.l_run : 0.0f, n > 0, out_row, sm.rot,
+                          sm.q[x] + (warp & 7) * kOutWarp);
         }
     }
     if (failed && p.error_flag != nullptr) atomicExch(p.error_flag, 1);
@@ -1317,40 +1438,119 @@ prefill_attn_kernel(const PrefillParams p) {
     if (warp == kSoftmaxWarps) tmem_dealloc(sm.tmem_base, kCols);
 }
 
+// Puts the parts of a unit together.  CTA: 32 rows of a unit; lane = row, warp = 16 head-dims; parts are read by whole columns.
+constexpr int kMergeThreads = 256;
+template <typename T>
+__global__ void __launch_bounds__(kMergeThreads)
+prefill_merge_kernel(const PrefillParams p) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = 32 * blockIdx.y + lane;
+    grid_dependency_wait();
+    AttnWork w;
+    if (!find_work<true>(p, p.tokens_per_tile, p.whole + blockIdx.x, w) || w.parts < 2) return;
+    const int parts = w.parts, tl = row / p.G, tk = w.first_tok + tl;
+    if (tl >= p.tokens_per_tile || tk >= w.q_len) return;
+    const float* const first = p.parts + w.slot * kPartFloats + row;
+    float m = -INFINITY;
+    for (int i = 0; i < parts; ++i) m = fmaxf(m, first[i * kPartFloats + kPfRows * kHeadDim]);
+    float l = 0.0f, acc[16];
+#pragma unroll
+    for (int d = 0; d < 16; ++d) acc[d] = 0.0f;
+#pragma unroll 2
+    for (int i = 0; i < parts; ++i) {
+        const float* const part = first + i * kPartFloats;
+        const float m_part = part[kPfRows * kHeadDim];
+        const float weight = m_part == -INFINITY ? 0.0f : pf_ex2(m_part - m);        // (0: a part in which the row sees no key)
+        l += weight * part[kPfRows * kHeadDim + kPfRows];
+#pragma unroll
+        for (int d = 0; d < 16; ++d) acc[d] += weight * part[(16 * warp + d) * kPfRows];
+    }
+    const float inv_l = l > 0.0f ? 1.0f / l : 0.0f;
+    uint32_t out[8];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {                        // rotation block: head-dims 16 warp + 4b .. + 3
+        float o[4], y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] = pf_round<T>(acc[(4 * b + e) ^ 1] * inv_l);        // column d holds head-dim d ^ 1
+        const float* r = p.rotation + (16 * warp + 4 * b) * (kHeadDim + 1);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float4 rr = __ldg(reinterpret_cast<const float4*>(r + k * kHeadDim));
+            y[0] = k ? __fmaf_rn(o[k], rr.x, y[0]) : __fmul_rn(o[0], rr.x);
+            y[1] = k ? __fmaf_rn(o[k], rr.y, y[1]) : __fmul_rn(o[0], rr.y);
+            y[2] = k ? __fmaf_rn(o[k], rr.z, y[2]) : __fmul_rn(o[0], rr.z);
+            y[3] = k ? __fmaf_rn(o[k], rr.w, y[3]) : __fmul_rn(o[0], rr.w);
+        }
+        out[2 * b] = pf_pack<T>(y[0], y[1]);
+        out[2 * b + 1] = pf_pack<T>(y[2], y[3]);
+    }
+    T* const dst = static_cast<T*>(p.out) + (w.q_begin + tk) * p.o_stride_tok +
+                   static_cast<int64_t>(w.kvh * p.G + row % p.G) * p.o_stride_head + 16 * warp;
+    reinterpret_cast<uint4*>(dst)[0] = make_uint4(out[0], out[1], out[2], out[3]);
+    reinterpret_cast<uint4*>(dst)[1] = make_uint4(out[4], out[5], out[6], out[7]);
+}
+
 // ---- host side --------------------------------------------------------------------------------
+
+// Results of parts, behind the records; none where no context is long enough to be divided.
+static long long part_room(int key_tiles) { return key_tiles < 2 * kMinPart ? 0 : 6LL * sm_count(); }
+
+// How the attention of a batch is laid out: whether two tiles share a CTA, else which units are divided by keys and how finely:
+// those behind the last full wave of CTAs (two per SM), where all of them see long contexts; all units where there are fewer than
+// a wave.  `longest`: bound of the query tokens of a sequence, `units`, `pairs`: CTAs with one and with two tiles.
+//
+// Before and after, whole call in us: units without division against divided ones 16 tokens after 8000, 32 / 8 heads 123 / 49, 64 after
+// 16000 236 / 72, 4 x 64 after 16000 277 / 133, 512 after 30000 508 / 284; 12 single tokens after up to 6000 128 / 88.
+// One tile per CTA and two, contexts above 16384 tokens being where the second was taken before: 2048 tokens after 30000 990 (the last
+// wave divided) / 960 with the GPU at its power limit, 940 / 975 out of rest; 2048 after 18000 653 / 625.  So two tiles count 0.88 there.
+static bool two_tiles(PrefillParams& p, int longest, long long units, long long pairs) {
+    const int tiles = p.stage_tiles_per_seq;
+    const long long room = part_room(tiles), sms = sm_count(), slots = 2 * sms;
+    // time of `ctas` CTAs in key tiles: set-up and output are worth 6, and CTAs alone on their SMs take 0.7 of the time
+    auto waves = [&](long long ctas, double key_tiles) {
+        return (ctas <= sms ? 0.7 : 1.0) * ((ctas + slots - 1) / slots) * (key_tiles + 6.0);
+    };
+    const long long whole = units / slots * slots, tail = units - whole;
+    const int seen = whole == 0 ? tiles : (tiles * kPfKeys - longest) / kPfKeys;       // by the units behind `whole`, at least
+    p.units = static_cast<int>(units);
+    p.whole = p.units;
+    p.max_parts = 1;
+    double least = waves(tail, tiles);
+    for (int parts = 2; p.parts != nullptr && tail > 0 && parts <= seen / kMinPart && tail * parts <= room; ++parts) {
+        const double time = waves(tail * parts, static_cast<double>(seen) / parts) + 3.0;              // 3: the merge
+        if (time < (p.max_parts == 1 ? 0.97 * waves(tail, seen) : least)) { p.max_parts = parts; p.whole = static_cast<int>(whole); least = time; }
+    }
+    const bool two = tiles > 16384 / kPfKeys && whole > 0 && p.num_tokens > 1LL * p.num_seqs * p.tokens_per_tile &&
+                     0.88 * ((pairs + sms - 1) / sms) * (tiles + 6.0) < whole / slots * (tiles + 6.0) + least;
+    if (two) {
+        p.units = p.whole = static_cast<int>(pairs);
+        p.max_parts = 1;
+    }
+    return two;
+}
 
 template <typename T, int KB, int VB>
 static int launch_prefill(const PrefillParams& p, int m_tiles, int num_seqs, cudaStream_t st) {
     if (p.stage != nullptr) {
         dim3 sgrid(p.stage_tiles_per_seq, p.H, num_seqs);
         if (int e = launch_dependent("rq_prefill_int8 stage launch", prefill_stage_kernel<T, KB, VB>, sgrid, dim3(128), 0, st, p)) return e;
-        // Units of work: at most tokens / (tokens of a unit) + one partial unit per sequence, found by the CTAs
-        // themselves (a grid of longest sequence x sequences was mostly empty CTAs for batches of mixed lengths).
-        // One tile per CTA, two CTAs per SM, is the faster form for short contexts, as one CTA's queries and output run under
-        // the other's loop; two tiles per CTA read K/V half as often.  Both, in us (one / two): 300 tokens 20.5 / 24.6,
-        // 19 prompts of 34 to 283 67 / 77, 64 x 256 282 / 300, 16 x 1024 371 / 377, 8 x 2048 480 / 479, 4 x 4096 696 / 687; 2048 tokens
-        // after 2000 141 / 135, 8192 327 / 314, 12000 453 / 437, 18000 653 / 625, 30000 1042 / 999.  So for prompts alone the
-        // two cross near 2000 to 4000 keys, and the line at 16384 gives up 2 to 5 % between there and itself.  It stands there
-        // for the sake of batches that also have running requests of one token, where the form with fewer, longer units
-        // wins or loses with the last wave: after up to 6000, 28 heads, one prompt of 2048 with 12 of them 265 / 253, with 30 284 / 313,
-        // one of 512 with 60 231 / 256; 32 heads, 2048 with 12 300 / 328, with 30 420 / 410 (and 30 with 2 prompts of up to 1500 after
-        // 4000, 28 heads 205 / 197).  Behind the line one tile is kept where most sequences have no second one (4 x 64 after
-        // 16000 277 / 284) or there are too few tiles for every SM.
+        // Units of work: at most tokens / (tokens of a unit) + one partial unit per sequence, found by the CTAs themselves.
         auto units = [&](long long per) {
             const long long by_tokens = p.num_tokens / per + num_seqs;
             const long long by_longest = num_seqs * ((1LL * m_tiles * p.tokens_per_tile + per - 1) / per);
             return (by_tokens < by_longest ? by_tokens : by_longest) * p.H;
         };
-        auto attend = [&](auto tiles) {
-            constexpr int kTiles = decltype(tiles)::value;
-            const size_t smem = sizeof(AttnSmem<kTiles>);
-            if (int e = ensure_smem(prefill_attn_kernel<T, kTiles>, smem)) return e;
-            return launch_dependent("rq_prefill_int8 attention launch", prefill_attn_kernel<T, kTiles>,
-                                    dim3(static_cast<unsigned>(units(1LL * p.tokens_per_tile * kTiles))), dim3(kAttnThreads<kTiles>), smem, st, p);
+        PrefillParams q = p;
+        const bool two = two_tiles(q, m_tiles * p.tokens_per_tile, units(p.tokens_per_tile), units(2LL * p.tokens_per_tile));
+        const int divided = q.units - q.whole;
+        auto attend = [&](auto kernel, int threads, size_t smem) -> int {
+            if (int e = ensure_smem(kernel, smem)) return e;
+            return launch_dependent("rq_prefill_int8 attention launch", kernel, dim3(static_cast<unsigned>(q.units + divided * (q.max_parts - 1))),
+                                    dim3(threads), smem, st, q);
         };
-        const bool one = p.stage_tiles_per_seq <= 16384 / kPfKeys || units(p.tokens_per_tile) <= sm_count() ||
-                         p.num_tokens <= 1LL * num_seqs * p.tokens_per_tile;
-        return one ? attend(std::integral_constant<int, 1>{}) : attend(std::integral_constant<int, 2>{});
+        if (two) return attend(prefill_attn_kernel<T, 2, false>, kAttnThreads<2>, sizeof(AttnSmem<2>));
+        if (divided == 0) return attend(prefill_attn_kernel<T, 1, false>, kAttnThreads<1>, sizeof(AttnSmem<1>));
+        if (int e = attend(prefill_attn_kernel<T, 1, true>, kAttnThreads<1>, sizeof(AttnSmem<1>))) return e;
+        return launch_dependent("rq_prefill_int8 merge launch", prefill_merge_kernel<T>, dim3(static_cast<unsigned>(divided), 4), dim3(kMergeThreads), 0, st, q);
     }
     dim3 grid(m_tiles, p.H, num_seqs);
     const size_t smem = sizeof(PrefillSmem);
@@ -1367,10 +1567,13 @@ static int dispatch_prefill(const PrefillParams& p, int m_tiles, int num_seqs, i
     return launch_prefill<T, 4, 4>(p, m_tiles, num_seqs, st);
 }
 
-static size_t stage_bytes(int num_seqs, int num_kv_heads, int max_seq_len) {
+static size_t record_bytes(int num_seqs, int num_kv_heads, int max_seq_len) {
     if (num_seqs <= 0 || num_kv_heads <= 0 || max_seq_len <= 0) return 0;
     const size_t tiles = (static_cast<size_t>(max_seq_len) + kPfKeys - 1) / kPfKeys;
     return static_cast<size_t>(num_seqs) * tiles * num_kv_heads * kStageRecord;
+}
+static size_t part_bytes(int max_seq_len) {
+    return static_cast<size_t>(part_room((max_seq_len + kPfKeys - 1) / kPfKeys)) * sizeof(float) * kPartFloats;
 }
 
 }  // namespace rq
@@ -1378,7 +1581,8 @@ static size_t stage_bytes(int num_seqs, int num_kv_heads, int max_seq_len) {
 using namespace rq;
 
 extern "C" size_t rq_prefill_workspace_bytes(int num_seqs, int num_kv_heads, int max_seq_len) {
-    return stage_bytes(num_seqs, num_kv_heads, max_seq_len);
+    const size_t records = record_bytes(num_seqs, num_kv_heads, max_seq_len);
+    return records > 0 ? records + part_bytes(max_seq_len) : 0;
 }
 
 static int prefill_impl(const void* q, void* out, int dtype, int64_t q_stride_tok,
@@ -1439,7 +1643,7 @@ static int prefill_impl(const void* q, void* out, int dtype, int64_t q_stride_to
     if (workspace != nullptr) {
         if (max_seq_len <= 0)
             return fail(RQ_ERR_INVALID_ARG, "rq_prefill_int8_staged: max_seq_len must be positive");
-        const size_t need = stage_bytes(num_seqs, num_kv_heads, max_seq_len);
+        const size_t need = record_bytes(num_seqs, num_kv_heads, max_seq_len);
         if (workspace_bytes < need)
             return fail(RQ_ERR_WORKSPACE, "rq_prefill_int8_staged: workspace of %zu bytes needed, %zu given", need,
                         workspace_bytes);
@@ -1447,6 +1651,8 @@ static int prefill_impl(const void* q, void* out, int dtype, int64_t q_stride_to
             return fail(RQ_ERR_ALIGNMENT, "rq_prefill_int8_staged: workspace must be 128-byte aligned");
         p.stage = static_cast<uint8_t*>(workspace);
         p.stage_tiles_per_seq = (max_seq_len + kPfKeys - 1) / kPfKeys;
+        const size_t extra = part_bytes(max_seq_len);
+        if (extra > 0 && workspace_bytes >= need + extra) p.parts = reinterpret_cast<float*>(p.stage + need);
     }
     const int longest = (max_q_len > 0 && max_q_len < num_tokens) ? max_q_len : num_tokens;
     const int m_tiles = (longest + p.tokens_per_tile - 1) / p.tokens_per_tile;

@@ -1,0 +1,82 @@
+"""Prefill with units whose keys are divided between CTAs, against the fused kernel, which divides none.
+
+The two agree in the INT8 scores; a divided row has its probabilities rounded against another reference maximum in every part.
+With u the rounding unit of the type, the two results differ by four independent roundings of relative size u / sqrt(3)
+or less (probabilities and output, of either), 1.2 u together; the bound is 4 u.  Rows of units that are not divided
+agree bit for bit."""
+
+import pytest
+import torch
+
+import gpu_util
+from gpu_util import DEV
+from rotorquant_vllm import cuda as rq
+from rotorquant_vllm import synthetic as syn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,HQ,ctx,q,whole", [
+    (8, 32, [1920], [40], True),                                  # 15 key tiles: too few for two parts
+    (8, 32, [1921], [40], False),                                 # 16: two parts
+    (2, 8, [2049, 5, 0, 3000, 700], [33, 5, 0, 1, 700], False),   # whole units among the others, an empty sequence
+    (1, 4, [2300], [2300], False),                                # causal: units of 1 to 18 key tiles
+    (4, 28, [4097, 2100], [1, 37], False),                        # rows without a token
+    (2, 2, [6000], [129], False),                                 # one head a tile, one row in the second
+    (8, 8, [8000], [5000], False),                                # a full wave of whole units, the others divided
+])
+@pytest.mark.parametrize("dtype,u", [(torch.bfloat16, 2.0 ** -9), (torch.float16, 2.0 ** -12)])
+def test_divided_units(H, HQ, ctx, q, whole, dtype, u):
+    p = {k: v.to(DEV) for k, v in gpu_util.params("iso_fast", 3, 4).items()}
+    lens = torch.tensor(ctx, dtype=torch.int32)
+    table, blocks = syn.make_block_table(lens, 16, len(ctx))
+    slots = syn.slot_mapping_for(table, lens, 16).to(DEV)
+    key, value = (t.to(DEV) for t in syn.make_kv(int(lens.sum()), H, 128, dtype, 3))
+    cache = torch.full((blocks, 16, H * 256), 0xFF, dtype=torch.uint8, device=DEV)
+    rq.compress_and_store(key, value, cache, slots, p["R"], p["k_boundaries"], p["v_boundaries"])
+    queries = syn.make_queries(sum(q), HQ, 128, dtype, 4).to(DEV)
+    cu = torch.tensor([0] + q).cumsum(0).to(torch.int32).to(DEV)
+    args = (queries, cache, table.to(DEV), lens.to(DEV), p["k_centroids"], p["v_centroids"], p["R"], H, 128, 16)
+    flag = torch.zeros(1, dtype=torch.int32, device=DEV)
+    kw = {"cu_seqlens_q": cu, "max_q_len": max(q), "max_seq_len": max(ctx), "error_flag": flag}
+    got = rq.fused_paged_rq_int8_prefill(*args, staged=True, **kw)
+    again = rq.fused_paged_rq_int8_prefill(*args, staged=True, **kw)
+    want = rq.fused_paged_rq_int8_prefill(*args, staged=False, **kw)
+    assert int(flag.item()) == 0, "a bounded device-side wait expired"
+    assert torch.equal(got, again)
+    if whole:
+        assert torch.equal(got, want)
+        return
+    assert not torch.equal(got, want)                             # something was divided
+    for s in range(len(ctx)):
+        if q[s]:
+            a, b = got[cu[s]:cu[s + 1]].double(), want[cu[s]:cu[s + 1]].double()
+            assert (a - b).norm() <= 4 * u * b.norm(), (s, float((a - b).norm() / b.norm()))
+            if ctx[s] <= 15 * 128:
+                assert torch.equal(a, b)
+    # scratch that holds the records only: nothing is divided
+    records = len(ctx) * (-(-max(ctx) // 128)) * H * 49664
+    small = torch.empty(records, dtype=torch.uint8, device=DEV)
+    assert torch.equal(rq.fused_paged_rq_int8_prefill(*args, workspace=small, **kw), want)
+
+
+@pytest.mark.parametrize("H,HQ,q", [(32, 32, [257, 129, 300, 140, 260]), (4, 28, [700, 36, 19, 0, 640]), (8, 32, [65, 1300, 31])])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_two_tiles_per_cta(H, HQ, q, dtype):
+    """Enough tiles for every SM under a bound above 16384 tokens: pairs of tiles, none divided, the fused kernel's bits."""
+    ctx = [n + 60 * i for i, n in enumerate(q)]
+    p = {k: v.to(DEV) for k, v in gpu_util.params("planar", 4, 3).items()}
+    lens = torch.tensor(ctx, dtype=torch.int32)
+    table, blocks = syn.make_block_table(lens, 16, 1)
+    slots = syn.slot_mapping_for(table, lens, 16).to(DEV)
+    key, value = (t.to(DEV) for t in syn.make_kv(int(lens.sum()), H, 128, dtype, 5))
+    cache = torch.full((blocks, 16, H * 256), 0xFF, dtype=torch.uint8, device=DEV)
+    rq.compress_and_store(key, value, cache, slots, p["R"], p["k_boundaries"], p["v_boundaries"])
+    queries = syn.make_queries(sum(q), HQ, 128, dtype, 6).to(DEV)
+    cu = torch.tensor([0] + q).cumsum(0).to(torch.int32).to(DEV)
+    args = (queries, cache, table.to(DEV), lens.to(DEV), p["k_centroids"], p["v_centroids"], p["R"], H, 128, 16)
+    flag = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got, want = (rq.fused_paged_rq_int8_prefill(*args, cu_seqlens_q=cu, max_q_len=max(q), max_seq_len=16385, error_flag=flag, staged=s)
+                 for s in (True, False))
+    assert int(flag.item()) == 0, "a bounded device-side wait expired"
+    assert torch.equal(got, want)
