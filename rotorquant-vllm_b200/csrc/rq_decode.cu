@@ -89,6 +89,7 @@ struct DecodeParams {
     int layer_ctas;                        // CTAs per launch layer (SM count) when pieces are weighted, else 0
     int num_layers;
     int layer_w[kMaxLayers];               // piece weight of the CTAs of each launch layer
+    uint64_t inv_weight;                   // 2^64 / weight of all CTAs, rounded down
 };
 
 //
@@ -108,10 +109,12 @@ __host__ __device__ inline int64_t weight_cum(int64_t n, int layer_ctas, int num
     return acc;
 }
 // A batch with no more tiles than groups (short sequences under a wide block table) gives every group one tile.
+// The quotient is taken with the reciprocal, at most one below the true one and ascending with g: a 64-bit division is
+// several hundred clocks at the start of every CTA.
 __device__ __forceinline__ int64_t piece_begin(const DecodeParams& p, int64_t g, int64_t total, int J) {
     if (total <= p.groups) return g < total ? g : total;
-    return total * weight_cum(g * J, p.layer_ctas, p.num_layers, p.layer_w) /
-           weight_cum(static_cast<int64_t>(p.groups) * J, p.layer_ctas, p.num_layers, p.layer_w);
+    if (g >= p.groups) return total;
+    return static_cast<int64_t>(__umul64hi(total * weight_cum(g * J, p.layer_ctas, p.num_layers, p.layer_w), p.inv_weight));
 }
 
 // ---- small PTX wrappers ------------------------------------------------------
@@ -421,6 +424,13 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         if (hit) { seq = base + __ffs(hit) - 1; break; }
     }
 
+    // The sequence's length, and the tiles before it; the next one's length is fetched while this one is worked on.
+    int pre = 0, seq_len = 0;
+    if (seq < p.num_seqs) {
+        pre = prefix[seq];
+        seq_len = max(__ldg(p.seq_lens + seq), 0);
+    }
+
     float cmax_k = 0.0f;                      // largest |K centroid|
 #pragma unroll
     for (int i = 0; i < NK; ++i) cmax_k = fmaxf(cmax_k, fabsf(sm.cb[0][i]));
@@ -435,8 +445,13 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
 
 #pragma unroll 1
     while (x < x_end && seq < p.num_seqs) {
-        const int pre = prefix[seq], n_s = prefix[seq + 1] - pre;
-        if (n_s <= 0 || x >= static_cast<int64_t>(pre) + n_s) { ++seq; continue; }
+        const int n_s = (seq_len + kUTile - 1) / kUTile;
+        if (n_s == 0 || x >= static_cast<int64_t>(pre) + n_s) {
+            pre += n_s;
+            seq_len = ++seq < p.num_seqs ? max(__ldg(p.seq_lens + seq), 0) : 0;
+            continue;
+        }
+        const int next_len = seq + 1 < p.num_seqs ? max(__ldg(p.seq_lens + seq + 1), 0) : 0;
         const int t_begin = static_cast<int>(x - pre);
         const int64_t reach = t_begin + (x_end - x);
         const int t_end = reach < n_s ? static_cast<int>(reach) : n_s;
@@ -449,9 +464,25 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         const int kvh = item / p.head_groups, hg = item % p.head_groups;
         const int heads_here = min(kHeadsPerCta, p.G - hg * kHeadsPerCta);
         const int first_qh = kvh * p.G + hg * kHeadsPerCta;
-        const int seq_len = max(__ldg(p.seq_lens + seq), 0);
         const int32_t* bt_row = p.block_table + seq * p.bt_stride;
         const int last_blk = static_cast<int>(p.num_blocks) - 1;
+
+        // The queries and this lane's rotation block are requested before anything that waits for the block table, for all
+        // heads at once: 3500 -> 700 clocks between the staging request and the query tile.  Whole call, us, with the lengths
+        // fetched a sequence ahead and the piece boundaries without divisions: 64 x 4096 tokens 106.2 -> 104.9, 16 of 2048 to 32768 on
+        // one KV head 45.3 -> 43.6, 200 of 100 to 2000, 28 / 4 heads 79.2 -> 75.8, 48 of 500 to 9000, 64 / 8 heads 104.6 -> 102.5; 256 of
+        // 512 to 8192, 28 / 4 heads 287 either way.  (Staging the first tile of the next sequence under the last one of this: 293 and
+        // 106.9 for the last two, as every tile pays for the choice.)
+        uint2 q_raw[NH / 4];
+        float4 rot[4];
+#pragma unroll
+        for (int round = 0; round < NH / 4; ++round)
+            q_raw[round] = __ldg(reinterpret_cast<const uint2*>(
+                static_cast<const T*>(p.q) + seq * p.q_stride_seq +
+                static_cast<int64_t>(first_qh + min(4 * round + warp, heads_here - 1)) * p.q_stride_head + 4 * lane));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            rot[j] = __ldg(reinterpret_cast<const float4*>(p.rotation + (4 * lane + j) * kHeadDim + 4 * lane));
 
         // Index words and norms of this thread's token, fetched one tile ahead.  Past the end of the
         // sequence nothing is fetched and the norm is 0, which zeroes the value of every table entry;
@@ -572,24 +603,20 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         }
 
         // ---- queries of this item: rotate, round, quantise to signed digit planes (B operand) ----
-#pragma unroll 1
+#pragma unroll
         for (int round = 0; round < NH / 4; ++round) {
             const int h = 4 * round + warp;
-            float r[4] = {0.f, 0.f, 0.f, 0.f};
-            if (h < heads_here) {
-                const T* qp = static_cast<const T*>(p.q) + seq * p.q_stride_seq +
-                              static_cast<int64_t>(first_qh + h) * p.q_stride_head + 4 * lane;
-                const uint2 raw = __ldg(reinterpret_cast<const uint2*>(qp));
-                const float2 x01 = unpack_pair<T>(raw.x), x23 = unpack_pair<T>(raw.y);
+            float r[4];
+            {
+                const bool used = h < heads_here;
+                const float2 x01 = unpack_pair<T>(q_raw[round].x), x23 = unpack_pair<T>(q_raw[round].y);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float4 rr = __ldg(reinterpret_cast<const float4*>(
-                        p.rotation + (4 * lane + j) * kHeadDim + 4 * lane));
-                    float acc = __fmul_rn(x01.x, rr.x);
-                    acc = __fmaf_rn(x01.y, rr.y, acc);
-                    acc = __fmaf_rn(x23.x, rr.z, acc);
-                    acc = __fmaf_rn(x23.y, rr.w, acc);
-                    r[j] = round_to<T>(acc);
+                    float acc = __fmul_rn(x01.x, rot[j].x);
+                    acc = __fmaf_rn(x01.y, rot[j].y, acc);
+                    acc = __fmaf_rn(x23.x, rot[j].z, acc);
+                    acc = __fmaf_rn(x23.y, rot[j].w, acc);
+                    r[j] = used ? round_to<T>(acc) : 0.0f;
                 }
             }
             float mx = fmaxf(fmaxf(fabsf(r[0]), fabsf(r[1])), fmaxf(fabsf(r[2]), fabsf(r[3])));
@@ -858,7 +885,11 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         __syncthreads();
 
         x += t_end - t_begin;
-        if (t_end == n_s) ++seq;
+        if (t_end == n_s) {
+            ++seq;
+            pre += n_s;
+            seq_len = next_len;
+        }
     }
 
     if (dead) {
@@ -960,7 +991,8 @@ decode_merge_kernel(const DecodeParams p) {
             min_w = p.layer_w[0];
             for (int i = 1; i < p.num_layers; ++i) min_w = min(min_w, p.layer_w[i]);
         }
-        const bool dense = total <= p.groups || total * J * min_w >=
+        // (a thousandth more than a tile, as the boundaries may be one below the true quotient)
+        const bool dense = total <= p.groups || total * J * min_w / 1024 * 1023 >=
                            weight_cum(static_cast<int64_t>(p.groups) * J, p.layer_ctas, p.num_layers, p.layer_w);
         float m_all = -INFINITY;
         for (int g0 = g_first + sub; g0 <= g_last; g0 += 32 * W) {                  // normally one round
@@ -1349,6 +1381,7 @@ static int decode_impl(const void* q, void* out, int dtype, int64_t q_stride_seq
     for (int i = 0; i < kMaxLayers; ++i)
         p.layer_w[i] = env.n_weights > 0 ? env.weights[i < env.n_weights ? i : env.n_weights - 1] : kDefaultWeights[i];
     if (!env.equal_pieces && ctas > 1LL * (kCtasPerSm - 1) * sms) p.layer_ctas = sms;
+    p.inv_weight = UINT64_MAX / static_cast<uint64_t>(weight_cum(ctas, p.layer_ctas, p.num_layers, p.layer_w));
     p.out = out; p.o_stride_seq = o_stride_seq; p.o_stride_head = o_stride_head;
     p.num_peers = num_peers;
     for (int g = 0; g < num_peers; ++g) p.peer_out[g] = peer_out[g];
