@@ -106,6 +106,21 @@ int rq_decompress_blocks(const uint8_t* kv_cache, int64_t num_blocks, int block_
                          int n_centroids_v, void* out_k, void* out_v, int out_dtype, void* stream);
 
 /*
+ * rq_block_union and rq_decompress_blocks in one call, the second launch right behind the first: for callers that need the
+ * number of blocks only when both are under way.
+ *
+ *   blocks_out, remapped_out   as rq_block_union
+ *   count_out     device memory: the number of referenced blocks, -1 when an entry is out of range (nothing is expanded then)
+ *   count_host    the same number for the host (pinned memory, written as soon as it is known), or NULL
+ *   out_k, out_v  room for most_blocks >= min(num_seqs * max_blocks, num_blocks) blocks; the first count_out are written
+ */
+int rq_gather_blocks(const uint8_t* kv_cache, int64_t num_blocks, int block_size, int total_bytes, int num_kv_heads,
+                     int head_dim, const int32_t* block_table, int64_t block_table_stride, int num_seqs, int max_blocks,
+                     const int32_t* seq_lens, const float* centroids_k, int n_centroids_k, const float* centroids_v,
+                     int n_centroids_v, int32_t* blocks_out, int32_t* remapped_out, int32_t* count_out, int32_t* count_host,
+                     void* out_k, void* out_v, int64_t most_blocks, int out_dtype, void* stream);
+
+/*
  * The physical blocks a batch references (the torch.unique and renumbering part of
  * RQAttentionImpl._decompress_cache_paged), in one launch.
  *

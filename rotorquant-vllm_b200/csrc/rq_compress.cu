@@ -454,11 +454,12 @@ decompress_rows_kernel(const uint8_t* __restrict__ packed, const float* __restri
 
 // Paged decompress: the K (blockIdx.y == 0) and V rows of whole cache blocks, picked by a list of physical block
 // numbers, straight out of the slot layout.  Output row of (listed block j, position t, head h):
-// (j * block_size + t) * H + h.
+// (j * block_size + t) * H + h.  `count`: the number of listed blocks where the host does not know it (device memory); `rows` is
+// then its bound.
 template <typename T>
 __global__ void __launch_bounds__(kExpandThreads)
 decompress_blocks_kernel(const uint8_t* __restrict__ cache, int total_bytes, uint32_t block_size, int bs_shift, uint32_t H,
-                         int h_shift, const int32_t* __restrict__ blocks, uint32_t rows, int64_t num_blocks,
+                         int h_shift, const int32_t* __restrict__ blocks, const int32_t* count, uint32_t rows, int64_t num_blocks,
                          const float* __restrict__ cent_k, int n_k, const float* __restrict__ cent_v, int n_v,
                          T* __restrict__ out_k, T* __restrict__ out_v) {
     using E = Expand<T>;
@@ -466,6 +467,10 @@ decompress_blocks_kernel(const uint8_t* __restrict__ cache, int total_bytes, uin
     __shared__ float cb[16];
     if (threadIdx.x < 16) cb[threadIdx.x] = threadIdx.x < (kind ? n_v : n_k) ? (kind ? cent_v : cent_k)[threadIdx.x] : 0.f;
     __syncthreads();
+    if (count != nullptr) {                // behind the launch that lists the blocks: how many there are
+        grid_dependency_wait();
+        rows = min(rows, static_cast<uint32_t>(max(*count, 0)) * block_size * H);
+    }
     const SlotLayout lay = slot_layout(H);
     const int idx_off = kind ? lay.v_idx : lay.k_idx, norm_off = kind ? lay.v_norm : lay.k_norm;
     T* out = kind ? out_v : out_k;
@@ -507,20 +512,21 @@ constexpr int64_t kUnionMaxEntries = 1 << 20;
 __global__ void __launch_bounds__(kUnionThreads)
 block_union_kernel(const int32_t* __restrict__ table, int64_t stride, int num_seqs, int width,
                    const int32_t* __restrict__ seq_lens, int block_size, int num_blocks, int32_t* __restrict__ listed,
-                   int32_t* __restrict__ remapped, int32_t* count) {
+                   int32_t* __restrict__ remapped, int32_t* count, int32_t* count_host) {
     extern __shared__ uint32_t bits[];
     const int words = (num_blocks + 31) / 32, tid = threadIdx.x;
     int* prefix = reinterpret_cast<int*>(bits + words);
     __shared__ int warp_sums[32];
+    grid_launch_dependents();              // the launch that expands the blocks waits for this one's end
     for (int i = tid; i < words; i += kUnionThreads) bits[i] = 0u;
     __syncthreads();
     const int entries = num_seqs * width;
     bool bad = false;
     for (int e = tid; e < entries; e += kUnionThreads) {
         const int s = e / width, w = e - s * width;
-        const int64_t need = (static_cast<int64_t>(max(__ldg(seq_lens + s), 0)) + block_size - 1) / block_size;
-        if (w < need) {
-            const int b = __ldg(table + s * stride + w);
+        const int b = __ldg(table + s * stride + w);               // (beside the length, not behind it)
+        const int64_t len = max(__ldg(seq_lens + s), 0);
+        if (static_cast<int64_t>(w) * block_size < len) {
             if (b < 0 || b >= num_blocks) bad = true;
             else atomicOr(&bits[b >> 5], 1u << (b & 31));
         }
@@ -544,7 +550,10 @@ block_union_kernel(const int32_t* __restrict__ table, int64_t stride, int num_se
         prefix[i] = at;
         for (uint32_t b = bits[i]; b != 0; b &= b - 1) listed[at++] = 32 * i + __ffs(b) - 1;
     }
-    if (tid == kUnionThreads - 1) *count = bad ? -1 : at;      // every run of the last thread lies behind all others
+    if (tid == kUnionThreads - 1) {                            // every run of the last thread lies behind all others
+        *count = bad ? -1 : at;
+        if (count_host != nullptr) *static_cast<volatile int32_t*>(count_host) = bad ? -1 : at;
+    }
     __syncthreads();
     for (int e = tid; e < entries; e += kUnionThreads) {
         const int s = e / width, w = e - s * width;
@@ -610,14 +619,19 @@ static void launch_expand_rows(const uint8_t* packed, const float* norms, int64_
         packed, norms, num_rows, centroids, n_centroids, static_cast<T*>(out));
 }
 template <typename T>
-static void launch_expand_blocks(const uint8_t* cache, int total_bytes, int block_size, int H, const int32_t* blocks,
-                                 int64_t rows, int64_t num_blocks, const float* cent_k, int n_k, const float* cent_v,
+static int launch_expand_blocks(const uint8_t* cache, int total_bytes, int block_size, int H, const int32_t* blocks, const int32_t* count,
+                                int64_t rows, int64_t num_blocks, const float* cent_k, int n_k, const float* cent_v,
                                  int n_v, void* out_k, void* out_v, cudaStream_t st) {
     const int64_t units = rows << Expand<T>::kShift, per = kExpandThreads * kExpandUnits;
     const dim3 grid(static_cast<unsigned>((units + per - 1) / per), 2);
+    if (count != nullptr)
+        return launch_dependent("rq_gather_blocks launch", decompress_blocks_kernel<T>, grid, dim3(kExpandThreads), 0, st,
+                                cache, total_bytes, static_cast<uint32_t>(block_size), shift_of(block_size), static_cast<uint32_t>(H), shift_of(H), blocks, count,
+                                static_cast<uint32_t>(rows), num_blocks, cent_k, n_k, cent_v, n_v, static_cast<T*>(out_k), static_cast<T*>(out_v));
     decompress_blocks_kernel<T><<<grid, kExpandThreads, 0, st>>>(
-        cache, total_bytes, block_size, shift_of(block_size), H, shift_of(H), blocks, static_cast<uint32_t>(rows), num_blocks,
+        cache, total_bytes, block_size, shift_of(block_size), H, shift_of(H), blocks, nullptr, static_cast<uint32_t>(rows), num_blocks,
         cent_k, n_k, cent_v, n_v, static_cast<T*>(out_k), static_cast<T*>(out_v));
+    return check_cuda(cudaGetLastError(), "rq_decompress_blocks launch");
 }
 
 }  // namespace rq
@@ -724,10 +738,10 @@ extern "C" int rq_decompress(const uint8_t* packed, const float* norms, int64_t 
     return check_cuda(cudaGetLastError(), "rq_decompress launch");
 }
 
-extern "C" int rq_decompress_blocks(const uint8_t* kv_cache, int64_t num_blocks, int block_size, int total_bytes,
+static int expand_blocks(const uint8_t* kv_cache, int64_t num_blocks, int block_size, int total_bytes,
                                     int num_kv_heads, int head_dim, const int32_t* blocks, int64_t num_listed,
-                                    const float* centroids_k, int n_centroids_k, const float* centroids_v,
-                                    int n_centroids_v, void* out_k, void* out_v, int out_dtype, void* stream) {
+                         const int32_t* count, const float* centroids_k, int n_centroids_k, const float* centroids_v,
+                         int n_centroids_v, void* out_k, void* out_v, int out_dtype, void* stream) {
     if (num_blocks < 0 || block_size <= 0 || num_kv_heads <= 0 || num_listed < 0)
         return fail(RQ_ERR_INVALID_ARG, "rq_decompress_blocks: negative or zero size");
     if (head_dim != kHeadDim)
@@ -749,20 +763,27 @@ extern "C" int rq_decompress_blocks(const uint8_t* kv_cache, int64_t num_blocks,
     if (rows > 0x7fffffffLL) return fail(RQ_ERR_UNSUPPORTED, "rq_decompress_blocks: too many rows for one launch");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto launch = [&](auto tag) {
-        launch_expand_blocks<decltype(tag)>(kv_cache, total_bytes, block_size, num_kv_heads, blocks, rows, num_blocks, centroids_k,
-                                            n_centroids_k, centroids_v, n_centroids_v, out_k, out_v, st);
+        return launch_expand_blocks<decltype(tag)>(kv_cache, total_bytes, block_size, num_kv_heads, blocks, count, rows, num_blocks, centroids_k,
+                                                   n_centroids_k, centroids_v, n_centroids_v, out_k, out_v, st);
     };
     switch (out_dtype) {
-        case RQ_DTYPE_F32: launch(float{}); break;
-        case RQ_DTYPE_F16: launch(__half{}); break;
-        default: launch(__nv_bfloat16{}); break;
+        case RQ_DTYPE_F32: return launch(float{});
+        case RQ_DTYPE_F16: return launch(__half{});
+        default: return launch(__nv_bfloat16{});
     }
-    return check_cuda(cudaGetLastError(), "rq_decompress_blocks launch");
 }
 
-extern "C" int rq_block_union(const int32_t* block_table, int64_t block_table_stride, int num_seqs, int max_blocks,
-                              const int32_t* seq_lens, int block_size, int64_t num_blocks, int32_t* blocks_out,
-                              int32_t* remapped_out, int32_t* count_out, void* stream) {
+extern "C" int rq_decompress_blocks(const uint8_t* kv_cache, int64_t num_blocks, int block_size, int total_bytes,
+                                    int num_kv_heads, int head_dim, const int32_t* blocks, int64_t num_listed,
+                                    const float* centroids_k, int n_centroids_k, const float* centroids_v,
+                                    int n_centroids_v, void* out_k, void* out_v, int out_dtype, void* stream) {
+    return expand_blocks(kv_cache, num_blocks, block_size, total_bytes, num_kv_heads, head_dim, blocks, num_listed, nullptr, centroids_k,
+                         n_centroids_k, centroids_v, n_centroids_v, out_k, out_v, out_dtype, stream);
+}
+
+static int list_blocks(const int32_t* block_table, int64_t block_table_stride, int num_seqs, int max_blocks,
+                       const int32_t* seq_lens, int block_size, int64_t num_blocks, int32_t* blocks_out,
+                       int32_t* remapped_out, int32_t* count_out, int32_t* count_host, void* stream) {
     if (num_seqs <= 0 || max_blocks <= 0 || block_size <= 0 || num_blocks <= 0)
         return fail(RQ_ERR_INVALID_ARG, "rq_block_union: negative or zero size");
     if (num_blocks > kUnionMaxBlocks || static_cast<int64_t>(num_seqs) * max_blocks > kUnionMaxEntries)
@@ -775,6 +796,26 @@ extern "C" int rq_block_union(const int32_t* block_table, int64_t block_table_st
     if (int e = ensure_smem(block_union_kernel, smem)) return e;
     block_union_kernel<<<1, kUnionThreads, smem, static_cast<cudaStream_t>(stream)>>>(
         block_table, block_table_stride, num_seqs, max_blocks, seq_lens, block_size, static_cast<int>(num_blocks), blocks_out,
-        remapped_out, count_out);
+        remapped_out, count_out, count_host);
     return check_cuda(cudaGetLastError(), "rq_block_union launch");
+}
+
+extern "C" int rq_block_union(const int32_t* block_table, int64_t block_table_stride, int num_seqs, int max_blocks,
+                              const int32_t* seq_lens, int block_size, int64_t num_blocks, int32_t* blocks_out,
+                              int32_t* remapped_out, int32_t* count_out, void* stream) {
+    return list_blocks(block_table, block_table_stride, num_seqs, max_blocks, seq_lens, block_size, num_blocks, blocks_out, remapped_out,
+                       count_out, nullptr, stream);
+}
+
+extern "C" int rq_gather_blocks(const uint8_t* kv_cache, int64_t num_blocks, int block_size, int total_bytes, int num_kv_heads,
+                                int head_dim, const int32_t* block_table, int64_t block_table_stride, int num_seqs, int max_blocks,
+                                const int32_t* seq_lens, const float* centroids_k, int n_centroids_k, const float* centroids_v,
+                                int n_centroids_v, int32_t* blocks_out, int32_t* remapped_out, int32_t* count_out, int32_t* count_host,
+                                void* out_k, void* out_v, int64_t most_blocks, int out_dtype, void* stream) {
+    if (most_blocks <= 0) return fail(RQ_ERR_INVALID_ARG, "rq_gather_blocks: no room for blocks");
+    if (int e = list_blocks(block_table, block_table_stride, num_seqs, max_blocks, seq_lens, block_size, num_blocks, blocks_out, remapped_out,
+                            count_out, count_host, stream))
+        return e;
+    return expand_blocks(kv_cache, num_blocks, block_size, total_bytes, num_kv_heads, head_dim, blocks_out, most_blocks, count_out, centroids_k,
+                         n_centroids_k, centroids_v, n_centroids_v, out_k, out_v, out_dtype, stream);
 }

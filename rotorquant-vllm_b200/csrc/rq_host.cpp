@@ -36,6 +36,7 @@ struct Entry {
     decltype(&rq_decompress) decompress;
     decltype(&rq_decompress_blocks) decompress_blocks;
     decltype(&rq_block_union) block_union;
+    decltype(&rq_gather_blocks) gather_blocks;
     decltype(&rq_decode_workspace_bytes) decode_workspace_bytes;
     decltype(&rq_decode) decode;
     decltype(&rq_prefill_workspace_bytes) prefill_workspace_bytes;
@@ -153,12 +154,13 @@ PyObject* bind(PyObject*, PyObject* dict) {
     set(fn.decompress, dict, "rq_decompress");
     set(fn.decompress_blocks, dict, "rq_decompress_blocks");
     set(fn.block_union, dict, "rq_block_union");
+    set(fn.gather_blocks, dict, "rq_gather_blocks");
     set(fn.decode_workspace_bytes, dict, "rq_decode_workspace_bytes");
     set(fn.decode, dict, "rq_decode");
     set(fn.prefill_workspace_bytes, dict, "rq_prefill_workspace_bytes");
     set(fn.prefill_int8_staged, dict, "rq_prefill_int8_staged");
     set(fn.last_error, dict, "rq_last_error");
-    bound = fn.compress_store && fn.compress && fn.decompress && fn.decompress_blocks && fn.block_union && fn.decode_workspace_bytes && fn.decode &&
+    bound = fn.compress_store && fn.compress && fn.decompress && fn.decompress_blocks && fn.block_union && fn.gather_blocks && fn.decode_workspace_bytes && fn.decode &&
             fn.prefill_workspace_bytes && fn.prefill_int8_staged && fn.last_error;
     if (PyErr_Occurred()) return nullptr;
     if (!bound) { PyErr_SetString(PyExc_RuntimeError, "bind: an entry point is missing"); return nullptr; }
@@ -420,13 +422,65 @@ PyObject* gather(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const int64_t nb = cache->size(0), bs = cache->size(1);
     const auto index = static_cast<c10::DeviceIndex>(dev.index);
     const c10::cuda::CUDAGuard guard(index);
-    const at::Tensor listed = at::empty({std::min(table->numel(), nb)}, table->options());
+    const int64_t most = std::min(table->numel(), nb);
+    const at::Tensor listed = at::empty({most + 1}, table->options());                   // the last one is the count
     const at::Tensor remapped = at::empty({table->size(0), table->size(1)}, table->options());
     // the count lands in pinned memory of this thread, which the kernel writes directly
     static thread_local at::Tensor landing;
     if (!landing.defined()) landing = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
     auto* count = static_cast<volatile int32_t*>(landing.data_ptr());
     const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(index);
+    const at::ScalarType types[3] = {at::kFloat, at::kHalf, at::kBFloat16};
+    const auto options = cache->options().dtype(types[code]);
+    auto results = [&](const at::Tensor& k, const at::Tensor& v) -> PyObject* {
+        PyObject* out[3] = {THPVariable_Wrap(k), THPVariable_Wrap(v), THPVariable_Wrap(remapped)};
+        PyObject* all = out[0] && out[1] && out[2] ? PyTuple_Pack(3, out[0], out[1], out[2]) : nullptr;
+        for (PyObject* o : out) Py_XDECREF(o);
+        return all;
+    };
+    // Where all blocks that the table can name take little memory, the results are allocated for as many, the blocks are expanded
+    // right behind the launch that lists them, and the host meanwhile waits for their number alone, which sizes the tensors
+    // (and their storages) then.  Otherwise the results are allocated when the number is known, with the GPU idle until
+    // then.  4 sequences of 700 to 2048 tokens, 8 KV heads: 25.6 us that way, 14.2 this way.
+    constexpr int64_t kMostBytes = int64_t{192} << 20;
+    const int64_t block_elements = bs * heads * 128;
+    if (most * block_elements <= kMostBytes / (2 * static_cast<int64_t>(c10::elementSize(types[code])))) {
+        const at::Tensor k = at::empty({most, bs, heads, 128}, options), v = at::empty({most, bs, heads, 128}, options);
+        constexpr int32_t kUnknown = INT32_MIN;
+        *count = kUnknown;
+        cudaError_t err = cudaSuccess;
+        const int status = unlocked([&] {
+            const int st = fn.gather_blocks(static_cast<const uint8_t*>(cache->const_data_ptr()), nb, static_cast<int>(bs),
+                                            static_cast<int>(cache->size(2)), static_cast<int>(heads), 128,
+                                            static_cast<const int32_t*>(table->const_data_ptr()), table->stride(0),
+                                            static_cast<int>(table->size(0)), static_cast<int>(table->size(1)),
+                                            static_cast<const int32_t*>(lens->const_data_ptr()),
+                                            static_cast<const float*>(ck->const_data_ptr()), static_cast<int>(ck->numel()),
+                                            static_cast<const float*>(cv->const_data_ptr()), static_cast<int>(cv->numel()),
+                                            static_cast<int32_t*>(listed.data_ptr()), static_cast<int32_t*>(remapped.data_ptr()),
+                                            static_cast<int32_t*>(listed.data_ptr()) + most, static_cast<int32_t*>(landing.data_ptr()),
+                                            k.data_ptr(), v.data_ptr(), most, static_cast<int>(code), stream.stream());
+            if (st != RQ_OK) return st;
+            for (int spin = 0; *count == kUnknown; ++spin) {     // a stream that ends, or fails, without the number ends the wait
+                if (spin % 1024 != 0) continue;
+                err = cudaStreamQuery(stream.stream());
+                if (err == cudaErrorNotReady) err = cudaSuccess;
+                else break;
+            }
+            return st;
+        });
+        if (status == RQ_ERR_UNSUPPORTED) return none();
+        if (raised(status)) return nullptr;
+        if (err == cudaSuccess && *count == kUnknown) err = cudaErrorUnknown;
+        if (err != cudaSuccess) { PyErr_SetString(PyExc_RuntimeError, cudaGetErrorString(err)); return nullptr; }
+        const int64_t n = *count;
+        if (n < 0) return none();
+        for (const at::Tensor* t : {&k, &v}) {
+            t->unsafeGetTensorImpl()->set_sizes_contiguous({n, bs, heads, 128});
+            t->storage().unsafeGetStorageImpl()->set_nbytes(static_cast<size_t>(n * block_elements) * t->element_size());
+        }
+        return results(k, v);
+    }
     int status = unlocked([&] {
         return fn.block_union(static_cast<const int32_t*>(table->const_data_ptr()), table->stride(0),
                               static_cast<int>(table->size(0)), static_cast<int>(table->size(1)),
@@ -440,8 +494,7 @@ PyObject* gather(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (err != cudaSuccess) { PyErr_SetString(PyExc_RuntimeError, cudaGetErrorString(err)); return nullptr; }
     const int64_t n = *count;
     if (n < 0) return none();
-    const at::ScalarType types[3] = {at::kFloat, at::kHalf, at::kBFloat16};
-    const at::Tensor k = at::empty({n, bs, heads, 128}, cache->options().dtype(types[code])), v = at::empty_like(k);
+    const at::Tensor k = at::empty({n, bs, heads, 128}, options), v = at::empty_like(k);
     status = unlocked([&] {
         return fn.decompress_blocks(static_cast<const uint8_t*>(cache->const_data_ptr()), nb, static_cast<int>(bs),
                                     static_cast<int>(cache->size(2)), static_cast<int>(heads), 128,
@@ -451,10 +504,7 @@ PyObject* gather(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
                                     k.data_ptr(), v.data_ptr(), static_cast<int>(code), stream.stream());
     });
     if (raised(status)) return nullptr;
-    PyObject* out[3] = {THPVariable_Wrap(k), THPVariable_Wrap(v), THPVariable_Wrap(remapped)};
-    PyObject* all = out[0] && out[1] && out[2] ? PyTuple_Pack(3, out[0], out[1], out[2]) : nullptr;
-    for (PyObject* o : out) Py_XDECREF(o);
-    return all;
+    return results(k, v);
 }
 
 // The functions as Python calls them: an exception must not reach the interpreter's C frames, which end the process.

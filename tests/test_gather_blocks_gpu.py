@@ -1,0 +1,40 @@
+"""The paged decompress against its definition (the referenced blocks in ascending order, expanded one by one), where the blocks
+are expanded before the host knows their number and where they are not (room for all blocks of the table is too much)."""
+
+import pytest
+import torch
+
+from gpu_util import DEV, params
+from rotorquant_vllm.cuda.decompress import decompress_blocks, decompress_cache_paged
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,bs,blocks,width,lens", [
+    (8, 16, 9, 40, [1, 129, 0, 17]), (1, 16, 5, 2, [0, 0]), (1, 64, 3, 1, [64]), (4, 24, 30, 12, [24 * 12, 25]),
+    (2, 16, 700, 200, [1600, 3200, 31]),
+    (1, 16, 30000, 8192, [20000, 1, 3]),                         # 24576 blocks at most
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_gather(H, bs, blocks, width, lens, dtype):
+    p = {k: v.to(DEV) for k, v in params("iso_fast", 3, 4).items()}
+    gen = torch.Generator().manual_seed(len(lens))
+    cache = torch.randint(0, 256, (blocks, bs, H * 256), generator=gen, dtype=torch.uint8) & 0x77
+    table = torch.full((len(lens), width), blocks + 5, dtype=torch.int32)            # entries that no sequence reaches may be anything
+    for s, n in enumerate(lens):
+        need = -(-n // bs)
+        table[s, :need] = torch.randint(blocks, (need,), generator=gen).to(torch.int32)
+    cache, table, seq_lens = cache.to(DEV), table.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV)
+    used = torch.unique(torch.cat([table[s, :-(-n // bs)] for s, n in enumerate(lens)]))
+    want_k, want_v = decompress_blocks(cache, used, H, p["k_centroids"], p["v_centroids"], dtype)
+    for _ in range(3):
+        k, v, remapped = decompress_cache_paged(cache, table, seq_lens, H, p["k_centroids"], p["v_centroids"], dtype)
+        assert k.shape == want_k.shape and torch.equal(k, want_k) and torch.equal(v, want_v)
+        assert k._base is None and k.is_contiguous() and k.untyped_storage().nbytes() == k.numel() * k.element_size()
+        for s, n in enumerate(lens):
+            need = -(-n // bs)
+            assert torch.equal(used[remapped[s, :need].long()], table[s, :need])
+    if any(lens):
+        table[0 if lens[0] else 1, 0] = blocks
+        with pytest.raises(ValueError, match="refers to block"):
+            decompress_cache_paged(cache, table, seq_lens, H, p["k_centroids"], p["v_centroids"], dtype)
