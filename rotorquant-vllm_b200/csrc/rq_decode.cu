@@ -471,7 +471,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         // heads at once: 3500 -> 700 clocks between the staging request and the query tile.  Whole call, us, with the lengths
         // fetched a sequence ahead and the piece boundaries without divisions: 64 x 4096 tokens 106.2 -> 104.9, 16 of 2048 to 32768 on
         // one KV head 45.3 -> 43.6, 200 of 100 to 2000, 28 / 4 heads 79.2 -> 75.8, 48 of 500 to 9000, 64 / 8 heads 104.6 -> 102.5; 256 of
-        // 512 to 8192, 28 / 4 heads 287 either way.  (Staging the first tile of the next sequence under the last one of this: 293 and
+        // 512 to 8192, 28 / 4 heads 287 -> 281.  (Staging the first tile of the next sequence under the last one of this: 293 and
         // 106.9 for the last two, as every tile pays for the choice.)
         uint2 q_raw[NH / 4];
         float4 rot[4];
@@ -524,8 +524,11 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
             const int t = tile * kUTile + 32 * warp + (lane & 16);
             return (tile < t_end && t < seq_len) ? __ldg(bt_row + (t >> p.bs_shift)) : 0;
         };
-        // Completes one phase of bar_in[warp].  Not after a wait for the phase before has expired (stop): it may be open still.
+        // Completes one phase of bar_in[warp] for a tile before t_end.  Not after a wait for the phase before has expired (stop): it
+        // may be open still.  (With the test of the tile at the callers the code comes out slower with 4-bit keys: 287 us for 256
+        // sequences of 512 to 8192 tokens, 281 this way.)
         [[maybe_unused]] auto issue_tile = [&](int tile, int blk, bool stop) {
+            if (tile >= t_end) return;
             const int t = tile * kUTile + 32 * warp + (lane & 16);
             blk = blk < 0 ? 0 : (blk > last_blk ? last_blk : blk);
             const int gslot = (blk << p.bs_shift) + (t & (p.block_size - 1));
@@ -646,7 +649,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
                 fetch_staged(0, kw, nk);
                 fetch_staged(1, vw, nv);
                 __syncwarp();
-                if (t_begin + 1 < t_end) issue_tile(t_begin + 1, pf_blk, failed_in);
+                issue_tile(t_begin + 1, pf_blk, failed_in);
                 pf_blk = load_blk(t_begin + 2);
             }
         }
@@ -749,7 +752,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
                 v_rows_landed();
                 if (tile + 1 < t_end) fetch_staged(1, vw, nv);
                 __syncwarp();                            // the staging rows are free again
-                if (tile + 2 < t_end) issue_tile(tile + 2, pf_blk, failed);
+                issue_tile(tile + 2, pf_blk, failed);
                 pf_blk = load_blk(tile + 3);
             } else {
                 fetch_direct(1, next_slot, vw, nv);
